@@ -103,6 +103,18 @@ SB_API int sb_spmm_csr_f32(int64_t m, int64_t n, int64_t k, int64_t nnz, const i
                            const void* plan, int64_t plan_segments, void* scratch,
                            size_t scratch_bytes, void* stream);
 
+/* The same product for a matrix that has no plan (one that is multiplied once, or whose structure
+ * changes from call to call): the kernel cuts the stored entries into equal tiles, so rows of any
+ * length are balanced without looking at them first and nothing is read back to the host.  Any
+ * SB_* dtype, any alignment.  `ws`: sb_spmm_csr_once_workspace_bytes(dtype, k, nnz) bytes,
+ * 16-byte aligned, contents undefined before and after; bias may be NULL; with `accumulate` the
+ * present contents of C are added (before bias and ReLU). */
+SB_API size_t sb_spmm_csr_once_workspace_bytes(int dtype, int64_t k, int64_t nnz);
+SB_API int sb_spmm_csr_once(int dtype, int64_t m, int64_t n, int64_t k, int64_t nnz, const int32_t* pos,
+                            const int32_t* crd, const void* val, const void* B, int64_t ldb,
+                            const void* bias, int relu, int accumulate, void* C, int64_t ldc, void* ws,
+                            size_t ws_bytes, void* stream);
+
 /* Accumulating form:  C[i, 0:k] = act( bias + C[i, 0:k] + sum_p ... ), same arguments.  A product
  * whose dense operand arrives in pieces (row chunks of B, each with the matrix entries whose
  * columns fall in it) is the first piece through sb_spmm_csr_f32 and the others through this

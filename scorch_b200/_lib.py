@@ -34,6 +34,9 @@ SIGNATURES = {
                                _ptr, _i64, _i64, _i64, _i64, _i64, _ptr, _i64, _ptr, _sz, _ptr]),
     "sb_spmm_csr_acc_f32": (_int, [_i64, _i64, _i64, _i64, _ptr, _ptr, _ptr, _ptr, _i64, _ptr, _int,
                                    _ptr, _i64, _i64, _i64, _i64, _i64, _ptr, _i64, _ptr, _sz, _ptr]),
+    "sb_spmm_csr_once_workspace_bytes": (_sz, [_int, _i64, _i64]),
+    "sb_spmm_csr_once": (_int, [_int, _i64, _i64, _i64, _i64, _ptr, _ptr, _ptr, _ptr, _i64, _ptr, _int,
+                                _int, _ptr, _i64, _ptr, _sz, _ptr]),
     "sb_spmm_wide_select": (_int, [_int]),
     "sb_spmm_wide_status": (_int, []),
     "sb_probe_l2_gather": (_int, [_ptr, _i64, _i64, _i64, _ptr, _ptr]),

@@ -1,0 +1,397 @@
+// SpMM over tiles of stored entries: the form for one matrix, with no row plan.
+//
+// What it is for: rows of very different lengths (power-law matrices) and short rows.  With a warp
+// or lane group per row, most of the GPU waits for the few that got long rows.  Here a CTA takes
+// the rows that begin in a window of TE consecutive entries, so every CTA has about the same number
+// of entries, and inside it a row is taken by whatever suits its length:
+//   up to kGroupRow entries    one lane group (L lanes across the operand's columns)
+//   up to kWarpRow             the lane groups of a warp, a slice each
+//   longer                     all lane groups of the CTA, in units of kUnit entries; the unit sums
+//                              of a row of several units are added in order by a second launch
+//                              (which also writes the rows without entries)
+// Nothing is built beforehand and no host decision depends on the matrix.  Which sums are formed in
+// which order depends on a row's own length only, not on where the row lies: the same bits on every
+// run, and for a block of rows the same as for the whole matrix.
+// The window's indices and values go to shared memory by cp.async while the first row is looked
+// for; gathers keep U operand rows per lane group in flight.
+// Bound: L2 -> SM gathers of operand rows (17 TB/s measured for random rows of 64 bytes and more)
+// where the operand stays in L2, else DRAM on the gathers.
+#pragma once
+
+#include "spmm_kernels.cuh"
+
+namespace sb {
+
+constexpr int kTileThreadsMm = 256;
+constexpr int kTileWarps = kTileThreadsMm / 32;
+constexpr int kUnit = 512;             // a window's last row or unit reaches up to this far behind it
+// Largest window.  Wide rows (L = 32) have work enough in 1536 entries and lose residency to more
+// (6 M entries, 256 columns: 371 us, 415 with 3072); narrow ones gain by having their start-up
+// spread over twice as many (0.8 M entries in rows of 8, 64 columns: 27.0 us, 22.9 with 3072).
+constexpr int tile_window(int L) { return L == 32 ? 1536 : 3072; }
+// Rows of up to this length go to a lane group.  32 lets the warp's other groups help with a row of
+// a power-law graph (2 M rows, 64 columns: 6.10 ms with 64, 5.66 with 32); the 8 groups of four
+// lanes have too little of a 33-entry row each (27 entries per row, 16 float64 columns: 53.6 us
+// with 32, 49.6 with 64).
+template <int L>
+constexpr int kGroupRow = L == 4 ? 64 : 32;
+constexpr int kWarpRow = 192;
+constexpr int kTileRowCap = 1024;      // row pointers kept in shared memory at a time
+constexpr int kTileLists = 96;         // rows of the window that a warp / the CTA takes
+static_assert(tile_window(8) / 33 + 2 <= kTileLists && tile_window(4) / 65 + 2 <= kTileLists &&
+              tile_window(32) / 33 + 2 <= kTileLists, "rows longer than kGroupRow of a window");
+static_assert(tile_window(8) / kWarpRow + tile_window(8) / kUnit + 4 <= kTileLists, "units of a window");
+
+// Resident CTAs per SM the kernels are compiled for (64 / 80 registers; measured per lane count).
+constexpr int tile_ctas(int L) { return L == 32 ? 4 : 3; }
+// Entries per window, a multiple of 32: as few full waves of CTAs over the chip as windows of at
+// most tile_window(L) allow (a last wave that is half empty costs as much as a full one), at least 64
+// and at least four per lane group.
+inline int tile_entries(int64_t nnz, int L) {
+  const int64_t slots = 148 * tile_ctas(L);
+  const int64_t waves = std::max<int64_t>(1, ceil_div(nnz, slots * tile_window(L)));
+  const int64_t te = ceil_div(ceil_div(nnz, slots * waves), 32) * 32;
+  return (int)std::min<int64_t>(std::max<int64_t>(te, std::max(64, 1024 / L)), tile_window(L));
+}
+
+template <typename T>
+struct TileArgs {
+  int nnz, entries, tiles;
+  T* first;         // [nnz / kUnit + 1][k] sums of the first units of rows of several units ...
+  T* rest;          // ... and of their other units; index = first entry of the unit / kUnit
+};
+
+// One stored entry in shared memory, read by one load.
+template <typename T>
+struct alignas(sizeof(T) == 4 ? 8 : 16) Entry {
+  T a;
+  int j;
+};
+
+struct TileUnit {
+  int row, begin, len;
+};
+
+template <typename T, int L, int VEC, int W>
+struct TileSmem {
+  Pack<T, W> part[kTileWarps][VEC][L];
+  Entry<T> entry[tile_window(L) + kUnit];
+  int pos[kTileRowCap + 2];
+  TileUnit by_warp[kTileLists], by_cta[kTileLists];
+  int n_warp, n_cta, next_warp, next_row;
+  int count[kTileWarps];
+};
+
+template <int BYTES>
+__device__ __forceinline__ void cp_async(void* smem, const void* gmem) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(s), "l"(gmem), "n"(BYTES) : "memory");
+}
+
+// Row of entry p: the largest r with pos[r] <= p < pos[m]; the whole CTA calls it.  Matrices of up
+// to 32 rows per thread are looked at in one go (one round of loads in flight together instead of
+// one dependent round per factor of 256); `s_count`: one int per warp.
+__device__ __forceinline__ int tile_row_of(const int* __restrict__ pos, int m, int p, int* s_count) {
+  if (m <= 32 * kTileThreadsMm) {
+    int c = 0;
+    for (int r = threadIdx.x; r < m; r += 8 * kTileThreadsMm) {
+#pragma unroll
+      for (int q = 0; q < 8; q++) {
+        const int x = r + q * kTileThreadsMm;
+        c += x < m && __ldg(pos + x) <= p;
+      }
+    }
+    c = __reduce_add_sync(FULL, c);
+    if ((threadIdx.x & 31) == 0) s_count[threadIdx.x >> 5] = c;
+    __syncthreads();
+    c = 0;
+#pragma unroll
+    for (int w = 0; w < kTileWarps; w++) c += s_count[w];
+    __syncthreads();
+    return c - 1;
+  }
+  int lo = 0, hi = m;
+  while (true) {
+    const int span = hi - lo;
+    const int step = (span + kTileThreadsMm - 1) / kTileThreadsMm;
+    const long long r = (long long)lo + (long long)threadIdx.x * step;
+    const int c = __syncthreads_count(r < hi && __ldg(pos + r) <= p);
+    lo += (c - 1) * step;
+    if (step == 1) return lo;
+    hi = min(hi, lo + step);
+  }
+}
+
+template <typename T, int L, int VEC, int W>
+__device__ __forceinline__ void tile_store_row(const SpmmArgs<T>& a, int row, int col0, const bool (&col_ok)[VEC],
+                                               const Pack<T, W> (&sum)[VEC]) {
+  T* crow = a.C + (long long)row * a.ldc;
+#pragma unroll
+  for (int v = 0; v < VEC; v++) {
+    const int col = col0 + v * L * W;
+    if (!col_ok[v]) continue;
+    Pack<T, W> s = sum[v];
+    if (a.accumulate) {
+      const Pack<T, W> old = ld_l2<T, W>(crow + col);
+#pragma unroll
+      for (int w = 0; w < W; w++) s.v[w] += old.v[w];
+    }
+    st_stream<T, W>(crow + col, epilogue<T, W>(s, a.bias, col, a.relu));
+  }
+}
+
+// acc += the entries [b, e) of the window, one after the other, U operand rows in flight.  Lanes
+// beyond the last column read the first one's slice (`Bcol` points there) and drop the result.
+template <typename T, int VEC, int W, int U>
+__device__ __forceinline__ void tile_add(Pack<T, W> (&acc)[VEC], const Entry<T>* entry, int b, int e,
+                                         const char* const (&Bcol)[VEC], unsigned pitch) {
+  int p = b;
+#pragma unroll 1
+  for (; p + U <= e; p += U) {
+    Entry<T> x[U];
+    Pack<T, W> bv[U][VEC];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      x[u] = entry[p + u];
+#pragma unroll
+      for (int v = 0; v < VEC; v++)
+        bv[u][v] = ld_dense<T, W>(reinterpret_cast<const T*>(Bcol[v] + (unsigned long long)(unsigned)x[u].j * pitch));
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+#pragma unroll
+      for (int v = 0; v < VEC; v++) {
+#pragma unroll
+        for (int w = 0; w < W; w++) acc[v].v[w] = mul_add(x[u].a, bv[u][v].v[w], acc[v].v[w]);
+      }
+    }
+  }
+  if (p < e) {
+    Entry<T> x[U];
+    Pack<T, W> bv[U][VEC];
+#pragma unroll
+    for (int u = 0; u + 1 < U; u++) {
+      x[u].a = T(0);
+      if (p + u < e) {
+        x[u] = entry[p + u];
+#pragma unroll
+        for (int v = 0; v < VEC; v++)
+          bv[u][v] =
+              ld_dense<T, W>(reinterpret_cast<const T*>(Bcol[v] + (unsigned long long)(unsigned)x[u].j * pitch));
+      } else {
+#pragma unroll
+        for (int v = 0; v < VEC; v++) {
+#pragma unroll
+          for (int w = 0; w < W; w++) bv[u][v].v[w] = T(0);
+        }
+      }
+    }
+#pragma unroll
+    for (int u = 0; u + 1 < U; u++) {
+#pragma unroll
+      for (int v = 0; v < VEC; v++) {
+#pragma unroll
+        for (int w = 0; w < W; w++) acc[v].v[w] = mul_add(x[u].a, bv[u][v].v[w], acc[v].v[w]);
+      }
+    }
+  }
+}
+
+template <typename T, int L, int VEC, int W>
+__global__ void __launch_bounds__(kTileThreadsMm, tile_ctas(L))
+spmm_tile_kernel(SpmmArgs<T> a, TileArgs<T> t) {
+  using Smem = TileSmem<T, L, VEC, W>;
+  constexpr int G = 32 / L, NG = kTileWarps * G;
+  constexpr int UMAX = SB_SPMM_INFLIGHT * 4 / (VEC * W * (int)sizeof(T));
+  constexpr int U = UMAX >= 8 ? 8 : UMAX >= 4 ? 4 : 2;
+  extern __shared__ __align__(32) unsigned char smem_raw[];
+  Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, l = lane % L, g = lane / L;
+  const int col0 = blockIdx.y * (L * W * VEC) + l * W;
+  bool col_ok[VEC];
+  const char* Bcol[VEC];
+#pragma unroll
+  for (int v = 0; v < VEC; v++) {
+    col_ok[v] = (col0 + v * L * W) < a.k;
+    Bcol[v] = reinterpret_cast<const char*>(a.B + (col_ok[v] ? col0 + v * L * W : 0));
+  }
+  const unsigned pitch = (unsigned)(a.ldb * (long long)sizeof(T));
+  const int e0 = (int)blockIdx.x * t.entries, e1 = min(t.nnz, e0 + t.entries);
+  const int staged = min(t.nnz, e1 + kUnit) - e0;
+  for (int i = tid; i < staged; i += kTileThreadsMm) {
+    cp_async<4>(&sm.entry[i].j, a.crd + e0 + i);
+    cp_async<(int)sizeof(T)>(&sm.entry[i].a, a.val + e0 + i);
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+
+  // rows in turns of kTileRowCap, from the one that holds the first entry not dealt with
+  for (int next = e0; next < e1;) {
+    const int r0 = tile_row_of(a.pos, a.m, next, sm.count);
+    for (int i = tid; i < kTileRowCap + 1; i += kTileThreadsMm) sm.pos[i] = __ldg(a.pos + min(a.m, r0 + i));
+    if (tid == 0) { sm.n_warp = sm.n_cta = sm.next_warp = sm.next_row = 0; }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    // rows and units too long for a lane group, as far as they begin in the window
+    int rows = 0;                        // rows of this turn that begin before e1
+    for (int i = tid; i < kTileRowCap; i += kTileThreadsMm) {
+      const int b = sm.pos[i], len = sm.pos[i + 1] - b;
+      const bool here = b < e1 && r0 + i < a.m;
+      rows += here;
+      if (!here || len <= kGroupRow<L>) continue;
+      if (len <= kWarpRow) {
+        if (b >= next) sm.by_warp[atomicAdd(&sm.n_warp, 1)] = TileUnit{r0 + i, b, len};
+      } else {
+        // (first unit at or behind the window's start; a row that began before a later turn's first
+        // entry was dealt with by the turn before)
+        int u = b >= next ? 0 : (next == e0 ? (e0 - b + kUnit - 1) / kUnit : INT32_MAX / kUnit);
+        for (; u < (len + kUnit - 1) / kUnit && b + u * kUnit < e1; u++)
+          sm.by_cta[atomicAdd(&sm.n_cta, 1)] = TileUnit{r0 + i, b + u * kUnit, min(kUnit, len - u * kUnit)};
+      }
+    }
+    rows = __reduce_add_sync(FULL, rows);
+    if (lane == 0) sm.count[warp] = rows;
+    __syncthreads();
+    rows = 0;
+#pragma unroll
+    for (int w = 0; w < kTileWarps; w++) rows += sm.count[w];
+    const int n_cta = sm.n_cta, n_warp = sm.n_warp;
+
+    for (int i = 0; i < n_cta; i++) {
+      const TileUnit q = sm.by_cta[i];
+      const int slice = (q.len + NG - 1) / NG, w0 = min(q.len, (warp * G + g) * slice);
+      const int b = q.begin - e0 + w0;
+      Pack<T, W> s[VEC];
+      zero_acc<T, VEC, W>(s);
+      tile_add<T, VEC, W, U>(s, sm.entry, b, b + min(slice, q.len - w0), Bcol, pitch);
+      reduce_groups<T, L, VEC, W>(s);
+      if (lane < L) {
+#pragma unroll
+        for (int v = 0; v < VEC; v++) sm.part[warp][v][l] = s[v];
+      }
+      __syncthreads();
+      if (warp == (i % kTileWarps) && lane < L) {
+#pragma unroll
+        for (int v = 0; v < VEC; v++) {
+          s[v] = sm.part[0][v][l];
+#pragma unroll
+          for (int w2 = 1; w2 < kTileWarps; w2++) {
+            const Pack<T, W> x = sm.part[w2][v][l];
+#pragma unroll
+            for (int w = 0; w < W; w++) s[v].v[w] += x.v[w];
+          }
+        }
+        const int rb = __ldg(a.pos + q.row);
+        if (__ldg(a.pos + q.row + 1) - rb <= kUnit) {
+          tile_store_row<T, L, VEC, W>(a, q.row, col0, col_ok, s);
+        } else {
+          T* dst = (q.begin == rb ? t.first : t.rest) + (long long)(q.begin / kUnit) * a.k + col0;
+#pragma unroll
+          for (int v = 0; v < VEC; v++)
+            if (col_ok[v]) store_plain<T, W>(dst + v * L * W, s[v]);
+        }
+      }
+      __syncthreads();
+    }
+
+    while (true) {
+      int i = 0;
+      if (lane == 0) i = atomicAdd(&sm.next_warp, 1);
+      i = __shfl_sync(FULL, i, 0);
+      if (i >= n_warp) break;
+      const TileUnit q = sm.by_warp[i];
+      const int slice = (q.len + G - 1) / G, w0 = min(q.len, g * slice);
+      const int b = q.begin - e0 + w0;
+      Pack<T, W> s[VEC];
+      zero_acc<T, VEC, W>(s);
+      tile_add<T, VEC, W, U>(s, sm.entry, b, b + min(slice, q.len - w0), Bcol, pitch);
+      reduce_groups<T, L, VEC, W>(s);
+      if (lane < L) tile_store_row<T, L, VEC, W>(a, q.row, col0, col_ok, s);
+    }
+
+    while (true) {
+      int i = 0;
+      if (lane == 0) i = atomicAdd(&sm.next_row, G);
+      i = __shfl_sync(FULL, i, 0);
+      if (i >= rows) break;
+      i += g;
+      const int b = sm.pos[i < rows ? i : 0], len = i < rows ? sm.pos[i + 1] - b : 0;
+      if (b < next || len == 0 || len > kGroupRow<L>) continue;
+      Pack<T, W> s[VEC];
+      zero_acc<T, VEC, W>(s);
+      tile_add<T, VEC, W, U>(s, sm.entry, b - e0, b - e0 + len, Bcol, pitch);
+      tile_store_row<T, L, VEC, W>(a, r0 + i, col0, col_ok, s);
+    }
+    next = sm.pos[kTileRowCap];
+    __syncthreads();
+  }
+}
+
+// Rows without entries (zeros, or act(bias)), and rows of several units: their unit sums in order.
+// A warp looks at 32 rows and takes those that need something, a lane per column.
+template <typename T>
+__global__ void __launch_bounds__(kTileThreadsMm)
+spmm_tile_rows_kernel(SpmmArgs<T> a, TileArgs<T> t) {
+  const int lane = threadIdx.x & 31;
+  const long long r0 = ((long long)blockIdx.x * kTileWarps + (threadIdx.x >> 5)) * 32;
+  int b = 0, len = 1;
+  if (r0 + lane < a.m) {
+    b = __ldg(a.pos + r0 + lane);
+    len = __ldg(a.pos + r0 + lane + 1) - b;
+  }
+  unsigned todo = __ballot_sync(FULL, len == 0 || len > kUnit);
+  asm volatile("griddepcontrol.wait;" ::: "memory");   // the tile kernel's results
+  while (todo) {
+    const int i = __ffs(todo) - 1;
+    todo &= todo - 1;
+    const int rb = __shfl_sync(FULL, b, i), units = (__shfl_sync(FULL, len, i) + kUnit - 1) / kUnit;
+    T* crow = a.C + (r0 + i) * a.ldc;
+    for (int col = blockIdx.y * 32 + lane; col < a.k; col += gridDim.y * 32) {
+      T s = T(0);
+      if (units > 0) s = t.first[(long long)(rb / kUnit) * a.k + col];
+#pragma unroll 8
+      for (int u = 1; u < units; u++) s += t.rest[((long long)(rb / kUnit) + u) * a.k + col];
+      Pack<T, 1> x;
+      x.v[0] = s + (a.accumulate ? crow[col] : T(0));
+      st_stream<T, 1>(crow + col, epilogue<T, 1>(x, a.bias, col, a.relu));
+    }
+  }
+}
+
+// (two unit sums per kUnit entries)
+inline size_t tile_workspace_bytes(size_t size, int64_t k, int64_t nnz) {
+  return nnz <= kUnit ? 0 : 2 * (size_t)(nnz / kUnit + 1) * (size_t)k * size;
+}
+
+template <typename T, int L, int VEC, int W>
+static int launch_tiles(const SpmmArgs<T>& a, int64_t nnz, void* ws, cudaStream_t st) {
+  using Smem = TileSmem<T, L, VEC, W>;
+  const unsigned panels = (unsigned)ceil_div(a.k, L * W * VEC);
+  if (panels > 65535)
+    return fail(SB_ERR_UNSUPPORTED, "spmm: at most %lld columns with this layout, got %d",
+                65535ll * (L * W * VEC), a.k);
+  TileArgs<T> t;
+  t.nnz = (int)nnz;
+  t.entries = tile_entries(nnz, L);
+  t.tiles = (int)ceil_div(nnz, t.entries);
+  t.first = static_cast<T*>(ws);
+  t.rest = t.first + (size_t)(nnz / kUnit + 1) * a.k;
+  if (t.tiles > 0) {
+    auto kernel = spmm_tile_kernel<T, L, VEC, W>;
+    static bool sized[64] = {};   // per device: the attribute is set once
+    int dev = 0;
+    SB_CUDA(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64 || !sized[dev]) {
+      SB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem)));
+      if (dev >= 0 && dev < 64) sized[dev] = true;
+    }
+    kernel<<<dim3((unsigned)t.tiles, panels), kTileThreadsMm, sizeof(Smem), st>>>(a, t);
+    SB_LAUNCH_CHECK("spmm_tile_kernel");
+  }
+  // (may be set up while the tiles still run: it waits for them itself)
+  SB_CUDA(launch_early(spmm_tile_rows_kernel<T>,
+                       dim3((unsigned)ceil_div(a.m, kTileThreadsMm), (unsigned)std::min<int64_t>(ceil_div(a.k, 32), 64)),
+                       kTileThreadsMm, st, a, t));
+  return SB_OK;
+}
+
+}  // namespace sb

@@ -349,7 +349,9 @@ def spmm_csr(pos, crd, val, B, bias=None, relu: bool = False, plan: Optional[Csr
     """C = act(bias + A @ B) for CSR A.  ``B`` is (n, k) or (batch, n, k); ``val`` is (nnz,) —
     shared by all batch items — or (batch, nnz).  Returns (m, k) or (batch, m, k).
     2-D ``B`` / ``out`` may be column slices of wider row-major buffers (row pitch > k).
-    ``accumulate``: act(bias + out + A @ B), ``out`` required."""
+    ``accumulate``: act(bias + out + A @ B), ``out`` required.
+    One matrix runs over equal tiles of its entries and needs no ``plan``; a batch uses the plan of
+    its long rows (``plan_for(pos)`` when none is given)."""
     pos = _dev(pos, torch.int32, "pos")
     crd = _dev(crd, torch.int32, "crd")
     m, nnz = pos.numel() - 1, crd.numel()
@@ -393,11 +395,15 @@ def spmm_csr(pos, crd, val, B, bias=None, relu: bool = False, plan: Optional[Csr
             if out.stride(1) != 1 or out.stride(0) < k:
                 raise ValueError("out rows must be contiguous")
             ldc = out.stride(0)
+    L = _lib.lib()
+    use_blocks = (block_plan is not None and not accumulate and block_plan.blocks > 0 and k in _BLOCKED_SPMM_K
+                  and ldb % 4 == 0 and ldc % 4 == 0)
+    if batch == 1 and stride_val == 0 and not use_blocks and not (k >= 512 and L.sb_spmm_wide_select(-1) == 1):
+        _spmm_once(pos, crd, val, B, nb if n is None else n, ldb, bias, relu, accumulate, out, ldc)
+        return _wrote(out)
     if plan is None:
         plan = plan_for(pos, nnz)
-    L = _lib.lib()
-    if (block_plan is not None and not accumulate and block_plan.blocks > 0 and plan.segments == 0
-            and k in _BLOCKED_SPMM_K and ldb % 4 == 0 and ldc % 4 == 0):
+    if use_blocks and plan.segments == 0:
         with torch.cuda.device(B.device):
             check(L.sb_spmm_csr_blocked_f32(m, nb if n is None else n, k, nnz, pos.data_ptr(),
                                             crd.data_ptr(), val.data_ptr(), B.data_ptr(), ldb,
@@ -416,6 +422,17 @@ def spmm_csr(pos, crd, val, B, bias=None, relu: bool = False, plan: Optional[Csr
     return _wrote(out)
 
 
+def _spmm_once(pos, crd, val, B, n, ldb, bias, relu, accumulate, out, ldc):
+    L = _lib.lib()
+    code, k, nnz = _DTYPE_CODE[val.dtype], out.shape[-1], crd.numel()
+    wbytes = L.sb_spmm_csr_once_workspace_bytes(code, k, nnz)
+    with torch.cuda.device(B.device):
+        ws = torch.empty(wbytes, dtype=torch.uint8, device=B.device)
+        check(L.sb_spmm_csr_once(code, pos.numel() - 1, n, k, nnz, pos.data_ptr(), crd.data_ptr(), val.data_ptr(),
+                                 B.data_ptr(), ldb, _ptr(bias), int(bool(relu)), int(bool(accumulate)),
+                                 out.data_ptr(), ldc, ws.data_ptr(), wbytes, _stream()))
+
+
 def _spmm_typed(pos, crd, val, B, n):
     code = _DTYPE_CODE.get(val.dtype)
     if code is None:
@@ -424,12 +441,8 @@ def _spmm_typed(pos, crd, val, B, n):
     B = _dev(B, val.dtype, "B")
     if B.dim() != 2:
         raise ValueError("typed SpMM takes a 2-D dense operand")
-    m, nnz, k = pos.numel() - 1, crd.numel(), B.shape[1]
-    out = torch.empty((m, k), dtype=val.dtype, device=B.device)
-    with torch.cuda.device(B.device):
-        check(_lib.lib().sb_spmm_csr_typed(code, m, B.shape[0] if n is None else n, k, nnz,
-                                           pos.data_ptr(), crd.data_ptr(), val.data_ptr(),
-                                           B.data_ptr(), k, out.data_ptr(), k, _stream()))
+    out = torch.empty((pos.numel() - 1, B.shape[1]), dtype=val.dtype, device=B.device)
+    _spmm_once(pos, crd, val, B, B.shape[0] if n is None else n, B.shape[1], None, False, False, out, B.shape[1])
     return out
 
 
