@@ -123,6 +123,25 @@ def lib():
     return _lib
 
 
+_host = None
+
+
+def host():
+    """The native front end (``csrc/host.cpp``) bound to the library: its functions take tensors in
+    the plain form and return None for any other, which the Python path then handles."""
+    global _host
+    if _host is None:
+        lib()
+        try:
+            from . import _host as module
+        except ImportError as e:
+            raise ImportError(f"scorch_b200._host is missing: build it with `python -m scorch_b200.build` ({e})")
+        import torch
+        module.bind(LIB_PATH, ScorchB200Error, torch.OutOfMemoryError)
+        _host = module
+    return _host
+
+
 def check(status: int) -> None:
     if status != SB_OK:
         raise ScorchB200Error(status, lib().sb_last_error().decode("utf-8", "replace"))

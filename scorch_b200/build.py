@@ -18,6 +18,7 @@ CSRC = os.path.join(HERE, "csrc")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 OBJDIR = os.path.join(CSRC, "build")
 LIB = os.path.join(HERE, "libscorch_b200.so")
+HOST = os.path.join(HERE, "_host.so")          # CPython module of the native front end (csrc/host.cpp)
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
@@ -44,6 +45,20 @@ def _stale(target: str, deps: list[str]) -> bool:
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def _host_command() -> list[str]:
+    import sysconfig
+    import torch
+    from torch.utils import cpp_extension as ext
+    cmd = [_host_cxx(), "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f"-I{INCLUDE}",
+           f"-I{sysconfig.get_paths()['include']}"]
+    for d in ext.include_paths("cuda"):
+        cmd += ["-isystem", d]
+    libs = os.path.join(os.path.dirname(torch.__file__), "lib")
+    return cmd + [os.path.join(CSRC, "host.cpp"), "-o", HOST, f"-L{libs}", "-lc10", "-lc10_cuda", "-ltorch_cpu",
+                  "-ltorch_python", "-ldl"]
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
     os.makedirs(OBJDIR, exist_ok=True)
     headers = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".h"))]
@@ -64,6 +79,10 @@ def build(force: bool = False, verbose: bool = False) -> str:
             print(" ".join(cmd))
         log = open(os.path.join(OBJDIR, src[:-3] + ".ptxas.log"), "w")
         procs.append((src, subprocess.Popen(cmd, stdout=log, stderr=subprocess.STDOUT), log))
+    host_src = os.path.join(CSRC, "host.cpp")
+    if force or _stale(HOST, [host_src] + headers):
+        log = open(os.path.join(OBJDIR, "host.log"), "w")
+        procs.append(("host.cpp", subprocess.Popen(_host_command(), stdout=log, stderr=subprocess.STDOUT), log))
     failed = []
     for src, p, log in procs:
         rc = p.wait()

@@ -1,0 +1,256 @@
+// Native front end of the small calls: one CPython call checks the tensors, allocates the result
+// and the workspace from torch's allocator and calls the C ABI.
+//
+// Why: a product over a small matrix is a few microseconds of GPU work, and the Python path to it
+// (argument checks, torch.empty, a device guard and a 17-argument ctypes call) costs 20 to 30.  The
+// functions here return None for any operand that is not in the plain form (CUDA, contiguous,
+// matching types and sizes); the caller then takes the Python path, which converts or raises, so
+// every check and message lives in one place.
+#define PY_SSIZE_T_CLEAN
+#include <Python.h>
+
+#include <dlfcn.h>
+#include <stdlib.h>
+
+#include <ATen/ATen.h>
+#include <ATen/SparseCsrTensorUtils.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include "scorch_b200.h"
+
+namespace {
+
+struct Abi {
+  decltype(&sb_last_error) last_error;
+  decltype(&sb_spmm_csr_once_workspace_bytes) spmm_once_bytes;
+  decltype(&sb_spmm_csr_once) spmm_once;
+  decltype(&sb_spmm_wide_select) spmm_wide_select;
+  decltype(&sb_spmv_csr_scratch_bytes) spmv_bytes;
+  decltype(&sb_spmv_csr_f32) spmv_f32;
+  decltype(&sb_spmv_csr_typed) spmv_typed;
+  decltype(&sb_sddmm_coo_f32) sddmm_coo;
+  decltype(&sb_sddmm_csr_f32) sddmm_csr;
+} abi;
+bool bound = false;
+PyObject *error_class = nullptr, *oom_class = nullptr;
+
+// A tensor argument, or null when the object is not a torch.Tensor.
+const at::Tensor* tensor(PyObject* o) { return THPVariable_Check(o) ? &THPVariable_Unpack(o) : nullptr; }
+
+bool plain(const at::Tensor& t, at::ScalarType type) {
+  return t.is_cuda() && t.layout() == at::kStrided && t.scalar_type() == type && t.is_contiguous();
+}
+bool indices(const at::Tensor& t) { return plain(t, at::kInt) && t.dim() == 1; }
+
+int dtype_code(at::ScalarType t) {
+  switch (t) {
+    case at::kFloat: return SB_F32;
+    case at::kDouble: return SB_F64;
+    case at::kInt: return SB_I32;
+    case at::kLong: return SB_I64;
+    default: return -1;
+  }
+}
+
+PyObject* fail(int rc) {
+  PyObject* args = Py_BuildValue("(is)", rc, abi.last_error());
+  if (args) {
+    PyObject* e = PyObject_CallObject(error_class, args);
+    Py_DECREF(args);
+    if (e) {
+      PyErr_SetObject(error_class, e);
+      Py_DECREF(e);
+    }
+  }
+  return nullptr;
+}
+
+// The caller asked for every operand to be checked: the Python path does that.
+bool checking() {
+  const char* v = getenv("SCORCH_B200_VALIDATE");
+  return v && v[0] == '1' && v[1] == 0;
+}
+
+at::Tensor workspace(size_t bytes, const at::Tensor& like) {
+  return at::empty({(int64_t)(bytes > 16 ? bytes : 16)}, like.options().dtype(at::kByte));
+}
+
+void* stream_of(const at::Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.get_device()).stream(); }
+
+// C++ exceptions (the allocator out of memory, ...) as Python ones; None = not in the plain form.
+template <typename F>
+PyObject* guarded(F&& f) {
+  if (!bound) Py_RETURN_NONE;
+  try {
+    return f();
+  } catch (const c10::OutOfMemoryError& e) {
+    PyErr_SetString(oom_class, e.what());
+  } catch (const std::exception& e) {
+    PyErr_SetString(PyExc_RuntimeError, e.what());
+  }
+  return nullptr;
+}
+
+// pos, crd, val of a matrix times B (rows x k): the common part of the entry points below.
+PyObject* spmm(const at::Tensor& pos, const at::Tensor& crd, const at::Tensor& val, const at::Tensor& B,
+               const at::Tensor* bias, bool relu, int64_t n) {
+  const int code = dtype_code(val.scalar_type());
+  if (code < 0 || !indices(pos) || !indices(crd) || !plain(val, val.scalar_type()) || val.dim() != 1 ||
+      B.dim() != 2 || !plain(B, val.scalar_type()) || val.numel() != crd.numel() || pos.numel() < 1 ||
+      (n >= 0 && n != B.size(0)) || checking())
+    Py_RETURN_NONE;
+  const int64_t m = pos.numel() - 1, k = B.size(1), nnz = crd.numel();
+  if (bias && (code != SB_F32 || !plain(*bias, at::kFloat) || bias->numel() != k)) Py_RETURN_NONE;
+  if (code == SB_F32 ? (k >= 512 && abi.spmm_wide_select(-1) == 1) : (k > 65535 * 32 || relu)) Py_RETURN_NONE;
+  const c10::cuda::CUDAGuard device(B.device());
+  at::Tensor out = at::empty({m, k}, val.options());
+  const size_t bytes = abi.spmm_once_bytes(code, k, nnz);
+  at::Tensor ws = workspace(bytes, out);
+  const int rc = abi.spmm_once(code, m, B.size(0), k, nnz, pos.const_data_ptr<int>(), crd.const_data_ptr<int>(),
+                               val.const_data_ptr(), B.const_data_ptr(), k, bias ? bias->const_data_ptr() : nullptr,
+                               relu, 0, out.data_ptr(), k, ws.data_ptr(), bytes > 16 ? bytes : 16, stream_of(B));
+  return rc == SB_OK ? THPVariable_Wrap(std::move(out)) : fail(rc);
+}
+
+PyObject* spmv(const at::Tensor& pos, const at::Tensor& crd, const at::Tensor& val, const at::Tensor& x) {
+  const int code = dtype_code(val.scalar_type());
+  if (code < 0 || !indices(pos) || !indices(crd) || !plain(val, val.scalar_type()) || val.dim() != 1 ||
+      x.dim() != 1 || !plain(x, val.scalar_type()) || val.numel() != crd.numel() || pos.numel() < 1 || checking())
+    Py_RETURN_NONE;
+  const int64_t m = pos.numel() - 1, nnz = crd.numel();
+  const c10::cuda::CUDAGuard device(x.device());
+  at::Tensor y = at::empty({m}, val.options());
+  int rc;
+  if (code == SB_F32) {
+    const size_t bytes = abi.spmv_bytes(nnz);
+    at::Tensor ws = workspace(bytes, y);
+    rc = abi.spmv_f32(m, x.numel(), nnz, pos.const_data_ptr<int>(), crd.const_data_ptr<int>(),
+                      val.const_data_ptr<float>(), x.const_data_ptr<float>(), y.data_ptr<float>(), ws.data_ptr(),
+                      bytes, stream_of(x));
+  } else {
+    rc = abi.spmv_typed(code, m, x.numel(), nnz, pos.const_data_ptr<int>(), crd.const_data_ptr<int>(),
+                        val.const_data_ptr(), x.const_data_ptr(), y.data_ptr(), stream_of(x));
+  }
+  return rc == SB_OK ? THPVariable_Wrap(std::move(y)) : fail(rc);
+}
+
+// ---- Python functions ---------------------------------------------------------------------------
+// bind(path of libscorch_b200.so, class of ABI errors, class of allocation errors)
+PyObject* py_bind(PyObject*, PyObject* args) {
+  const char* path;
+  PyObject *cls, *oom;
+  if (!PyArg_ParseTuple(args, "sOO", &path, &cls, &oom)) return nullptr;
+  void* lib = dlopen(path, RTLD_NOW | RTLD_LOCAL);
+  if (!lib) return PyErr_Format(PyExc_ImportError, "%s", dlerror());
+  bool ok = true;
+  auto find = [&](auto& f, const char* name) {
+    f = reinterpret_cast<std::decay_t<decltype(f)>>(dlsym(lib, name));
+    ok = ok && f;
+  };
+  find(abi.last_error, "sb_last_error");
+  find(abi.spmm_once_bytes, "sb_spmm_csr_once_workspace_bytes");
+  find(abi.spmm_once, "sb_spmm_csr_once");
+  find(abi.spmm_wide_select, "sb_spmm_wide_select");
+  find(abi.spmv_bytes, "sb_spmv_csr_scratch_bytes");
+  find(abi.spmv_f32, "sb_spmv_csr_f32");
+  find(abi.spmv_typed, "sb_spmv_csr_typed");
+  find(abi.sddmm_coo, "sb_sddmm_coo_f32");
+  find(abi.sddmm_csr, "sb_sddmm_csr_f32");
+  if (!ok) return PyErr_Format(PyExc_ImportError, "%s lacks a symbol of the C ABI", path);
+  Py_INCREF(cls);
+  Py_INCREF(oom);
+  Py_XDECREF(error_class);
+  Py_XDECREF(oom_class);
+  error_class = cls;
+  oom_class = oom;
+  bound = true;
+  Py_RETURN_NONE;
+}
+
+// spmm(pos, crd, val, B, bias | None, relu, n | -1) -> (m, k) tensor or None
+PyObject* py_spmm(PyObject*, PyObject* const* a, Py_ssize_t count) {
+  return guarded([&]() -> PyObject* {
+    if (count != 7) Py_RETURN_NONE;
+    const at::Tensor *pos = tensor(a[0]), *crd = tensor(a[1]), *val = tensor(a[2]), *B = tensor(a[3]);
+    const at::Tensor* bias = a[4] == Py_None ? nullptr : tensor(a[4]);
+    if (!pos || !crd || !val || !B || (a[4] != Py_None && !bias)) Py_RETURN_NONE;
+    const int relu = PyObject_IsTrue(a[5]);
+    const long long n = PyLong_AsLongLong(a[6]);
+    if (relu < 0 || (n == -1 && PyErr_Occurred())) return nullptr;
+    return spmm(*pos, *crd, *val, *B, bias, relu == 1, n);
+  });
+}
+
+PyObject* py_spmv(PyObject*, PyObject* const* a, Py_ssize_t count) {
+  return guarded([&]() -> PyObject* {
+    if (count != 4) Py_RETURN_NONE;
+    const at::Tensor *pos = tensor(a[0]), *crd = tensor(a[1]), *val = tensor(a[2]), *x = tensor(a[3]);
+    if (!pos || !crd || !val || !x) Py_RETURN_NONE;
+    return spmv(*pos, *crd, *val, *x);
+  });
+}
+
+// matmul_csr(A torch CSR, B dense matrix or vector) -> tensor or None
+PyObject* py_matmul_csr(PyObject*, PyObject* const* a, Py_ssize_t count) {
+  return guarded([&]() -> PyObject* {
+    if (count != 2) Py_RETURN_NONE;
+    const at::Tensor *A = tensor(a[0]), *B = tensor(a[1]);
+    if (!A || !B || A->layout() != at::kSparseCsr || A->dim() != 2 || B->layout() != at::kStrided || B->dim() < 1)
+      Py_RETURN_NONE;
+    const auto* csr = at::sparse_csr::get_sparse_csr_impl(*A);
+    const at::Tensor &pos = csr->compressed_indices(), &crd = csr->plain_indices(), &val = csr->values();
+    if (B->dim() == 1) return spmv(pos, crd, val, *B);
+    return spmm(pos, crd, val, *B, nullptr, false, -1);
+  });
+}
+
+// sddmm(row or pos, col, mask_val, Q, K, csr) -> values, or (values, row, col) for a CSR mask, or None
+PyObject* py_sddmm(PyObject*, PyObject* const* a, Py_ssize_t count) {
+  return guarded([&]() -> PyObject* {
+    if (count != 6) Py_RETURN_NONE;
+    const at::Tensor *row = tensor(a[0]), *col = tensor(a[1]), *val = tensor(a[2]), *Q = tensor(a[3]), *K = tensor(a[4]);
+    const int csr = PyObject_IsTrue(a[5]);
+    if (csr < 0) return nullptr;
+    if (!row || !col || !val || !Q || !K || !indices(*row) || !indices(*col) || !plain(*val, at::kFloat) ||
+        !plain(*Q, at::kFloat) || !plain(*K, at::kFloat) || Q->dim() != 2 || K->dim() != 2 ||
+        Q->size(1) != K->size(1) || val->numel() != col->numel() ||
+        (csr ? row->numel() != Q->size(0) + 1 : row->numel() != col->numel()) || checking())
+      Py_RETURN_NONE;
+    const int64_t m = Q->size(0), n = K->size(0), d = Q->size(1), nnz = col->numel();
+    const c10::cuda::CUDAGuard device(Q->device());
+    at::Tensor out = at::empty({nnz}, Q->options());
+    int rc;
+    if (!csr) {
+      rc = abi.sddmm_coo(m, n, d, nnz, row->const_data_ptr<int>(), col->const_data_ptr<int>(),
+                         val->const_data_ptr<float>(), Q->const_data_ptr<float>(), d, K->const_data_ptr<float>(), d,
+                         out.data_ptr<float>(), 1, 0, 0, 0, stream_of(*Q));
+      return rc == SB_OK ? THPVariable_Wrap(std::move(out)) : fail(rc);
+    }
+    at::Tensor orow = at::empty({nnz}, row->options()), ocol = at::empty({nnz}, row->options());
+    rc = abi.sddmm_csr(m, n, d, nnz, row->const_data_ptr<int>(), col->const_data_ptr<int>(),
+                       val->const_data_ptr<float>(), Q->const_data_ptr<float>(), d, K->const_data_ptr<float>(), d,
+                       out.data_ptr<float>(), orow.data_ptr<int>(), ocol.data_ptr<int>(), 1, 0, 0, 0, stream_of(*Q));
+    if (rc != SB_OK) return fail(rc);
+    return Py_BuildValue("(NNN)", THPVariable_Wrap(std::move(out)), THPVariable_Wrap(std::move(orow)),
+                         THPVariable_Wrap(std::move(ocol)));
+  });
+}
+
+PyMethodDef methods[] = {
+    {"bind", py_bind, METH_VARARGS, "bind(path, error_class, oom_class): resolve the C ABI"},
+    {"spmm", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_spmm)), METH_FASTCALL,
+     "spmm(pos, crd, val, B, bias, relu, n) -> tensor, or None for the general path"},
+    {"spmv", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_spmv)), METH_FASTCALL,
+     "spmv(pos, crd, val, x) -> tensor, or None for the general path"},
+    {"matmul_csr", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_matmul_csr)), METH_FASTCALL,
+     "matmul_csr(A, B) for a torch CSR tensor A -> tensor, or None for the general path"},
+    {"sddmm", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_sddmm)), METH_FASTCALL,
+     "sddmm(row_or_pos, col, mask_val, Q, K, csr) -> tensor(s), or None for the general path"},
+    {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__host(void) { return PyModule_Create(&module); }

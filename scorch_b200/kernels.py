@@ -352,6 +352,10 @@ def spmm_csr(pos, crd, val, B, bias=None, relu: bool = False, plan: Optional[Csr
     ``accumulate``: act(bias + out + A @ B), ``out`` required.
     One matrix runs over equal tiles of its entries and needs no ``plan``; a batch uses the plan of
     its long rows (``plan_for(pos)`` when none is given)."""
+    if out is None and block_plan is None and not accumulate:
+        r = _lib.host().spmm(pos, crd, val, B, bias, relu, -1 if n is None else n)
+        if r is not None:
+            return r
     pos = _dev(pos, torch.int32, "pos")
     crd = _dev(crd, torch.int32, "crd")
     m, nnz = pos.numel() - 1, crd.numel()
@@ -449,6 +453,9 @@ def _spmm_typed(pos, crd, val, B, n):
 def spmv_csr(pos, crd, val, x, plan: Optional[CsrPlan] = None) -> torch.Tensor:
     """y = A @ x for CSR A (``plan`` is accepted for symmetry with ``spmm_csr`` and not needed:
     the fp32 kernel is balanced by entries, not rows)."""
+    r = _lib.host().spmv(pos, crd, val, x)
+    if r is not None:
+        return r
     pos = _dev(pos, torch.int32, "pos")
     crd = _dev(crd, torch.int32, "crd")
     m, nnz = pos.numel() - 1, crd.numel()

@@ -15,6 +15,7 @@ from typing import Any, Callable, List, Mapping, Optional, Sequence, Tuple, Unio
 
 import torch
 
+from . import _lib
 from . import scorch_ops as native_ops
 from .stensor import STensor, TensorFormat, TensorIndex, parse_format
 
@@ -115,9 +116,29 @@ def _wrap(result_cpp, shape, fmt) -> STensor:
                    value=result_cpp.storage.value)
 
 
+def _matmul_on_device(a, b) -> Optional[torch.Tensor]:
+    """CSR x dense operands that already lie on the GPU in the layout the kernels take: straight to
+    the native front end.  None: the general path below."""
+    if not isinstance(b, torch.Tensor) or not b.is_cuda:
+        return None
+    if isinstance(a, STensor):
+        index = a.storage.index
+        if index.tensor_format.levels != ("d", "s") or index.mode_order != [0, 1]:
+            return None
+        pos, crd = index.mode_indices[1]
+        if b.dim() == 2:
+            return _lib.host().spmm(pos, crd, a.storage.value, b, None, False, -1)
+        return _lib.host().spmv(pos, crd, a.storage.value, b) if b.dim() == 1 else None
+    return _lib.host().matmul_csr(a, b)
+
+
 def matmul(a: Union[torch.Tensor, STensor], b: Union[torch.Tensor, STensor], **kwargs: Any
            ) -> Union[torch.Tensor, STensor]:
     """Matrix product with the reference's dispatch (src/scorch/ops.py:248-372)."""
+    if not kwargs:
+        r = _matmul_on_device(a, b)
+        if r is not None:
+            return r
     if isinstance(a, torch.Tensor) and isinstance(b, torch.Tensor):
         a_sp = a.layout != torch.strided
         b_sp = b.layout != torch.strided
@@ -161,6 +182,22 @@ def matmul(a: Union[torch.Tensor, STensor], b: Union[torch.Tensor, STensor], **k
     return result.to_torch() if result.format.is_dense() else result
 
 
+def _sddmm_on_device(S, Q, K) -> Optional[STensor]:
+    """SDDMM of a sparse mask and dense Q, K that already lie on the GPU (see _matmul_on_device)."""
+    if not isinstance(S, STensor) or not S.values.is_cuda:
+        return None
+    index = S.storage.index
+    levels = index.tensor_format.levels
+    if levels == ("o", "o"):
+        (row,), (col,) = index.mode_indices
+        v = _lib.host().sddmm(row, col, S.storage.value, Q, K, False)
+        return None if v is None else STensor(S.shape, index=TensorIndex(index.mode_indices, S.format), value=v)
+    if levels == ("d", "s"):
+        r = _lib.host().sddmm(*index.mode_indices[1], S.storage.value, Q, K, True)
+        return None if r is None else STensor(S.shape, index=TensorIndex([[r[1]], [r[2]]], "o,o"), value=r[0])
+    return None
+
+
 _SDDMM_EXPRS = ("ij,ik,jk->ij", "ij,ik,kj->ij")
 
 
@@ -175,8 +212,12 @@ def einsum(expression: str, *tensors: Union[torch.Tensor, STensor], **kwargs: An
     * ``"ijk,km->ijm"`` (TTM) and ``"ijk,jm,km->im"`` (MTTKRP) with a ``d,s,s`` / ``s,s,s`` (or dense)
       3-D tensor and dense matrices -> dense result (``tensor3``).
     """
-    ts = tuple(STensor.from_torch(t) if isinstance(t, torch.Tensor) else t for t in tensors)
     expr = expression.replace(" ", "")
+    if expr == "ij,ik,jk->ij" and len(tensors) == 3:
+        r = _sddmm_on_device(*tensors)
+        if r is not None:
+            return r
+    ts = tuple(STensor.from_torch(t) if isinstance(t, torch.Tensor) else t for t in tensors)
     if expr in _SDDMM_EXPRS and len(ts) == 3:
         S, A, B = ts
         if not (str(A.format) == "d,d" and str(B.format) == "d,d" and S.dtype == torch.float32):
@@ -270,6 +311,11 @@ def spmm_bias_act(a: Union[torch.Tensor, STensor], b: torch.Tensor, bias: torch.
                   relu: bool) -> torch.Tensor:
     """Fused ``act(A @ B + bias)`` — the kernel ``@scorch.compile`` reaches for a GCN layer
     (reference: src/scorch/trace.py:232-301 -> csrc/spmm.h:28-89)."""
+    if isinstance(a, STensor) and a.storage.index.tensor_format.levels == ("d", "s") and b.is_cuda:
+        pos, crd = a.storage.index.mode_indices[1]
+        r = _lib.host().spmm(pos, crd, a.storage.value, b, bias, relu, -1)
+        if r is not None:
+            return r
     if isinstance(a, torch.Tensor):
         a = STensor.from_torch(a)
     bs = STensor.from_torch(b)
