@@ -34,11 +34,11 @@ static int short_rows_wanted(int64_t m, int64_t k, int64_t nnz) {
 }
 
 template <typename T>
-static SpmmArgs<T> spmm_args(int64_t m, int64_t k, int64_t nnz, const int* pos, const int* crd, const T* val,
+static SpmmArgs<T> spmm_args(int64_t m, int64_t n, int64_t k, int64_t nnz, const int* pos, const int* crd, const T* val,
                              const T* B, int64_t ldb, const T* bias, int relu, T* C, int64_t ldc,
                              int64_t stride_val, int64_t stride_b, int64_t stride_c) {
   SpmmArgs<T> a{};
-  a.m = (int)m; a.k = (int)k; a.pos = pos; a.end = pos + 1; a.crd = crd; a.val = val; a.B = B; a.ldb = ldb;
+  a.m = (int)m; a.n = (int)n; a.k = (int)k; a.pos = pos; a.end = pos + 1; a.crd = crd; a.val = val; a.B = B; a.ldb = ldb;
   a.bias = bias; a.relu = relu; a.C = C; a.ldc = ldc;
   a.stride_val = stride_val; a.stride_b = stride_b; a.stride_c = stride_c;
   a.short_rows = short_rows_wanted(m, k, nnz);
@@ -52,7 +52,7 @@ int spmm_remainder(int64_t m, int64_t k, const int* rem_pos, const int* rem_ent,
                    const float* val, const float* B, int64_t ldb, const float* bias, int relu,
                    float* C, int64_t ldc, int64_t batch, int64_t stride_val, int64_t stride_b,
                    int64_t stride_c, int val_compact, cudaStream_t st) {
-  SpmmArgs<float> a = spmm_args<float>(m, k, 0, rem_pos, crd, val, B, ldb, bias, relu, C, ldc, stride_val,
+  SpmmArgs<float> a = spmm_args<float>(m, m, k, 0, rem_pos, crd, val, B, ldb, bias, relu, C, ldc, stride_val,
                                        stride_b, stride_c);
   a.ent = rem_ent; a.val_compact = val_compact; a.accumulate = 1; a.short_rows = 1;
   return spmm_dispatch_f32(a, batch, nullptr, 0, 0, nullptr, nullptr, st);
@@ -75,10 +75,10 @@ static int check_common(int64_t m, int64_t n, int64_t k, int64_t nnz, const void
 }
 
 template <typename T>
-static int spmm_typed(int64_t m, int64_t k, int64_t nnz, const int32_t* pos, const int32_t* crd, const void* val,
+static int spmm_typed(int64_t m, int64_t n, int64_t k, int64_t nnz, const int32_t* pos, const int32_t* crd, const void* val,
                       const void* B, int64_t ldb, const void* bias, int relu, int accumulate, void* C,
                       int64_t ldc, void* tile_ws, cudaStream_t st) {
-  SpmmArgs<T> a = spmm_args<T>(m, k, nnz, pos, crd, (const T*)val, (const T*)B, ldb, (const T*)bias, relu, (T*)C,
+  SpmmArgs<T> a = spmm_args<T>(m, n, k, nnz, pos, crd, (const T*)val, (const T*)B, ldb, (const T*)bias, relu, (T*)C,
                                ldc, 0, 0, 0);
   a.accumulate = accumulate ? 1 : 0;
   return spmm_dispatch_typed<T>(a, nnz, tile_ws, st);
@@ -130,7 +130,7 @@ static int spmm_csr_f32_impl(int64_t m, int64_t n, int64_t k, int64_t nnz, const
   // wide operands, no heavy rows: optionally the bulk-copy kernel of spmm_wide.cu
   if (k >= 512 && batch == 1 && vec_ok && !accumulate && !(plan && plan_segments != 0) && spmm_wide_wanted())
     return spmm_wide_launch(m, k, pos, crd, val, B, ldb, bias, relu, C, ldc, st);
-  SpmmArgs<float> a = spmm_args<float>(m, k, nnz, pos, crd, val, B, ldb, bias, relu, C, ldc, stride_val,
+  SpmmArgs<float> a = spmm_args<float>(m, n, k, nnz, pos, crd, val, B, ldb, bias, relu, C, ldc, stride_val,
                                        stride_b, stride_c);
   a.skip_heavy = (plan && plan_segments != 0) ? 1 : 0;
   a.accumulate = accumulate ? 1 : 0;
@@ -178,16 +178,16 @@ int sb_spmm_csr_once(int dtype, int64_t m, int64_t n, int64_t k, int64_t nnz, co
   cudaStream_t st = (cudaStream_t)stream;
   switch (dtype) {
     case SB_F32: {
-      SpmmArgs<float> a = spmm_args<float>(m, k, nnz, pos, crd, (const float*)val, (const float*)B, ldb,
+      SpmmArgs<float> a = spmm_args<float>(m, n, k, nnz, pos, crd, (const float*)val, (const float*)B, ldb,
                                            (const float*)bias, relu, (float*)C, ldc, 0, 0, 0);
       a.accumulate = accumulate ? 1 : 0;
       return spmm_dispatch_f32(a, 1, nullptr, nnz, 0, nullptr, ws, st);
     }
-    case SB_F64: return spmm_typed<double>(m, k, nnz, pos, crd, val, B, ldb, bias, relu, accumulate, C, ldc, ws, st);
+    case SB_F64: return spmm_typed<double>(m, n, k, nnz, pos, crd, val, B, ldb, bias, relu, accumulate, C, ldc, ws, st);
     case SB_I32:  // unsigned arithmetic: same bits as the reference's wrapping int32 math
-      return spmm_typed<unsigned int>(m, k, nnz, pos, crd, val, B, ldb, bias, relu, accumulate, C, ldc, ws, st);
+      return spmm_typed<unsigned int>(m, n, k, nnz, pos, crd, val, B, ldb, bias, relu, accumulate, C, ldc, ws, st);
     default:
-      return spmm_typed<unsigned long long>(m, k, nnz, pos, crd, val, B, ldb, bias, relu, accumulate, C, ldc, ws, st);
+      return spmm_typed<unsigned long long>(m, n, k, nnz, pos, crd, val, B, ldb, bias, relu, accumulate, C, ldc, ws, st);
   }
 }
 
@@ -206,11 +206,11 @@ int sb_spmm_csr_typed(int dtype, int64_t m, int64_t n, int64_t k, int64_t nnz, c
       return sb_spmm_csr_f32(m, n, k, nnz, pos, crd, (const float*)val, (const float*)B, ldb,
                              nullptr, 0, (float*)C, ldc, 1, 0, 0, 0, nullptr, 0, nullptr, 0, stream);
     case SB_F64:
-      return spmm_typed<double>(m, k, nnz, pos, crd, val, B, ldb, nullptr, 0, 0, C, ldc, nullptr, st);
+      return spmm_typed<double>(m, n, k, nnz, pos, crd, val, B, ldb, nullptr, 0, 0, C, ldc, nullptr, st);
     case SB_I32:  // unsigned arithmetic: same bits as the reference's wrapping int32 math
-      return spmm_typed<unsigned int>(m, k, nnz, pos, crd, val, B, ldb, nullptr, 0, 0, C, ldc, nullptr, st);
+      return spmm_typed<unsigned int>(m, n, k, nnz, pos, crd, val, B, ldb, nullptr, 0, 0, C, ldc, nullptr, st);
     case SB_I64:
-      return spmm_typed<unsigned long long>(m, k, nnz, pos, crd, val, B, ldb, nullptr, 0, 0, C, ldc, nullptr, st);
+      return spmm_typed<unsigned long long>(m, n, k, nnz, pos, crd, val, B, ldb, nullptr, 0, 0, C, ldc, nullptr, st);
     default:
       return fail(SB_ERR_UNSUPPORTED, "spmm_typed: unknown dtype %d", dtype);
   }

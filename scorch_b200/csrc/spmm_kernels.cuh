@@ -43,6 +43,7 @@ constexpr int kWarpsPerCta = 8;
 template <typename T>
 struct SpmmArgs {
   int m;
+  int n;               // rows of B
   int k;
   const int* pos;      // first entry of each row ...
   const int* end;      // ... and the one after its last (pos + 1 unless only part of a row is taken)

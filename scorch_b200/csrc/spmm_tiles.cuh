@@ -46,7 +46,7 @@ static_assert(tile_window(8) / kWarpRow + tile_window(8) / kUnit + 4 <= kTileLis
 constexpr int tile_ctas(int L) { return L == 32 ? 4 : 3; }
 // Entries per window, a multiple of 32: as few full waves of CTAs over the chip as windows of at
 // most tile_window(L) allow (a last wave that is half empty costs as much as a full one), at least 64
-// and at least four per lane group.
+// and at least four per lane group. 
 inline int tile_entries(int64_t nnz, int L) {
   const int64_t slots = 148 * tile_ctas(L);
   const int64_t waves = std::max<int64_t>(1, ceil_div(nnz, slots * tile_window(L)));
@@ -56,7 +56,7 @@ inline int tile_entries(int64_t nnz, int L) {
 
 template <typename T>
 struct TileArgs {
-  int nnz, entries, tiles;
+  int nnz, entries, tiles, panels;
   T* first;         // [nnz / kUnit + 1][k] sums of the first units of rows of several units ...
   T* rest;          // ... and of their other units; index = first entry of the unit / kUnit
 };
@@ -207,14 +207,6 @@ spmm_tile_kernel(SpmmArgs<T> a, TileArgs<T> t) {
   extern __shared__ __align__(32) unsigned char smem_raw[];
   Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, l = lane % L, g = lane / L;
-  const int col0 = blockIdx.y * (L * W * VEC) + l * W;
-  bool col_ok[VEC];
-  const char* Bcol[VEC];
-#pragma unroll
-  for (int v = 0; v < VEC; v++) {
-    col_ok[v] = (col0 + v * L * W) < a.k;
-    Bcol[v] = reinterpret_cast<const char*>(a.B + (col_ok[v] ? col0 + v * L * W : 0));
-  }
   const unsigned pitch = (unsigned)(a.ldb * (long long)sizeof(T));
   const int e0 = (int)blockIdx.x * t.entries, e1 = min(t.nnz, e0 + t.entries);
   const int staged = min(t.nnz, e1 + kUnit) - e0;
@@ -255,6 +247,16 @@ spmm_tile_kernel(SpmmArgs<T> a, TileArgs<T> t) {
 #pragma unroll
     for (int w = 0; w < kTileWarps; w++) rows += sm.count[w];
     const int n_cta = sm.n_cta, n_warp = sm.n_warp;
+
+    for (int panel = blockIdx.y; panel < t.panels; panel += gridDim.y) {
+    const int col0 = panel * (L * W * VEC) + l * W;
+    bool col_ok[VEC];
+    const char* Bcol[VEC];
+#pragma unroll
+    for (int v = 0; v < VEC; v++) {
+      col_ok[v] = (col0 + v * L * W) < a.k;
+      Bcol[v] = reinterpret_cast<const char*>(a.B + (col_ok[v] ? col0 + v * L * W : 0));
+    }
 
     for (int i = 0; i < n_cta; i++) {
       const TileUnit q = sm.by_cta[i];
@@ -321,6 +323,10 @@ spmm_tile_kernel(SpmmArgs<T> a, TileArgs<T> t) {
       tile_add<T, VEC, W, U>(s, sm.entry, b - e0, b - e0 + len, Bcol, pitch);
       tile_store_row<T, L, VEC, W>(a, r0 + i, col0, col_ok, s);
     }
+    __syncthreads();
+    if (tid == 0) sm.next_warp = sm.next_row = 0;
+    __syncthreads();
+    }
     next = sm.pos[kTileRowCap];
     __syncthreads();
   }
@@ -371,7 +377,15 @@ static int launch_tiles(const SpmmArgs<T>& a, int64_t nnz, void* ws, cudaStream_
                 65535ll * (L * W * VEC), a.k);
   TileArgs<T> t;
   t.nnz = (int)nnz;
-  t.entries = tile_entries(nnz, L);
+  t.panels = (int)panels;
+  // Column panels.  An operand that L2 holds whole: every (window, panel) is a CTA of its own, windows
+  // sized for all of them together (81,724 entries, 8 panels of 4 MB: 63 us with the next form, 45
+  // with this).  A larger one, all windows resident at once: every CTA goes through the panels
+  // itself; its start-up is paid once, and the CTAs, equally loaded, stay at about the same panel,
+  // which L2 holds (262,144 entries, 16 panels of 32 MB: 286 us panel by panel, 249 this way).
+  // Otherwise panel after panel on grid.y.
+  const bool in_l2 = (double)a.n * a.ldb * sizeof(T) <= 64e6;
+  t.entries = tile_entries(in_l2 ? nnz * panels : nnz, L);
   t.tiles = (int)ceil_div(nnz, t.entries);
   t.first = static_cast<T*>(ws);
   t.rest = t.first + (size_t)(nnz / kUnit + 1) * a.k;
@@ -384,7 +398,8 @@ static int launch_tiles(const SpmmArgs<T>& a, int64_t nnz, void* ws, cudaStream_
       SB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem)));
       if (dev >= 0 && dev < 64) sized[dev] = true;
     }
-    kernel<<<dim3((unsigned)t.tiles, panels), kTileThreadsMm, sizeof(Smem), st>>>(a, t);
+    const bool resident = !in_l2 && t.tiles <= 148 * tile_ctas(L);
+    kernel<<<dim3((unsigned)t.tiles, resident ? 1 : panels), kTileThreadsMm, sizeof(Smem), st>>>(a, t);
     SB_LAUNCH_CHECK("spmm_tile_kernel");
   }
   // (may be set up while the tiles still run: it waits for them itself)
