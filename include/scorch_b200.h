@@ -391,6 +391,27 @@ SB_API int sb_spgemm_numeric(int dtype, int64_t m, int64_t kb, int64_t n, const 
                              const int32_t* Bcrd, const void* Bval, const int32_t* Cpos,
                              int32_t* Ccrd, void* Cval, void* ws, size_t ws_bytes, void* stream);
 
+/* The same product in one pass: every row is expanded and sorted once, its entries written at the
+ * row's product offset (an upper bound of its entry offset) and moved together at the end.  Costs
+ * memory for all products instead of a second expansion.
+ *   sb_spgemm_begin   product offsets off[m + 1], rows per bin (counts_host[5]) and the number of
+ *                     products; synchronises.  off is valid where products <= INT32_MAX.
+ *   sb_spgemm_rows    the rows into tcrd / tval (one slot per product), Cpos[m + 1] and the total;
+ *                     synchronises; SB_ERR_OVERFLOW as for sb_spgemm_symbolic.  `ws` and counts as
+ *                     sb_spgemm_begin left them.
+ *   sb_spgemm_finish  the rows to their places in Ccrd / Cval. */
+SB_API int sb_spgemm_begin(int64_t m, int64_t kb, int64_t n, const int32_t* Apos, const int32_t* Acrd,
+                           const int32_t* Bpos, int32_t* off, int64_t* counts_host,
+                           int64_t* products_host, void* ws, size_t ws_bytes, void* stream);
+SB_API int sb_spgemm_rows(int dtype, int64_t m, int64_t kb, int64_t n, const int32_t* Apos,
+                          const int32_t* Acrd, const void* Aval, const int32_t* Bpos,
+                          const int32_t* Bcrd, const void* Bval, const int32_t* off,
+                          const int64_t* counts_host, int32_t* tcrd, void* tval, int32_t* Cpos,
+                          int64_t* total_nnz_host, void* ws, size_t ws_bytes, void* stream);
+SB_API int sb_spgemm_finish(int dtype, int64_t m, int64_t nnz, const int32_t* off, const int32_t* tcrd,
+                            const void* tval, const int32_t* Cpos, int32_t* Ccrd, void* Cval,
+                            void* stream);
+
 /* --------------------------------------------------------------------------------------------
  * Element-wise product / sum of two CSR matrices of the same shape, CSR out with ascending columns:
  *   SB_EWISE_MUL  C = A .* B, stored where both operands store an entry;

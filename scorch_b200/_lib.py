@@ -82,6 +82,11 @@ SIGNATURES = {
                                   C.POINTER(_i64), _ptr, _sz, _ptr]),
     "sb_spgemm_numeric": (_int, [_int, _i64, _i64, _i64, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr,
                                  _ptr, _ptr, _ptr, _sz, _ptr]),
+    "sb_spgemm_begin": (_int, [_i64, _i64, _i64, _ptr, _ptr, _ptr, _ptr, C.POINTER(_i64), C.POINTER(_i64), _ptr,
+                               _sz, _ptr]),
+    "sb_spgemm_rows": (_int, [_int, _i64, _i64, _i64, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, C.POINTER(_i64),
+                              _ptr, _ptr, _ptr, C.POINTER(_i64), _ptr, _sz, _ptr]),
+    "sb_spgemm_finish": (_int, [_int, _i64, _i64, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr]),
     "sb_csr_ewise_workspace_bytes": (_sz, [_i64]),
     "sb_csr_ewise_symbolic": (_int, [_int, _i64, _ptr, _ptr, _ptr, _ptr, _ptr, C.POINTER(_i64), _ptr, _sz, _ptr]),
     "sb_csr_ewise_numeric": (_int, [_int, _int, _i64, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr]),

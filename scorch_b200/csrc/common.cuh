@@ -167,6 +167,41 @@ __device__ __forceinline__ int row_of_entry(const int* __restrict__ pos, int lo,
   return lo;
 }
 
+// Row of entry p: the largest r with pos[r] <= p < pos[m]; the whole CTA calls it.  Matrices of up
+// to 32 rows per thread are looked at in one go (one round of loads in flight together instead of
+// one dependent round per factor of 256); `s_count`: one int per warp.
+template <int NT>
+__device__ __forceinline__ int cta_row_of(const int* __restrict__ pos, int m, int p, int* s_count) {
+  if (m <= 32 * NT) {
+    int c = 0;
+    for (int r = threadIdx.x; r < m; r += 8 * NT) {
+#pragma unroll
+      for (int q = 0; q < 8; q++) {
+        const int x = r + q * NT;
+        c += x < m && __ldg(pos + x) <= p;
+      }
+    }
+    c = __reduce_add_sync(FULL, c);
+    if ((threadIdx.x & 31) == 0) s_count[threadIdx.x >> 5] = c;
+    __syncthreads();
+    c = 0;
+#pragma unroll
+    for (int w = 0; w < NT / 32; w++) c += s_count[w];
+    __syncthreads();
+    return c - 1;
+  }
+  int lo = 0, hi = m;
+  while (true) {
+    const int span = hi - lo;
+    const int step = (span + NT - 1) / NT;
+    const long long r = (long long)lo + (long long)threadIdx.x * step;
+    const int c = __syncthreads_count(r < hi && __ldg(pos + r) <= p);
+    lo += (c - 1) * step;
+    if (step == 1) return lo;
+    hi = min(hi, lo + step);
+  }
+}
+
 #endif  // __CUDACC__
 
 }  // namespace sb

@@ -32,6 +32,10 @@ struct Abi {
   decltype(&sb_spmv_csr_typed) spmv_typed;
   decltype(&sb_sddmm_coo_f32) sddmm_coo;
   decltype(&sb_sddmm_csr_f32) sddmm_csr;
+  decltype(&sb_spgemm_workspace_bytes) spgemm_bytes;
+  decltype(&sb_spgemm_begin) spgemm_begin;
+  decltype(&sb_spgemm_rows) spgemm_rows;
+  decltype(&sb_spgemm_finish) spgemm_finish;
 } abi;
 bool bound = false;
 PyObject *error_class = nullptr, *oom_class = nullptr;
@@ -158,6 +162,10 @@ PyObject* py_bind(PyObject*, PyObject* args) {
   find(abi.spmv_typed, "sb_spmv_csr_typed");
   find(abi.sddmm_coo, "sb_sddmm_coo_f32");
   find(abi.sddmm_csr, "sb_sddmm_csr_f32");
+  find(abi.spgemm_bytes, "sb_spgemm_workspace_bytes");
+  find(abi.spgemm_begin, "sb_spgemm_begin");
+  find(abi.spgemm_rows, "sb_spgemm_rows");
+  find(abi.spgemm_finish, "sb_spgemm_finish");
   if (!ok) return PyErr_Format(PyExc_ImportError, "%s lacks a symbol of the C ABI", path);
   Py_INCREF(cls);
   Py_INCREF(oom);
@@ -238,6 +246,70 @@ PyObject* py_sddmm(PyObject*, PyObject* const* a, Py_ssize_t count) {
   });
 }
 
+// spgemm(Apos, Acrd, Aval, Bpos, Bcrd, Bval, n) -> (Cpos, Ccrd, Cval), or None: not in the plain
+// form, or more products than the one-pass form has memory for
+constexpr int64_t kOnePassBytes = (int64_t)16 << 30;
+
+PyObject* py_spgemm(PyObject*, PyObject* const* a, Py_ssize_t count) {
+  return guarded([&]() -> PyObject* {
+    if (count != 7) Py_RETURN_NONE;
+    const at::Tensor* t[6];
+    for (int i = 0; i < 6; i++)
+      if (!(t[i] = tensor(a[i]))) Py_RETURN_NONE;
+    const long long n = PyLong_AsLongLong(a[6]);
+    if (n == -1 && PyErr_Occurred()) return nullptr;
+    const at::Tensor &apos = *t[0], &acrd = *t[1], &aval = *t[2], &bpos = *t[3], &bcrd = *t[4], &bval = *t[5];
+    const int code = dtype_code(aval.scalar_type());
+    if (code < 0 || !indices(apos) || !indices(acrd) || !indices(bpos) || !indices(bcrd) ||
+        !plain(aval, aval.scalar_type()) || !plain(bval, aval.scalar_type()) || aval.dim() != 1 || bval.dim() != 1 ||
+        aval.numel() != acrd.numel() || bval.numel() != bcrd.numel() || apos.numel() < 1 || bpos.numel() < 1 ||
+        checking())
+      Py_RETURN_NONE;
+    const int64_t m = apos.numel() - 1, kb = bpos.numel() - 1, size = aval.element_size();
+    const c10::cuda::CUDAGuard device(aval.device());
+    void* stream = stream_of(aval);
+    const size_t bytes = abi.spgemm_bytes(m, n, code);
+    at::Tensor ws = workspace(bytes, aval), off = at::empty({m + 1}, apos.options());
+    int64_t counts[5], products = 0, total = 0;
+    const int *ap = apos.const_data_ptr<int>(), *ac = acrd.const_data_ptr<int>();
+    const int *bp = bpos.const_data_ptr<int>(), *bc = bcrd.const_data_ptr<int>();
+    int rc = abi.spgemm_begin(m, kb, n, ap, ac, bp, off.data_ptr<int>(), counts, &products, ws.data_ptr(), bytes,
+                              stream);
+    if (rc != SB_OK) return fail(rc);
+    if (products > INT32_MAX || products * (4 + size) > kOnePassBytes) Py_RETURN_NONE;
+    at::Tensor cpos = at::empty({m + 1}, apos.options()), ccrd, cval;
+    {
+      at::Tensor tcrd, tval;
+      try {
+        tcrd = at::empty({products}, apos.options());
+        tval = at::empty({products}, aval.options());
+      } catch (const c10::OutOfMemoryError&) {
+        Py_RETURN_NONE;
+      }
+      rc = abi.spgemm_rows(code, m, kb, n, ap, ac, aval.const_data_ptr(), bp, bc, bval.const_data_ptr(),
+                           off.data_ptr<int>(), counts, tcrd.data_ptr<int>(), tval.data_ptr(), cpos.data_ptr<int>(),
+                           &total, ws.data_ptr(), bytes, stream);
+      if (rc != SB_OK) return fail(rc);
+      if (total == products) {     // no two products met: the rows are in place already
+        ccrd = tcrd;
+        cval = tval;
+      } else {
+        try {
+          ccrd = at::empty({total}, apos.options());
+          cval = at::empty({total}, aval.options());
+        } catch (const c10::OutOfMemoryError&) {
+          Py_RETURN_NONE;
+        }
+        rc = abi.spgemm_finish(code, m, total, off.data_ptr<int>(), tcrd.data_ptr<int>(), tval.data_ptr(),
+                               cpos.data_ptr<int>(), ccrd.data_ptr<int>(), cval.data_ptr(), stream);
+        if (rc != SB_OK) return fail(rc);
+      }
+    }
+    return Py_BuildValue("(NNN)", THPVariable_Wrap(std::move(cpos)), THPVariable_Wrap(std::move(ccrd)),
+                         THPVariable_Wrap(std::move(cval)));
+  });
+}
+
 PyMethodDef methods[] = {
     {"bind", py_bind, METH_VARARGS, "bind(path, error_class, oom_class): resolve the C ABI"},
     {"spmm", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_spmm)), METH_FASTCALL,
@@ -248,6 +320,8 @@ PyMethodDef methods[] = {
      "matmul_csr(A, B) for a torch CSR tensor A -> tensor, or None for the general path"},
     {"sddmm", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_sddmm)), METH_FASTCALL,
      "sddmm(row_or_pos, col, mask_val, Q, K, csr) -> tensor(s), or None for the general path"},
+    {"spgemm", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_spgemm)), METH_FASTCALL,
+     "spgemm(Apos, Acrd, Aval, Bpos, Bcrd, Bval, n) -> (Cpos, Ccrd, Cval), or None for the two-phase path"},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

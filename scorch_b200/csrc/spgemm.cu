@@ -1,198 +1,227 @@
-// CSR x CSR SpGEMM (Gustavson) for sm_100a, two phases (symbolic / numeric) like the reference.
+// CSR x CSR SpGEMM (Gustavson) for sm_100a.
 //
 // Rows of A are binned by their product upper bound U_i = sum over the row's entries of the
 // length of the matching B row:
-//   bin 0  U <= 32      one warp per row, 64-slot hash set/accumulator in shared memory
-//   bin 1  U <= 128     one warp per row, 256 slots
-//   bin 2  U <= 512     one 128-thread CTA per row, 1024 slots
-//   bin 3  U <= 2048    one 256-thread CTA per row, 4096 slots
-//   bin 4  U <= 8192    one 512-thread CTA per row, 16384 slots
-//   bin 5  U  > 8192    dense bitmap (+ dense accumulator) of n columns in the workspace; the
-//                       rows' entries are spread over the GPU as (row, chunk) tasks
-// Hash bins: open addressing with atomicCAS on the column key (+ atomicAdd on the value), load
-// factor <= 0.5 by construction.  The numeric phase compacts each row's table in place and sorts
-// the occupied part in shared memory (bitonic) so columns come out ascending like the
-// reference's per-row sort; the dense bin emits columns in bitmap order, which is already
-// ascending.  The structure is the symbolic union: a slot whose value cancels to 0 is kept.
-// Row pointers come from a three-kernel exclusive scan in int64, stored as int32 with an
-// overflow check.
+//   bin 0  U <= 128     one warp per row, products sorted by (column, ordinal) in registers
+//   bin 1  U <= 512     one 64-thread CTA per row, the same network across its warps
+//   bin 2  U <= 2048    one 128-thread CTA per row
+//   bin 3  U <= 8192    one 512-thread CTA per row, its columns in segments of a warp each
+//   bin 4  U  > 8192    the row's columns are cut into buckets of some 700 products, the products
+//                       scattered to their buckets in global memory and every bucket sorted by a CTA
+// (spgemm_rows.cuh: the sorting kernels of bins 0-3.)  Columns come out ascending like the
+// reference's per-row sort; the structure is the symbolic union: an entry whose value cancels to 0
+// is kept.  Two ways to run it:
+//   two phases (sb_spgemm_symbolic / _numeric, like the reference): count, then the same kernels
+//     again with values;
+//   one pass (sb_spgemm_begin / _rows / _finish): every row's entries are written at the row's
+//     product offset (an upper bound of its entry offset) and moved together afterwards - one
+//     expansion and sort less for one copy of the result more.
+// Row pointers come from an exclusive scan in int64, stored as int32 with an overflow check.
 //
-// Values are reproducible bit for bit from run to run.  Several products may land on one output
-// entry and the hardware serves their atomic additions in any order, so floating-point sums are
-// not added as floats: every product is computed exactly in double, scaled by a power of two
-// chosen per output row so that no partial sum can overflow (2^61 / (sum |a| of the row * max |b|)),
-// rounded to a 64-bit integer and added with integer atomics, whose result does not depend on
-// the order.  The total is converted back once per entry.  The rounding step is 2^-61 of the
-// row's bound, far below fp32 (and fp64) resolution of the sum itself.  Rows whose bound is not
-// finite (Inf / NaN operands) are added as floats like before, so those values propagate.
-// Integer dtypes wrap like the reference's and need none of this.
+// Values are reproducible bit for bit from run to run.  Bins 0-3 sum the products of an entry in the
+// order of their ordinals.  A bucket's products arrive in no order; where several land on one
+// entry, every product is computed exactly in double, scaled by a power of two chosen per output row
+// so that no partial sum can overflow (2^61 / (sum |a| of the row * max |b|)), rounded to a 64-bit
+// integer and added as an integer, whose result does not depend on the order.  The rounding step is
+// 2^-61 of the row's bound, far below fp32 (and fp64) resolution of the sum itself.  Rows whose bound
+// is not finite add floats.  Integer dtypes wrap like the reference's and need none of this.
 #include <limits.h>
 #include <string.h>
 
 #include <algorithm>
+#include <vector>
 
-#include "common.cuh"
+#include "spgemm_rows.cuh"
 
 namespace sb {
 
-constexpr int kBins = 6;
-constexpr int kEmpty = INT_MAX;
-constexpr int kDenseWorkersMax = 296;  // 2 CTAs per SM on a 148-SM part
-constexpr size_t kDenseBudget = (size_t)4 << 30;
+constexpr int kBins = 5;
 
-// Workspace header (int64 words): [0..5] rows per bin, [8] total nnz of C.
+// Long rows (bin 4) are handled in batches of at most `products` products (the area's capacity); a
+// single row with more than that takes the dense kernel, whose bitmap and accumulator of n columns
+// lie in the same area.
+constexpr int64_t kBigProductsMax = (int64_t)1 << 26;
+constexpr int64_t kBucketProducts = 1024;      // buckets per row: U / this, rounded up to a power of two
+constexpr int kBucketSort = 2048;              // products a bucket's sorting kernel takes
+constexpr int kBigTasks = 1 << 17;
+
+static int64_t big_products(int64_t m, int64_t n) {
+  return std::min<int64_t>(kBigProductsMax, std::max<int64_t>((int64_t)1 << 20, 64 * (m + n)));
+}
+static int64_t big_buckets(int64_t products) { return products / (kBucketProducts / 2) + 64; }
+
 struct WsLayout {
-  long long* hdr;       // 16 int64
+  long long* hdr;       // 16 int64: [0..4] rows per bin, [8] total of the last scan
   int* bin_cursor;      // kBins ints (+ padding)
-  int* upper;           // m ints: product upper bound per row (saturating)
+  int* upper;           // m + 1 ints: product upper bound per row (saturating)
   int* bin_rows;        // kBins * m ints
   int* row_cnt;         // m ints
-  double* row_scale;    // m doubles: fixed-point scale of each output row (numeric phase)
   unsigned long long* max_b;  // bit pattern of max |b| over the right operand
   long long* block_sum; // scan temporaries
-  int* dense_ctl;       // task prefix, per-row done counters and queue of the dense bin
-  unsigned* bitmap;     // workers * words
-  void* dense_acc;      // workers * n * sizeof(T)
-  int workers;
-  long long words;      // bitmap words per worker
+  char* area;           // long rows
+  int64_t products;     // its capacity
+  size_t area_bytes;
   size_t total;
 };
 
 static size_t align_up(size_t x) { return (x + 255) & ~(size_t)255; }
-// every accumulator slot is 8 bytes: 64-bit fixed point for the float types, the type itself
-// (in the low bytes) for the integer ones
-static size_t dtype_size(int) { return 8; }
 
-static WsLayout ws_layout(void* base, int64_t m, int64_t n, int dtype) {
+struct alignas(16) BigRecord {
+  unsigned col, pad;
+  Slot prod;
+};
+
+// Arrays of a batch of long rows inside the area.
+struct BigArea {
+  int* row;             // [rows] row id
+  int* p0;              // [rows + 1] first bucket
+  int* shift;           // [rows] bucket of a column = first bucket + (column >> shift)
+  int* tasks;           // [tasks][3] row index, first and last + 1 entry of A
+  double* scale;        // [rows] fixed-point scale
+  int *cnt, *off, *cursor, *bucket_row, *ucnt, *uoff;   // per bucket
+  long long* block_sum;
+  unsigned* key;        // products, symbolic phase: the column
+  BigRecord *rec, *rec2; // numeric phase (the same memory), and a second copy for rewritten buckets
+  size_t bytes;
+};
+static BigArea big_area(char* p, int64_t products) {
+  BigArea b;
+  const size_t nb = (size_t)big_buckets(products) + 1;
+  size_t off = 0;
+  auto take = [&](size_t bytes) { char* q = p + off; off += align_up(bytes); return q; };
+  b.row = (int*)take(nb * 4); b.p0 = (int*)take(nb * 4); b.shift = (int*)take(nb * 4);
+  b.tasks = (int*)take((size_t)kBigTasks * 12);
+  b.scale = (double*)take(nb * 8);
+  b.cnt = (int*)take(nb * 4); b.off = (int*)take(nb * 4); b.cursor = (int*)take(nb * 4);
+  b.bucket_row = (int*)take(nb * 4); b.ucnt = (int*)take(nb * 4); b.uoff = (int*)take(nb * 4);
+  b.block_sum = (long long*)take((nb / 4096 + 4) * 8);
+  b.rec = (BigRecord*)take((size_t)products * sizeof(BigRecord));
+  b.rec2 = (BigRecord*)take((size_t)products * sizeof(BigRecord));
+  b.key = (unsigned*)b.rec;
+  b.bytes = off;
+  return b;
+}
+
+// Dense fallback: one bitmap + accumulator of n columns.
+static size_t dense_words(int64_t n) { return (size_t)((n + 31) / 32); }
+static size_t dense_bytes(int64_t n) { return align_up(4096) + align_up(dense_words(n) * 4) + align_up((size_t)n * 8); }
+
+static WsLayout ws_layout(void* base, int64_t m, int64_t n) {
   WsLayout w;
   char* p = static_cast<char*>(base);
   size_t off = 0;
-  w.hdr = reinterpret_cast<long long*>(p + off); off += align_up(16 * 8);
-  w.bin_cursor = reinterpret_cast<int*>(p + off); off += align_up(16 * 4);
-  w.upper = reinterpret_cast<int*>(p + off); off += align_up((size_t)m * 4);
-  w.bin_rows = reinterpret_cast<int*>(p + off); off += align_up((size_t)m * 4 * kBins);
-  w.row_cnt = reinterpret_cast<int*>(p + off); off += align_up((size_t)m * 4);
-  w.row_scale = reinterpret_cast<double*>(p + off); off += align_up((size_t)m * 8);
-  w.max_b = reinterpret_cast<unsigned long long*>(p + off); off += align_up(8);
-  w.block_sum = reinterpret_cast<long long*>(p + off);
-  off += align_up((size_t)(ceil_div(m > 0 ? m : 1, 4096) + 1) * 8);
-  w.dense_ctl = reinterpret_cast<int*>(p + off); off += align_up((size_t)(2 * kDenseWorkersMax + 8) * 4);
-  w.words = (n + 31) / 32;
-  const size_t per_worker = (size_t)w.words * 4 + (size_t)n * dtype_size(dtype);
-  long long workers = per_worker ? (long long)(kDenseBudget / per_worker) : kDenseWorkersMax;
-  if (workers < 1) workers = 1;
-  if (workers > kDenseWorkersMax) workers = kDenseWorkersMax;
-  w.workers = (int)workers;
-  w.bitmap = reinterpret_cast<unsigned*>(p + off); off += align_up((size_t)w.workers * w.words * 4);
-  w.dense_acc = p + off; off += align_up((size_t)w.workers * (size_t)n * dtype_size(dtype));
+  auto take = [&](size_t bytes) { char* q = p + off; off += align_up(bytes); return q; };
+  w.hdr = (long long*)take(16 * 8);
+  w.bin_cursor = (int*)take(16 * 4);
+  w.upper = (int*)take((size_t)(m + 1) * 4);
+  w.bin_rows = (int*)take((size_t)m * 4 * kBins);
+  w.row_cnt = (int*)take((size_t)(m + 1) * 4);
+  w.max_b = (unsigned long long*)take(8);
+  w.block_sum = (long long*)take((size_t)(ceil_div(m > 0 ? m : 1, 4096) + 1) * 8);
+  w.products = big_products(m, n);
+  w.area_bytes = std::max(big_area(nullptr, w.products).bytes, dense_bytes(n));
+  w.area = take(w.area_bytes);
   w.total = off;
   return w;
 }
 
 // ---- binning ---------------------------------------------------------------------------------
-__device__ __forceinline__ int bin_of(int u) {
-  if (u <= 32) return 0;
-  if (u <= 128) return 1;
-  if (u <= 512) return 2;
-  if (u <= 2048) return 3;
-  if (u <= 8192) return 4;
-  return 5;
+// U_i of every row of A and the row's bin.  A CTA takes 1024 rows: 8 lanes per row, rows of more
+// than 64 entries by a warp, of more than 2048 by the CTA (8 lanes alone needed 2 ms for the hub rows
+// of a 2 M-row matrix); it appends them to the bins' lists with one atomic per bin (one per warp and
+// bin is 0.4 ms there: five addresses for everybody).  Rows with U = 0 get row_cnt = 0 and join no bin.
+constexpr int kBinThreads = 1024, kBinRows = 1024, kBinLaneRow = 64, kBinWarpRow = 2048;
+
+// Products of the entries b + x, b + x + step, ... before e.
+__device__ __forceinline__ long long count_products(const int* __restrict__ Acrd, const int* __restrict__ Bpos,
+                                                    int b, int e, int x, int step) {
+  long long u = 0;
+#pragma unroll 4
+  for (int p = b + x; p < e; p += step) {
+    const int j = ld_stream(Acrd + p);
+    u += __ldg(Bpos + j + 1) - __ldg(Bpos + j);
+  }
+  return u;
 }
 
-// 8 lanes per row of A: U_i and the row's bin; rows are appended to their bin's list with one
-// atomic per (warp, bin).  Rows with U = 0 get row_cnt = 0 and join no bin.
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kBinThreads)
 spgemm_bin_kernel(int m, const int* __restrict__ Apos, const int* __restrict__ Acrd,
                   const int* __restrict__ Bpos, int* __restrict__ upper, int* __restrict__ bin_rows,
                   int* __restrict__ bin_cursor, int* __restrict__ row_cnt) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long row = t >> 3;
-  const int l = (int)(t & 7), lane = threadIdx.x & 31;
-  long long u = 0;
-  if (row < m) {
-    const int b = __ldg(Apos + row), e = __ldg(Apos + row + 1);
-    for (int p = b + l; p < e; p += 8) {
-      const int j = ld_stream(Acrd + p);
-      u += __ldg(Bpos + j + 1) - __ldg(Bpos + j);
+  __shared__ int s_u[kBinRows], s_pos[kBinRows + 1];
+  __shared__ int s_warp_rows[kBinRows], s_cta_rows[kBinRows];
+  __shared__ int s_nwarp, s_ncta, s_next;
+  __shared__ long long s_part[32];
+  __shared__ int s_cnt[kBins], s_base[kBins];
+  const int tid = threadIdx.x, l = tid & 7, warp = tid >> 5, lane = tid & 31;
+  const long long row0 = (long long)blockIdx.x * kBinRows;
+  const int rows = (int)min((long long)kBinRows, m - row0);
+  if (tid < kBins) s_cnt[tid] = 0;
+  if (tid == 0) s_nwarp = s_ncta = s_next = 0;
+  for (int x = tid; x <= rows; x += kBinThreads) s_pos[x] = __ldg(Apos + row0 + x);
+  __syncthreads();
+#pragma unroll 2
+  for (int q = 0; q < kBinRows / (kBinThreads / 8); q++) {
+    const int x = q * (kBinThreads / 8) + (tid >> 3);
+    long long u = 0;
+    bool put = false;
+    if (x < rows) {
+      const int b = s_pos[x], e = s_pos[x + 1];
+      if (e - b <= kBinLaneRow) {
+        u = count_products(Acrd, Bpos, b, e, l, 8);
+        put = l == 0;
+      } else if (l == 0) {
+        if (e - b <= kBinWarpRow) s_warp_rows[atomicAdd(&s_nwarp, 1)] = x;
+        else s_cta_rows[atomicAdd(&s_ncta, 1)] = x;
+      }
     }
+    u += __shfl_xor_sync(FULL, u, 4);
+    u += __shfl_xor_sync(FULL, u, 2);
+    u += __shfl_xor_sync(FULL, u, 1);
+    if (put) s_u[x] = (int)min(u, (long long)INT_MAX);
   }
-  u += __shfl_xor_sync(FULL, u, 4);
-  u += __shfl_xor_sync(FULL, u, 2);
-  u += __shfl_xor_sync(FULL, u, 1);
-  const int ui = u > INT_MAX ? INT_MAX : (int)u;
-  const bool owner = (l == 0) && (row < m);
-  int bin = -1;
-  if (owner) {
-    upper[row] = ui;
-    if (ui == 0) row_cnt[row] = 0; else bin = bin_of(ui);
-  }
+  __syncthreads();
+  const int nwarp = s_nwarp, ncta = s_ncta;
+  for (int i = 0; i < ncta; i++) {
+    const int x = s_cta_rows[i];
+    long long u = count_products(Acrd, Bpos, s_pos[x], s_pos[x + 1], tid, kBinThreads);
 #pragma unroll
-  for (int b = 0; b < kBins; b++) {
-    const unsigned mask = __ballot_sync(FULL, bin == b);
-    if (mask == 0) continue;
-    const int leader = __ffs(mask) - 1;
-    int base = 0;
-    if (lane == leader) base = atomicAdd(&bin_cursor[b], __popc(mask));
-    base = __shfl_sync(FULL, base, leader);
-    if (bin == b) bin_rows[(long long)b * m + base + __popc(mask & ((1u << lane) - 1))] = (int)row;
+    for (int o = 16; o > 0; o >>= 1) u += __shfl_xor_sync(FULL, u, o);
+    if (lane == 0) s_part[warp] = u;
+    __syncthreads();
+    if (tid == 0) {
+      for (int w = 1; w < 32; w++) u += s_part[w];
+      s_u[x] = (int)min(u, (long long)INT_MAX);
+    }
+    __syncthreads();
   }
-}
-
-// ---- hash + sort primitives ------------------------------------------------------------------
-template <int S>
-__device__ __forceinline__ int hash_slot(int c) {
-  return (int)(((unsigned)c * 0x9E3779B1u) >> (32 - __builtin_ctz(S)));
-}
-
-// Slot of column c in the table, inserting it when absent (`fresh` = it was).
-template <int S>
-__device__ __forceinline__ int hash_find_or_insert(int* keys, int c, int& fresh) {
-  int h = hash_slot<S>(c);
   while (true) {
-    const int old = atomicCAS(&keys[h], kEmpty, c);
-    if (old == kEmpty || old == c) {
-      fresh += (old == kEmpty);
-      return h;
-    }
-    h = (h + 1) & (S - 1);
+    int i = 0;
+    if (lane == 0) i = atomicAdd(&s_next, 1);
+    i = __shfl_sync(FULL, i, 0);
+    if (i >= nwarp) break;
+    const int x = s_warp_rows[i];
+    long long u = count_products(Acrd, Bpos, s_pos[x], s_pos[x + 1], lane, 32);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) u += __shfl_xor_sync(FULL, u, o);
+    if (lane == 0) s_u[x] = (int)min(u, (long long)INT_MAX);
   }
+  __syncthreads();
+  int bin = -1, slot = 0;
+  if (tid < rows) {
+    const int u = s_u[tid];
+    upper[row0 + tid] = u;
+    if (u == 0) row_cnt[row0 + tid] = 0;
+    else bin = (u > 128) + (u > 512) + (u > 2048) + (u > 8192);
+  }
+  if (bin >= 0) slot = atomicAdd(&s_cnt[bin], 1);
+  __syncthreads();
+  if (tid < kBins && s_cnt[tid]) s_base[tid] = atomicAdd(&bin_cursor[tid], s_cnt[tid]);
+  __syncthreads();
+  if (bin >= 0) bin_rows[(long long)bin * m + s_base[bin] + slot] = (int)(row0 + tid);
 }
 
-// ---- order-independent accumulation ------------------------------------------------------------
-// An accumulator slot is 8 bytes.  Float types: a 64-bit fixed-point sum of the exactly computed,
-// scaled products (integer atomics: the same bits whatever the order); with `fixed` false (the
-// row's bound is not finite) the slot's low bytes hold a plain T added with float atomics.
-// Integer types: the slot's low bytes hold T, added with wrapping integer atomics.
-typedef unsigned long long Slot;
-
-template <typename T> struct IsFloat { static constexpr bool value = false; };
-template <> struct IsFloat<float> { static constexpr bool value = true; };
-template <> struct IsFloat<double> { static constexpr bool value = true; };
-
-template <typename T>
-__device__ __forceinline__ void acc_add(Slot* slot, T a, T b, double scale, bool fixed) {
-  if constexpr (IsFloat<T>::value) {
-    if (fixed) {
-      const long long q = __double2ll_rn((double)a * (double)b * scale);
-      atomicAdd(slot, (Slot)q);
-    } else {
-      atomicAdd(reinterpret_cast<T*>(slot), a * b);
-    }
-  } else {
-    atomicAdd(reinterpret_cast<T*>(slot), a * b);
-  }
-}
-
-template <typename T>
-__device__ __forceinline__ T acc_value(Slot v, double inv_scale, bool fixed) {
-  if constexpr (IsFloat<T>::value) {
-    if (fixed) return (T)((double)(long long)v * inv_scale);
-  }
-  T out;
-  memcpy(&out, &v, sizeof(T));
-  return out;
-}
-
+// ---- long rows: fixed-point accumulation ------------------------------------------------------
 // scale = 2^(61 - exponent of bound); NaN marks "not fixed point"
 __device__ __forceinline__ double scale_for_bound(double bound) {
   if (!(bound < 1.0e300)) return __longlong_as_double(0x7ff8000000000000LL);  // Inf / NaN
@@ -202,242 +231,289 @@ __device__ __forceinline__ double scale_for_bound(double bound) {
   return ldexp(1.0, 61 - e);        // bound * scale < 2^61
 }
 
-// Bitonic sort of the first P slots (P a power of two <= S) by key, values carried along.
-template <typename T, int NT, bool WARP_SCOPE>
-__device__ __forceinline__ void bitonic_sort(int* keys, T* vals, int P, int tid) {
-  for (int k = 2; k <= P; k <<= 1) {
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      for (int t = tid; t < P / 2; t += NT) {
-        const int i = ((t & ~(j - 1)) << 1) | (t & (j - 1));
-        const int x = i | j;
-        const bool up = (i & k) == 0;
-        const int a = keys[i], b = keys[x];
-        if ((a > b) == up) {
-          keys[i] = b; keys[x] = a;
-          const T va = vals[i]; vals[i] = vals[x]; vals[x] = va;
-        }
-      }
-      if (WARP_SCOPE) __syncwarp(); else __syncthreads();
-    }
-  }
+
+template <typename T>
+__device__ __forceinline__ Slot to_fixed(Slot bits, double scale) {
+  return (Slot)__double2ll_rn(__longlong_as_double((long long)bits) * scale);
+}
+template <typename T>
+__device__ __forceinline__ T from_fixed(Slot sum, double scale) {
+  return (T)((double)(long long)sum * (1.0 / scale));
+}
+template <typename T>
+__device__ __forceinline__ T one_product(Slot bits) {
+  if constexpr (kIsFloat<T>) return (T)__longlong_as_double((long long)bits);
+  else return (T)bits;
 }
 
-// Moves the occupied slots of a hash table to the front, in place, NT slots per round: a round
-// reads its slots into registers, scans the occupancy, and writes them at the running offset,
-// which never runs ahead of the slots already read.  Then pads up to the next power of two with
-// empty keys and returns that size (what the sort has to cover).  One warp (WARP_SCOPE) or one
-// CTA of NT threads; `s_scan` is NT/32 + 1 ints of shared memory (unused for a warp).
-template <typename T, int S, int NT, bool WARP_SCOPE>
-__device__ __forceinline__ int compact_table(int* keys, T* vals, int tid, int* s_scan) {
-  const int lane = tid & 31, warp = tid >> 5;
-  int run = 0;
-  for (int r0 = 0; r0 < S; r0 += NT) {
-    const int key = keys[r0 + tid];
-    const T val = vals[r0 + tid];
-    const bool occ = key != kEmpty;
-    const unsigned ball = __ballot_sync(FULL, occ);
-    int off = __popc(ball & ((1u << lane) - 1));
-    int total = __popc(ball);
-    if (!WARP_SCOPE) {
-      if (lane == 0) s_scan[warp] = total;
-      __syncthreads();  // also: every slot of this round has been read
-      int before = 0;
-      total = 0;
-#pragma unroll
-      for (int w = 0; w < NT / 32; w++) {
-        const int c = s_scan[w];
-        if (w < warp) before += c;
-        total += c;
-      }
-      off += before;
-      __syncthreads();  // s_scan is rewritten next round
-    } else {
-      __syncwarp();
-    }
-    if (occ) {
-      keys[run + off] = key;
-      vals[run + off] = val;
-    }
-    run += total;
-    if (WARP_SCOPE) __syncwarp(); else __syncthreads();
-  }
-  int P = 1;
-  while (P < run) P <<= 1;
-  for (int t = run + tid; t < P; t += NT) keys[t] = kEmpty;
-  if (WARP_SCOPE) __syncwarp(); else __syncthreads();
-  return P;
-}
-
-struct CsrIn {
-  const int* Apos; const int* Acrd; const void* Aval;
-  const int* Bpos; const int* Bcrd; const void* Bval;
-  const double* row_scale;   // numeric phase, float types: fixed-point scale per output row
-};
-
-// The products of A entries [pa0, pa1) (at most 32, one per lane) spread evenly over the lanes
-// of a warp: lane l looks up the B row of entry pa0 + l, a warp scan of the row lengths numbers
-// the products, and every lane then takes products lane, lane + 32, ... — a 5-step search over
-// the scanned lengths tells which entry a product belongs to.  No lane idles on a short B row and
-// the index loads of 32 entries are in flight together, instead of one dependent chain
-// (A entry -> B row pointers -> B entries) per entry.  `emit(a_value, pb)` is called once per
-// product with the value of its A entry (T(0) in the symbolic phase) and its position in B.
-// `defer(pa, len)` may take an entry out of the warp's share (it returns true and deals with the
-// entry's products itself): the dense rows hand B rows of hub length to the whole CTA that way.
-template <typename T, bool NUMERIC, typename F, typename D>
-__device__ __forceinline__ void expand_products(const CsrIn& in, int pa0, int pa1, int lane, F&& emit,
-                                                D&& defer) {
-  const int pa = pa0 + lane;
-  int bb = 0, len = 0;
-  T a = T(0);
-  if (pa < pa1) {
-    const int j = __ldg(in.Acrd + pa);
-    bb = __ldg(in.Bpos + j);
-    len = __ldg(in.Bpos + j + 1) - bb;
-    if (defer(pa, len)) len = 0;
-    if (NUMERIC) a = static_cast<const T*>(in.Aval)[pa];
-  }
-  int incl = len;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int y = __shfl_up_sync(FULL, incl, o);
-    if (lane >= o) incl += y;
-  }
-  const int total = __shfl_sync(FULL, incl, 31);
-  const int excl = incl - len;
-  for (int q0 = 0; q0 < total; q0 += 32) {
-    const int q = q0 + lane;
-    // largest e with excl[e] <= q (lanes past the end search too: shuffles need the whole warp)
-    int e = 0;
-#pragma unroll
-    for (int step = 16; step > 0; step >>= 1) {
-      const int v = __shfl_sync(FULL, excl, e + step);
-      if (v <= q) e += step;
-    }
-    const int e_excl = __shfl_sync(FULL, excl, e);
-    const int e_bb = __shfl_sync(FULL, bb, e);
-    T e_a;
-    if constexpr (sizeof(T) == 8) {
-      const long long bits = __shfl_sync(FULL, *reinterpret_cast<const long long*>(&a), e);
-      memcpy(&e_a, &bits, 8);
-    } else {
-      const int bits = __shfl_sync(FULL, *reinterpret_cast<const int*>(&a), e);
-      memcpy(&e_a, &bits, 4);
-    }
-    if (q < total) emit(e_a, e_bb + (q - e_excl));
-  }
-}
-
-// One warp per row (bins 0, 1): 32 A entries at a time, their products spread over the lanes.
-template <typename T, int S, bool NUMERIC>
-__global__ void __launch_bounds__(128)
-spgemm_warp_kernel(const int* __restrict__ rows, int nrows, CsrIn in, int* __restrict__ row_cnt,
-                   const int* __restrict__ Cpos, int* __restrict__ Ccrd, T* __restrict__ Cval) {
-  __shared__ int s_keys[4][S];
-  __shared__ Slot s_vals[4][NUMERIC ? S : 1];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int r = blockIdx.x * 4 + warp;
-  if (r >= nrows) return;
-  const int i = __ldg(rows + r);
-  int* keys = s_keys[warp];
-  Slot* vals = s_vals[warp];
-  for (int t = lane; t < S; t += 32) {
-    keys[t] = kEmpty;
-    if (NUMERIC) vals[t] = 0;
-  }
-  __syncwarp();
-  double scale = 1.0;
-  if (NUMERIC && IsFloat<T>::value) scale = in.row_scale[i];
-  const bool fixed = scale == scale;
-  const T* Bval = static_cast<const T*>(in.Bval);
-  const int ab = __ldg(in.Apos + i), ae = __ldg(in.Apos + i + 1);
-  int fresh = 0;
-  for (int pa0 = ab; pa0 < ae; pa0 += 32) {
-    expand_products<T, NUMERIC>(in, pa0, min(ae, pa0 + 32), lane, [&](T a, int pb) {
-      const int c = __ldg(in.Bcrd + pb);
-      const int h = hash_find_or_insert<S>(keys, c, fresh);
-      if (NUMERIC) acc_add<T>(vals + h, a, Bval[pb], scale, fixed);
-    }, [](int, int) { return false; });
-  }
-  __syncwarp();
-  if (!NUMERIC) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) fresh += __shfl_xor_sync(FULL, fresh, o);
-    if (lane == 0) row_cnt[i] = fresh;
+// Sum of products that arrive in no particular order (`fixed` false: the row's bound is not finite).
+template <typename T>
+__device__ __forceinline__ void acc_add(Slot* slot, Slot bits, double scale, bool fixed) {
+  if constexpr (kIsFloat<T>) {
+    if (fixed) atomicAdd(slot, to_fixed<T>(bits, scale));
+    else atomicAdd(reinterpret_cast<double*>(slot), __longlong_as_double((long long)bits));
   } else {
-    const int P = compact_table<Slot, S, 32, true>(keys, vals, lane, nullptr);
-    bitonic_sort<Slot, 32, true>(keys, vals, P, lane);
-    const int base = __ldg(Cpos + i), cnt = __ldg(Cpos + i + 1) - base;
-    const double inv = 1.0 / scale;
-    for (int t = lane; t < cnt; t += 32) {
-      Ccrd[base + t] = keys[t];
-      Cval[base + t] = acc_value<T>(vals[t], inv, fixed);
-    }
+    atomicAdd(slot, bits);
   }
 }
+template <typename T>
+__device__ __forceinline__ T acc_value(Slot v, double scale, bool fixed) {
+  if constexpr (kIsFloat<T>) return fixed ? from_fixed<T>(v, scale) : (T)__longlong_as_double((long long)v);
+  else return (T)v;
+}
 
-// One CTA per row (bins 2-4): warps take alternate slabs of 32 entries of the A row.
-template <typename T, int S, int NT, bool NUMERIC>
-__global__ void __launch_bounds__(NT)
-spgemm_cta_kernel(const int* __restrict__ rows, int nrows, CsrIn in, int* __restrict__ row_cnt,
-                  const int* __restrict__ Cpos, int* __restrict__ Ccrd, T* __restrict__ Cval) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  Slot* vals = reinterpret_cast<Slot*>(smem_raw);                 // S accumulators (numeric only)
-  int* keys = reinterpret_cast<int*>(smem_raw + (NUMERIC ? sizeof(Slot) * S : 0));
-  __shared__ int s_fresh;
-  __shared__ int s_scan[NT / 32 + 1];
+template <typename T>
+__global__ void spgemm_max_abs_kernel(const int* __restrict__ nnz_ptr, const T* __restrict__ val, unsigned long long* out) {
+  const long long nnz = *nnz_ptr;
+  double mx = 0.0;
+  bool bad = false;
+  for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < nnz;
+       p += (long long)gridDim.x * blockDim.x) {
+    const double v = fabs((double)val[p]);
+    if (!(v < 1.0e300)) bad = true; else mx = fmax(mx, v);
+  }
+  if (bad) mx = __longlong_as_double(0x7ff0000000000000LL);  // +inf: sorts above every finite bit pattern
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(FULL, mx, o));
+  // non-negative doubles order like their bit patterns
+  if ((threadIdx.x & 31) == 0) atomicMax(out, (unsigned long long)__double_as_longlong(mx));
+}
+
+
+constexpr int kHistBuckets = 2048;    // buckets counted in shared memory
+
+// Buckets of every row of the batch: their row; counts zeroed.
+__global__ void big_setup_kernel(BigArea b, int rows) {
   const int r = blockIdx.x;
-  if (r >= nrows) return;
-  const int i = __ldg(rows + r);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  for (int t = tid; t < S; t += NT) {
-    keys[t] = kEmpty;
-    if (NUMERIC) vals[t] = 0;
+  const int p1 = b.p0[r + 1];
+  for (int p = b.p0[r] + threadIdx.x; p < p1; p += blockDim.x) {
+    b.bucket_row[p] = r;
+    b.cnt[p] = 0;
   }
-  if (tid == 0) s_fresh = 0;
-  __syncthreads();
-  double scale = 1.0;
-  if (NUMERIC && IsFloat<T>::value) scale = in.row_scale[i];
-  const bool fixed = scale == scale;
-  const T* Bval = static_cast<const T*>(in.Bval);
-  const int ab = __ldg(in.Apos + i), ae = __ldg(in.Apos + i + 1);
-  int fresh = 0;
-  // warps take slabs of 32 A entries; a slab's products are spread over the warp's lanes
-  for (int pa0 = ab + 32 * warp; pa0 < ae; pa0 += NT) {
-    expand_products<T, NUMERIC>(in, pa0, min(ae, pa0 + 32), lane, [&](T a, int pb) {
-      const int c = __ldg(in.Bcrd + pb);
-      const int h = hash_find_or_insert<S>(keys, c, fresh);
-      if (NUMERIC) acc_add<T>(vals + h, a, Bval[pb], scale, fixed);
-    }, [](int, int) { return false; });
-  }
-  if (!NUMERIC) {
+}
+
+// Fixed-point scale of every row of the batch, from sum |a| over the row and max |b|.
+template <typename T>
+__global__ void __launch_bounds__(256)
+big_scale_kernel(BigArea b, const int* __restrict__ Apos, const T* __restrict__ Aval,
+                 const unsigned long long* __restrict__ max_b) {
+  __shared__ double s_part[8];
+  const int row = b.row[blockIdx.x], e = __ldg(Apos + row + 1);
+  double s = 0.0;
+  for (int p = __ldg(Apos + row) + threadIdx.x; p < e; p += 256) s += fabs((double)Aval[p]);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) fresh += __shfl_xor_sync(FULL, fresh, o);
-    if (lane == 0 && fresh) atomicAdd(&s_fresh, fresh);
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(FULL, s, o);
+  if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; w++) s += s_part[w];
+    b.scale[blockIdx.x] = scale_for_bound(s * __longlong_as_double((long long)*max_b));
+  }
+}
+
+// One task = some entries of one long row of A.  SCATTER false: products per bucket; true: every
+// product's column (and value) to the next free place of its bucket.
+// (One 16-byte record per product: a column and a value array cost a third scattered access.)
+template <typename T, bool NUMERIC, bool SCATTER>
+__global__ void __launch_bounds__(256)
+big_expand_kernel(BigArea b, CsrIn in) {
+  __shared__ int s_hist[SCATTER ? 1 : kHistBuckets];
+  __shared__ ExpandSmem<T, 256> s_expand;
+  const int tid = threadIdx.x;
+  const int r = b.tasks[3 * blockIdx.x], ab = b.tasks[3 * blockIdx.x + 1], ae = b.tasks[3 * blockIdx.x + 2];
+  const int p0 = b.p0[r], buckets = b.p0[r + 1] - p0, shift = b.shift[r];
+  const bool in_smem = !SCATTER && buckets <= kHistBuckets;
+  if (in_smem) {
+    for (int p = tid; p < buckets; p += 256) s_hist[p] = 0;
     __syncthreads();
-    if (tid == 0) row_cnt[i] = s_fresh;
-  } else {
+  }
+  const T* Bval = static_cast<const T*>(in.Bval);
+  expand_cta<T, NUMERIC, 256>(in, ab, ae, s_expand, tid, [&](int, T a, int pb) {
+    const int c = __ldg(in.Bcrd + pb), p = c >> shift;
+    if (!SCATTER) {
+      atomicAdd(in_smem ? &s_hist[p] : &b.cnt[p0 + p], 1);
+    } else {
+      const Slot v = NUMERIC ? product_bits<T>(a, __ldg(Bval + pb)) : 0;
+      const int slot = atomicAdd(&b.cursor[p0 + p], 1);
+      if (NUMERIC) b.rec[slot] = BigRecord{(unsigned)c, 0u, v};
+      else b.key[slot] = (unsigned)c;
+    }
+  });
+  if (in_smem) {
     __syncthreads();
-    const int P = compact_table<Slot, S, NT, false>(keys, vals, tid, s_scan);
-    bitonic_sort<Slot, NT, false>(keys, vals, P, tid);
-    const int base = __ldg(Cpos + i), cnt = __ldg(Cpos + i + 1) - base;
-    const double inv = 1.0 / scale;
-    for (int t = tid; t < cnt; t += NT) {
-      Ccrd[base + t] = keys[t];
-      Cval[base + t] = acc_value<T>(vals[t], inv, fixed);
+    for (int p = tid; p < buckets; p += 256) {
+      const int c = s_hist[p];
+      if (c) atomicAdd(&b.cnt[p0 + p], c);
     }
   }
 }
 
-// Bin 5 (rows whose products do not fit a shared-memory table): dense bitmap (+ accumulator) of
-// n columns per row in the workspace.  Rows are handled in batches of up to `slots` rows, one
+// Buckets of at most kBucketSort products: sorted by column, the sums of equal columns left, in
+// place, at the bucket's start.  ucnt: distinct columns.
+template <typename T, bool NUMERIC, typename KEY>
+__global__ void __launch_bounds__(128)
+big_sort_kernel(BigArea b) {
+  constexpr int NT = 128;
+  __shared__ __align__(16) KEY s_keys[kBucketSort];
+  __shared__ Slot s_prods[NUMERIC ? kBucketSort : 1];
+  __shared__ int s_part[NT / 32];
+  const int p = blockIdx.x, tid = threadIdx.x;
+  const int o = b.off[p], count = b.off[p + 1] - o;
+  if (count > kBucketSort) return;
+  if (count == 0) {
+    if (tid == 0) b.ucnt[p] = 0;
+    return;
+  }
+  const int r = b.bucket_row[p], shift = b.shift[r], lo = (int)((unsigned)(p - b.p0[r]) << shift);
+  constexpr int kOrd = 11;   // 2048 ordinals
+  for (int x = tid; x < count; x += NT) {
+    unsigned c;
+    if (NUMERIC) {
+      const BigRecord q = b.rec[o + x];
+      c = q.col;
+      s_prods[x] = q.prod;
+    } else {
+      c = b.key[o + x];
+    }
+    s_keys[x] = ((KEY)(c - (unsigned)lo) << kOrd) | (KEY)x;
+  }
+  __syncthreads();
+  if (count <= 4 * NT) sort_keys<KEY, 4, NT>(s_keys, count, tid);
+  else if (count <= 8 * NT) sort_keys<KEY, 8, NT>(s_keys, count, tid);
+  else sort_keys<KEY, 16, NT>(s_keys, count, tid);
+  double scale = 1.0;
+  if (NUMERIC && kIsFloat<T>) scale = b.scale[r];
+  const bool fixed = scale == scale;
+  const int u = emit_runs<KEY, NT, NUMERIC>(s_keys, count, kOrd, tid, s_part, lo, o,
+                                            [&](long long at, int col, int x, int last) {
+    const KEY mask = ((KEY)1 << kOrd) - 1;
+    T v;
+    if (last == x + 1) {
+      v = one_product<T>(s_prods[(int)(s_keys[x] & mask)]);
+    } else {
+      // (the ordinals are the order of arrival: sums that do not depend on it)
+      Slot s = 0;
+      double f = 0.0;
+      for (; x < last; x++) {
+        const Slot q = s_prods[(int)(s_keys[x] & mask)];
+        if (!kIsFloat<T>) s += q;
+        else if (fixed) s += to_fixed<T>(q, scale);
+        else f += __longlong_as_double((long long)q);
+      }
+      v = kIsFloat<T> && !fixed ? (T)f : acc_value<T>(s, scale, true);
+    }
+    b.rec[at].col = (unsigned)col;
+    *reinterpret_cast<T*>(&b.rec[at].prod) = v;
+  });
+  if (tid == 0) b.ucnt[p] = u;
+}
+
+// Larger buckets (columns that many products share): windows of kWindow columns, the bucket's
+// products run through once per window and added to accumulators in shared memory.  The result goes
+// to the second copy of the bucket, since the products are read again for the next window.
+constexpr int kWindow = 8192;
+template <typename T, bool NUMERIC>
+__global__ void __launch_bounds__(512)
+big_window_kernel(BigArea b, int buckets, long long n) {
+  constexpr int NT = 512;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  unsigned* bits = reinterpret_cast<unsigned*>(smem_raw);           // kWindow / 32 words
+  Slot* acc = reinterpret_cast<Slot*>(smem_raw + kWindow / 8);
+  __shared__ int s_part[NT / 32];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  for (int q0 = blockIdx.x * NT; q0 < buckets; q0 += gridDim.x * NT) {
+    const bool mine = q0 + tid < buckets && b.off[q0 + tid + 1] - b.off[q0 + tid] > kBucketSort;
+    if (!__syncthreads_or(mine)) continue;
+    for (int p = q0; p < min(buckets, q0 + NT); p++) {
+      const int o = b.off[p], count = b.off[p + 1] - o;
+      if (count <= kBucketSort) continue;
+      const int r = b.bucket_row[p], shift = b.shift[r];
+      const long long lo = (long long)(p - b.p0[r]) << shift, hi = min(n, lo + (1ll << shift));
+      double scale = 1.0;
+      if (NUMERIC && kIsFloat<T>) scale = b.scale[r];
+      const bool fixed = scale == scale;
+      int done = 0;
+      for (long long w0 = lo; w0 < hi; w0 += kWindow) {
+        __syncthreads();
+        for (int x = tid; x < kWindow / 32; x += NT) bits[x] = 0;
+        if (NUMERIC)
+          for (int x = tid; x < kWindow; x += NT) acc[x] = 0;
+        __syncthreads();
+        for (int x = tid; x < count; x += NT) {
+          const long long d = (long long)(NUMERIC ? b.rec[o + x].col : b.key[o + x]) - w0;
+          if (d < 0 || d >= kWindow) continue;
+          atomicOr(&bits[d >> 5], 1u << (d & 31));
+          if (NUMERIC) acc_add<T>(&acc[d], b.rec[o + x].prod, scale, fixed);
+        }
+        __syncthreads();
+        // 256 words: threads 0..255 take one each, in column order
+        unsigned m = tid < kWindow / 32 ? bits[tid] : 0;
+        const int c = __popc(m);
+        int incl = c;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+          const int y = __shfl_up_sync(FULL, incl, d);
+          if (lane >= d) incl += y;
+        }
+        if (lane == 31) s_part[warp] = incl;
+        __syncthreads();
+        int before = 0, total = 0;
+#pragma unroll
+        for (int w = 0; w < NT / 32; w++) {
+          const int v = s_part[w];
+          if (w < warp) before += v;
+          total += v;
+        }
+        if (NUMERIC) {
+          int at = o + done + before + incl - c;
+          while (m) {
+            const int d = tid * 32 + __ffs(m) - 1;
+            m &= m - 1;
+            b.rec2[at].col = (unsigned)(w0 + d);
+            *reinterpret_cast<T*>(&b.rec2[at].prod) = acc_value<T>(acc[d], scale, fixed);
+            at++;
+          }
+        }
+        done += total;
+      }
+      if (tid == 0) b.ucnt[p] = done;
+      __syncthreads();
+    }
+  }
+}
+
+// Distinct columns per row of the batch.
+__global__ void big_count_rows_kernel(BigArea b, int rows, int* __restrict__ row_cnt) {
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r < rows) row_cnt[b.row[r]] = b.uoff[b.p0[r + 1]] - b.uoff[b.p0[r]];
+}
+
+// The buckets' results to their rows: a warp per bucket.
+template <typename T>
+__global__ void __launch_bounds__(256)
+big_store_kernel(BigArea b, int buckets, RowsOut out) {
+  const int p = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (p >= buckets) return;
+  const int o = b.off[p], u = b.ucnt[p], r = b.bucket_row[p];
+  const bool second = b.off[p + 1] - o > kBucketSort;
+  const BigRecord* rec = (second ? b.rec2 : b.rec) + o;
+  const long long dst = (long long)out.off[b.row[r]] + (b.uoff[p] - b.uoff[b.p0[r]]);
+#pragma unroll 4
+  for (int x = lane; x < u; x += 32) {
+    const BigRecord q = rec[x];
+    out.crd[dst + x] = (int)q.col;
+    static_cast<T*>(out.val)[dst + x] = *reinterpret_cast<const T*>(&q.prod);
+  }
+}
+
+// ---- rows of more products than the area holds -------------------------------------------------
+// Dense bitmap (+ accumulator) of n columns in the area.  Rows are handled in batches of up to `slots` rows, one
 // slot each; a row's A entries are cut into chunks of kDenseChunk entries and the (row, chunk)
 // tasks of a batch are handed out through an atomic queue, so a hub row with hundreds of
 // thousands of entries is spread over the whole GPU.  The CTA that finishes a row's last chunk
 // (a counter per row, no spinning) walks the row's bitmap in ascending column order, emits the
 // row and leaves bitmap and accumulator all-zero for the next batch.
 constexpr int kDenseChunk = 2048;     // A entries per task
-constexpr int kLongBRow = 2048;       // B rows at least this long are walked by the whole CTA
-constexpr int kDeferCap = 64;
 
 struct DenseCtl {
   int* task_pref;  // [slots + 1]
@@ -465,21 +541,18 @@ template <typename T, bool NUMERIC>
 __global__ void __launch_bounds__(256)
 spgemm_dense_kernel(const int* __restrict__ rows, int r0, int nb, CsrIn in, long long words,
                     unsigned* __restrict__ bitmap_all, Slot* __restrict__ acc_all, long long n,
-                    DenseCtl ctl, int* __restrict__ row_cnt, const int* __restrict__ Cpos,
+                    DenseCtl ctl, const double* __restrict__ row_scale, int* __restrict__ row_cnt,
+                    const int* __restrict__ Cpos,
                     int* __restrict__ Ccrd, T* __restrict__ Cval) {
   __shared__ int s_warp[8];
   __shared__ int s_base;
   __shared__ int s_task;
   __shared__ int s_last;
-  __shared__ int s_ndefer;
-  __shared__ int s_defer[kDeferCap];
+  __shared__ ExpandSmem<T, 256> s_expand;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int total = __ldg(ctl.task_pref + nb);
   while (true) {
-    if (tid == 0) {
-      s_task = atomicAdd(ctl.queue, 1);
-      s_ndefer = 0;
-    }
+    if (tid == 0) s_task = atomicAdd(ctl.queue, 1);
     __syncthreads();
     const int task = s_task;
     if (task >= total) return;
@@ -496,35 +569,16 @@ spgemm_dense_kernel(const int* __restrict__ rows, int r0, int nb, CsrIn in, long
     unsigned* bitmap = bitmap_all + (long long)k * words;
     Slot* acc = NUMERIC ? acc_all + (long long)k * n : nullptr;
     double scale = 1.0;
-    if (NUMERIC && IsFloat<T>::value) scale = in.row_scale[i];
+    if (NUMERIC && kIsFloat<T>) scale = row_scale[k];
     const bool fixed = scale == scale;
     const int ab = __ldg(in.Apos + i) + chunk * kDenseChunk;
     const int ae = min(__ldg(in.Apos + i + 1), ab + kDenseChunk);
-    // warps take slabs of 32 A entries; a slab's products are spread over the warp's lanes.  B
-    // rows of hub length are put aside and walked by the whole CTA afterwards.
     auto add = [&](T av, int pb) {
       const int c = __ldg(in.Bcrd + pb);
-      if (NUMERIC) acc_add<T>(acc + c, av, static_cast<const T*>(in.Bval)[pb], scale, fixed);
+      if (NUMERIC) acc_add<T>(acc + c, product_bits<T>(av, static_cast<const T*>(in.Bval)[pb]), scale, fixed);
       atomicOr(&bitmap[c >> 5], 1u << (c & 31));
     };
-    for (int pa0 = ab + 32 * warp; pa0 < ae; pa0 += 256) {
-      expand_products<T, NUMERIC>(in, pa0, min(ae, pa0 + 32), lane, add, [&](int pa, int len) {
-        if (len < kLongBRow) return false;
-        const int slot = atomicAdd(&s_ndefer, 1);
-        if (slot >= kDeferCap) return false;
-        s_defer[slot] = pa;
-        return true;
-      });
-    }
-    __syncthreads();
-    const int nd = min(s_ndefer, kDeferCap);
-    for (int q = 0; q < nd; q++) {
-      const int pa = s_defer[q];
-      const int j = __ldg(in.Acrd + pa);
-      const T av = NUMERIC ? static_cast<const T*>(in.Aval)[pa] : T(0);
-      const int bb = __ldg(in.Bpos + j), be = __ldg(in.Bpos + j + 1);
-      for (int pb = bb + tid; pb < be; pb += 256) add(av, pb);
-    }
+    expand_cta<T, NUMERIC, 256>(in, ab, ae, s_expand, tid, [&](int, T a, int pb) { add(a, pb); });
     // publish this chunk, then find out whether it was the row's last one
     __threadfence();
     __syncthreads();
@@ -568,7 +622,7 @@ spgemm_dense_kernel(const int* __restrict__ rows, int r0, int nb, CsrIn in, long
           bits &= bits - 1;
           const long long c = w * 32 + bit;
           Ccrd[o] = (int)c;
-          Cval[o] = acc_value<T>(__ldcg(acc + c), 1.0 / scale, fixed);
+          Cval[o] = acc_value<T>(__ldcg(acc + c), scale, fixed);
           acc[c] = 0;
           o++;
         }
@@ -577,7 +631,7 @@ spgemm_dense_kernel(const int* __restrict__ rows, int r0, int nb, CsrIn in, long
       if (tid == 0) s_base = base + step_total;
       __syncthreads();
     }
-    if (!NUMERIC && tid == 0) row_cnt[i] = s_base;
+    if (row_cnt && tid == 0) row_cnt[i] = s_base;
     __syncthreads();
   }
 }
@@ -606,17 +660,38 @@ scan_reduce_kernel(int m, const int* __restrict__ cnt, long long* __restrict__ b
   }
 }
 
-__global__ void scan_blocks_kernel(int nb, long long* block_sum, long long* hdr_total) {
-  // single thread block, sequential over at most a few thousand tiles
-  if (threadIdx.x == 0) {
-    long long run = 0;
-    for (int b = 0; b < nb; b++) {
-      const long long v = block_sum[b];
-      block_sum[b] = run;
-      run += v;
+// Exclusive scan of the tiles' sums by one CTA, 1024 at a time.
+__global__ void __launch_bounds__(1024)
+scan_blocks_kernel(int nb, long long* block_sum, long long* hdr_total) {
+  __shared__ long long s[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  long long run = 0;
+  for (int b0 = 0; b0 < nb; b0 += 1024) {
+    const int b = b0 + threadIdx.x;
+    const long long v = b < nb ? block_sum[b] : 0;
+    long long incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const long long y = __shfl_up_sync(FULL, incl, o);
+      if (lane >= o) incl += y;
     }
-    *hdr_total = run;
+    if (lane == 31) s[warp] = incl;
+    __syncthreads();
+    if (warp == 0) {
+      long long w = s[lane];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const long long y = __shfl_up_sync(FULL, w, o);
+        if (lane >= o) w += y;
+      }
+      s[lane] = w;
+    }
+    __syncthreads();
+    if (b < nb) block_sum[b] = run + (warp ? s[warp - 1] : 0) + incl - v;
+    run += s[31];
+    __syncthreads();
   }
+  if (threadIdx.x == 0) *hdr_total = run;
 }
 
 __global__ void __launch_bounds__(1024)
@@ -674,105 +749,318 @@ int exclusive_scan_i32(int n, const int* cnt, int* out, long long* block_sum, lo
   const int nb = (int)ceil_div(n, kScanTile);
   scan_reduce_kernel<<<nb, 1024, 0, st>>>(n, cnt, block_sum);
   SB_LAUNCH_CHECK("scan_reduce_kernel");
-  scan_blocks_kernel<<<1, 32, 0, st>>>(nb, block_sum, total_dev);
+  scan_blocks_kernel<<<1, 1024, 0, st>>>(nb, block_sum, total_dev);
   SB_LAUNCH_CHECK("scan_blocks_kernel");
   scan_write_kernel<<<nb, 1024, 0, st>>>(n, cnt, block_sum, out);
   SB_LAUNCH_CHECK("scan_write_kernel");
   return SB_OK;
 }
 
-// ---- fixed-point scales of the numeric phase (float types) ---------------------------------------
-template <typename T>
-__global__ void spgemm_max_abs_kernel(long long nnz, const T* __restrict__ val, unsigned long long* out) {
-  double mx = 0.0;
-  bool bad = false;
-  for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < nnz;
-       p += (long long)gridDim.x * blockDim.x) {
-    const double v = fabs((double)val[p]);
-    if (!(v < 1.0e300)) bad = true; else mx = fmax(mx, v);
-  }
-  if (bad) mx = __longlong_as_double(0x7ff0000000000000LL);  // +inf: sorts above every finite bit pattern
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(FULL, mx, o));
-  // non-negative doubles order like their bit patterns
-  if ((threadIdx.x & 31) == 0) atomicMax(out, (unsigned long long)__double_as_longlong(mx));
-}
-
-// 8 lanes per row: scale of row i from sum |a| over the row and max |b|.
+// ---- one-pass form: the rows' entries from their product offsets to their place ------------------
+// A CTA moves kMoveTile consecutive entries of the result, whatever the rows' lengths (a warp per row
+// left the hub rows to a warp each: 4.7 ms for 272 M entries); a thread finds the row of its entry
+// among the tile's row pointers in shared memory.
+constexpr int kMoveTile = 8192, kMoveRows = 1024;
 template <typename T>
 __global__ void __launch_bounds__(256)
-spgemm_row_scale_kernel(int m, const int* __restrict__ Apos, const T* __restrict__ Aval,
-                        const unsigned long long* __restrict__ max_b, double* __restrict__ row_scale) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long row = t >> 3;
-  const int l = (int)(t & 7);
-  double s = 0.0;
-  if (row < m) {
-    const int b = __ldg(Apos + row), e = __ldg(Apos + row + 1);
-    for (int p = b + l; p < e; p += 8) s += fabs((double)Aval[p]);
+spgemm_move_kernel(int m, int nnz, const int* __restrict__ off, const int* __restrict__ Cpos,
+                   const int* __restrict__ tcrd, const T* __restrict__ tval, int* __restrict__ Ccrd,
+                   T* __restrict__ Cval) {
+  __shared__ int s_pos[kMoveRows + 1], s_shift[kMoveRows];
+  __shared__ int s_count[8];
+  const int tid = threadIdx.x;
+  const int e1 = min((long long)nnz, ((long long)blockIdx.x + 1) * kMoveTile);
+  for (int e = blockIdx.x * kMoveTile; e < e1;) {
+    const int r0 = cta_row_of<256>(Cpos, m, e, s_count);
+    for (int x = tid; x < kMoveRows + 1; x += 256) {
+      const int r = min(m, r0 + x), p = __ldg(Cpos + r);
+      s_pos[x] = p;
+      if (x < kMoveRows && r < m) s_shift[x] = __ldg(off + r) - p;
+    }
+    __syncthreads();
+    const int stop = min(e1, s_pos[kMoveRows]);
+#pragma unroll 4
+    for (int o = e + tid; o < stop; o += 256) {
+      int lo = 0, hi = kMoveRows;
+#pragma unroll
+      for (int step = 0; step < 10; step++) {
+        const int mid = (lo + hi) >> 1;
+        const bool right = s_pos[mid] <= o;
+        lo = right ? mid : lo;
+        hi = right ? hi : mid;
+      }
+      const int src = o + s_shift[lo];
+      Ccrd[o] = __ldg(tcrd + src);
+      Cval[o] = __ldg(tval + src);
+    }
+    e = stop;
+    __syncthreads();
   }
-  s += __shfl_xor_sync(FULL, s, 4);
-  s += __shfl_xor_sync(FULL, s, 2);
-  s += __shfl_xor_sync(FULL, s, 1);
-  if (l == 0 && row < m) row_scale[row] = scale_for_bound(s * __longlong_as_double((long long)*max_b));
 }
 
 // ---- host side ---------------------------------------------------------------------------------
+__global__ void big_info_kernel(const int* __restrict__ rows, int count, const int* __restrict__ upper,
+                                const int* __restrict__ Apos, int4* __restrict__ info) {
+  const int x = blockIdx.x * blockDim.x + threadIdx.x;
+  if (x >= count) return;
+  const int i = rows[x];
+  info[x] = make_int4(i, upper[i], Apos[i], Apos[i + 1]);
+}
+
+static int ceil_log2(int64_t x) {
+  int b = 0;
+  while (((int64_t)1 << b) < x) b++;
+  return b;
+}
+
+// Rows with more products than the area holds, one after the other.
 template <typename T, bool NUMERIC>
-static int launch_bins(const WsLayout& w, const long long* counts, int64_t m, int64_t n,
-                       const CsrIn& in, const int* Cpos, int* Ccrd, T* Cval, cudaStream_t st) {
-  const int* rows0 = w.bin_rows;
-  if (counts[0] > 0) {
-    spgemm_warp_kernel<T, 64, NUMERIC><<<(unsigned)ceil_div(counts[0], 4), 128, 0, st>>>(
-        rows0, (int)counts[0], in, w.row_cnt, Cpos, Ccrd, Cval);
-    SB_LAUNCH_CHECK("spgemm_warp_kernel<64>");
-  }
-  if (counts[1] > 0) {
-    spgemm_warp_kernel<T, 256, NUMERIC><<<(unsigned)ceil_div(counts[1], 4), 128, 0, st>>>(
-        rows0 + m, (int)counts[1], in, w.row_cnt, Cpos, Ccrd, Cval);
-    SB_LAUNCH_CHECK("spgemm_warp_kernel<256>");
-  }
-#define SB_CTA_BIN(IDX, SLOTS, THREADS)                                                        \
-  if (counts[IDX] > 0) {                                                                      \
-    constexpr int S = SLOTS;                                                                  \
-    const size_t smem = (size_t)S * 4 + (NUMERIC ? (size_t)S * sizeof(Slot) : 0);             \
-    auto k = spgemm_cta_kernel<T, S, THREADS, NUMERIC>;                                       \
-    SB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-    k<<<(unsigned)counts[IDX], THREADS, smem, st>>>(rows0 + (long long)IDX * m, (int)counts[IDX], \
-                                                    in, w.row_cnt, Cpos, Ccrd, Cval);         \
-    SB_LAUNCH_CHECK("spgemm_cta_kernel");                                                     \
-  }
-  SB_CTA_BIN(2, 1024, 128)
-  SB_CTA_BIN(3, 4096, 256)
-  SB_CTA_BIN(4, 16384, 512)
-#undef SB_CTA_BIN
-  if (counts[5] > 0) {
-    DenseCtl ctl{w.dense_ctl, w.dense_ctl + kDenseWorkersMax + 1, w.dense_ctl + 2 * kDenseWorkersMax + 2};
-    const int grid = 4 * sm_count();
-    for (long long r0 = 0; r0 < counts[5]; r0 += w.workers) {
-      const int nb = (int)((counts[5] - r0) < w.workers ? (counts[5] - r0) : w.workers);
-      dense_batch_setup_kernel<<<1, 32, 0, st>>>(rows0 + 5 * m, (int)r0, nb, in.Apos, ctl);
-      SB_LAUNCH_CHECK("dense_batch_setup_kernel");
-      spgemm_dense_kernel<T, NUMERIC><<<grid, 256, 0, st>>>(
-          rows0 + 5 * m, (int)r0, nb, in, w.words, w.bitmap, static_cast<Slot*>(w.dense_acc),
-          (long long)n, ctl, w.row_cnt, Cpos, Ccrd, Cval);
-      SB_LAUNCH_CHECK("spgemm_dense_kernel");
+static int dense_row(const WsLayout& w, int row, int64_t n, const CsrIn& in, const RowsOut& out, cudaStream_t st) {
+  char* p = w.area;
+  int* ctl = reinterpret_cast<int*>(p);                         // [0..1] tasks, [2] done, [3] queue, [4] row
+  double* scale = reinterpret_cast<double*>(p + 64);
+  unsigned* bitmap = reinterpret_cast<unsigned*>(p + align_up(4096));
+  Slot* acc = reinterpret_cast<Slot*>(p + align_up(4096) + align_up(dense_words(n) * 4));
+  SB_CUDA(cudaMemsetAsync(bitmap, 0, dense_words(n) * 4, st));
+  SB_CUDA(cudaMemcpyAsync(ctl + 4, &row, 4, cudaMemcpyHostToDevice, st));
+  if (NUMERIC) {
+    SB_CUDA(cudaMemsetAsync(acc, 0, (size_t)n * 8, st));
+    if constexpr (kIsFloat<T>) {
+      BigArea b{};
+      b.row = ctl + 4;
+      b.scale = scale;
+      big_scale_kernel<T><<<1, 256, 0, st>>>(b, in.Apos, static_cast<const T*>(in.Aval), w.max_b);
+      SB_LAUNCH_CHECK("big_scale_kernel");
     }
+  }
+  DenseCtl c{ctl, ctl + 2, ctl + 3};
+  dense_batch_setup_kernel<<<1, 32, 0, st>>>(ctl + 4, 0, 1, in.Apos, c);
+  SB_LAUNCH_CHECK("dense_batch_setup_kernel");
+  spgemm_dense_kernel<T, NUMERIC><<<4 * sm_count(), 256, 0, st>>>(
+      ctl + 4, 0, 1, in, (long long)dense_words(n), bitmap, acc, (long long)n, c, scale, out.row_cnt, out.off, out.crd,
+      static_cast<T*>(out.val));
+  SB_LAUNCH_CHECK("spgemm_dense_kernel");
+  return SB_OK;
+}
+
+// One batch of long rows whose plan (rows, first buckets, shifts, tasks) is in host memory.
+template <typename T, bool NUMERIC>
+static int big_batch(const WsLayout& w, const std::vector<int>& row, const std::vector<int>& p0,
+                     const std::vector<int>& shift, const std::vector<int>& tasks, int64_t n, const CsrIn& in,
+                     const RowsOut& out, cudaStream_t st) {
+  const BigArea b = big_area(w.area, w.products);
+  const int rows = (int)row.size(), buckets = p0.back();
+  SB_CUDA(cudaMemcpyAsync(b.row, row.data(), row.size() * 4, cudaMemcpyHostToDevice, st));
+  SB_CUDA(cudaMemcpyAsync(b.p0, p0.data(), p0.size() * 4, cudaMemcpyHostToDevice, st));
+  SB_CUDA(cudaMemcpyAsync(b.shift, shift.data(), shift.size() * 4, cudaMemcpyHostToDevice, st));
+  SB_CUDA(cudaMemcpyAsync(b.tasks, tasks.data(), tasks.size() * 4, cudaMemcpyHostToDevice, st));
+  const unsigned ntasks = (unsigned)(tasks.size() / 3);
+  big_setup_kernel<<<rows, 128, 0, st>>>(b, rows);
+  SB_LAUNCH_CHECK("big_setup_kernel");
+  if constexpr (NUMERIC && kIsFloat<T>) {
+    big_scale_kernel<T><<<rows, 256, 0, st>>>(b, in.Apos, static_cast<const T*>(in.Aval), w.max_b);
+    SB_LAUNCH_CHECK("big_scale_kernel");
+  }
+  big_expand_kernel<T, false, false><<<ntasks, 256, 0, st>>>(b, in);
+  SB_LAUNCH_CHECK("big_expand_kernel");
+  int rc = exclusive_scan_i32(buckets, b.cnt, b.off, b.block_sum, w.hdr + 8, st);
+  if (rc != SB_OK) return rc;
+  SB_CUDA(cudaMemcpyAsync(b.cursor, b.off, (size_t)buckets * 4, cudaMemcpyDeviceToDevice, st));
+  big_expand_kernel<T, NUMERIC, true><<<ntasks, 256, 0, st>>>(b, in);
+  SB_LAUNCH_CHECK("big_expand_kernel");
+  const int widest = *std::max_element(shift.begin(), shift.end());
+  if (widest + 11 <= 32) big_sort_kernel<T, NUMERIC, unsigned><<<buckets, 128, 0, st>>>(b);
+  else big_sort_kernel<T, NUMERIC, unsigned long long><<<buckets, 128, 0, st>>>(b);
+  SB_LAUNCH_CHECK("big_sort_kernel");
+  auto window = big_window_kernel<T, NUMERIC>;
+  const int smem = kWindow / 8 + (NUMERIC ? kWindow * 8 : 0);
+  SB_CUDA(cudaFuncSetAttribute(window, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  window<<<(unsigned)std::min<int64_t>(ceil_div(buckets, 512), 2 * sm_count()), 512, smem, st>>>(b, buckets, n);
+  SB_LAUNCH_CHECK("big_window_kernel");
+  rc = exclusive_scan_i32(buckets, b.ucnt, b.uoff, b.block_sum, w.hdr + 8, st);
+  if (rc != SB_OK) return rc;
+  if (out.row_cnt) {
+    big_count_rows_kernel<<<(unsigned)ceil_div(rows, 128), 128, 0, st>>>(b, rows, out.row_cnt);
+    SB_LAUNCH_CHECK("big_count_rows_kernel");
+  }
+  if (NUMERIC) {
+    big_store_kernel<T><<<(unsigned)ceil_div(buckets, 8), 256, 0, st>>>(b, buckets, out);
+    SB_LAUNCH_CHECK("big_store_kernel");
   }
   return SB_OK;
 }
 
+template <typename T, bool NUMERIC>
+static int big_rows(const WsLayout& w, int64_t count, int64_t m, int64_t kb, int64_t n, const CsrIn& in,
+                    const RowsOut& out, cudaStream_t st) {
+  if (NUMERIC && kIsFloat<T>) {
+    SB_CUDA(cudaMemsetAsync(w.max_b, 0, 8, st));
+    spgemm_max_abs_kernel<T><<<8 * sm_count(), 256, 0, st>>>(in.Bpos + kb, static_cast<const T*>(in.Bval), w.max_b);
+    SB_LAUNCH_CHECK("spgemm_max_abs_kernel");
+  }
+  std::vector<int4> info((size_t)count);
+  const int64_t room = (int64_t)(w.area_bytes / sizeof(int4));
+  for (int64_t x0 = 0; x0 < count; x0 += room) {
+    const int part = (int)std::min<int64_t>(room, count - x0);
+    big_info_kernel<<<(unsigned)ceil_div(part, 256), 256, 0, st>>>(w.bin_rows + (kBins - 1) * m + x0, part, w.upper,
+                                                                   in.Apos, reinterpret_cast<int4*>(w.area));
+    SB_LAUNCH_CHECK("big_info_kernel");
+    SB_CUDA(cudaMemcpyAsync(info.data() + x0, w.area, (size_t)part * sizeof(int4), cudaMemcpyDeviceToHost, st));
+    SB_CUDA(cudaStreamSynchronize(st));
+  }
+  const int nbits = ceil_log2(std::max<int64_t>(n, 1));
+  std::vector<int> row, p0{0}, shift, tasks;
+  int64_t products = 0;
+  auto flush = [&]() -> int {
+    if (row.empty()) return SB_OK;
+    const int rc = big_batch<T, NUMERIC>(w, row, p0, shift, tasks, n, in, out, st);
+    row.clear(); shift.clear(); tasks.clear();
+    p0.assign(1, 0);
+    products = 0;
+    return rc;
+  };
+  for (const int4& x : info) {
+    if (x.y > w.products) {
+      int rc = flush();
+      if (rc == SB_OK) rc = dense_row<T, NUMERIC>(w, x.x, n, in, out, st);
+      if (rc != SB_OK) return rc;
+      continue;
+    }
+    const int s = std::max(0, nbits - ceil_log2(ceil_div(x.y, kBucketProducts)));
+    const int buckets = (int)((n - 1) >> s) + 1;
+    const int len = x.w - x.z;
+    int chunk = 512;                     // A entries per task
+    while (ceil_div(len, chunk) > kBigTasks / 4) chunk *= 2;
+    if (products + x.y > w.products || p0.back() + buckets > big_buckets(w.products) ||
+        (int64_t)tasks.size() / 3 + ceil_div(len, chunk) > kBigTasks) {
+      const int rc = flush();
+      if (rc != SB_OK) return rc;
+    }
+    for (int b = x.z; b < x.w; b += chunk) {
+      tasks.push_back((int)row.size());
+      tasks.push_back(b);
+      tasks.push_back((int)std::min<int64_t>((int64_t)b + chunk, x.w));
+    }
+    row.push_back(x.x);
+    shift.push_back(s);
+    p0.push_back(p0.back() + buckets);
+    products += x.y;
+  }
+  return flush();
+}
+
+template <typename T, bool NUMERIC, typename KEY>
+static int launch_warp_bin(const int* rows, int64_t count, const WsLayout& w, const CsrIn& in, int shift,
+                           const RowsOut& out, cudaStream_t st) {
+  constexpr int WARPS = 4;
+  spgemm_warp_kernel<T, NUMERIC, KEY, WARPS><<<(unsigned)ceil_div(count, WARPS), 32 * WARPS, 0, st>>>(
+      rows, (int)count, w.upper, in, shift, out);
+  SB_LAUNCH_CHECK("spgemm_warp_kernel");
+  return SB_OK;
+}
+
+template <typename T, bool NUMERIC, typename KEY, int NT, int RMAX>
+static int launch_cta_bin(const int* rows, int64_t count, const WsLayout& w, const CsrIn& in, int shift,
+                          const RowsOut& out, cudaStream_t st) {
+  auto k = spgemm_cta_kernel<T, NUMERIC, KEY, NT, RMAX>;
+  const int smem = RMAX * NT * (int)(sizeof(KEY) + (NUMERIC ? sizeof(Slot) : 0));
+  SB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  k<<<(unsigned)count, NT, smem, st>>>(rows, w.upper, in, shift, out);
+  SB_LAUNCH_CHECK("spgemm_cta_kernel");
+  return SB_OK;
+}
+
+template <typename T, bool NUMERIC>
+static int launch_split_bin(const int* rows, int64_t count, const WsLayout& w, const CsrIn& in, int nbits,
+                            const RowsOut& out, cudaStream_t st) {
+  auto k = spgemm_split_kernel<T, NUMERIC>;
+  const int smem = kSplitCap * (int)(sizeof(unsigned) + (NUMERIC ? sizeof(Slot) : 0));
+  SB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  k<<<(unsigned)count, kSplitThreads, smem, st>>>(rows, w.upper, in, std::max(0, nbits - 5), out);
+  SB_LAUNCH_CHECK("spgemm_split_kernel");
+  return SB_OK;
+}
+
+// All rows; the longest first, so that the short ones fill in behind them.  A key holds the column
+// above the product's ordinal: 32 bits where both fit.
+template <typename T, bool NUMERIC>
+static int launch_bins(const WsLayout& w, const long long* counts, int64_t m, int64_t kb, int64_t n,
+                       const CsrIn& in, const RowsOut& out, cudaStream_t st) {
+  const int nbits = ceil_log2(std::max<int64_t>(n, 1));
+  int rc = SB_OK;
+  if (counts[4] > 0) rc = big_rows<T, NUMERIC>(w, counts[4], m, kb, n, in, out, st);
+  if (rc != SB_OK) return rc;
+  typedef unsigned K32;
+  typedef unsigned long long K64;
+  const int* rows = w.bin_rows;
+  if (counts[3] > 0) {
+    // (a segment's part of the column and 13 bits of ordinal fit one key up to 2^24 columns)
+    rc = nbits <= 24 ? launch_split_bin<T, NUMERIC>(rows + 3 * m, counts[3], w, in, nbits, out, st)
+                     : launch_cta_bin<T, NUMERIC, K64, 512, 16>(rows + 3 * m, counts[3], w, in, 13, out, st);
+    if (rc != SB_OK) return rc;
+  }
+  if (counts[2] > 0) {
+    rc = nbits <= 21 ? launch_cta_bin<T, NUMERIC, K32, 128, 16>(rows + 2 * m, counts[2], w, in, 11, out, st)
+                     : launch_cta_bin<T, NUMERIC, K64, 128, 16>(rows + 2 * m, counts[2], w, in, 11, out, st);
+    if (rc != SB_OK) return rc;
+  }
+  if (counts[1] > 0) {
+    rc = nbits <= 23 ? launch_cta_bin<T, NUMERIC, K32, 64, 8>(rows + m, counts[1], w, in, 9, out, st)
+                     : launch_cta_bin<T, NUMERIC, K64, 64, 8>(rows + m, counts[1], w, in, 9, out, st);
+    if (rc != SB_OK) return rc;
+  }
+  if (counts[0] > 0)
+    rc = nbits <= 25 ? launch_warp_bin<T, NUMERIC, K32>(rows, counts[0], w, in, 7, out, st)
+                     : launch_warp_bin<T, NUMERIC, K64>(rows, counts[0], w, in, 7, out, st);
+  return rc;
+}
+
+template <bool NUMERIC>
+static int launch_bins_typed(int dtype, const WsLayout& w, const long long* counts, int64_t m, int64_t kb, int64_t n,
+                             const CsrIn& in, const RowsOut& out, cudaStream_t st) {
+  switch (dtype) {
+    case SB_F32: return launch_bins<float, NUMERIC>(w, counts, m, kb, n, in, out, st);
+    case SB_F64: return launch_bins<double, NUMERIC>(w, counts, m, kb, n, in, out, st);
+    case SB_I32: return launch_bins<unsigned int, NUMERIC>(w, counts, m, kb, n, in, out, st);
+    default: return launch_bins<unsigned long long, NUMERIC>(w, counts, m, kb, n, in, out, st);
+  }
+}
+
 static int check_spgemm(int64_t m, int64_t kb, int64_t n, const void* Apos, const void* Bpos,
-                        void* ws, size_t ws_bytes, int dtype) {
+                        void* ws, size_t ws_bytes) {
   SB_CHECK_ARG(m >= 0 && kb >= 0 && n >= 0, "spgemm: negative size");
   SB_CHECK_ARG(m < INT32_MAX / 8 && kb < INT32_MAX && n < INT32_MAX - 1,
                "spgemm: dimension exceeds the supported int32 range");
   SB_CHECK_ARG(Apos && Bpos, "spgemm: null row pointers");
   SB_CHECK_ARG(ws && aligned16(ws), "spgemm: workspace is null or misaligned");
-  (void)dtype;
   const size_t need = sb_spgemm_workspace_bytes(m, n, SB_F32);  // the same for every dtype
   if (ws_bytes < need)
     return fail(SB_ERR_WORKSPACE, "spgemm: workspace has %zu bytes, needs %zu", ws_bytes, need);
+  return SB_OK;
+}
+
+// Product bounds and bins of the rows.
+static int bin_rows(const WsLayout& w, int64_t m, const int32_t* Apos, const int32_t* Acrd, const int32_t* Bpos,
+                    cudaStream_t st) {
+  SB_CUDA(cudaMemsetAsync(w.hdr, 0, 16 * 8, st));
+  SB_CUDA(cudaMemsetAsync(w.bin_cursor, 0, 16 * 4, st));
+  spgemm_bin_kernel<<<(unsigned)ceil_div(m, kBinRows), kBinThreads, 0, st>>>((int)m, Apos, Acrd, Bpos, w.upper,
+                                                                            w.bin_rows, w.bin_cursor, w.row_cnt);
+  SB_LAUNCH_CHECK("spgemm_bin_kernel");
+  return SB_OK;
+}
+
+// Row pointers from the rows' counts; the total, checked against int32.
+static int row_pointers(const WsLayout& w, int64_t m, int32_t* Cpos, int64_t* total_host, cudaStream_t st) {
+  int rc = exclusive_scan_i32((int)m, w.row_cnt, Cpos, w.block_sum, w.hdr + 8, st);
+  if (rc != SB_OK) return rc;
+  long long total = 0;
+  SB_CUDA(cudaMemcpyAsync(&total, w.hdr + 8, 8, cudaMemcpyDeviceToHost, st));
+  SB_CUDA(cudaStreamSynchronize(st));
+  *total_host = total;
+  if (total > INT32_MAX)
+    return fail(SB_ERR_OVERFLOW, "spgemm: the product has %lld stored entries, which does not fit "
+                "the int32 row pointers", total);
   return SB_OK;
 }
 
@@ -783,58 +1071,38 @@ using namespace sb;
 extern "C" {
 
 size_t sb_spgemm_workspace_bytes(int64_t m, int64_t n, int dtype) {
-  if (m < 0) m = 0;
-  if (n < 0) n = 0;
-  // One size for all dtypes (the symbolic phase does not know the numeric dtype): the largest
-  // of the per-dtype layouts.
-  (void)dtype;
-  const size_t a = ws_layout(nullptr, m, n, SB_F32).total;
-  const size_t b = ws_layout(nullptr, m, n, SB_F64).total;
-  return a > b ? a : b;
+  (void)dtype;   // one size for all: the symbolic phase does not know the numeric dtype
+  return ws_layout(nullptr, m < 0 ? 0 : m, n < 0 ? 0 : n).total;
 }
 
 int sb_spgemm_symbolic(int64_t m, int64_t kb, int64_t n, const int32_t* Apos, const int32_t* Acrd,
                        const int32_t* Bpos, const int32_t* Bcrd, int32_t* Cpos,
                        int64_t* total_nnz_host, void* ws, size_t ws_bytes, void* stream) {
-  int rc = check_spgemm(m, kb, n, Apos, Bpos, ws, ws_bytes, SB_F32);
+  int rc = check_spgemm(m, kb, n, Apos, Bpos, ws, ws_bytes);
   if (rc != SB_OK) return rc;
   SB_CHECK_ARG(Cpos && total_nnz_host, "spgemm_symbolic: null output");
   cudaStream_t st = (cudaStream_t)stream;
-  // the symbolic phase only needs the bitmaps; lay the workspace out for the smallest dtype so
-  // that any numeric dtype (whose layout is recomputed there) fits the caller's buffer
-  WsLayout w = ws_layout(ws, m, n, SB_F32);
+  const WsLayout w = ws_layout(ws, m, n);
   *total_nnz_host = 0;
-  SB_CUDA(cudaMemsetAsync(w.hdr, 0, 16 * 8, st));
-  SB_CUDA(cudaMemsetAsync(w.bin_cursor, 0, 16 * 4, st));
   if (m == 0) {
+    SB_CUDA(cudaMemsetAsync(w.hdr, 0, 16 * 8, st));
     SB_CUDA(cudaMemsetAsync(Cpos, 0, 4, st));
     SB_CUDA(cudaStreamSynchronize(st));
     return SB_OK;
   }
-  spgemm_bin_kernel<<<(unsigned)ceil_div(m * 8, 256), 256, 0, st>>>(
-      (int)m, Apos, Acrd, Bpos, w.upper, w.bin_rows, w.bin_cursor, w.row_cnt);
-  SB_LAUNCH_CHECK("spgemm_bin_kernel");
+  rc = bin_rows(w, m, Apos, Acrd, Bpos, st);
+  if (rc != SB_OK) return rc;
   int cursors[kBins];
   SB_CUDA(cudaMemcpyAsync(cursors, w.bin_cursor, sizeof(cursors), cudaMemcpyDeviceToHost, st));
   SB_CUDA(cudaStreamSynchronize(st));
   long long counts[kBins];
   for (int b = 0; b < kBins; b++) counts[b] = cursors[b];
-  if (counts[kBins - 1] > 0) SB_CUDA(cudaMemsetAsync(w.bitmap, 0, (size_t)w.workers * w.words * 4, st));
-  CsrIn in{Apos, Acrd, nullptr, Bpos, Bcrd, nullptr, nullptr};
-  rc = launch_bins<float, false>(w, counts, m, n, in, nullptr, nullptr, nullptr, st);
-  if (rc != SB_OK) return rc;
-  rc = exclusive_scan_i32((int)m, w.row_cnt, Cpos, w.block_sum, w.hdr + 8, st);
+  const CsrIn in{Apos, Acrd, nullptr, Bpos, Bcrd, nullptr};
+  rc = launch_bins<float, false>(w, counts, m, kb, n, in, RowsOut{w.row_cnt, nullptr, nullptr, nullptr}, st);
   if (rc != SB_OK) return rc;
   // keep the bin sizes in the workspace header for the numeric phase
   SB_CUDA(cudaMemcpyAsync(w.hdr, counts, sizeof(counts), cudaMemcpyHostToDevice, st));
-  long long total = 0;
-  SB_CUDA(cudaMemcpyAsync(&total, w.hdr + 8, 8, cudaMemcpyDeviceToHost, st));
-  SB_CUDA(cudaStreamSynchronize(st));
-  *total_nnz_host = total;
-  if (total > INT32_MAX)
-    return fail(SB_ERR_OVERFLOW, "spgemm: the product has %lld stored entries, which does not fit "
-                "the int32 row pointers", total);
-  return SB_OK;
+  return row_pointers(w, m, Cpos, total_nnz_host, st);
 }
 
 int sb_spgemm_numeric(int dtype, int64_t m, int64_t kb, int64_t n, const int32_t* Apos,
@@ -842,13 +1110,12 @@ int sb_spgemm_numeric(int dtype, int64_t m, int64_t kb, int64_t n, const int32_t
                       const int32_t* Bcrd, const void* Bval, const int32_t* Cpos, int32_t* Ccrd,
                       void* Cval, void* ws, size_t ws_bytes, void* stream) {
   SB_CHECK_ARG(dtype >= SB_F32 && dtype <= SB_I64, "spgemm_numeric: unknown dtype");
-  int rc = check_spgemm(m, kb, n, Apos, Bpos, ws, ws_bytes, dtype);
+  int rc = check_spgemm(m, kb, n, Apos, Bpos, ws, ws_bytes);
   if (rc != SB_OK) return rc;
   SB_CHECK_ARG(Cpos, "spgemm_numeric: Cpos is null");
   if (m == 0) return SB_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  // the row bins sit at dtype-independent offsets; the dense area is re-laid-out for `dtype`
-  WsLayout w = ws_layout(ws, m, n, dtype);
+  const WsLayout w = ws_layout(ws, m, n);
   long long counts[kBins];
   SB_CUDA(cudaMemcpyAsync(counts, w.hdr, sizeof(counts), cudaMemcpyDeviceToHost, st));
   SB_CUDA(cudaStreamSynchronize(st));
@@ -861,41 +1128,79 @@ int sb_spgemm_numeric(int dtype, int64_t m, int64_t kb, int64_t n, const int32_t
   SB_CHECK_ARG(binned <= m, "spgemm_numeric: workspace does not hold the bins of a symbolic call");
   if (binned == 0) return SB_OK;
   SB_CHECK_ARG(Ccrd && Cval && Aval && Bval, "spgemm_numeric: null pointer");
-  if (counts[kBins - 1] > 0) {
-    SB_CUDA(cudaMemsetAsync(w.bitmap, 0, (size_t)w.workers * w.words * 4, st));
-    SB_CUDA(cudaMemsetAsync(w.dense_acc, 0, (size_t)w.workers * (size_t)n * dtype_size(dtype), st));
+  const CsrIn in{Apos, Acrd, Aval, Bpos, Bcrd, Bval};
+  return launch_bins_typed<true>(dtype, w, counts, m, kb, n, in, RowsOut{nullptr, Cpos, Ccrd, Cval}, st);
+}
+
+int sb_spgemm_begin(int64_t m, int64_t kb, int64_t n, const int32_t* Apos, const int32_t* Acrd,
+                    const int32_t* Bpos, int32_t* off, int64_t* counts_host, int64_t* products_host, void* ws,
+                    size_t ws_bytes, void* stream) {
+  int rc = check_spgemm(m, kb, n, Apos, Bpos, ws, ws_bytes);
+  if (rc != SB_OK) return rc;
+  SB_CHECK_ARG(off && counts_host && products_host, "spgemm_begin: null output");
+  cudaStream_t st = (cudaStream_t)stream;
+  const WsLayout w = ws_layout(ws, m, n);
+  for (int b = 0; b < kBins; b++) counts_host[b] = 0;
+  *products_host = 0;
+  if (m == 0) return SB_OK;
+  rc = bin_rows(w, m, Apos, Acrd, Bpos, st);
+  if (rc != SB_OK) return rc;
+  rc = exclusive_scan_i32((int)m, w.upper, off, w.block_sum, w.hdr + 8, st);
+  if (rc != SB_OK) return rc;
+  struct { long long hdr[32]; int cursors[16]; } h;   // header and cursors are neighbours
+  static_assert(sizeof(long long) * 32 == 256, "the header takes one 256-byte unit of the workspace");
+  SB_CUDA(cudaMemcpyAsync(&h, w.hdr, sizeof(h), cudaMemcpyDeviceToHost, st));
+  SB_CUDA(cudaStreamSynchronize(st));
+  for (int b = 0; b < kBins; b++) counts_host[b] = h.cursors[b];
+  *products_host = h.hdr[8];
+  return SB_OK;
+}
+
+int sb_spgemm_rows(int dtype, int64_t m, int64_t kb, int64_t n, const int32_t* Apos, const int32_t* Acrd,
+                   const void* Aval, const int32_t* Bpos, const int32_t* Bcrd, const void* Bval, const int32_t* off,
+                   const int64_t* counts_host, int32_t* tcrd, void* tval, int32_t* Cpos, int64_t* total_nnz_host,
+                   void* ws, size_t ws_bytes, void* stream) {
+  SB_CHECK_ARG(dtype >= SB_F32 && dtype <= SB_I64, "spgemm_rows: unknown dtype");
+  int rc = check_spgemm(m, kb, n, Apos, Bpos, ws, ws_bytes);
+  if (rc != SB_OK) return rc;
+  SB_CHECK_ARG(off && counts_host && Cpos && total_nnz_host, "spgemm_rows: null pointer");
+  cudaStream_t st = (cudaStream_t)stream;
+  const WsLayout w = ws_layout(ws, m, n);
+  *total_nnz_host = 0;
+  if (m == 0) {
+    SB_CUDA(cudaMemsetAsync(Cpos, 0, 4, st));
+    return SB_OK;
   }
-  CsrIn in{Apos, Acrd, Aval, Bpos, Bcrd, Bval, w.row_scale};
-  if (dtype == SB_F32 || dtype == SB_F64) {
-    long long bnnz = 0;   // stored entries of B = its last row pointer
-    SB_CUDA(cudaMemcpyAsync(&bnnz, Bpos + kb, 4, cudaMemcpyDeviceToHost, st));
-    SB_CUDA(cudaMemsetAsync(w.max_b, 0, 8, st));
-    SB_CUDA(cudaStreamSynchronize(st));
-    bnnz &= 0xffffffffLL;
-    if (bnnz > 0) {
-      const unsigned blocks = (unsigned)std::min<long long>(ceil_div(bnnz, 256), 8LL * sm_count());
-      if (dtype == SB_F32) spgemm_max_abs_kernel<float><<<blocks, 256, 0, st>>>(bnnz, (const float*)Bval, w.max_b);
-      else spgemm_max_abs_kernel<double><<<blocks, 256, 0, st>>>(bnnz, (const double*)Bval, w.max_b);
-      SB_LAUNCH_CHECK("spgemm_max_abs_kernel");
-    }
-    const unsigned grid = (unsigned)ceil_div(m * 8, 256);
-    if (dtype == SB_F32)
-      spgemm_row_scale_kernel<float><<<grid, 256, 0, st>>>((int)m, Apos, (const float*)Aval, w.max_b, w.row_scale);
-    else
-      spgemm_row_scale_kernel<double><<<grid, 256, 0, st>>>((int)m, Apos, (const double*)Aval, w.max_b, w.row_scale);
-    SB_LAUNCH_CHECK("spgemm_row_scale_kernel");
+  long long counts[kBins], binned = 0;
+  for (int b = 0; b < kBins; b++) {
+    counts[b] = counts_host[b];
+    SB_CHECK_ARG(counts[b] >= 0 && counts[b] <= m, "spgemm_rows: counts are not those of sb_spgemm_begin");
+    binned += counts[b];
   }
-  switch (dtype) {
-    case SB_F32:
-      return launch_bins<float, true>(w, counts, m, n, in, Cpos, Ccrd, (float*)Cval, st);
-    case SB_F64:
-      return launch_bins<double, true>(w, counts, m, n, in, Cpos, Ccrd, (double*)Cval, st);
-    case SB_I32:
-      return launch_bins<unsigned int, true>(w, counts, m, n, in, Cpos, Ccrd, (unsigned int*)Cval, st);
-    default:
-      return launch_bins<unsigned long long, true>(w, counts, m, n, in, Cpos, Ccrd,
-                                                   (unsigned long long*)Cval, st);
-  }
+  SB_CHECK_ARG(binned <= m, "spgemm_rows: counts are not those of sb_spgemm_begin");
+  SB_CHECK_ARG(binned == 0 || (tcrd && tval && Aval && Bval), "spgemm_rows: null pointer");
+  const CsrIn in{Apos, Acrd, Aval, Bpos, Bcrd, Bval};
+  rc = launch_bins_typed<true>(dtype, w, counts, m, kb, n, in, RowsOut{w.row_cnt, off, tcrd, tval}, st);
+  if (rc != SB_OK) return rc;
+  return row_pointers(w, m, Cpos, total_nnz_host, st);
+}
+
+int sb_spgemm_finish(int dtype, int64_t m, int64_t nnz, const int32_t* off, const int32_t* tcrd, const void* tval,
+                     const int32_t* Cpos, int32_t* Ccrd, void* Cval, void* stream) {
+  SB_CHECK_ARG(dtype >= SB_F32 && dtype <= SB_I64, "spgemm_finish: unknown dtype");
+  SB_CHECK_ARG(m >= 0 && m < INT32_MAX / 32 && nnz >= 0 && nnz <= INT32_MAX, "spgemm_finish: bad size");
+  if (m == 0 || nnz == 0) return SB_OK;
+  SB_CHECK_ARG(off && tcrd && tval && Cpos && Ccrd && Cval, "spgemm_finish: null pointer");
+  cudaStream_t st = (cudaStream_t)stream;
+  const unsigned grid = (unsigned)ceil_div(nnz, kMoveTile);
+  if (dtype == SB_F32 || dtype == SB_I32)
+    spgemm_move_kernel<unsigned><<<grid, 256, 0, st>>>((int)m, (int)nnz, off, Cpos, tcrd, (const unsigned*)tval, Ccrd,
+                                                       (unsigned*)Cval);
+  else
+    spgemm_move_kernel<unsigned long long><<<grid, 256, 0, st>>>(
+        (int)m, (int)nnz, off, Cpos, tcrd, (const unsigned long long*)tval, Ccrd, (unsigned long long*)Cval);
+  SB_LAUNCH_CHECK("spgemm_move_kernel");
+  return SB_OK;
 }
 
 }  // extern "C"

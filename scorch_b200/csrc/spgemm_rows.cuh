@@ -1,0 +1,522 @@
+// Sorting kernels of the SpGEMM (see spgemm.cu): one output row, or one bucket of a long row, per
+// warp or CTA.
+//
+// The products of a row are expanded into shared memory, each with a key (column, ordinal of the
+// product) in one 32- or 64-bit word, and the keys are sorted in registers by a bitonic network
+// (R keys per thread; strides below R inside the thread, then shuffles, then shared memory).  Equal
+// columns are then neighbours in the order of their ordinals: a run is summed in that order, so the
+// result has the same bits on every run without atomics, and the values move once (they are looked
+// up by ordinal).  Hash tables with 64-bit atomics, a compaction and a sort of key-value pairs did
+// the same at 5.8 G products/s.
+// Bound: the gather of B's rows (12 entries each on a power-law matrix: two or three sectors per
+// row and array) and the issue rate of the network: about 2 instructions per key and 512-key row.
+#pragma once
+
+#include <limits.h>
+
+#include <type_traits>
+
+#include "common.cuh"
+
+namespace sb {
+
+typedef unsigned long long Slot;   // bits of a product: double for the float types, else the integer
+
+template <typename T>
+constexpr bool kIsFloat = std::is_same<T, float>::value || std::is_same<T, double>::value;
+
+template <typename T>
+__device__ __forceinline__ Slot product_bits(T a, T b) {
+  if constexpr (kIsFloat<T>) return (Slot)__double_as_longlong((double)a * (double)b);
+  else return (Slot)(T)(a * b);
+}
+
+struct CsrIn {
+  const int* Apos; const int* Acrd; const void* Aval;
+  const int* Bpos; const int* Bcrd; const void* Bval;
+};
+
+// Sum of a run of products in a fixed order.  float: the products are exact in double.  double:
+// the rounding errors of the additions are carried along (two-sum), as exact as the 64-bit
+// fixed-point sums of the long rows.
+template <typename T>
+struct RunSum {
+  double s = 0.0, c = 0.0;
+  T i = T(0);
+  __device__ __forceinline__ void add(Slot bits) {
+    if constexpr (std::is_same<T, float>::value) {
+      s += __longlong_as_double((long long)bits);
+    } else if constexpr (std::is_same<T, double>::value) {
+      const double x = __longlong_as_double((long long)bits), t = s + x, z = t - s;
+      c += (s - (t - z)) + (x - z);
+      s = t;
+    } else {
+      i += (T)bits;
+    }
+  }
+  __device__ __forceinline__ T value() const {
+    if constexpr (std::is_same<T, float>::value) return (float)s;
+    else if constexpr (std::is_same<T, double>::value) return fabs(s) <= 1.7976931348623157e308 ? s + c : s;
+    else return i;
+  }
+};
+
+// ---- bitonic network ---------------------------------------------------------------------------
+// Ascending sort of NT * R keys, thread t holding elements t * R .. t * R + R - 1.  `xch`: NT * R
+// keys of shared memory (used when the CTA has more than one warp).
+// (Only the steps inside a thread are unrolled: the register file is indexed by constants, and the
+// loops over sizes and thread distances keep the code small.)
+template <typename KEY, int R>
+__device__ __forceinline__ void compare_inside(KEY (&k)[R], int stride, bool up) {
+#pragma unroll
+  for (int i = 0; i < R; i++) {
+    const int j = i ^ stride;
+    if (j > i) {
+      const KEY lo = k[i] < k[j] ? k[i] : k[j], hi = k[i] < k[j] ? k[j] : k[i];
+      k[i] = up ? lo : hi;
+      k[j] = up ? hi : lo;
+    }
+  }
+}
+
+template <typename KEY, int R, int NT>
+__device__ __forceinline__ void bitonic_sort(KEY (&k)[R], KEY* xch, int tid) {
+  // sizes up to R / 2: the direction depends on the place inside the thread
+#pragma unroll
+  for (int size = 2; size < R; size <<= 1) {
+#pragma unroll
+    for (int stride = size >> 1; stride > 0; stride >>= 1) {
+#pragma unroll
+      for (int i = 0; i < R; i++) {
+        const int j = i ^ stride;
+        if (j > i) {
+          const KEY lo = k[i] < k[j] ? k[i] : k[j], hi = k[i] < k[j] ? k[j] : k[i];
+          k[i] = (i & size) == 0 ? lo : hi;
+          k[j] = (i & size) == 0 ? hi : lo;
+        }
+      }
+    }
+  }
+  // sizes R, 2 R, ...: `span` threads are merged
+#pragma unroll 1
+  for (int span = 1; span <= NT; span <<= 1) {
+    const bool up = (tid & span) == 0;
+#pragma unroll 1
+    for (int ts = span >> 1; ts > 0; ts >>= 1) {
+      const bool keep_min = up == ((tid & ts) == 0);
+      if (NT == 32 || ts < 32) {
+#pragma unroll
+        for (int i = 0; i < R; i++) {
+          const KEY o = __shfl_xor_sync(FULL, k[i], ts);
+          k[i] = (k[i] < o) == keep_min ? k[i] : o;
+        }
+      } else {
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < R; i++) xch[i * NT + tid] = k[i];
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < R; i++) {
+          const KEY o = xch[i * NT + (tid ^ ts)];
+          k[i] = (k[i] < o) == keep_min ? k[i] : o;
+        }
+      }
+    }
+#pragma unroll
+    for (int stride = R >> 1; stride > 0; stride >>= 1) compare_inside<KEY, R>(k, stride, up);
+  }
+}
+
+template <int NT>
+__device__ __forceinline__ void group_sync() {
+  if (NT == 32) __syncwarp(); else __syncthreads();
+}
+
+// Sorts the first `count` <= NT * R keys of `keys` in place (groups of several warps use the rest of
+// the NT * R slots as well).
+template <typename KEY, int R, int NT>
+__device__ __forceinline__ void sort_keys(KEY* keys, int count, int tid) {
+  KEY k[R];
+#pragma unroll
+  for (int i = 0; i < R; i++) {
+    const int e = tid + i * NT;      // (any assignment will do: the keys are in no order yet)
+    k[i] = e < count ? keys[e] : ~KEY(0);
+  }
+  bitonic_sort<KEY, R, NT>(k, keys, tid);
+  group_sync<NT>();
+#pragma unroll
+  for (int i = 0; i < R; i++)
+    if (tid * R + i < count) keys[tid * R + i] = k[i];
+  group_sync<NT>();
+}
+
+// ---- emission -------------------------------------------------------------------------------------
+// Distinct columns (key >> shift) among the sorted keys [b, e) of a row that begins at keys[0]: their
+// number, a warp together.
+template <typename KEY>
+__device__ __forceinline__ int count_runs(const KEY* keys, int b, int e, int shift, int lane) {
+  int heads = 0;
+  for (int x0 = b; x0 < e; x0 += 32) {
+    const int x = x0 + lane;
+    const bool head = x < e && (x == 0 || (keys[x] >> shift) != (keys[x - 1] >> shift));
+    heads += __popc(__ballot_sync(FULL, head));
+  }
+  return heads;
+}
+// ... and for each one write(o, column, first, last): o = at, at + 1, ..., [first, last) its run of
+// sorted keys (which may end behind e, at most at `count`).
+template <typename KEY, typename F>
+__device__ __forceinline__ void write_runs(const KEY* keys, int b, int e, int count, int shift, int lane, int col0,
+                                           long long at, F&& write) {
+  for (int x0 = b; x0 < e; x0 += 32) {
+    const int x = x0 + lane;
+    const KEY col = x < e ? keys[x] >> shift : KEY(0);
+    const bool head = x < e && (x == 0 || col != (keys[x - 1] >> shift));
+    const unsigned heads = __ballot_sync(FULL, head);
+    if (head) {
+      int last = x + 1;
+      while (last < count && (keys[last] >> shift) == col) last++;
+      const long long o = at + __popc(heads & ((1u << lane) - 1u));
+      write(o, col0 + (int)col, x, last);
+    }
+    at += __popc(heads);
+  }
+}
+// Both for a group of NT threads, every warp a contiguous part (s_part: one int per warp); returns
+// the number of distinct columns.
+template <typename KEY, int NT, bool EMIT, typename F>
+__device__ __forceinline__ int emit_runs(const KEY* keys, int count, int shift, int tid, int* s_part, int col0,
+                                         long long base, F&& write) {
+  constexpr int NW = NT / 32;
+  const int warp = tid >> 5, lane = tid & 31;
+  const int per = NW == 1 ? count : ((count + NT - 1) / NT) * 32;
+  const int b = NW == 1 ? 0 : min(count, warp * per), e = NW == 1 ? count : min(count, b + per);
+  int before = 0, total = 0;
+  if (NW > 1 || !EMIT) {
+    total = count_runs<KEY>(keys, b, e, shift, lane);
+    if (NW > 1) {
+      if (lane == 0) s_part[warp] = total;
+      __syncthreads();
+      total = 0;
+#pragma unroll
+      for (int w = 0; w < NW; w++) {
+        const int h = s_part[w];
+        if (w < warp) before += h;
+        total += h;
+      }
+    }
+  }
+  if (EMIT) {
+    if (NW == 1) total = count_runs<KEY>(keys, b, e, shift, lane);
+    write_runs<KEY>(keys, b, e, count, shift, lane, col0, base + before, write);
+  }
+  return total;
+}
+
+// ---- expansion ------------------------------------------------------------------------------------
+// The products of A entries [pa0, pa1) (at most 32, one per lane) spread evenly over the lanes
+// of a warp: lane l looks up the B row of entry pa0 + l, a warp scan of the row lengths numbers
+// the products, and every lane then takes products lane, lane + 32, ... — a 5-step search over
+// the scanned lengths tells which entry a product belongs to.  No lane idles on a short B row and
+// the index loads of 32 entries are in flight together, instead of one dependent chain
+// (A entry -> B row pointers -> B entries) per entry.  `emit(ordinal, a_value, pb)` is called once
+// per product with its number in this group, the value of its A entry (T(0) in the symbolic phase)
+// and its position in B; the number of products is returned.
+template <typename T, bool NUMERIC, typename F>
+__device__ __forceinline__ int expand_products(const CsrIn& in, int pa0, int pa1, int lane, F&& emit) {
+  const int pa = pa0 + lane;
+  int bb = 0, len = 0;
+  T a = T(0);
+  if (pa < pa1) {
+    const int j = __ldg(in.Acrd + pa);
+    bb = __ldg(in.Bpos + j);
+    len = __ldg(in.Bpos + j + 1) - bb;
+    if (NUMERIC) a = static_cast<const T*>(in.Aval)[pa];
+  }
+  int incl = len;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(FULL, incl, o);
+    if (lane >= o) incl += y;
+  }
+  const int total = __shfl_sync(FULL, incl, 31);
+  const int excl = incl - len;
+#pragma unroll 4
+  for (int q0 = 0; q0 < total; q0 += 32) {
+    const int q = q0 + lane;
+    // largest e with excl[e] <= q (lanes past the end search too: shuffles need the whole warp)
+    int e = 0;
+#pragma unroll
+    for (int step = 16; step > 0; step >>= 1) {
+      const int v = __shfl_sync(FULL, excl, e + step);
+      if (v <= q) e += step;
+    }
+    const int off = __shfl_sync(FULL, bb - excl, e);
+    const T e_a = NUMERIC ? __shfl_sync(FULL, a, e) : T(0);
+    if (q < total) emit(q, e_a, off + q);
+  }
+  return total;
+}
+
+// The same for a CTA of NT threads, NT entries at a time: product q goes to thread q % NT whatever the
+// lengths of the B rows are, the search runs over the scanned lengths in shared memory.  (With a
+// warp per 32 entries, a row whose products come mostly from one long B row - the usual long row of
+// a power-law matrix - kept one warp busy and the rest waiting.)
+template <typename T, int NT>
+struct ExpandSmem {
+  int excl[NT], off[NT];
+  T a[NT];
+  int part[NT / 32];
+};
+template <typename T, bool NUMERIC, int NT, typename F>
+__device__ __forceinline__ void expand_cta(const CsrIn& in, int ab, int ae, ExpandSmem<T, NT>& sm, int tid, F&& emit) {
+  const int warp = tid >> 5, lane = tid & 31;
+  int first = 0;
+  for (int p0 = ab; p0 < ae; p0 += NT) {
+    const int pa = p0 + tid;
+    int bb = 0, len = 0;
+    if (pa < ae) {
+      const int j = __ldg(in.Acrd + pa);
+      bb = __ldg(in.Bpos + j);
+      len = __ldg(in.Bpos + j + 1) - bb;
+      if (NUMERIC) sm.a[tid] = static_cast<const T*>(in.Aval)[pa];
+    }
+    int incl = len;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(FULL, incl, o);
+      if (lane >= o) incl += y;
+    }
+    if (lane == 31) sm.part[warp] = incl;
+    __syncthreads();
+    int excl = incl - len, total = 0;
+#pragma unroll
+    for (int w = 0; w < NT / 32; w++) {
+      const int c = sm.part[w];
+      if (w < warp) excl += c;
+      total += c;
+    }
+    sm.excl[tid] = excl;
+    sm.off[tid] = bb - excl;
+    __syncthreads();
+#pragma unroll 4
+    for (int q = tid; q < total; q += NT) {
+      int e = 0;   // largest e with excl[e] <= q
+#pragma unroll
+      for (int step = NT / 2; step > 0; step >>= 1)
+        if (sm.excl[e + step] <= q) e += step;
+      emit(first + q, NUMERIC ? sm.a[e] : T(0), sm.off[e] + q);
+    }
+    first += total;
+    __syncthreads();
+  }
+}
+
+// All products of A row [ab, ae) to shared memory: keys[o] = column << shift | o, prods[o]; their
+// number is known beforehand.  One warp (`sm` unused) or a CTA.  COLUMNS: keys[o] = column alone.
+template <typename T, bool NUMERIC, typename KEY, int NT, bool COLUMNS = false>
+__device__ __forceinline__ void expand_row(const CsrIn& in, int ab, int ae, int shift, KEY* keys, Slot* prods,
+                                           int tid, ExpandSmem<T, NT>* sm) {
+  const T* Bval = static_cast<const T*>(in.Bval);
+  auto put = [&](int o, T a, int pb) {
+    const KEY c = (KEY)(unsigned)__ldg(in.Bcrd + pb);
+    keys[o] = COLUMNS ? c : (c << shift) | (KEY)o;
+    if (NUMERIC) prods[o] = product_bits<T>(a, __ldg(Bval + pb));
+  };
+  if constexpr (NT == 32) {
+    int first = 0;
+    for (int p0 = ab; p0 < ae; p0 += 32)
+      first += expand_products<T, NUMERIC>(in, p0, min(ae, p0 + 32), tid, [&](int o, T a, int pb) {
+        put(first + o, a, pb);
+      });
+    __syncwarp();
+  } else {
+    expand_cta<T, NUMERIC, NT>(in, ab, ae, *sm, tid, put);
+  }
+}
+
+struct RowsOut {
+  int* row_cnt;         // distinct columns per row (null: not wanted)
+  const int* off;       // [row] where the row's entries go (numeric)
+  int* crd;
+  void* val;
+};
+
+template <typename T, bool NUMERIC, typename KEY, int R, int NT>
+__device__ __forceinline__ int sort_and_emit(KEY* keys, const Slot* prods, int count, int shift, int tid, int* s_part,
+                                             long long base, const RowsOut& out) {
+  sort_keys<KEY, R, NT>(keys, count, tid);
+  T* val = static_cast<T*>(out.val);
+  const KEY mask = ((KEY)1 << shift) - 1;
+  return emit_runs<KEY, NT, NUMERIC>(keys, count, shift, tid, s_part, 0, base,
+                                     [&](long long o, int col, int x, int last) {
+    out.crd[o] = col;
+    RunSum<T> s;
+    for (; x < last; x++) s.add(prods[(int)(keys[x] & mask)]);
+    val[o] = s.value();
+  });
+}
+
+// Rows of at most 128 products: a warp each, the network as long as the row needs.
+constexpr int kWarpCap = 128;
+template <typename T, bool NUMERIC, typename KEY, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS)
+spgemm_warp_kernel(const int* __restrict__ rows, int nrows, const int* __restrict__ upper, CsrIn in, int shift,
+                   RowsOut out) {
+  __shared__ KEY s_keys[WARPS][kWarpCap];
+  __shared__ Slot s_prods[WARPS][NUMERIC ? kWarpCap : 1];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int r = blockIdx.x * WARPS + warp;
+  if (r >= nrows) return;
+  const int i = __ldg(rows + r);
+  const int count = __ldg(upper + i), ab = __ldg(in.Apos + i), ae = __ldg(in.Apos + i + 1);
+  const long long base = NUMERIC ? __ldg(out.off + i) : 0;
+  KEY* keys = s_keys[warp];
+  Slot* prods = s_prods[warp];
+  expand_row<T, NUMERIC, KEY, 32>(in, ab, ae, shift, keys, prods, lane, nullptr);
+  int u;
+#define SB_SORT(R) u = sort_and_emit<T, NUMERIC, KEY, R, 32>(keys, prods, count, shift, lane, nullptr, base, out)
+  if (count <= 32) SB_SORT(1);
+  else if (count <= 64) SB_SORT(2);
+  else SB_SORT(4);
+#undef SB_SORT
+  if (out.row_cnt && lane == 0) out.row_cnt[i] = u;
+}
+
+// Rows of at most RMAX NT products: a CTA of NT threads each.  (A single warp for 129 to 512
+// products took 57 ns per thousand products, serial in its slabs of A entries.)
+template <typename T, bool NUMERIC, typename KEY, int NT, int RMAX>
+__global__ void __launch_bounds__(NT)
+spgemm_cta_kernel(const int* __restrict__ rows, const int* __restrict__ upper, CsrIn in, int shift, RowsOut out) {
+  constexpr int CAP = RMAX * NT;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  Slot* prods = reinterpret_cast<Slot*>(smem_raw);
+  KEY* keys = reinterpret_cast<KEY*>(smem_raw + (NUMERIC ? sizeof(Slot) * CAP : 0));
+  __shared__ ExpandSmem<T, NT> s_expand;
+  int* s_part = s_expand.part;
+  const int i = __ldg(rows + blockIdx.x), tid = threadIdx.x;
+  const int count = __ldg(upper + i), ab = __ldg(in.Apos + i), ae = __ldg(in.Apos + i + 1);
+  const long long base = NUMERIC ? __ldg(out.off + i) : 0;
+  expand_row<T, NUMERIC, KEY, NT>(in, ab, ae, shift, keys, prods, tid, &s_expand);
+  int u;
+  if (count <= RMAX / 2 * NT)
+    u = sort_and_emit<T, NUMERIC, KEY, RMAX / 2, NT>(keys, prods, count, shift, tid, s_part, base, out);
+  else
+    u = sort_and_emit<T, NUMERIC, KEY, RMAX, NT>(keys, prods, count, shift, tid, s_part, base, out);
+  if (out.row_cnt && tid == 0) out.row_cnt[i] = u;
+}
+
+// Rows of 2049 to 8192 products: a CTA each, the row's columns cut into up to 32 segments that a warp
+// sorts each.  The network over the whole row would need 64-bit keys (21 bits of column and 13 of
+// ordinal on a 2 M-column matrix), 128 KB of shared memory and ten exchanges through it: 4.6 ms
+// for 10,562 rows where the segments take 1.9 ms.  Segments of more than 512 products (columns
+// crowded together) are sorted by the CTA in shared memory.
+constexpr int kSplitThreads = 512, kSplitCap = 8192, kSegments = 32, kSegmentSort = 512, kSplitOrd = 13;
+
+// Ascending sort of any number of keys in shared memory by NT threads: the bitonic network in the form
+// in which every comparison puts the smaller key first, so that places behind the end need no key.
+template <typename KEY, int NT>
+__device__ __noinline__ void sort_in_smem(KEY* keys, int count, int tid) {
+  for (int size = 2; size < 2 * count; size <<= 1) {
+    for (int stride = size >> 1; stride > 0; stride >>= 1) {
+      const int flip = stride == size >> 1 ? size - 1 : stride;
+      __syncthreads();
+      for (int x = tid; x < count; x += NT) {
+        const int y = x ^ flip;
+        if (y > x && y < count && keys[y] < keys[x]) {
+          const KEY t = keys[x];
+          keys[x] = keys[y];
+          keys[y] = t;
+        }
+      }
+    }
+  }
+  __syncthreads();
+}
+
+template <typename T, bool NUMERIC>
+__global__ void __launch_bounds__(kSplitThreads, 2)
+spgemm_split_kernel(const int* __restrict__ rows, const int* __restrict__ upper, CsrIn in, int seg_shift,
+                    RowsOut out) {
+  constexpr int NT = kSplitThreads, NW = NT / 32, R = kSplitCap / NT;
+  typedef unsigned KEY;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  Slot* prods = reinterpret_cast<Slot*>(smem_raw);
+  KEY* keys = reinterpret_cast<KEY*>(smem_raw + (NUMERIC ? sizeof(Slot) * kSplitCap : 0));
+  __shared__ ExpandSmem<T, NT> s_expand;
+  __shared__ int s_cnt[kSegments], s_start[kSegments + 1], s_u[kSegments];
+  const int i = __ldg(rows + blockIdx.x), tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int count = __ldg(upper + i), ab = __ldg(in.Apos + i), ae = __ldg(in.Apos + i + 1);
+  const long long base = NUMERIC ? __ldg(out.off + i) : 0;
+  if (tid < kSegments) s_cnt[tid] = 0;
+  expand_row<T, NUMERIC, KEY, NT, true>(in, ab, ae, 0, keys, prods, tid, &s_expand);
+  // columns to their segments (in any order: the sort brings it), the ordinal below the column
+  KEY c[R];
+  int rank[R];
+#pragma unroll
+  for (int q = 0; q < R; q++) {
+    const int x = tid + q * NT;
+    if (x < count) {
+      c[q] = keys[x];
+      rank[q] = atomicAdd(&s_cnt[c[q] >> seg_shift], 1);
+    }
+  }
+  __syncthreads();
+  if (warp == 0) {
+    const int v = s_cnt[lane];
+    int incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(FULL, incl, o);
+      if (lane >= o) incl += y;
+    }
+    s_start[lane + 1] = incl;
+    if (lane == 0) s_start[0] = 0;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < R; q++) {
+    const int x = tid + q * NT;
+    if (x < count) {
+      const int seg = c[q] >> seg_shift;
+      keys[s_start[seg] + rank[q]] = ((c[q] & (((KEY)1 << seg_shift) - 1)) << kSplitOrd) | (KEY)x;
+    }
+  }
+  __syncthreads();
+  for (int seg = 0; seg < kSegments; seg++) {
+    const int n = s_start[seg + 1] - s_start[seg];
+    if (n > kSegmentSort) sort_in_smem<KEY, NT>(keys + s_start[seg], n, tid);
+  }
+  for (int seg = warp; seg < kSegments; seg += NW) {
+    const int b = s_start[seg], n = s_start[seg + 1] - b;
+    if (n <= kSegmentSort) {
+      if (n > 256) sort_keys<KEY, 16, 32>(keys + b, n, lane);
+      else if (n > 128) sort_keys<KEY, 8, 32>(keys + b, n, lane);
+      else if (n > 1) sort_keys<KEY, 4, 32>(keys + b, n, lane);
+    }
+    const int u = count_runs<KEY>(keys + b, 0, n, kSplitOrd, lane);
+    if (lane == 0) s_u[seg] = u;
+  }
+  __syncthreads();
+  if (out.row_cnt && warp == 0) {
+    const int u = __reduce_add_sync(FULL, s_u[lane]);
+    if (lane == 0) out.row_cnt[i] = u;
+  }
+  if (NUMERIC) {
+    T* val = static_cast<T*>(out.val);
+    for (int seg = warp; seg < kSegments; seg += NW) {
+      const int b = s_start[seg], n = s_start[seg + 1] - b;
+      const int before = __reduce_add_sync(FULL, lane < seg ? s_u[lane] : 0);
+      const KEY* k = keys + b;
+      write_runs<KEY>(k, 0, n, n, kSplitOrd, lane, seg << seg_shift, base + before,
+                      [&](long long o, int col, int x, int last) {
+        out.crd[o] = col;
+        RunSum<T> s;
+        for (; x < last; x++) s.add(prods[(int)(k[x] & (kSplitCap - 1))]);
+        val[o] = s.value();
+      });
+    }
+  }
+}
+
+}  // namespace sb

@@ -88,40 +88,6 @@ __device__ __forceinline__ void cp_async(void* smem, const void* gmem) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(s), "l"(gmem), "n"(BYTES) : "memory");
 }
 
-// Row of entry p: the largest r with pos[r] <= p < pos[m]; the whole CTA calls it.  Matrices of up
-// to 32 rows per thread are looked at in one go (one round of loads in flight together instead of
-// one dependent round per factor of 256); `s_count`: one int per warp.
-__device__ __forceinline__ int tile_row_of(const int* __restrict__ pos, int m, int p, int* s_count) {
-  if (m <= 32 * kTileThreadsMm) {
-    int c = 0;
-    for (int r = threadIdx.x; r < m; r += 8 * kTileThreadsMm) {
-#pragma unroll
-      for (int q = 0; q < 8; q++) {
-        const int x = r + q * kTileThreadsMm;
-        c += x < m && __ldg(pos + x) <= p;
-      }
-    }
-    c = __reduce_add_sync(FULL, c);
-    if ((threadIdx.x & 31) == 0) s_count[threadIdx.x >> 5] = c;
-    __syncthreads();
-    c = 0;
-#pragma unroll
-    for (int w = 0; w < kTileWarps; w++) c += s_count[w];
-    __syncthreads();
-    return c - 1;
-  }
-  int lo = 0, hi = m;
-  while (true) {
-    const int span = hi - lo;
-    const int step = (span + kTileThreadsMm - 1) / kTileThreadsMm;
-    const long long r = (long long)lo + (long long)threadIdx.x * step;
-    const int c = __syncthreads_count(r < hi && __ldg(pos + r) <= p);
-    lo += (c - 1) * step;
-    if (step == 1) return lo;
-    hi = min(hi, lo + step);
-  }
-}
-
 template <typename T, int L, int VEC, int W>
 __device__ __forceinline__ void tile_store_row(const SpmmArgs<T>& a, int row, int col0, const bool (&col_ok)[VEC],
                                                const Pack<T, W> (&sum)[VEC]) {
@@ -218,7 +184,7 @@ spmm_tile_kernel(SpmmArgs<T> a, TileArgs<T> t) {
 
   // rows in turns of kTileRowCap, from the one that holds the first entry not dealt with
   for (int next = e0; next < e1;) {
-    const int r0 = tile_row_of(a.pos, a.m, next, sm.count);
+    const int r0 = cta_row_of<kTileThreadsMm>(a.pos, a.m, next, sm.count);
     for (int i = tid; i < kTileRowCap + 1; i += kTileThreadsMm) sm.pos[i] = __ldg(a.pos + min(a.m, r0 + i));
     if (tid == 0) { sm.n_warp = sm.n_cta = sm.next_warp = sm.next_row = 0; }
     asm volatile("cp.async.wait_group 0;" ::: "memory");

@@ -559,7 +559,13 @@ def csr_row_softmax(pos, val, scale: float = 1.0, out: Optional[torch.Tensor] = 
 
 def spgemm_csr(Apos, Acrd, Aval, Bpos, Bcrd, Bval, n: int, timings: Optional[dict] = None
                ) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
-    """C = A @ B for CSR operands.  Returns (Cpos int32, Ccrd int32 ascending per row, Cval)."""
+    """C = A @ B for CSR operands.  Returns (Cpos int32, Ccrd int32 ascending per row, Cval).
+    One pass where memory for all products is there (16 GB at most); else, and when ``timings`` asks
+    for the phases, symbolic + numeric."""
+    if timings is None:
+        r = _lib.host().spgemm(Apos, Acrd, Aval, Bpos, Bcrd, Bval, n)
+        if r is not None:
+            return r
     Apos, Acrd = _dev(Apos, torch.int32, "Apos"), _dev(Acrd, torch.int32, "Acrd")
     Bpos, Bcrd = _dev(Bpos, torch.int32, "Bpos"), _dev(Bcrd, torch.int32, "Bcrd")
     code = _DTYPE_CODE.get(Aval.dtype)
