@@ -87,16 +87,18 @@ int spmm_wide_launch(int64_t m, int64_t k, const int* pos, const int* crd, const
                      int64_t ldb, const float* bias, int relu, float* C, int64_t ldc, cudaStream_t st);
 
 #ifdef __CUDACC__
-// Launch of a kernel whose first act is griddepcontrol.wait: its CTAs may be set up while the kernel
-// before it on the stream still runs (a follow-up launch costs about a microsecond less).
+// Launch of a kernel that waits for the kernel before it on the stream itself (griddepcontrol.wait):
+// its CTAs may be set up while that one still runs (a follow-up launch costs about a microsecond less).
 template <typename... P, typename... A>
-inline cudaError_t launch_early(void (*kernel)(P...), dim3 grid, unsigned threads, cudaStream_t st, A... args) {
+inline cudaError_t launch_early(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st,
+                                A... args) {
   cudaLaunchAttribute attr{};
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;

@@ -126,7 +126,8 @@ static WsLayout ws_layout(void* base, int64_t m, int64_t n) {
 }
 
 // ---- binning ---------------------------------------------------------------------------------
-// U_i of every row of A and the row's bin.  A CTA takes 1024 rows: 8 lanes per row, rows of more
+// U_i of every row of A and the row's bin.  A CTA takes up to 1024 rows (fewer where that leaves SMs
+// idle): 8 lanes per row, rows of more
 // than 64 entries by a warp, of more than 2048 by the CTA (8 lanes alone needed 2 ms for the hub rows
 // of a 2 M-row matrix); it appends them to the bins' lists with one atomic per bin (one per warp and
 // bin is 0.4 ms there: five addresses for everybody).  Rows with U = 0 get row_cnt = 0 and join no bin.
@@ -145,7 +146,7 @@ __device__ __forceinline__ long long count_products(const int* __restrict__ Acrd
 }
 
 __global__ void __launch_bounds__(kBinThreads)
-spgemm_bin_kernel(int m, const int* __restrict__ Apos, const int* __restrict__ Acrd,
+spgemm_bin_kernel(int m, int rows_per_cta, const int* __restrict__ Apos, const int* __restrict__ Acrd,
                   const int* __restrict__ Bpos, int* __restrict__ upper, int* __restrict__ bin_rows,
                   int* __restrict__ bin_cursor, int* __restrict__ row_cnt) {
   __shared__ int s_u[kBinRows], s_pos[kBinRows + 1];
@@ -154,15 +155,15 @@ spgemm_bin_kernel(int m, const int* __restrict__ Apos, const int* __restrict__ A
   __shared__ long long s_part[32];
   __shared__ int s_cnt[kBins], s_base[kBins];
   const int tid = threadIdx.x, l = tid & 7, warp = tid >> 5, lane = tid & 31;
-  const long long row0 = (long long)blockIdx.x * kBinRows;
-  const int rows = (int)min((long long)kBinRows, m - row0);
+  const long long row0 = (long long)blockIdx.x * rows_per_cta;
+  const int rows = (int)min((long long)rows_per_cta, m - row0);
   if (tid < kBins) s_cnt[tid] = 0;
   if (tid == 0) s_nwarp = s_ncta = s_next = 0;
   for (int x = tid; x <= rows; x += kBinThreads) s_pos[x] = __ldg(Apos + row0 + x);
   __syncthreads();
 #pragma unroll 2
-  for (int q = 0; q < kBinRows / (kBinThreads / 8); q++) {
-    const int x = q * (kBinThreads / 8) + (tid >> 3);
+  for (int x0 = 0; x0 < rows; x0 += kBinThreads / 8) {
+    const int x = x0 + (tid >> 3);
     long long u = 0;
     bool put = false;
     if (x < rows) {
@@ -256,6 +257,22 @@ __device__ __forceinline__ void acc_add(Slot* slot, Slot bits, double scale, boo
     atomicAdd(slot, bits);
   }
 }
+// The same for a slot in shared memory, where a 64-bit atomic addition is a compare-and-swap loop: two
+// 32-bit additions, the carry of the lower one into the upper one.
+template <typename T>
+__device__ __forceinline__ void acc_add_smem(Slot* slot, Slot bits, double scale, bool fixed) {
+  if constexpr (kIsFloat<T>) {
+    if (!fixed) {
+      atomicAdd(reinterpret_cast<double*>(slot), __longlong_as_double((long long)bits));
+      return;
+    }
+    bits = to_fixed<T>(bits, scale);
+  }
+  unsigned* half = reinterpret_cast<unsigned*>(slot);
+  const unsigned lo = (unsigned)bits, old = atomicAdd(half, lo);
+  if constexpr (sizeof(T) == 8 || kIsFloat<T>) atomicAdd(half + 1, (unsigned)(bits >> 32) + (old + lo < old));
+}
+
 template <typename T>
 __device__ __forceinline__ T acc_value(Slot v, double scale, bool fixed) {
   if constexpr (kIsFloat<T>) return fixed ? from_fixed<T>(v, scale) : (T)__longlong_as_double((long long)v);
@@ -443,7 +460,7 @@ big_window_kernel(BigArea b, int buckets, long long n) {
           const long long d = (long long)(NUMERIC ? b.rec[o + x].col : b.key[o + x]) - w0;
           if (d < 0 || d >= kWindow) continue;
           atomicOr(&bits[d >> 5], 1u << (d & 31));
-          if (NUMERIC) acc_add<T>(&acc[d], b.rec[o + x].prod, scale, fixed);
+          if (NUMERIC) acc_add_smem<T>(&acc[d], b.rec[o + x].prod, scale, fixed);
         }
         __syncthreads();
         // 256 words: threads 0..255 take one each, in column order
@@ -737,6 +754,49 @@ scan_write_kernel(int m, const int* __restrict__ cnt, const long long* __restric
   }
 }
 
+// All of it by one CTA, for short arrays: a warp per contiguous part, 32 counts at a time.
+constexpr int kScanSmall = 32768;
+__global__ void __launch_bounds__(1024)
+scan_small_kernel(int m, const int* __restrict__ cnt, int* __restrict__ out, long long* __restrict__ total) {
+  constexpr int STEPS = kScanSmall / 1024;
+  __shared__ long long s[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int steps = (m + 1023) / 1024, b = warp * steps * 32;
+  int c[STEPS];
+  long long mine = 0;
+#pragma unroll
+  for (int i = 0; i < STEPS; i++) {
+    const int x = b + i * 32 + lane;
+    c[i] = i < steps && x < m ? cnt[x] : 0;
+    mine += c[i];
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(FULL, mine, o);
+  if (lane == 0) s[warp] = mine;
+  __syncthreads();
+  long long run = 0, all = 0;
+#pragma unroll
+  for (int w = 0; w < 32; w++) {
+    const long long v = s[w];
+    if (w < warp) run += v;
+    all += v;
+  }
+  if (threadIdx.x == 0) { out[0] = 0; *total = all; }
+#pragma unroll
+  for (int i = 0; i < STEPS; i++) {
+    if (i >= steps) break;
+    long long incl = c[i];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const long long y = __shfl_up_sync(FULL, incl, o);
+      if (lane >= o) incl += y;
+    }
+    const int x = b + i * 32 + lane;
+    if (x < m) out[x + 1] = (int)(run + incl);
+    run += __shfl_sync(FULL, incl, 31);
+  }
+}
+
 // Exclusive scan of n int counts into out[0..n] (int32), running total in int64 at *total_dev.
 // `block_sum` needs ceil(n / 4096) + 1 int64 slots.
 int exclusive_scan_i32(int n, const int* cnt, int* out, long long* block_sum, long long* total_dev,
@@ -744,6 +804,11 @@ int exclusive_scan_i32(int n, const int* cnt, int* out, long long* block_sum, lo
   if (n <= 0) {
     SB_CUDA(cudaMemsetAsync(out, 0, 4, st));
     SB_CUDA(cudaMemsetAsync(total_dev, 0, 8, st));
+    return SB_OK;
+  }
+  if (n <= kScanSmall) {
+    scan_small_kernel<<<1, 1024, 0, st>>>(n, cnt, out, total_dev);
+    SB_LAUNCH_CHECK("scan_small_kernel");
     return SB_OK;
   }
   const int nb = (int)ceil_div(n, kScanTile);
@@ -754,6 +819,90 @@ int exclusive_scan_i32(int n, const int* cnt, int* out, long long* block_sum, lo
   scan_write_kernel<<<nb, 1024, 0, st>>>(n, cnt, block_sum, out);
   SB_LAUNCH_CHECK("scan_write_kernel");
   return SB_OK;
+}
+
+// ---- long rows of a matrix of few columns ---------------------------------------------------------
+// Bitmap and accumulators of all n columns in shared memory (n up to kSmemColumns): one CTA per row,
+// no plan, no read-back, one launch instead of the bucket path's ten (20,011 columns, ten rows of
+// 8,200 to 80,000 products: 190 us there, 92 us here, beside the other bins' kernels).
+constexpr int kSmemColumns = 24576, kSmemThreads = 1024;
+template <typename T, bool NUMERIC>
+__global__ void __launch_bounds__(kSmemThreads)
+spgemm_smem_kernel(const int* __restrict__ rows, CsrIn in, int n, const unsigned long long* __restrict__ max_b,
+                   RowsOut out) {
+  constexpr int NT = kSmemThreads, NW = NT / 32;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  unsigned* bits = reinterpret_cast<unsigned*>(smem_raw);            // kSmemColumns / 32 words
+  Slot* acc = reinterpret_cast<Slot*>(smem_raw + kSmemColumns / 8);
+  __shared__ ExpandSmem<T, NT> s_expand;
+  __shared__ double s_abs[NW];
+  __shared__ int s_part[NW], s_at[kSmemColumns / 32];
+  let_next_begin();
+  const int i = __ldg(rows + blockIdx.x), tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int ab = __ldg(in.Apos + i), ae = __ldg(in.Apos + i + 1);
+  for (int x = tid; x < kSmemColumns / 32; x += NT) bits[x] = 0;
+  if (NUMERIC)
+    for (int x = tid; x < n; x += NT) acc[x] = 0;
+  double scale = 1.0;
+  if constexpr (NUMERIC && kIsFloat<T>) {
+    double s = 0.0;
+    for (int p = ab + tid; p < ae; p += NT) s += fabs((double)static_cast<const T*>(in.Aval)[p]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(FULL, s, o);
+    if (lane == 0) s_abs[warp] = s;
+    __syncthreads();
+    s = 0.0;
+    for (int w = 0; w < NW; w++) s += s_abs[w];
+    scale = scale_for_bound(s * __longlong_as_double((long long)*max_b));
+  }
+  const bool fixed = scale == scale;
+  __syncthreads();
+  const T* Bval = static_cast<const T*>(in.Bval);
+  expand_cta<T, NUMERIC, NT>(in, ab, ae, s_expand, tid, [&](int, T a, int pb) {
+    const int c = __ldg(in.Bcrd + pb);
+    const unsigned bit = 1u << (c & 31);
+    if (!(bits[c >> 5] & bit)) atomicOr(&bits[c >> 5], bit);
+    if (NUMERIC) acc_add_smem<T>(&acc[c], product_bits<T>(a, __ldg(Bval + pb)), scale, fixed);
+  });
+  __syncthreads();
+  // kSmemColumns / 32 = 768 words: one per thread, in column order
+  unsigned m = tid < kSmemColumns / 32 ? bits[tid] : 0;
+  const int c = __popc(m);
+  int incl = c;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int y = __shfl_up_sync(FULL, incl, d);
+    if (lane >= d) incl += y;
+  }
+  if (lane == 31) s_part[warp] = incl;
+  __syncthreads();
+  int before = 0, total = 0;
+#pragma unroll
+  for (int w = 0; w < NW; w++) {
+    const int v = s_part[w];
+    if (w < warp) before += v;
+    total += v;
+  }
+  if (out.row_cnt && tid == 0) out.row_cnt[i] = total;
+  if (NUMERIC) {
+    // a warp per word, a lane per column
+    if (tid < kSmemColumns / 32) s_at[tid] = before + incl - c;
+    __syncthreads();
+    const long long base = __ldg(out.off + i);
+    const double inv = 1.0 / scale;
+    for (int w = warp; w < kSmemColumns / 32; w += NW) {
+      const unsigned word = bits[w];
+      if (!(word >> lane & 1)) continue;
+      const long long at = base + s_at[w] + __popc(word & ((1u << lane) - 1u));
+      const Slot v = acc[w * 32 + lane];
+      out.crd[at] = w * 32 + lane;
+      T value;
+      if constexpr (kIsFloat<T>) value = fixed ? (T)((double)(long long)v * inv) : (T)__longlong_as_double((long long)v);
+      else value = (T)v;
+      static_cast<T*>(out.val)[at] = value;
+    }
+  }
+  end_after_previous();
 }
 
 // ---- one-pass form: the rows' entries from their product offsets to their place ------------------
@@ -890,14 +1039,28 @@ static int big_batch(const WsLayout& w, const std::vector<int>& row, const std::
   return SB_OK;
 }
 
+// max |b|, for the fixed-point scales of the long rows.
+template <typename T>
+static int max_abs(const WsLayout& w, const CsrIn& in, int64_t kb, cudaStream_t st) {
+  SB_CUDA(cudaMemsetAsync(w.max_b, 0, 8, st));
+  spgemm_max_abs_kernel<T><<<8 * sm_count(), 256, 0, st>>>(in.Bpos + kb, static_cast<const T*>(in.Bval), w.max_b);
+  SB_LAUNCH_CHECK("spgemm_max_abs_kernel");
+  return SB_OK;
+}
+
 template <typename T, bool NUMERIC>
-static int big_rows(const WsLayout& w, int64_t count, int64_t m, int64_t kb, int64_t n, const CsrIn& in,
+static int launch_smem_bin(const int* rows, int64_t count, const WsLayout& w, int64_t n, const CsrIn& in,
+                           const RowsOut& out, cudaStream_t st) {
+  auto k = spgemm_smem_kernel<T, NUMERIC>;
+  const int smem = kSmemColumns / 8 + (NUMERIC ? (int)n * 8 : 0);
+  SB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  SB_CUDA(launch_early(k, dim3((unsigned)count), kSmemThreads, smem, st, rows, in, (int)n, w.max_b, out));
+  return SB_OK;
+}
+
+template <typename T, bool NUMERIC>
+static int big_rows(const WsLayout& w, int64_t count, int64_t m, int64_t n, const CsrIn& in,
                     const RowsOut& out, cudaStream_t st) {
-  if (NUMERIC && kIsFloat<T>) {
-    SB_CUDA(cudaMemsetAsync(w.max_b, 0, 8, st));
-    spgemm_max_abs_kernel<T><<<8 * sm_count(), 256, 0, st>>>(in.Bpos + kb, static_cast<const T*>(in.Bval), w.max_b);
-    SB_LAUNCH_CHECK("spgemm_max_abs_kernel");
-  }
   std::vector<int4> info((size_t)count);
   const int64_t room = (int64_t)(w.area_bytes / sizeof(int4));
   for (int64_t x0 = 0; x0 < count; x0 += room) {
@@ -953,9 +1116,8 @@ template <typename T, bool NUMERIC, typename KEY>
 static int launch_warp_bin(const int* rows, int64_t count, const WsLayout& w, const CsrIn& in, int shift,
                            const RowsOut& out, cudaStream_t st) {
   constexpr int WARPS = 4;
-  spgemm_warp_kernel<T, NUMERIC, KEY, WARPS><<<(unsigned)ceil_div(count, WARPS), 32 * WARPS, 0, st>>>(
-      rows, (int)count, w.upper, in, shift, out);
-  SB_LAUNCH_CHECK("spgemm_warp_kernel");
+  SB_CUDA(launch_early(spgemm_warp_kernel<T, NUMERIC, KEY, WARPS>, dim3((unsigned)ceil_div(count, WARPS)), 32 * WARPS,
+                       0, st, rows, (int)count, w.upper, in, shift, out));
   return SB_OK;
 }
 
@@ -965,8 +1127,7 @@ static int launch_cta_bin(const int* rows, int64_t count, const WsLayout& w, con
   auto k = spgemm_cta_kernel<T, NUMERIC, KEY, NT, RMAX>;
   const int smem = RMAX * NT * (int)(sizeof(KEY) + (NUMERIC ? sizeof(Slot) : 0));
   SB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  k<<<(unsigned)count, NT, smem, st>>>(rows, w.upper, in, shift, out);
-  SB_LAUNCH_CHECK("spgemm_cta_kernel");
+  SB_CUDA(launch_early(k, dim3((unsigned)count), NT, smem, st, rows, w.upper, in, shift, out));
   return SB_OK;
 }
 
@@ -981,14 +1142,21 @@ static int launch_split_bin(const int* rows, int64_t count, const WsLayout& w, c
   return SB_OK;
 }
 
-// All rows; the longest first, so that the short ones fill in behind them.  A key holds the column
+// All rows; the longest first, so that the short ones fill in behind them: a bin's kernel lets the
+// next one start as soon as its own CTAs have (they do not depend on one another) and ends after the
+// one before it.  A key holds the column
 // above the product's ordinal: 32 bits where both fit.
 template <typename T, bool NUMERIC>
 static int launch_bins(const WsLayout& w, const long long* counts, int64_t m, int64_t kb, int64_t n,
                        const CsrIn& in, const RowsOut& out, cudaStream_t st) {
   const int nbits = ceil_log2(std::max<int64_t>(n, 1));
   int rc = SB_OK;
-  if (counts[4] > 0) rc = big_rows<T, NUMERIC>(w, counts[4], m, kb, n, in, out, st);
+  const bool in_smem = n <= kSmemColumns;
+  if constexpr (NUMERIC && kIsFloat<T>) {
+    if (counts[4] > 0) rc = max_abs<T>(w, in, kb, st);
+    if (rc != SB_OK) return rc;
+  }
+  if (counts[4] > 0 && !in_smem) rc = big_rows<T, NUMERIC>(w, counts[4], m, n, in, out, st);
   if (rc != SB_OK) return rc;
   typedef unsigned K32;
   typedef unsigned long long K64;
@@ -1009,9 +1177,13 @@ static int launch_bins(const WsLayout& w, const long long* counts, int64_t m, in
                      : launch_cta_bin<T, NUMERIC, K64, 64, 8>(rows + m, counts[1], w, in, 9, out, st);
     if (rc != SB_OK) return rc;
   }
-  if (counts[0] > 0)
+  if (counts[0] > 0) {
     rc = nbits <= 25 ? launch_warp_bin<T, NUMERIC, K32>(rows, counts[0], w, in, 7, out, st)
                      : launch_warp_bin<T, NUMERIC, K64>(rows, counts[0], w, in, 7, out, st);
+    if (rc != SB_OK) return rc;
+  }
+  if (counts[4] > 0 && in_smem)
+    rc = launch_smem_bin<T, NUMERIC>(rows + 4 * m, counts[4], w, n, in, out, st);
   return rc;
 }
 
@@ -1044,8 +1216,9 @@ static int bin_rows(const WsLayout& w, int64_t m, const int32_t* Apos, const int
                     cudaStream_t st) {
   SB_CUDA(cudaMemsetAsync(w.hdr, 0, 16 * 8, st));
   SB_CUDA(cudaMemsetAsync(w.bin_cursor, 0, 16 * 4, st));
-  spgemm_bin_kernel<<<(unsigned)ceil_div(m, kBinRows), kBinThreads, 0, st>>>((int)m, Apos, Acrd, Bpos, w.upper,
-                                                                            w.bin_rows, w.bin_cursor, w.row_cnt);
+  const int rows = (int)std::min<int64_t>(kBinRows, std::max<int64_t>(32, ceil_div(m, 2 * sm_count() * 32) * 32));
+  spgemm_bin_kernel<<<(unsigned)ceil_div(m, rows), kBinThreads, 0, st>>>((int)m, rows, Apos, Acrd, Bpos, w.upper,
+                                                                         w.bin_rows, w.bin_cursor, w.row_cnt);
   SB_LAUNCH_CHECK("spgemm_bin_kernel");
   return SB_OK;
 }

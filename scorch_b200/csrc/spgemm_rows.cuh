@@ -335,6 +335,11 @@ __device__ __forceinline__ void expand_row(const CsrIn& in, int ab, int ae, int 
   }
 }
 
+// The kernels of the bins run side by side: each lets the next launch begin at its own start and ends
+// only after the launch before it, so that what follows the last one follows all of them.
+__device__ __forceinline__ void let_next_begin() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void end_after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 struct RowsOut {
   int* row_cnt;         // distinct columns per row (null: not wanted)
   const int* off;       // [row] where the row's entries go (numeric)
@@ -367,7 +372,11 @@ spgemm_warp_kernel(const int* __restrict__ rows, int nrows, const int* __restric
   __shared__ Slot s_prods[WARPS][NUMERIC ? kWarpCap : 1];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int r = blockIdx.x * WARPS + warp;
-  if (r >= nrows) return;
+  let_next_begin();
+  if (r >= nrows) {
+    end_after_previous();
+    return;
+  }
   const int i = __ldg(rows + r);
   const int count = __ldg(upper + i), ab = __ldg(in.Apos + i), ae = __ldg(in.Apos + i + 1);
   const long long base = NUMERIC ? __ldg(out.off + i) : 0;
@@ -381,6 +390,7 @@ spgemm_warp_kernel(const int* __restrict__ rows, int nrows, const int* __restric
   else SB_SORT(4);
 #undef SB_SORT
   if (out.row_cnt && lane == 0) out.row_cnt[i] = u;
+  end_after_previous();
 }
 
 // Rows of at most RMAX NT products: a CTA of NT threads each.  (A single warp for 129 to 512
@@ -394,6 +404,7 @@ spgemm_cta_kernel(const int* __restrict__ rows, const int* __restrict__ upper, C
   KEY* keys = reinterpret_cast<KEY*>(smem_raw + (NUMERIC ? sizeof(Slot) * CAP : 0));
   __shared__ ExpandSmem<T, NT> s_expand;
   int* s_part = s_expand.part;
+  let_next_begin();
   const int i = __ldg(rows + blockIdx.x), tid = threadIdx.x;
   const int count = __ldg(upper + i), ab = __ldg(in.Apos + i), ae = __ldg(in.Apos + i + 1);
   const long long base = NUMERIC ? __ldg(out.off + i) : 0;
@@ -404,6 +415,7 @@ spgemm_cta_kernel(const int* __restrict__ rows, const int* __restrict__ upper, C
   else
     u = sort_and_emit<T, NUMERIC, KEY, RMAX, NT>(keys, prods, count, shift, tid, s_part, base, out);
   if (out.row_cnt && tid == 0) out.row_cnt[i] = u;
+  end_after_previous();
 }
 
 // Rows of 2049 to 8192 products: a CTA each, the row's columns cut into up to 32 segments that a warp
@@ -448,6 +460,7 @@ spgemm_split_kernel(const int* __restrict__ rows, const int* __restrict__ upper,
   const int i = __ldg(rows + blockIdx.x), tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int count = __ldg(upper + i), ab = __ldg(in.Apos + i), ae = __ldg(in.Apos + i + 1);
   const long long base = NUMERIC ? __ldg(out.off + i) : 0;
+  let_next_begin();
   if (tid < kSegments) s_cnt[tid] = 0;
   expand_row<T, NUMERIC, KEY, NT, true>(in, ab, ae, 0, keys, prods, tid, &s_expand);
   // columns to their segments (in any order: the sort brings it), the ordinal below the column
@@ -517,6 +530,7 @@ spgemm_split_kernel(const int* __restrict__ rows, const int* __restrict__ upper,
       });
     }
   }
+  end_after_previous();
 }
 
 }  // namespace sb

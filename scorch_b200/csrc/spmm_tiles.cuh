@@ -371,7 +371,7 @@ static int launch_tiles(const SpmmArgs<T>& a, int64_t nnz, void* ws, cudaStream_
   // (may be set up while the tiles still run: it waits for them itself)
   SB_CUDA(launch_early(spmm_tile_rows_kernel<T>,
                        dim3((unsigned)ceil_div(a.m, kTileThreadsMm), (unsigned)std::min<int64_t>(ceil_div(a.k, 32), 64)),
-                       kTileThreadsMm, st, a, t));
+                       kTileThreadsMm, 0, st, a, t));
   return SB_OK;
 }
 
