@@ -232,34 +232,18 @@ __global__ void attn_flag_init_kernel(int* flag) { *flag = 1; }
 // partial dot products are summed across the group's lanes, and the row's running maximum, sum
 // and unnormalised output are updated once per pair.  Scores are in log2 units like the block
 // kernel's.  The trip count is the longest row of the warp; finished groups idle.
+// Rows of more than kLongScattered entries (global tokens) are put aside and taken by all lane groups
+// of the CTA together, a slice each, whose running results are merged in slice order: alone, a
+// group needed 215 us for one row of 950 entries (1000 tokens, 12 heads: the whole call was 226 us).
 constexpr int kScatWarps = 8;
+constexpr int kLongScattered = 64;
+// Entries [b, e) of a row's scattered list (may be empty; per lane group) into the group's running
+// maximum, sum and output sums.  K, V: at this lane's 8 features.
 template <int L>
-__global__ void __launch_bounds__(kScatWarps * 32, 4)
-attn_scattered_kernel(AttnArgs a) {
-  constexpr int G = 32 / L;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int g = lane / L, l = lane % L;
-  const int row = (blockIdx.x * kScatWarps + warp) * G + g;
-  if ((blockIdx.x * kScatWarps + warp) * G >= a.m) return;
-  const long long bz = blockIdx.y;
-  const float* K = a.K + bz * a.stride_k + 8 * l;
-  const float* V = a.V + bz * a.stride_v + 8 * l;
-  const float scale = a.scale * 1.4426950408889634f;
-  const float* mask_val = (a.mask_val && !__ldg(a.mask_is_ones)) ? a.mask_val : nullptr;
-  const bool live = row < a.m;
-  int b = 0, e = 0;
-  Float8 q;
-#pragma unroll
-  for (int i = 0; i < 8; i++) q.v[i] = 0.f;
-  if (live) {
-    b = __ldg(a.rem_pos + row);
-    e = __ldg(a.rem_pos + row + 1);
-    q = ldg8(a.Q + bz * a.stride_q + (size_t)((unsigned long long)(unsigned)row * a.ldq) + 8 * l);
-  }
+__device__ __forceinline__ void attn_scatter_range(const AttnArgs& a, const float* mask_val, const float* K,
+                                                   const float* V, const Float8& q, float scale, int b, int e, int l,
+                                                   float& M, float& Ls, float (&acc)[8]) {
   const int longest = __reduce_max_sync(FULL, e - b);
-  float M = -INFINITY, Ls = 0.f, acc[8];
-#pragma unroll
-  for (int i = 0; i < 8; i++) acc[i] = 0.f;
   // the group's next L entries: column and mask value, one per lane, a chunk ahead
   int next_j = 0;
   float next_w = 1.f;
@@ -317,11 +301,94 @@ attn_scattered_kernel(AttnArgs a) {
       for (int i = 0; i < 8; i++) acc[i] = fmaf(p1e, vv[1].v[i], fmaf(p0e, vv[0].v[i], acc[i] * alpha));
     }
   }
+}
+
+template <int L>
+__global__ void __launch_bounds__(kScatWarps * 32, 4)
+attn_scattered_kernel(AttnArgs a) {
+  constexpr int G = 32 / L;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int g = lane / L, l = lane % L;
+  __shared__ int s_n, s_long[kScatWarps * G];
+  __shared__ float s_m[kScatWarps], s_l[kScatWarps], s_acc[kScatWarps][8 * L];
+  if (threadIdx.x == 0) s_n = 0;
+  __syncthreads();
+  const int row = (blockIdx.x * kScatWarps + warp) * G + g;
+  const long long bz = blockIdx.y;
+  const float* K = a.K + bz * a.stride_k + 8 * l;
+  const float* V = a.V + bz * a.stride_v + 8 * l;
+  const float scale = a.scale * 1.4426950408889634f;
+  const float* mask_val = (a.mask_val && !__ldg(a.mask_is_ones)) ? a.mask_val : nullptr;
+  const bool live = row < a.m;
+  int b = 0, e = 0;
+  Float8 q;
+#pragma unroll
+  for (int i = 0; i < 8; i++) q.v[i] = 0.f;
   if (live) {
+    b = __ldg(a.rem_pos + row);
+    e = __ldg(a.rem_pos + row + 1);
+    q = ldg8(a.Q + bz * a.stride_q + (size_t)((unsigned long long)(unsigned)row * a.ldq) + 8 * l);
+  }
+  float M = -INFINITY, Ls = 0.f, acc[8];
+#pragma unroll
+  for (int i = 0; i < 8; i++) acc[i] = 0.f;
+  const bool is_long = e - b > kLongScattered;
+  if (is_long && l == 0) s_long[atomicAdd(&s_n, 1)] = row;
+  attn_scatter_range<L>(a, mask_val, K, V, q, scale, b, is_long ? b : e, l, M, Ls, acc);
+  if (live && !is_long) {
     float* orow = a.O + bz * a.stride_o + (long long)row * a.ldo + 8 * l;
     *reinterpret_cast<float4*>(orow) = make_float4(acc[0], acc[1], acc[2], acc[3]);
     *reinterpret_cast<float4*>(orow + 4) = make_float4(acc[4], acc[5], acc[6], acc[7]);
     if (l == 0) a.stats[bz * a.m + row] = make_float2(M, Ls);
+  }
+  __syncthreads();
+  const int n_long = s_n;
+  for (int i = 0; i < n_long; i++) {
+    const int r = s_long[i];
+    b = __ldg(a.rem_pos + r);
+    e = __ldg(a.rem_pos + r + 1);
+    const int slice = (e - b + kScatWarps * G - 1) / (kScatWarps * G);
+    const int sb_ = min(e, b + (warp * G + g) * slice), se = min(e, sb_ + slice);
+    q = ldg8(a.Q + bz * a.stride_q + (size_t)((unsigned long long)(unsigned)r * a.ldq) + 8 * l);
+    M = -INFINITY;
+    Ls = 0.f;
+#pragma unroll
+    for (int c = 0; c < 8; c++) acc[c] = 0.f;
+    attn_scatter_range<L>(a, mask_val, K, V, q, scale, sb_, se, l, M, Ls, acc);
+    // groups of the warp, then warps, each time (max, sum, output) of both sides at the larger max
+#pragma unroll
+    for (int o = L; o < 32; o <<= 1) {
+      const float m2 = __shfl_xor_sync(FULL, M, o), l2 = __shfl_xor_sync(FULL, Ls, o);
+      const float nm = fmaxf(M, m2), ms = (nm == -INFINITY) ? 0.f : nm;
+      const float f1 = attn_exp2(M - ms), f2 = attn_exp2(m2 - ms);
+      // (the side with the lower lanes first: the same sum on both)
+      const bool low = (lane & o) == 0;
+      Ls = low ? Ls * f1 + l2 * f2 : l2 * f2 + Ls * f1;
+#pragma unroll
+      for (int c = 0; c < 8; c++) acc[c] = acc[c] * f1 + __shfl_xor_sync(FULL, acc[c], o) * f2;
+      M = nm;
+    }
+    if (g == 0) {
+      if (l == 0) { s_m[warp] = M; s_l[warp] = Ls; }
+#pragma unroll
+      for (int c = 0; c < 8; c++) s_acc[warp][8 * l + c] = acc[c];
+    }
+    __syncthreads();
+    if (threadIdx.x < 8 * L) {
+      float nm = -INFINITY, sum = 0.f, out = 0.f;
+#pragma unroll
+      for (int w = 0; w < kScatWarps; w++) nm = fmaxf(nm, s_m[w]);
+      const float ms = (nm == -INFINITY) ? 0.f : nm;
+#pragma unroll
+      for (int w = 0; w < kScatWarps; w++) {
+        const float f = attn_exp2(s_m[w] - ms);
+        sum += s_l[w] * f;
+        out += s_acc[w][threadIdx.x] * f;
+      }
+      a.O[bz * a.stride_o + (long long)r * a.ldo + threadIdx.x] = out;
+      if (threadIdx.x == 0) a.stats[bz * a.m + r] = make_float2(nm, sum);
+    }
+    __syncthreads();
   }
 }
 

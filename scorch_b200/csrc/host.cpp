@@ -32,6 +32,9 @@ struct Abi {
   decltype(&sb_spmv_csr_typed) spmv_typed;
   decltype(&sb_sddmm_coo_f32) sddmm_coo;
   decltype(&sb_sddmm_csr_f32) sddmm_csr;
+  decltype(&sb_sparse_attention_scratch_bytes) attention_bytes;
+  decltype(&sb_sparse_attention_csr_f32) attention_csr;
+  decltype(&sb_sparse_attention_band_f32) attention_band;
   decltype(&sb_spgemm_workspace_bytes) spgemm_bytes;
   decltype(&sb_spgemm_begin) spgemm_begin;
   decltype(&sb_spgemm_rows) spgemm_rows;
@@ -162,6 +165,9 @@ PyObject* py_bind(PyObject*, PyObject* args) {
   find(abi.spmv_typed, "sb_spmv_csr_typed");
   find(abi.sddmm_coo, "sb_sddmm_coo_f32");
   find(abi.sddmm_csr, "sb_sddmm_csr_f32");
+  find(abi.attention_bytes, "sb_sparse_attention_scratch_bytes");
+  find(abi.attention_csr, "sb_sparse_attention_csr_f32");
+  find(abi.attention_band, "sb_sparse_attention_band_f32");
   find(abi.spgemm_bytes, "sb_spgemm_workspace_bytes");
   find(abi.spgemm_begin, "sb_spgemm_begin");
   find(abi.spgemm_rows, "sb_spgemm_rows");
@@ -246,6 +252,47 @@ PyObject* py_sddmm(PyObject*, PyObject* const* a, Py_ssize_t count) {
   });
 }
 
+// attention(pos, crd, mask_val | None, Q, K, V, scale, plan buffer, plan rows, plan columns, blocks | -1
+// (band plan), entries outside) -> O or None
+PyObject* py_attention(PyObject*, PyObject* const* a, Py_ssize_t count) {
+  return guarded([&]() -> PyObject* {
+    if (count != 12) Py_RETURN_NONE;
+    const at::Tensor *pos = tensor(a[0]), *crd = tensor(a[1]), *Q = tensor(a[3]), *K = tensor(a[4]), *V = tensor(a[5]),
+                     *plan = tensor(a[7]);
+    const at::Tensor* val = a[2] == Py_None ? nullptr : tensor(a[2]);
+    if (!pos || !crd || !Q || !K || !V || !plan || (a[2] != Py_None && !val)) Py_RETURN_NONE;
+    const double scale = PyFloat_AsDouble(a[6]);
+    const long long pm = PyLong_AsLongLong(a[8]), pn = PyLong_AsLongLong(a[9]), blocks = PyLong_AsLongLong(a[10]),
+                    rem = PyLong_AsLongLong(a[11]);
+    if (PyErr_Occurred()) return nullptr;
+    if (!indices(*pos) || !indices(*crd) || (val && (!plain(*val, at::kFloat) || val->numel() != crd->numel())) ||
+        !plain(*Q, at::kFloat) || !plain(*K, at::kFloat) || !plain(*V, at::kFloat) || Q->dim() < 2 || Q->dim() > 3 ||
+        K->dim() != Q->dim() || K->sizes() != V->sizes() || checking())
+      Py_RETURN_NONE;
+    const bool batched = Q->dim() == 3;
+    const int64_t m = Q->size(-2), d = Q->size(-1), n = K->size(-2), nnz = crd->numel(), batch = batched ? Q->size(0) : 1;
+    if (pos->numel() != m + 1 || pm != m || pn != n || K->size(-1) != d || (batched && K->size(0) != batch) ||
+        (blocks < 0 ? d != 64 : (d != 32 && d != 64)))
+      Py_RETURN_NONE;
+    const c10::cuda::CUDAGuard device(Q->device());
+    at::Tensor out = at::empty(Q->sizes(), Q->options());
+    const size_t bytes = abi.attention_bytes(m, rem, batch);
+    at::Tensor ws = workspace(bytes, out);
+    const int *p = pos->const_data_ptr<int>(), *c = crd->const_data_ptr<int>();
+    const float *w = val ? val->const_data_ptr<float>() : nullptr, *q = Q->const_data_ptr<float>(),
+                *k = K->const_data_ptr<float>(), *v = V->const_data_ptr<float>();
+    const int rc =
+        blocks < 0
+            ? abi.attention_band(m, n, d, nnz, p, c, w, q, d, k, d, v, d, (float)scale, out.data_ptr<float>(), d, batch,
+                                 m * d, n * d, n * d, m * d, plan->const_data_ptr(), rem, ws.data_ptr(), bytes,
+                                 SB_ATTN_ALL_STAGES, stream_of(*Q))
+            : abi.attention_csr(m, n, d, nnz, p, c, w, q, d, k, d, v, d, (float)scale, out.data_ptr<float>(), d, batch,
+                                m * d, n * d, n * d, m * d, plan->const_data_ptr(), blocks, rem, ws.data_ptr(), bytes,
+                                SB_ATTN_ALL_STAGES, stream_of(*Q));
+    return rc == SB_OK ? THPVariable_Wrap(std::move(out)) : fail(rc);
+  });
+}
+
 // spgemm(Apos, Acrd, Aval, Bpos, Bcrd, Bval, n) -> (Cpos, Ccrd, Cval), or None: not in the plain
 // form, or more products than the one-pass form has memory for
 constexpr int64_t kOnePassBytes = (int64_t)16 << 30;
@@ -320,6 +367,8 @@ PyMethodDef methods[] = {
      "matmul_csr(A, B) for a torch CSR tensor A -> tensor, or None for the general path"},
     {"sddmm", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_sddmm)), METH_FASTCALL,
      "sddmm(row_or_pos, col, mask_val, Q, K, csr) -> tensor(s), or None for the general path"},
+    {"attention", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_attention)), METH_FASTCALL,
+     "attention(pos, crd, mask_val, Q, K, V, scale, plan, m, n, blocks, rem) -> tensor, or None for the general path"},
     {"spgemm", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_spgemm)), METH_FASTCALL,
      "spgemm(Apos, Acrd, Aval, Bpos, Bcrd, Bval, n) -> (Cpos, Ccrd, Cval), or None for the two-phase path"},
     {nullptr, nullptr, 0, nullptr}};

@@ -11,6 +11,8 @@
 // written back as one coalesced line per chunk.
 #include <math.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 
 // 128-bit K-row loads gathered together per lane (4 measured best on B200: 8 costs occupancy)
@@ -306,6 +308,146 @@ sddmm_kernel(SddmmArgs a) {
   }
 }
 
+// d = 8 G (32, 64, 128, 256) with 32-byte aligned rows: the form of the span kernel with one 256-bit
+// load per lane and entry.  Every warp takes the same number of consecutive 32-entry chunks and all
+// warps are resident at once, so there is no part-filled last wave (4663 warps of 8 chunks on 3552
+// slots took two full ones); kAhead K rows per lane group are in flight (four loads of 256 bits for
+// four entries instead of four of 128 for two).
+// Bound: L2 -> SM gathers of K rows, less what L1 keeps of a band.  1.19 M entries, d = 64: 48 us
+// before, NEWUS us.
+constexpr int kAhead = 4;
+
+struct Row8 { float v[8]; };
+__device__ __forceinline__ Row8 ld_row8(const float* p) {
+  Row8 r;
+  asm volatile("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=f"(r.v[0]), "=f"(r.v[1]), "=f"(r.v[2]), "=f"(r.v[3]), "=f"(r.v[4]), "=f"(r.v[5]),
+                 "=f"(r.v[6]), "=f"(r.v[7])
+               : "l"(p));
+  return r;
+}
+__device__ __forceinline__ float dot8(const Row8& a, const Row8& b) {
+  float s = 0.f, t = 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; i += 2) {
+    s = fmaf(a.v[i], b.v[i], s);
+    t = fmaf(a.v[i + 1], b.v[i + 1], t);
+  }
+  return s + t;
+}
+
+// Row of entry p (largest r in [lo, hi) with pos[r] <= p), the warp together: 32-fold per round.
+__device__ __forceinline__ int warp_row_of_entry(const int* __restrict__ pos, int lo, int hi, int p, int lane) {
+  while (hi - lo > 1) {
+    const int step = (hi - lo + 31) / 32;
+    const long long r = (long long)lo + (long long)lane * step;
+    const unsigned le = __ballot_sync(FULL, r < hi && __ldg(pos + r) <= p);
+    lo += (__popc(le) - 1) * step;
+    hi = min(hi, lo + step);
+  }
+  return lo;
+}
+
+template <int G>
+__global__ void __launch_bounds__(kSddmmWarps * 32, 4)
+sddmm_rows8_kernel(SddmmArgs a, int chunks_per_warp) {
+  constexpr int U = G < kAhead ? G : kAhead;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int l = lane % G, g0 = (lane / G) * G;
+  const long long first = ((long long)blockIdx.x * kSddmmWarps + warp) * chunks_per_warp * 32;
+  if (first >= a.nnz) return;
+  const int p_end = (int)min(a.nnz, first + (long long)chunks_per_warp * 32);
+  const long long bz = blockIdx.y;
+  const float* Q = a.Q + bz * a.stride_q + l * 8;
+  const float* K = a.K + bz * a.stride_k + l * 8;
+  float* out = a.out_val + bz * a.stride_out;
+  const unsigned ldq = (unsigned)a.ldq, ldk = (unsigned)a.ldk;
+  int next_j = 0, next_i = 0;
+  float next_s = 1.f;
+  auto fetch = [&](int p) {
+    if (p < p_end) {
+      next_j = ld_stream(a.crd + p);
+      if (a.mask_val) next_s = ld_stream(a.mask_val + p);
+      if (a.row) next_i = ld_stream(a.row + p);
+    }
+  };
+  int p0 = (int)first;
+  fetch(p0 + lane);
+  int r0 = a.pos ? warp_row_of_entry(a.pos, 0, a.m, p0, lane) : 0, q_row = -1;
+  Row8 q;
+#pragma unroll
+  for (int i = 0; i < 8; i++) q.v[i] = 0.f;
+#pragma unroll 1
+  for (; p0 < p_end; p0 += 32) {
+    const int cnt = min(32, p_end - p0);
+    const int my_j = next_j;
+    int my_i = next_i;
+    const float my_s = next_s;
+    fetch(p0 + 32 + lane);
+    bool one_row;                                  // warp-uniform
+    if (a.pos) {
+      r0 = advance_row(a.pos, a.m, r0, p0);
+      one_row = __ldg(a.pos + r0 + 1) >= p0 + cnt;
+      my_i = one_row ? r0 : row_of_entry(a.pos, r0, a.m, p0 + min(lane, cnt - 1));
+    } else {
+      r0 = __shfl_sync(FULL, my_i, 0);
+      one_row = __all_sync(FULL, lane >= cnt || my_i == r0);
+    }
+    if (bz == 0 && lane < cnt) {
+      if (a.out_row) a.out_row[p0 + lane] = my_i;
+      if (a.out_col) a.out_col[p0 + lane] = my_j;
+    }
+    float part[G];
+    if (one_row) {
+      if (r0 != q_row) {
+        q_row = r0;
+        q = ld_row8(Q + (size_t)((unsigned long long)(unsigned)r0 * ldq));
+      }
+#pragma unroll
+      for (int t0 = 0; t0 < G; t0 += U) {
+        Row8 k[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+          // (lanes past the end repeat entry 0: the result is dropped)
+          const unsigned j = (unsigned)__shfl_sync(FULL, my_j, g0 + t0 + u < cnt ? g0 + t0 + u : 0);
+          k[u] = ld_row8(K + (size_t)((unsigned long long)j * ldk));
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) part[t0 + u] = dot8(q, k[u]);
+      }
+    } else {
+      q_row = -1;
+#pragma unroll
+      for (int t0 = 0; t0 < G; t0 += 2) {
+        Row8 k[2], qq[2];
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+          const int idx = g0 + t0 + u < cnt ? g0 + t0 + u : 0;
+          const unsigned j = (unsigned)__shfl_sync(FULL, my_j, idx), i = (unsigned)__shfl_sync(FULL, my_i, idx);
+          k[u] = ld_row8(K + (size_t)((unsigned long long)j * ldk));
+          qq[u] = ld_row8(Q + (size_t)((unsigned long long)i * ldq));
+        }
+#pragma unroll
+        for (int u = 0; u < 2; u++) part[t0 + u] = dot8(qq[u], k[u]);
+      }
+    }
+    transpose_reduce<G>(part, lane);
+    if (lane < cnt) out[p0 + lane] = my_s * part[0];
+  }
+}
+
+template <int G>
+static int launch_rows8(const SddmmArgs& a, int64_t batch, cudaStream_t st) {
+  const int64_t chunks = ceil_div(a.nnz, 32);
+  // one wave over all batch items: 4 CTAs of 8 warps per SM
+  const int64_t slots = std::max<int64_t>(1, (int64_t)sm_count() * 4 * kSddmmWarps / batch);
+  const int per = (int)std::min<int64_t>(64, ceil_div(chunks, slots));
+  dim3 grid((unsigned)ceil_div(chunks, (int64_t)per * kSddmmWarps), (unsigned)batch);
+  sddmm_rows8_kernel<G><<<grid, kSddmmWarps * 32, 0, st>>>(a, per);
+  SB_LAUNCH_CHECK("sddmm_rows8_kernel");
+  return SB_OK;
+}
+
 // Any d / any alignment: one lane per entry, scalar loop over d.
 __global__ void sddmm_generic_kernel(SddmmArgs a) {
   const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -351,6 +493,14 @@ static int sddmm_dispatch(SddmmArgs a, int64_t batch, cudaStream_t st) {
     sddmm_generic_kernel<<<grid, 256, 0, st>>>(a);
     SB_LAUNCH_CHECK("sddmm_generic_kernel");
     return SB_OK;
+  }
+  const unsigned long long bits = (unsigned long long)reinterpret_cast<uintptr_t>(a.Q) | reinterpret_cast<uintptr_t>(a.K) |
+                                  4ull * (unsigned long long)(a.ldq | a.ldk | a.stride_q | a.stride_k);
+  if (!a.rowwise && !a.ent && !a.out_compact && (bits & 31) == 0) {
+    if (a.d == 32) return launch_rows8<4>(a, batch, st);
+    if (a.d == 64) return launch_rows8<8>(a, batch, st);
+    if (a.d == 128) return launch_rows8<16>(a, batch, st);
+    if (a.d == 256) return launch_rows8<32>(a, batch, st);
   }
   // G lanes share one dot product, each holding VEC float4 of the Q row (G*VEC*4 >= d); G
   // adjacent lanes read G*16 contiguous bytes of a K row, i.e. whole 128-byte lines for d >= 32.

@@ -282,6 +282,13 @@ def sparse_attention_csr(pos, crd, mask_val, Q, Kmat, V, scale: float = 1.0,
     a band on tcgen05, d = 64); default: the block plan.
     ``stages``: 3 = the whole call; 1, 2 = its two kernels one by one (scattered entries, then
     blocks / tiles; same arguments and ``out``), for callers that time them."""
+    if out is None and stages == 3 and attn_plan is not None and attn_plan.nnz == crd.numel() and (
+            mask_val is None or (mask_val.is_cuda and mask_val.dtype == torch.float32)):
+        r = _lib.host().attention(pos, crd, None if mask_val is None or _mask_is_all_ones(mask_val) else mask_val,
+                                  Q, Kmat, V, scale, attn_plan.buf, attn_plan.m, attn_plan.n,
+                                  -1 if isinstance(attn_plan, AttnBandPlan) else attn_plan.blocks, attn_plan.rem_nnz)
+        if r is not None:
+            return r
     pos = _dev(pos, torch.int32, "pos")
     crd = _dev(crd, torch.int32, "crd")
     m, nnz = pos.numel() - 1, crd.numel()
