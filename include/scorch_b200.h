@@ -169,6 +169,13 @@ SB_API int sb_spmv_csr_typed(int dtype, int64_t m, int64_t n, int64_t nnz, const
                              const int32_t* crd, const void* val, const void* x, void* y,
                              void* stream);
 
+/* The tiled form for every SB_* dtype (sb_spmv_csr_f32 is its SB_F32), with
+ * sb_spmv_csr_tiled_scratch_bytes(dtype, nnz) bytes of 16-byte aligned scratch. */
+SB_API size_t sb_spmv_csr_tiled_scratch_bytes(int dtype, int64_t nnz);
+SB_API int sb_spmv_csr_tiled(int dtype, int64_t m, int64_t n, int64_t nnz, const int32_t* pos,
+                             const int32_t* crd, const void* val, const void* x, void* y,
+                             void* scratch, size_t scratch_bytes, void* stream);
+
 /* SpMV that allocates nothing and asks the caller for no workspace.  (No counterpart in the
  * reference: its kernels malloc freely on the host.)  For callers that cannot call cudaMalloc —
  * a plugin living inside another runtime's device-memory arena, or a service that must not touch

@@ -45,6 +45,8 @@ SIGNATURES = {
     "sb_spmv_csr_scratch_bytes": (_sz, [_i64]),
     "sb_spmv_csr_f32": (_int, [_i64, _i64, _i64, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _sz, _ptr]),
     "sb_spmv_csr_typed": (_int, [_int, _i64, _i64, _i64, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr]),
+    "sb_spmv_csr_tiled_scratch_bytes": (_sz, [_int, _i64]),
+    "sb_spmv_csr_tiled": (_int, [_int, _i64, _i64, _i64, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _sz, _ptr]),
     "sb_spmv_csr_f32_static": (_int, [_i64, _i64, _i64, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr]),
     "sb_sddmm_csr_f32": (_int, [_i64, _i64, _i64, _i64, _ptr, _ptr, _ptr, _ptr, _i64, _ptr, _i64,
                                 _ptr, _ptr, _ptr, _i64, _i64, _i64, _i64, _ptr]),

@@ -27,9 +27,8 @@ struct Abi {
   decltype(&sb_spmm_csr_once_workspace_bytes) spmm_once_bytes;
   decltype(&sb_spmm_csr_once) spmm_once;
   decltype(&sb_spmm_wide_select) spmm_wide_select;
-  decltype(&sb_spmv_csr_scratch_bytes) spmv_bytes;
-  decltype(&sb_spmv_csr_f32) spmv_f32;
-  decltype(&sb_spmv_csr_typed) spmv_typed;
+  decltype(&sb_spmv_csr_tiled_scratch_bytes) spmv_bytes;
+  decltype(&sb_spmv_csr_tiled) spmv;
   decltype(&sb_sddmm_coo_f32) sddmm_coo;
   decltype(&sb_sddmm_csr_f32) sddmm_csr;
   decltype(&sb_sparse_attention_scratch_bytes) attention_bytes;
@@ -129,17 +128,10 @@ PyObject* spmv(const at::Tensor& pos, const at::Tensor& crd, const at::Tensor& v
   const int64_t m = pos.numel() - 1, nnz = crd.numel();
   const c10::cuda::CUDAGuard device(x.device());
   at::Tensor y = at::empty({m}, val.options());
-  int rc;
-  if (code == SB_F32) {
-    const size_t bytes = abi.spmv_bytes(nnz);
-    at::Tensor ws = workspace(bytes, y);
-    rc = abi.spmv_f32(m, x.numel(), nnz, pos.const_data_ptr<int>(), crd.const_data_ptr<int>(),
-                      val.const_data_ptr<float>(), x.const_data_ptr<float>(), y.data_ptr<float>(), ws.data_ptr(),
-                      bytes, stream_of(x));
-  } else {
-    rc = abi.spmv_typed(code, m, x.numel(), nnz, pos.const_data_ptr<int>(), crd.const_data_ptr<int>(),
-                        val.const_data_ptr(), x.const_data_ptr(), y.data_ptr(), stream_of(x));
-  }
+  const size_t bytes = abi.spmv_bytes(code, nnz);
+  at::Tensor ws = workspace(bytes, y);
+  const int rc = abi.spmv(code, m, x.numel(), nnz, pos.const_data_ptr<int>(), crd.const_data_ptr<int>(),
+                          val.const_data_ptr(), x.const_data_ptr(), y.data_ptr(), ws.data_ptr(), bytes, stream_of(x));
   return rc == SB_OK ? THPVariable_Wrap(std::move(y)) : fail(rc);
 }
 
@@ -160,9 +152,8 @@ PyObject* py_bind(PyObject*, PyObject* args) {
   find(abi.spmm_once_bytes, "sb_spmm_csr_once_workspace_bytes");
   find(abi.spmm_once, "sb_spmm_csr_once");
   find(abi.spmm_wide_select, "sb_spmm_wide_select");
-  find(abi.spmv_bytes, "sb_spmv_csr_scratch_bytes");
-  find(abi.spmv_f32, "sb_spmv_csr_f32");
-  find(abi.spmv_typed, "sb_spmv_csr_typed");
+  find(abi.spmv_bytes, "sb_spmv_csr_tiled_scratch_bytes");
+  find(abi.spmv, "sb_spmv_csr_tiled");
   find(abi.sddmm_coo, "sb_sddmm_coo_f32");
   find(abi.sddmm_csr, "sb_sddmm_csr_f32");
   find(abi.attention_bytes, "sb_sparse_attention_scratch_bytes");

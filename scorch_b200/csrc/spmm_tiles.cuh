@@ -69,7 +69,7 @@ struct alignas(sizeof(T) == 4 ? 8 : 16) Entry {
 };
 
 struct TileUnit {
-  int row, begin, len;
+  int row, begin, len, whole;   // whole: the row has no other unit
 };
 
 template <typename T, int L, int VEC, int W>
@@ -95,15 +95,21 @@ __device__ __forceinline__ void tile_store_row(const SpmmArgs<T>& a, int row, in
 #pragma unroll
   for (int v = 0; v < VEC; v++) {
     const int col = col0 + v * L * W;
-    if (!col_ok[v]) continue;
-    Pack<T, W> s = sum[v];
-    if (a.accumulate) {
-      const Pack<T, W> old = ld_l2<T, W>(crow + col);
-#pragma unroll
-      for (int w = 0; w < W; w++) s.v[w] += old.v[w];
-    }
-    st_stream<T, W>(crow + col, epilogue<T, W>(s, a.bias, col, a.relu));
+    if (col_ok[v]) st_stream<T, W>(crow + col, epilogue<T, W>(sum[v], a.bias, col, a.relu));
   }
+}
+
+// Initial sums of the lane group that will store the row: zero, or the row's present contents
+// (accumulation), loaded here so that they arrive with the first gathers.
+template <typename T, int L, int VEC, int W>
+__device__ __forceinline__ void tile_begin_row(Pack<T, W> (&s)[VEC], const SpmmArgs<T>& a, int row, int col0,
+                                               const bool (&col_ok)[VEC], bool owner) {
+  zero_acc<T, VEC, W>(s);
+  if (!a.accumulate || !owner) return;
+  const T* crow = a.C + (long long)row * a.ldc;
+#pragma unroll
+  for (int v = 0; v < VEC; v++)
+    if (col_ok[v]) s[v] = ld_l2<T, W>(crow + col0 + v * L * W);
 }
 
 // acc += the entries [b, e) of the window, one after the other, U operand rows in flight.  Lanes
@@ -197,13 +203,13 @@ spmm_tile_kernel(SpmmArgs<T> a, TileArgs<T> t) {
       rows += here;
       if (!here || len <= kGroupRow<L>) continue;
       if (len <= kWarpRow) {
-        if (b >= next) sm.by_warp[atomicAdd(&sm.n_warp, 1)] = TileUnit{r0 + i, b, len};
+        if (b >= next) sm.by_warp[atomicAdd(&sm.n_warp, 1)] = TileUnit{r0 + i, b, len, 1};
       } else {
         // (first unit at or behind the window's start; a row that began before a later turn's first
         // entry was dealt with by the turn before)
         int u = b >= next ? 0 : (next == e0 ? (e0 - b + kUnit - 1) / kUnit : INT32_MAX / kUnit);
         for (; u < (len + kUnit - 1) / kUnit && b + u * kUnit < e1; u++)
-          sm.by_cta[atomicAdd(&sm.n_cta, 1)] = TileUnit{r0 + i, b + u * kUnit, min(kUnit, len - u * kUnit)};
+          sm.by_cta[atomicAdd(&sm.n_cta, 1)] = TileUnit{r0 + i, b + u * kUnit, min(kUnit, len - u * kUnit), len <= kUnit};
       }
     }
     rows = __reduce_add_sync(FULL, rows);
@@ -229,7 +235,8 @@ spmm_tile_kernel(SpmmArgs<T> a, TileArgs<T> t) {
       const int slice = (q.len + NG - 1) / NG, w0 = min(q.len, (warp * G + g) * slice);
       const int b = q.begin - e0 + w0;
       Pack<T, W> s[VEC];
-      zero_acc<T, VEC, W>(s);
+      // (a row of several units gets its present contents from the kernel that adds the units)
+      tile_begin_row<T, L, VEC, W>(s, a, q.row, col0, col_ok, warp == 0 && lane < L && q.whole);
       tile_add<T, VEC, W, U>(s, sm.entry, b, b + min(slice, q.len - w0), Bcol, pitch);
       reduce_groups<T, L, VEC, W>(s);
       if (lane < L) {
@@ -248,11 +255,10 @@ spmm_tile_kernel(SpmmArgs<T> a, TileArgs<T> t) {
             for (int w = 0; w < W; w++) s[v].v[w] += x.v[w];
           }
         }
-        const int rb = __ldg(a.pos + q.row);
-        if (__ldg(a.pos + q.row + 1) - rb <= kUnit) {
+        if (q.whole) {
           tile_store_row<T, L, VEC, W>(a, q.row, col0, col_ok, s);
         } else {
-          T* dst = (q.begin == rb ? t.first : t.rest) + (long long)(q.begin / kUnit) * a.k + col0;
+          T* dst = (q.begin == __ldg(a.pos + q.row) ? t.first : t.rest) + (long long)(q.begin / kUnit) * a.k + col0;
 #pragma unroll
           for (int v = 0; v < VEC; v++)
             if (col_ok[v]) store_plain<T, W>(dst + v * L * W, s[v]);
@@ -270,7 +276,7 @@ spmm_tile_kernel(SpmmArgs<T> a, TileArgs<T> t) {
       const int slice = (q.len + G - 1) / G, w0 = min(q.len, g * slice);
       const int b = q.begin - e0 + w0;
       Pack<T, W> s[VEC];
-      zero_acc<T, VEC, W>(s);
+      tile_begin_row<T, L, VEC, W>(s, a, q.row, col0, col_ok, lane < L);
       tile_add<T, VEC, W, U>(s, sm.entry, b, b + min(slice, q.len - w0), Bcol, pitch);
       reduce_groups<T, L, VEC, W>(s);
       if (lane < L) tile_store_row<T, L, VEC, W>(a, q.row, col0, col_ok, s);
@@ -285,7 +291,7 @@ spmm_tile_kernel(SpmmArgs<T> a, TileArgs<T> t) {
       const int b = sm.pos[i < rows ? i : 0], len = i < rows ? sm.pos[i + 1] - b : 0;
       if (b < next || len == 0 || len > kGroupRow<L>) continue;
       Pack<T, W> s[VEC];
-      zero_acc<T, VEC, W>(s);
+      tile_begin_row<T, L, VEC, W>(s, a, r0 + i, col0, col_ok, true);
       tile_add<T, VEC, W, U>(s, sm.entry, b - e0, b - e0 + len, Bcol, pitch);
       tile_store_row<T, L, VEC, W>(a, r0 + i, col0, col_ok, s);
     }

@@ -1,9 +1,9 @@
 // CSR SpMV for sm_100a.
 //
-// fp32: entry-tiled kernel (below), balanced by stored entries.  x is gathered through the
+// Entry-tiled kernel (below), balanced by stored entries.  x is gathered through the
 // read-only path (it is L2 resident: 8 MB for 2M columns); the CSR streams are read once with
-// no-allocate loads.  The other registry dtypes (f64 / i32 / i64) use a plain G-lanes-per-row
-// kernel (G chosen from the mean row length).
+// no-allocate loads.  The entry point without scratch (sb_spmv_csr_typed) uses a plain
+// G-lanes-per-row kernel (G chosen from the mean row length).
 #include "common.cuh"
 
 namespace sb {
@@ -33,60 +33,69 @@ spmv_rows_kernel(int m, const int* __restrict__ pos, const int* __restrict__ crd
   if (write && l == 0) y[row] = acc;
 }
 
-// ---- fp32: entry-tiled kernel ------------------------------------------------------------------
+// ---- entry-tiled kernel --------------------------------------------------------------------------
 // The entry arrays are cut into tiles of kTile consecutive entries, one CTA per tile, whatever
-// the row lengths are (power-law rows included: a hub row simply spans many tiles).  A tile
-//   1. finds its first and last row with a 256-ary search over pos[] (3 rounds for 2M rows),
-//   2. streams its crd/val slices with 8 independent loads per thread, gathers x and leaves the
+// the row lengths are (power-law rows included: a hub row simply spans many tiles).  A first, small
+// kernel notes the row of every tile's first entry.  A tile
+//   1. streams its crd/val slices with 8 independent loads per thread, gathers x and leaves the
 //      products in shared memory,
-//   3. sums each row's segment (one thread per row for short rows, one warp per row for long
-//      ones) and writes y for rows that lie completely inside the tile.
-// A row cut by a tile border leaves partial sums in the scratch arrays; a second, tiny kernel
-// adds them in tile order, so the result does not depend on scheduling.
+//   2. sums each row's segment (one thread per row for short rows, one warp per row for long
+//      ones) and writes y for rows that lie completely inside the tile, empty ones included.
+// A row cut by a tile border leaves partial sums in the scratch arrays; a third kernel adds them in
+// tile order, so the result does not depend on scheduling.
+// Bound: the gather of x, one L1 tag look-up per entry and clock and SM (288 G entries/s measured for
+// random 4-byte loads: 83 us for the 23.8 M entries of a 2 M-row power-law matrix).  A search for the
+// rows in every tile, 256 scattered loads a round, took nearly as many look-ups as the gather: 174 us;
+// NEWUS us with the rows noted beforehand.
 constexpr int kTile = 2048;
 constexpr int kTileThreads = 256;
 
+template <typename T>
 struct TileScratch {
-  float* carry_first;  // partial sum of the tile's first row when that row began in an earlier tile
-  float* carry_last;   // partial sum of the tile's last row when it began here and continues
-  int* last_row;       // that last row, or -1
+  T* carry_first;   // partial sum of the tile's first row when that row began in an earlier tile
+  T* carry_last;    // partial sum of the tile's last row when it began here and continues
+  int* row;         // row of the tile's first entry (0 for the first tile)
 };
 
-// Largest r in [lo, hi) with pos[r] <= p, given pos[lo] <= p < pos[hi]; all threads of the CTA
-// call it together and get the same answer.
-__device__ __forceinline__ int find_row_cta(const int* __restrict__ pos, int lo, int hi, int p) {
-  const int tid = threadIdx.x;
-  while (true) {
-    const int span = hi - lo;
-    if (span <= kTileThreads) {
-      const int r = lo + tid;
-      const int c = __syncthreads_count(r < hi && __ldg(pos + r) <= p);
-      return lo + c - 1;
-    }
-    const int step = (span + kTileThreads - 1) / kTileThreads;
-    const long long r = (long long)lo + (long long)tid * step;
-    const int c = __syncthreads_count(r < hi && __ldg(pos + r) <= p);
-    lo = lo + (c - 1) * step;
-    hi = min(hi, lo + step);
-  }
+// (rows that end behind a tile's start and begin at or before it)
+__global__ void __launch_bounds__(256)
+spmv_tile_rows_kernel(int m, int tiles, const int* __restrict__ pos, int* __restrict__ row) {
+  const long long r = (long long)blockIdx.x * 256 + threadIdx.x;
+  if (r >= m) return;
+  const int b = __ldg(pos + r), e = __ldg(pos + r + 1);
+  if (r == 0) row[0] = 0;
+  for (int t = (b + kTile - 1) / kTile; t < tiles && (long long)t * kTile < e; t++)
+    if (t > 0) row[t] = (int)r;
 }
 
+__device__ __forceinline__ double ld_stream(const double* p) {
+  double v;
+  asm volatile("ld.global.nc.L1::no_allocate.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ unsigned ld_stream(const unsigned* p) {
+  return (unsigned)ld_stream(reinterpret_cast<const int*>(p));
+}
+__device__ __forceinline__ unsigned long long ld_stream(const unsigned long long* p) {
+  return (unsigned long long)__double_as_longlong(ld_stream(reinterpret_cast<const double*>(p)));
+}
+
+template <typename T>
 __global__ void __launch_bounds__(kTileThreads)
-spmv_tile_kernel(int m, int nnz, const int* __restrict__ pos, const int* __restrict__ crd,
-                 const float* __restrict__ val, const float* __restrict__ x, float* __restrict__ y,
-                 TileScratch sc) {
-  __shared__ float prod[kTile];
+spmv_tile_kernel(int m, int nnz, int tiles, const int* __restrict__ pos, const int* __restrict__ crd,
+                 const T* __restrict__ val, const T* __restrict__ x, T* __restrict__ y, TileScratch<T> sc) {
+  __shared__ T prod[kTile];
   const int t = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int e0 = t * kTile, e1 = min(nnz, e0 + kTile);
-  // products first: the loads are independent of the row search below
+  // products first: they do not need the rows
   {
     int j[kTile / kTileThreads];
-    float a[kTile / kTileThreads];
+    T a[kTile / kTileThreads];
 #pragma unroll
     for (int q = 0; q < kTile / kTileThreads; q++) {
       const int e = e0 + tid + q * kTileThreads;
       j[q] = 0;
-      a[q] = 0.f;
+      a[q] = T(0);
       if (e < e1) {
         j[q] = ld_stream(crd + e);
         a[q] = ld_stream(val + e);
@@ -95,11 +104,11 @@ spmv_tile_kernel(int m, int nnz, const int* __restrict__ pos, const int* __restr
 #pragma unroll
     for (int q = 0; q < kTile / kTileThreads; q++) {
       const int e = e0 + tid + q * kTileThreads;
-      prod[tid + q * kTileThreads] = (e < e1) ? a[q] * __ldg(x + j[q]) : 0.f;
+      prod[tid + q * kTileThreads] = (e < e1) ? a[q] * __ldg(x + j[q]) : T(0);
     }
   }
-  const int r_lo = find_row_cta(pos, 0, m, e0);
-  const int r_hi = find_row_cta(pos, r_lo, m, e1 - 1);
+  asm volatile("griddepcontrol.wait;" ::: "memory");   // the tiles' rows
+  const int r_lo = sc.row[t], r_hi = t + 1 < tiles ? sc.row[t + 1] : m - 1;
   __syncthreads();
   const int nr = r_hi - r_lo + 1;
   const bool thread_per_row = nr >= 128;
@@ -107,13 +116,15 @@ spmv_tile_kernel(int m, int nnz, const int* __restrict__ pos, const int* __restr
   const int stride = thread_per_row ? kTileThreads : kTileThreads / 32;
   for (int r = r_lo + first; r <= r_hi; r += stride) {
     const int rb = __ldg(pos + r), re = __ldg(pos + r + 1);
+    if (r == r_hi && rb >= e1 && t + 1 < tiles) continue;   // (begins with the next tile)
     const int b = max(rb, e0) - e0, e = min(re, e1) - e0;
-    float s = 0.f;
+    T s = T(0);
     if (thread_per_row) {
       for (int i = b; i < e; i++) s += prod[i];
     } else {
       for (int i = b + lane; i < e; i += 32) s += prod[i];
-      s = group_sum<32>(s);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(FULL, s, o);
       if (lane != 0) continue;
     }
     if (rb >= e0 && re <= e1) {
@@ -124,26 +135,40 @@ spmv_tile_kernel(int m, int nnz, const int* __restrict__ pos, const int* __restr
       sc.carry_last[t] = s;              // begins here, continues in the next tile
     }
   }
-  if (tid == 0) {
-    const int rb = __ldg(pos + r_hi), re = __ldg(pos + r_hi + 1);
-    sc.last_row[t] = (re > e1 && rb >= e0) ? r_hi : -1;
-  }
 }
 
 // Adds the pieces of every row that was cut by tile borders, in tile order.
-__global__ void spmv_tile_fixup_kernel(int ntiles, const int* __restrict__ pos, float* __restrict__ y,
-                                       TileScratch sc) {
+template <typename T>
+__global__ void spmv_tile_fixup_kernel(int ntiles, const int* __restrict__ pos, T* __restrict__ y, TileScratch<T> sc) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= ntiles) return;
-  const int r = sc.last_row[t];
-  if (r < 0) return;
-  const long long row_end = pos[r + 1];
-  float s = sc.carry_last[t];
-  for (int u = t + 1; u < ntiles; u++) {
-    s += sc.carry_first[u];
-    if (row_end <= (long long)(u + 1) * kTile) break;
-  }
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (t + 1 >= ntiles) return;
+  // the row that the next tile begins with, if it began in this tile
+  const int r = sc.row[t + 1];
+  const int rb = __ldg(pos + r), re = __ldg(pos + r + 1);
+  if (rb >= (t + 1) * kTile || rb < t * kTile) return;
+  T s = sc.carry_last[t];
+  const int last = (re - 1) / kTile;
+#pragma unroll 8
+  for (int u = t + 1; u <= last; u++) s += sc.carry_first[u];
   y[r] = s;
+}
+
+template <typename T>
+static int launch_tiles(int64_t m, int64_t nnz, const int32_t* pos, const int32_t* crd, const T* val, const T* x,
+                        T* y, void* scratch, size_t scratch_bytes, cudaStream_t st) {
+  const int tiles = (int)ceil_div(nnz, kTile);
+  const size_t stride = scratch_bytes / 3 / 256 * 256;
+  char* base = static_cast<char*>(scratch);
+  TileScratch<T> sc{reinterpret_cast<T*>(base), reinterpret_cast<T*>(base + stride),
+                    reinterpret_cast<int*>(base + 2 * stride)};
+  spmv_tile_rows_kernel<<<(unsigned)ceil_div(m, 256), 256, 0, st>>>((int)m, tiles, pos, sc.row);
+  SB_LAUNCH_CHECK("spmv_tile_rows_kernel");
+  SB_CUDA(launch_early(spmv_tile_kernel<T>, dim3((unsigned)tiles), kTileThreads, 0, st, (int)m, (int)nnz, tiles, pos,
+                       crd, val, x, y, sc));
+  if (tiles > 1)
+    SB_CUDA(launch_early(spmv_tile_fixup_kernel<T>, dim3((unsigned)ceil_div(tiles, 128)), 128, 0, st, tiles, pos, y, sc));
+  return SB_OK;
 }
 
 template <typename T>
@@ -189,30 +214,46 @@ size_t sb_spmv_csr_scratch_bytes(int64_t nnz) {
   return ((tiles * 4 + 255) / 256 * 256) * 3;
 }
 
-int sb_spmv_csr_f32(int64_t m, int64_t n, int64_t nnz, const int32_t* pos, const int32_t* crd,
-                    const float* val, const float* x, float* y, void* scratch, size_t scratch_bytes,
-                    void* stream) {
+size_t sb_spmv_csr_tiled_scratch_bytes(int dtype, int64_t nnz) {
+  if (nnz <= 0) return 0;
+  const size_t tiles = (size_t)ceil_div(nnz, kTile);
+  return ((tiles * (dtype == SB_F64 || dtype == SB_I64 ? 8 : 4) + 255) / 256 * 256) * 3;
+}
+
+int sb_spmv_csr_tiled(int dtype, int64_t m, int64_t n, int64_t nnz, const int32_t* pos, const int32_t* crd,
+                      const void* val, const void* x, void* y, void* scratch, size_t scratch_bytes, void* stream) {
   int rc = check_spmv(m, n, nnz, pos, crd, val, x, y);
   if (rc != SB_OK) return rc;
+  SB_CHECK_ARG(dtype >= SB_F32 && dtype <= SB_I64, "spmv: unknown dtype %d", dtype);
   if (m == 0) return SB_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  // rows without entries are not visited by any tile
-  SB_CUDA(cudaMemsetAsync(y, 0, (size_t)m * sizeof(float), st));
-  if (nnz == 0) return SB_OK;
-  const size_t need = sb_spmv_csr_scratch_bytes(nnz);
+  const bool wide = dtype == SB_F64 || dtype == SB_I64;
+  if (nnz == 0) {
+    SB_CUDA(cudaMemsetAsync(y, 0, (size_t)m * (wide ? 8 : 4), st));
+    return SB_OK;
+  }
+  const size_t need = sb_spmv_csr_tiled_scratch_bytes(dtype, nnz);
   SB_CHECK_ARG(scratch && aligned16(scratch), "spmv: scratch is null or misaligned");
   if (scratch_bytes < need)
     return fail(SB_ERR_WORKSPACE, "spmv: scratch has %zu bytes, needs %zu", scratch_bytes, need);
-  const int tiles = (int)ceil_div(nnz, kTile);
-  const size_t stride = need / 3;
-  char* base = static_cast<char*>(scratch);
-  TileScratch sc{reinterpret_cast<float*>(base), reinterpret_cast<float*>(base + stride),
-                 reinterpret_cast<int*>(base + 2 * stride)};
-  spmv_tile_kernel<<<tiles, kTileThreads, 0, st>>>((int)m, (int)nnz, pos, crd, val, x, y, sc);
-  SB_LAUNCH_CHECK("spmv_tile_kernel");
-  spmv_tile_fixup_kernel<<<(unsigned)ceil_div(tiles, 128), 128, 0, st>>>(tiles, pos, y, sc);
-  SB_LAUNCH_CHECK("spmv_tile_fixup_kernel");
-  return SB_OK;
+  switch (dtype) {
+    case SB_F32:
+      return launch_tiles<float>(m, nnz, pos, crd, (const float*)val, (const float*)x, (float*)y, scratch, need, st);
+    case SB_F64:
+      return launch_tiles<double>(m, nnz, pos, crd, (const double*)val, (const double*)x, (double*)y, scratch, need, st);
+    case SB_I32:  // unsigned arithmetic: same bits as the reference's wrapping int32 math
+      return launch_tiles<unsigned int>(m, nnz, pos, crd, (const unsigned int*)val, (const unsigned int*)x,
+                                        (unsigned int*)y, scratch, need, st);
+    default:
+      return launch_tiles<unsigned long long>(m, nnz, pos, crd, (const unsigned long long*)val,
+                                              (const unsigned long long*)x, (unsigned long long*)y, scratch, need, st);
+  }
+}
+
+int sb_spmv_csr_f32(int64_t m, int64_t n, int64_t nnz, const int32_t* pos, const int32_t* crd,
+                    const float* val, const float* x, float* y, void* scratch, size_t scratch_bytes,
+                    void* stream) {
+  return sb_spmv_csr_tiled(SB_F32, m, n, nnz, pos, crd, val, x, y, scratch, scratch_bytes, stream);
 }
 
 int sb_spmv_csr_typed(int dtype, int64_t m, int64_t n, int64_t nnz, const int32_t* pos,

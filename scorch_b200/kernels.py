@@ -459,7 +459,7 @@ def _spmm_typed(pos, crd, val, B, n):
 
 def spmv_csr(pos, crd, val, x, plan: Optional[CsrPlan] = None) -> torch.Tensor:
     """y = A @ x for CSR A (``plan`` is accepted for symmetry with ``spmm_csr`` and not needed:
-    the fp32 kernel is balanced by entries, not rows)."""
+    the kernel is balanced by entries, not rows)."""
     r = _lib.host().spmv(pos, crd, val, x)
     if r is not None:
         return r
@@ -475,14 +475,10 @@ def spmv_csr(pos, crd, val, x, plan: Optional[CsrPlan] = None) -> torch.Tensor:
     y = torch.empty(m, dtype=val.dtype, device=x.device)
     L = _lib.lib()
     with torch.cuda.device(x.device):
-        if code != SB_F32:
-            check(L.sb_spmv_csr_typed(code, m, x.numel(), nnz, pos.data_ptr(), crd.data_ptr(),
-                                      val.data_ptr(), x.data_ptr(), y.data_ptr(), _stream()))
-            return y
-        sbytes = L.sb_spmv_csr_scratch_bytes(nnz)
+        sbytes = L.sb_spmv_csr_tiled_scratch_bytes(code, nnz)
         scratch = torch.empty(max(sbytes, 16), dtype=torch.uint8, device=x.device)
-        check(L.sb_spmv_csr_f32(m, x.numel(), nnz, pos.data_ptr(), crd.data_ptr(), val.data_ptr(),
-                                x.data_ptr(), y.data_ptr(), scratch.data_ptr(), sbytes, _stream()))
+        check(L.sb_spmv_csr_tiled(code, m, x.numel(), nnz, pos.data_ptr(), crd.data_ptr(), val.data_ptr(),
+                                  x.data_ptr(), y.data_ptr(), scratch.data_ptr(), sbytes, _stream()))
     return y
 
 
