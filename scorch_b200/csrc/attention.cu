@@ -403,16 +403,20 @@ attn_scattered_kernel(AttnArgs a) {
 //               (u, g) = actual column g*KT + u), so a thread reads KT contiguous floats per V
 //               row and writes KT contiguous floats per output row.
 // Three CTAs per SM (168 registers; four spill, two leave the tensor pipe idle more often).
-constexpr int kAttnWarps = 4;  // row blocks per CTA (1 and 2 measured the same)
-template <int D16>  // head dimension d = 16 * D16 (of Q, K and V)
+// SPLIT > 1: as many warps share a row block, every SPLIT-th block each, and merge their running
+// softmax at the end.  For calls with fewer row blocks than the GPU holds warps, whose time is one
+// warp's serial chain of blocks (about 3 us per block at d = 64): 407 tokens, 2 heads, 8 blocks per
+// row block: 28.4 us with one warp, SPLITUS with four.
+constexpr int kAttnWarps = 4;  // warps per CTA (1 and 2 measured the same)
+template <int D16, int SPLIT>  // head dimension d = 16 * D16 (of Q, K and V)
 __global__ void __launch_bounds__(kAttnWarps * 32, 12 / kAttnWarps)
 attn_block_kernel(AttnArgs a) {
   constexpr int KT = 2 * D16;
   // the warp's Q rows as pre-split TF32 A fragments, one 128-bit word per lane and k-step
   __shared__ uint4 sq_hi[kAttnWarps][2 * D16][32], sq_lo[kAttnWarps][2 * D16][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int rb = blockIdx.x * kAttnWarps + warp;
-  if (rb >= a.RB) return;
+  const int rb = blockIdx.x * (kAttnWarps / SPLIT) + warp / SPLIT, part = warp % SPLIT;
+  if (SPLIT == 1 && rb >= a.RB) return;
   const int g = lane >> 2, t = lane & 3;
   const long long bz = blockIdx.y;
   const float* Q = a.Q + bz * a.stride_q;
@@ -420,7 +424,11 @@ attn_block_kernel(AttnArgs a) {
   const float* V = a.V + bz * a.stride_v;
   float* O = a.O + bz * a.stride_o;
   const int i0 = rb * 16;
-  const int kb = __ldg(a.rb_ptr + rb), ke = __ldg(a.rb_ptr + rb + 1);
+  int kb = 0, ke = 0;
+  if (rb < a.RB) {
+    ke = __ldg(a.rb_ptr + rb + 1);
+    kb = min(ke, __ldg(a.rb_ptr + rb) + part);
+  }
   const float scale = a.scale * 1.4426950408889634f;  // scores are kept in log2 units: exp2 below
   const float* mask_val = (a.mask_val && !__ldg(a.mask_is_ones)) ? a.mask_val : nullptr;
 
@@ -430,7 +438,7 @@ attn_block_kernel(AttnArgs a) {
   float o[KT][4];
 #pragma unroll
   for (int u = 0; u < KT; u++) o[u][0] = o[u][1] = o[u][2] = o[u][3] = 0.f;
-  if (a.has_rem) {
+  if (a.has_rem && part == 0) {
 #pragma unroll
     for (int r = 0; r < 2; r++) {
       const int row = i0 + g + 8 * r;
@@ -491,10 +499,10 @@ attn_block_kernel(AttnArgs a) {
       return x;
     };
     Desc d1 = load_desc(kb);                              // block b at the top of iteration b
-    Desc d2 = (kb + 1 < ke) ? load_desc(kb + 1) : d1;     // block b+1
+    Desc d2 = (kb + SPLIT < ke) ? load_desc(kb + SPLIT) : d1;   // the block after it
     load_k(d1.j0);
 #pragma unroll 1
-    for (int b = kb; b < ke; b++) {
+    for (int b = kb; b < ke; b += SPLIT) {
       const Desc cur = d1;
       const unsigned m0 = cur.m0, m1 = cur.m1;
       // warp-uniform: every entry of the block is stored (the blocks inside a band)
@@ -568,8 +576,8 @@ attn_block_kernel(AttnArgs a) {
       // K rows of the next block (its descriptor was read an iteration ago) and the descriptor
       // of the block after it: in flight during the softmax update and P V
       d1 = d2;
-      if (b + 1 < ke) load_k(d1.j0);
-      if (b + 2 < ke) d2 = load_desc(b + 2);
+      if (b + SPLIT < ke) load_k(d1.j0);
+      if (b + 2 * SPLIT < ke) d2 = load_desc(b + 2 * SPLIT);
       // the V rows of this block: in flight during the softmax update (issuing them before S
       // keeps 32 more registers live through it and measured 3 % slower)
       load_v();
@@ -655,6 +663,48 @@ attn_block_kernel(AttnArgs a) {
 #pragma unroll
           for (int u = 0; u < 4; u++) mma_tf32(o[u0 + u], ahi, bh[u][0], bh[u][1]);
         }
+      }
+    }
+  }
+
+  if constexpr (SPLIT > 1) {
+    // the parts' (maximum, sum, output) to the row block's first warp, added in order; the memory of
+    // the Q fragments (d / 2 words per lane and array) holds a part's accumulators (d / 2 words)
+    float* park = reinterpret_cast<float*>(&sq_hi[warp][0][0]);
+    float* park_lo = reinterpret_cast<float*>(&sq_lo[warp][0][0]);
+    __syncwarp();
+    if (part > 0) {
+#pragma unroll
+      for (int u = 0; u < KT; u++) {
+#pragma unroll
+        for (int e = 0; e < 4; e++) park[(u * 4 + e) * 32 + lane] = o[u][e];
+      }
+#pragma unroll
+      for (int r = 0; r < 2; r++) {
+        park_lo[(2 * r) * 32 + lane] = M[r];
+        park_lo[(2 * r + 1) * 32 + lane] = L[r];
+      }
+    }
+    __syncthreads();
+    if (part > 0 || rb >= a.RB) return;
+#pragma unroll 1
+    for (int p = 1; p < SPLIT; p++) {
+      const float* from = reinterpret_cast<const float*>(&sq_hi[warp + p][0][0]);
+      const float* from_lo = reinterpret_cast<const float*>(&sq_lo[warp + p][0][0]);
+      float f1[2], f2[2];
+#pragma unroll
+      for (int r = 0; r < 2; r++) {
+        const float m2 = from_lo[(2 * r) * 32 + lane], l2 = from_lo[(2 * r + 1) * 32 + lane];
+        const float nm = fmaxf(M[r], m2), ms = (nm == -INFINITY) ? 0.f : nm;
+        f1[r] = attn_exp2(M[r] - ms);
+        f2[r] = attn_exp2(m2 - ms);
+        L[r] = L[r] * f1[r] + l2 * f2[r];
+        M[r] = nm;
+      }
+#pragma unroll
+      for (int u = 0; u < KT; u++) {
+#pragma unroll
+        for (int e = 0; e < 4; e++) o[u][e] = o[u][e] * f1[e >> 1] + from[(u * 4 + e) * 32 + lane] * f2[e >> 1];
       }
     }
   }
@@ -823,9 +873,17 @@ int sb_sparse_attention_csr_f32(int64_t m, int64_t n, int64_t d, int64_t nnz, co
     if (rc != SB_OK) return rc;
   }
   if (stages & SB_ATTN_STAGE_BLOCKS) {
-    dim3 grid((unsigned)ceil_div(p.RB, kAttnWarps), (unsigned)batch);
-    if (d == 32) attn_block_kernel<2><<<grid, kAttnWarps * 32, 0, st>>>(a);
-    else attn_block_kernel<4><<<grid, kAttnWarps * 32, 0, st>>>(a);
+    // warps per row block: one where that fills the GPU (3 CTAs of 4 warps per SM), else two or four
+    const int64_t slots = 12 * (int64_t)sm_count(), work = p.RB * batch;
+    const int split = 4 * work <= slots ? 4 : 2 * work <= slots ? 2 : 1;
+    dim3 grid((unsigned)ceil_div(p.RB, kAttnWarps / split), (unsigned)batch);
+#define SB_BLOCKS(D16, SPLIT) attn_block_kernel<D16, SPLIT><<<grid, kAttnWarps * 32, 0, st>>>(a)
+    if (d == 32) {
+      if (split == 4) SB_BLOCKS(2, 4); else if (split == 2) SB_BLOCKS(2, 2); else SB_BLOCKS(2, 1);
+    } else {
+      if (split == 4) SB_BLOCKS(4, 4); else if (split == 2) SB_BLOCKS(4, 2); else SB_BLOCKS(4, 1);
+    }
+#undef SB_BLOCKS
     SB_LAUNCH_CHECK("attn_block_kernel");
   }
   return SB_OK;
