@@ -154,6 +154,21 @@ SB_API int sb_spmm_csr_typed(int dtype, int64_t m, int64_t n, int64_t k, int64_t
                              const void* B, int64_t ldb, void* C, int64_t ldc, void* stream);
 
 /* --------------------------------------------------------------------------------------------
+ * Dense C = A W, fp32 accuracy on the tensor cores (three bf16 parts per value, six products): the
+ * feature transforms of a graph layer, A tall (m x k, row pitch lda), W small (k x n).  k <= 32768 and
+ * lda multiples of 4, A 16-byte aligned; ldc a multiple of 8, C 32-byte aligned (SB_ERR_UNSUPPORTED
+ * otherwise); ws: sb_dense_matmul_workspace_bytes(n, k) bytes, 16-byte aligned.
+ * sb_dense_matmul_status() (synchronises): 0, or 1 when a wait inside the kernel ever ran out, or -1
+ * when it could not be read.
+ * Replaces: the torch.matmul(X, W) of the reference's caller, bench/bench_gcn.py:314-329.
+ * -------------------------------------------------------------------------------------------- */
+SB_API size_t sb_dense_matmul_workspace_bytes(int64_t n, int64_t k);
+SB_API int sb_dense_matmul_f32(int64_t m, int64_t n, int64_t k, const float* A, int64_t lda,
+                               const float* W, int64_t ldw, float* C, int64_t ldc, void* ws,
+                               size_t ws_bytes, void* stream);
+SB_API int sb_dense_matmul_status(void);
+
+/* --------------------------------------------------------------------------------------------
  * CSR SpMV: y[i] = sum_p val[p] * x[crd[p]].  Every y[i] is written.
  * Replaces: spmv_csr<T> csrc/kernels.h:12-49 (prebuilt_spmv_csr_{f32,f64,i32,i64}) and the
  *           compiler-emitted loop of scorch.ops.spmv (src/scorch/ops.py:48-136).

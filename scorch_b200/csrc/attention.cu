@@ -406,7 +406,7 @@ attn_scattered_kernel(AttnArgs a) {
 // SPLIT > 1: as many warps share a row block, every SPLIT-th block each, and merge their running
 // softmax at the end.  For calls with fewer row blocks than the GPU holds warps, whose time is one
 // warp's serial chain of blocks (about 3 us per block at d = 64): 407 tokens, 2 heads, 8 blocks per
-// row block: 28.4 us with one warp, SPLITUS with four.
+// row block: 28.4 us with one warp, block kernel 13.6 -> 5.7 us with four.
 constexpr int kAttnWarps = 4;  // warps per CTA (1 and 2 measured the same)
 template <int D16, int SPLIT>  // head dimension d = 16 * D16 (of Q, K and V)
 __global__ void __launch_bounds__(kAttnWarps * 32, 12 / kAttnWarps)

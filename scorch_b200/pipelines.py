@@ -7,9 +7,9 @@ on the device end to end.
   through one batched launch per stage, or — for masks with enough well-filled 16x16 blocks and
   head dimension 32 / 64 — through the single attention call that never writes the scores.
 * ``gcn_forward`` — H = ReLU(A_hat (X W1)), out = A_hat (H W2), transform first like the
-  reference's bench (bench/bench_gcn.py:314-329).  The dense X·W products are cuBLAS calls
-  through torch (outside the sparse path); the two A_hat products are the SpMM kernel, the first
-  with the fused ReLU epilogue.
+  reference's bench (bench/bench_gcn.py:314-329).  The dense X·W products of large graphs run on the
+  tensor cores in fp32 accuracy (``kernels.dense_matmul``), small ones through torch; the two A_hat
+  products are the SpMM kernel, the first with the fused ReLU epilogue.
 """
 from __future__ import annotations
 
@@ -76,9 +76,9 @@ def sparse_attention(pos: torch.Tensor, crd: torch.Tensor, mask_val: Optional[to
 
 
 def gcn_forward(pos, crd, val, X, W1, W2, plan: Optional[K.CsrPlan] = None) -> torch.Tensor:
-    xw = torch.matmul(X, W1)
+    xw = K.dense_matmul(X, W1)
     h = K.spmm_csr(pos, crd, val, xw, relu=True, plan=plan)
-    hw = torch.matmul(h, W2)
+    hw = K.dense_matmul(h, W2)
     return K.spmm_csr(pos, crd, val, hw, plan=plan)
 
 

@@ -1,0 +1,47 @@
+"""Dense transform on the tensor cores: edges of its tiles, chunks and panels, and values it cannot split."""
+from __future__ import annotations
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(X, W):
+    from scorch_b200 import _lib
+    L, (m, k), n = _lib.lib(), X.shape, W.shape[1]
+    out = torch.full((m + 1, n), 7.0, device="cuda")          # a guard row behind the result
+    ws = torch.empty(L.sb_dense_matmul_workspace_bytes(n, k), dtype=torch.uint8, device="cuda")
+    _lib.check(L.sb_dense_matmul_f32(m, n, k, X.data_ptr(), k, W.data_ptr(), n, out.data_ptr(), n, ws.data_ptr(),
+                                     ws.numel(), torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    assert L.sb_dense_matmul_status() == 0
+    assert (out[m] == 7.0).all()
+    return out[:m]
+
+
+@pytest.mark.parametrize("m", [1, 127, 128, 129, 148 * 128 + 5, 60000])
+@pytest.mark.parametrize("n,k", [(8, 4), (16, 32), (40, 36), (64, 256), (72, 100), (128, 64), (136, 128), (256, 260)])
+def test_dense_matmul(m, n, k):
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    X = torch.randn((m, k), generator=g, device="cuda")
+    W = torch.randn((k, n), generator=g, device="cuda") * k ** -0.5
+    want = X.double() @ W.double()
+    err = lambda c: ((c.double() - want).norm() / want.norm()).item()
+    # no further from float64 than a chain of fp32 FMAs is (2.9e-7 at k = 256)
+    assert err(_run(X, W)) <= 1.2e-7 + 1.7e-7 * (k / 256) ** 0.5
+    assert torch.equal(_run(X, W), _run(X, W))
+
+
+def test_values_beyond_the_split():
+    X = torch.randn((1000, 64), device="cuda")
+    W = torch.randn((64, 64), device="cuda") * 0.125
+    X[130, 3], X[131, 5], X[700, 0] = float("inf"), float("nan"), 3.0e38
+    got, want = _run(X, W), X.double() @ W.double()
+    assert torch.isinf(got[130]).all() and torch.isnan(got[131]).all()
+    fine = torch.isfinite(want.float())
+    assert torch.equal(fine, torch.isfinite(got))
+    assert torch.allclose(got[fine].double(), want[fine], rtol=1e-4, atol=1e-5)
+    W[3, 7] = float("nan")
+    got = _run(X, W)
+    assert torch.isnan(got[:, 7]).all() and torch.isfinite(got[0, :7]).all()
