@@ -115,6 +115,18 @@ SB_API int sb_spmm_csr_once(int dtype, int64_t m, int64_t n, int64_t k, int64_t 
                             const void* bias, int relu, int accumulate, void* C, int64_t ldc, void* ws,
                             size_t ws_bytes, void* stream);
 
+/* Column split of a CSR matrix (fp32 values, columns ascending per row) into `chunks` <= 64 matrices of
+ * the same rows: chunk c holds the entries with columns in [c * w, (c + 1) * w), w = ceil(n / chunks),
+ * column indices kept.  rpos[chunks * (m + 1)]: row pointers of each chunk, from 0; ccrd / cval[nnz]:
+ * the chunks' entries one after the other; counts_host[chunks]: their lengths.  For products whose
+ * dense operand is far larger than L2: sb_spmm_csr_once per chunk, accumulating.  Synchronises;
+ * SB_ERR_UNSUPPORTED when the columns of a row do not ascend. */
+SB_API size_t sb_csr_split_columns_workspace_bytes(int64_t m, int64_t chunks);
+SB_API int sb_csr_split_columns_f32(int64_t m, int64_t n, int64_t nnz, const int32_t* pos,
+                                    const int32_t* crd, const float* val, int64_t chunks, int32_t* rpos,
+                                    int32_t* ccrd, float* cval, int64_t* counts_host, void* ws,
+                                    size_t ws_bytes, void* stream);
+
 /* Accumulating form:  C[i, 0:k] = act( bias + C[i, 0:k] + sum_p ... ), same arguments.  A product
  * whose dense operand arrives in pieces (row chunks of B, each with the matrix entries whose
  * columns fall in it) is the first piece through sb_spmm_csr_f32 and the others through this

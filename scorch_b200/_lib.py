@@ -42,6 +42,9 @@ SIGNATURES = {
     "sb_probe_l2_gather": (_int, [_ptr, _i64, _i64, _i64, _ptr, _ptr]),
     "sb_spmm_csr_typed": (_int, [_int, _i64, _i64, _i64, _i64, _ptr, _ptr, _ptr, _ptr, _i64, _ptr,
                                  _i64, _ptr]),
+    "sb_csr_split_columns_workspace_bytes": (_sz, [_i64, _i64]),
+    "sb_csr_split_columns_f32": (_int, [_i64, _i64, _i64, _ptr, _ptr, _ptr, _i64, _ptr, _ptr, _ptr, C.POINTER(_i64),
+                                        _ptr, _sz, _ptr]),
     "sb_dense_matmul_workspace_bytes": (_sz, [_i64, _i64]),
     "sb_dense_matmul_f32": (_int, [_i64, _i64, _i64, _ptr, _i64, _ptr, _i64, _ptr, _i64, _ptr, _sz, _ptr]),
     "sb_dense_matmul_status": (_int, []),

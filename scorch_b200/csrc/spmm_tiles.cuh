@@ -316,7 +316,9 @@ spmm_tile_rows_kernel(SpmmArgs<T> a, TileArgs<T> t) {
     b = __ldg(a.pos + r0 + lane);
     len = __ldg(a.pos + r0 + lane + 1) - b;
   }
-  unsigned todo = __ballot_sync(FULL, len == 0 || len > kUnit);
+  // (an empty row of an accumulating product without bias or ReLU stays what it is)
+  const bool keep_empty = a.accumulate && !a.bias && !a.relu;
+  unsigned todo = __ballot_sync(FULL, (len == 0 && !keep_empty) || len > kUnit);
   asm volatile("griddepcontrol.wait;" ::: "memory");   // the tile kernel's results
   while (todo) {
     const int i = __ffs(todo) - 1;

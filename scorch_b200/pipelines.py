@@ -76,10 +76,14 @@ def sparse_attention(pos: torch.Tensor, crd: torch.Tensor, mask_val: Optional[to
 
 
 def gcn_forward(pos, crd, val, X, W1, W2, plan: Optional[K.CsrPlan] = None) -> torch.Tensor:
-    xw = K.dense_matmul(X, W1)
-    h = K.spmm_csr(pos, crd, val, xw, relu=True, plan=plan)
-    hw = K.dense_matmul(h, W2)
-    return K.spmm_csr(pos, crd, val, hw, plan=plan)
+    """Large graphs: the matrix is cut by columns once per call, and the products run chunk by chunk
+    with the operand in L2 (``kernels.split_chunks``)."""
+    n, hidden, width = X.shape[0], W1.shape[1], W2.shape[1]
+    split = K.ColumnSplit.of(pos, crd, val, n, max(hidden, width)) if W1.is_cuda and X.dtype == torch.float32 else None
+    # (an operand that L2 nearly holds whole is multiplied in one pass)
+    product = lambda B, relu: (split.matmul(B, relu) if split is not None and 4 * n * B.shape[1] > 1.3 * K.SPLIT_CHUNK_BYTES
+                               else K.spmm_csr(pos, crd, val, B, relu=relu, plan=plan))
+    return product(K.dense_matmul(product(K.dense_matmul(X, W1), True), W2), False)
 
 
 def chunk_bounds(units: int, chunks: int, shrink: bool = True) -> list:

@@ -1,0 +1,61 @@
+"""Column split of a CSR matrix and the chunked product."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+import torch
+
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _csr(lens, n, seed):
+    rng = np.random.default_rng(seed)
+    pos = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    crd = np.concatenate([np.sort(rng.choice(n, size=x, replace=False)) for x in lens]).astype(np.int32)
+    return pos, crd, rng.standard_normal(crd.size).astype(np.float32)
+
+
+@pytest.mark.parametrize("chunks", [1, 2, 5, 64])
+@pytest.mark.parametrize("k", [1, 40, 64, 200])
+def test_split_and_product(chunks, k):
+    from scorch_b200 import kernels as K
+    n = 3001
+    lens = [0, 0, 3000, 1, 0, 33, 700] + [int(x) for x in np.random.default_rng(1).integers(0, 40, 900)] + [0, 0]
+    pos, crd, val = _csr(lens, n, seed=chunks)
+    d = lambda a: torch.from_numpy(a).cuda()
+    split = K.ColumnSplit(d(pos), d(crd), d(val), n, chunks)
+    width, first = -(-n // chunks), 0
+    rows = np.repeat(np.arange(len(lens)), lens)
+    for c in range(chunks):
+        keep = crd // width == c
+        p = np.concatenate([[0], np.cumsum(np.bincount(rows[keep], minlength=len(lens)))])
+        assert split.counts[c] == keep.sum() and np.array_equal(split.pos[c].cpu().numpy(), p)
+        part = slice(first, first + split.counts[c])
+        assert np.array_equal(split.crd[part].cpu().numpy(), crd[keep])
+        assert np.array_equal(split.val[part].cpu().numpy(), val[keep])
+        first += split.counts[c]
+    B = np.random.default_rng(k).standard_normal((n, k)).astype(np.float32)
+    want = O.spmm_csr_acc64(pos, crd, val, B)
+    for relu in (False, True):
+        got = split.matmul(d(B), relu=relu).cpu().numpy()
+        assert O.allclose_report(got, np.maximum(want, 0) if relu else want, 1e-4, 1e-4)[0]
+
+
+def test_columns_that_do_not_ascend_are_not_split(monkeypatch):
+    from scorch_b200 import kernels as K, pipelines as P
+    monkeypatch.setattr(K, "SPLIT_CHUNK_BYTES", 2e5)
+    pos, crd, val = _csr([40] * 2000, 2000, seed=3)
+    g = torch.Generator().manual_seed(0)
+    X, W1, W2 = (torch.randn(s, generator=g).cuda() for s in ((2000, 64), (64, 64), (64, 40)))
+    d = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    assert K.ColumnSplit.of(d(pos), d(crd), d(val), 2000, 64) is not None
+    out = P.gcn_forward(d(pos), d(crd), d(val), X, W1, W2)
+    flip = lambda a: a.reshape(2000, 40)[:, ::-1].reshape(-1)
+    assert K.ColumnSplit.of(d(pos), d(flip(crd)), d(flip(val)), 2000, 64) is None
+    back = P.gcn_forward(d(pos), d(flip(crd)), d(flip(val)), X, W1, W2)
+    A = torch.sparse_csr_tensor(d(pos), d(crd), d(val), size=(2000, 2000)).to_dense().double()
+    want = A @ (torch.relu(A @ (X.double() @ W1.double())) @ W2.double())
+    for got in (out, back):
+        assert ((got.double() - want).norm() / want.norm()).item() < 1e-6
