@@ -125,7 +125,8 @@ __device__ __forceinline__ Pack<T, W> ld_dense(const T* p) {
 }
 
 // Present contents of an output slice, or a segment sum another CTA left in L2: not through L1.
-template <typename T, int W>
+// ONCE: read once and rewritten, marked for early eviction.
+template <typename T, int W, bool ONCE = false>
 __device__ __forceinline__ Pack<T, W> ld_l2(const T* p) {
   constexpr int N = W * (int)sizeof(T) / 4;
   unsigned r[N];
@@ -133,14 +134,16 @@ __device__ __forceinline__ Pack<T, W> ld_l2(const T* p) {
   if constexpr (N >= 4) {
 #pragma unroll
     for (int i = 0; i < N; i += 4) {
-      const uint4 x = __ldcg(reinterpret_cast<const uint4*>(q + i));
+      const uint4* s = reinterpret_cast<const uint4*>(q + i);
+      const uint4 x = ONCE ? __ldcs(s) : __ldcg(s);
       r[i] = x.x; r[i + 1] = x.y; r[i + 2] = x.z; r[i + 3] = x.w;
     }
   } else if constexpr (N == 2) {
-    const uint2 x = __ldcg(reinterpret_cast<const uint2*>(q));
+    const uint2* s = reinterpret_cast<const uint2*>(q);
+    const uint2 x = ONCE ? __ldcs(s) : __ldcg(s);
     r[0] = x.x; r[1] = x.y;
   } else {
-    r[0] = __ldcg(q);
+    r[0] = ONCE ? __ldcs(q) : __ldcg(q);
   }
   return unpack<T, W>(r);
 }

@@ -83,9 +83,10 @@ struct TileSmem {
 };
 
 template <int BYTES>
-__device__ __forceinline__ void cp_async(void* smem, const void* gmem) {
+__device__ __forceinline__ void cp_async(void* smem, const void* gmem, uint64_t policy) {
   const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(s), "l"(gmem), "n"(BYTES) : "memory");
+  asm volatile("cp.async.ca.shared.global.L2::cache_hint [%0], [%1], %2, %3;" ::"r"(s), "l"(gmem), "n"(BYTES), "l"(policy)
+               : "memory");
 }
 
 template <typename T, int L, int VEC, int W>
@@ -109,7 +110,7 @@ __device__ __forceinline__ void tile_begin_row(Pack<T, W> (&s)[VEC], const SpmmA
   const T* crow = a.C + (long long)row * a.ldc;
 #pragma unroll
   for (int v = 0; v < VEC; v++)
-    if (col_ok[v]) s[v] = ld_l2<T, W>(crow + col0 + v * L * W);
+    if (col_ok[v]) s[v] = ld_l2<T, W, true>(crow + col0 + v * L * W);
 }
 
 // acc += the entries [b, e) of the window, one after the other, U operand rows in flight.  Lanes
@@ -180,11 +181,17 @@ spmm_tile_kernel(SpmmArgs<T> a, TileArgs<T> t) {
   Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, l = lane % L, g = lane / L;
   const unsigned pitch = (unsigned)(a.ldb * (long long)sizeof(T));
+  // (set up while the kernel before it still runs; the operands may be that kernel's results)
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int e0 = (int)blockIdx.x * t.entries, e1 = min(t.nnz, e0 + t.entries);
   const int staged = min(t.nnz, e1 + kUnit) - e0;
+  // (read once: marked for early eviction, the operand's rows are what L2 should keep)
+  uint64_t once;
+  asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(once));
   for (int i = tid; i < staged; i += kTileThreadsMm) {
-    cp_async<4>(&sm.entry[i].j, a.crd + e0 + i);
-    cp_async<(int)sizeof(T)>(&sm.entry[i].a, a.val + e0 + i);
+    cp_async<4>(&sm.entry[i].j, a.crd + e0 + i, once);
+    cp_async<(int)sizeof(T)>(&sm.entry[i].a, a.val + e0 + i, once);
   }
   asm volatile("cp.async.commit_group;" ::: "memory");
 
@@ -310,6 +317,7 @@ template <typename T>
 __global__ void __launch_bounds__(kTileThreadsMm)
 spmm_tile_rows_kernel(SpmmArgs<T> a, TileArgs<T> t) {
   const int lane = threadIdx.x & 31;
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // (what follows waits for this kernel's end)
   const long long r0 = ((long long)blockIdx.x * kTileWarps + (threadIdx.x >> 5)) * 32;
   int b = 0, len = 1;
   if (r0 + lane < a.m) {
@@ -373,8 +381,7 @@ static int launch_tiles(const SpmmArgs<T>& a, int64_t nnz, void* ws, cudaStream_
       if (dev >= 0 && dev < 64) sized[dev] = true;
     }
     const bool resident = !in_l2 && t.tiles <= 148 * tile_ctas(L);
-    kernel<<<dim3((unsigned)t.tiles, resident ? 1 : panels), kTileThreadsMm, sizeof(Smem), st>>>(a, t);
-    SB_LAUNCH_CHECK("spmm_tile_kernel");
+    SB_CUDA(launch_early(kernel, dim3((unsigned)t.tiles, resident ? 1 : panels), kTileThreadsMm, sizeof(Smem), st, a, t));
   }
   // (may be set up while the tiles still run: it waits for them itself)
   SB_CUDA(launch_early(spmm_tile_rows_kernel<T>,

@@ -61,6 +61,7 @@ struct TileScratch {
 __global__ void __launch_bounds__(256)
 spmv_tile_rows_kernel(int m, int tiles, const int* __restrict__ pos, int* __restrict__ row) {
   const long long r = (long long)blockIdx.x * 256 + threadIdx.x;
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the tiles' products do not need this kernel
   if (r >= m) return;
   const int b = __ldg(pos + r), e = __ldg(pos + r + 1);
   if (r == 0) row[0] = 0;
