@@ -336,9 +336,12 @@ __device__ __forceinline__ void expand_row(const CsrIn& in, int ab, int ae, int 
 }
 
 // The kernels of the bins run side by side: each lets the next launch begin at its own start and ends
-// only after the launch before it, so that what follows the last one follows all of them.
+// only after the launch before it (its last CTA waits for that; the others free their places), so that
+// what follows the last one follows all of them.
 __device__ __forceinline__ void let_next_begin() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void end_after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void end_after_previous() {
+  if (blockIdx.x == gridDim.x - 1) asm volatile("griddepcontrol.wait;" ::: "memory");
+}
 
 struct RowsOut {
   int* row_cnt;         // distinct columns per row (null: not wanted)
