@@ -305,14 +305,12 @@ __device__ __forceinline__ void attn_scatter_range(const AttnArgs& a, const floa
 
 template <int L>
 __global__ void __launch_bounds__(kScatWarps * 32, 4)
-attn_scattered_kernel(AttnArgs a) {
+attn_scattered_kernel(const __grid_constant__ AttnArgs a) {
   constexpr int G = 32 / L;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane / L, l = lane % L;
   __shared__ int s_n, s_long[kScatWarps * G];
   __shared__ float s_m[kScatWarps], s_l[kScatWarps], s_acc[kScatWarps][8 * L];
-  if (threadIdx.x == 0) s_n = 0;
-  __syncthreads();
   const int row = (blockIdx.x * kScatWarps + warp) * G + g;
   const long long bz = blockIdx.y;
   const float* K = a.K + bz * a.stride_k + 8 * l;
@@ -333,7 +331,6 @@ attn_scattered_kernel(AttnArgs a) {
 #pragma unroll
   for (int i = 0; i < 8; i++) acc[i] = 0.f;
   const bool is_long = e - b > kLongScattered;
-  if (is_long && l == 0) s_long[atomicAdd(&s_n, 1)] = row;
   attn_scatter_range<L>(a, mask_val, K, V, q, scale, b, is_long ? b : e, l, M, Ls, acc);
   if (live && !is_long) {
     float* orow = a.O + bz * a.stride_o + (long long)row * a.ldo + 8 * l;
@@ -341,6 +338,10 @@ attn_scattered_kernel(AttnArgs a) {
     *reinterpret_cast<float4*>(orow + 4) = make_float4(acc[4], acc[5], acc[6], acc[7]);
     if (l == 0) a.stats[bz * a.m + row] = make_float2(M, Ls);
   }
+  if (!__syncthreads_or(is_long)) return;
+  if (threadIdx.x == 0) s_n = 0;
+  __syncthreads();
+  if (is_long && l == 0) s_long[atomicAdd(&s_n, 1)] = row;
   __syncthreads();
   const int n_long = s_n;
   for (int i = 0; i < n_long; i++) {

@@ -12,8 +12,7 @@
 // rows, lane 0 of the ninth issues the tensor-core work (so that issuing overlaps the others' work):
 //   1. Q tile and K window rows are read with plain loads (into registers ahead of the point where
 //      their shared-memory buffer is free), split into TF32 hi / lo parts and stored to shared
-//      memory in the tensor core's canonical K-major layout without swizzle (core matrix = 8 rows
-//      x 16 bytes, the cores of one 8-row group side by side);
+//      memory in the tensor core's K-major layout with the 128-byte swizzle;
 //   2. S = Q K^T  is issued as tcgen05.mma kind::tf32 (M 128, N 128, K 8) in three passes
 //      (lo*hi, hi*lo, hi*hi: the 3xTF32 split, fp32-level accuracy) into 384 TMEM columns, one K
 //      piece of 128 window columns at a time through two buffers;
@@ -163,41 +162,38 @@ struct BandArgs {
 };
 
 // Rows [row0, row0 + ROWS) of a row-major matrix (row pitch ld floats, rows outside [0, limit)
-// read as zeros) -> hi / lo parts in the canonical layout: 8-row groups of 8 * D floats; inside a
-// group the 16-byte pieces (4 features) of the 8 rows are contiguous (128 bytes per core matrix),
-// the D / 4 cores of the group side by side.  Lanes: 8 rows x 4 neighbouring cores = 512
-// contiguous bytes of shared memory per warp store, 64 contiguous bytes of each row per load.
+// read as zeros) -> hi / lo parts in the K-major layout with the 128-byte swizzle: D / 32 blocks of 32
+// features, in each block 128 bytes per row whose 16-byte pieces are permuted by the row's low three
+// bits.  16 neighbouring lanes take one row: a quarter warp loads 128 contiguous bytes and stores the
+// 8 pieces of one 128-byte line.  (The layout without swizzle keeps the bank of a piece fixed by its
+// row, so conflict-free stores need 8 rows per quarter warp, and its loads then touch 8 lines of 16
+// bytes each: fetching a tile's Q and K took 11,800 of its 42,400 cycles.)
 // Two halves, so that a piece can be loaded into registers while the buffer it goes to is still
 // being read by the tensor cores.
 template <int D, int ROWS>
 struct BandPiece {
-  static constexpr int QG = D / 16;                       // groups of 4 cores per row group
-  static constexpr int TASKS = (ROWS / 8) * QG;           // (row group, core group) pairs, one per warp pass
-  static constexpr int PASSES = TASKS / kBandWorkWarps;
-  static_assert(TASKS % kBandWorkWarps == 0, "staging tasks must divide over the warps");
+  static constexpr int QUADS = D / 4;                     // 16-byte pieces per row
+  static constexpr int STEP = kBandWorkWarps * 32 / QUADS;   // rows per pass
+  static constexpr int PASSES = ROWS / STEP;
+  static_assert(ROWS % STEP == 0, "rows must divide over the threads");
   float4 v[PASSES];
 
   __device__ __forceinline__ void load(const float* __restrict__ src, unsigned ld, int row0, int limit) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int r8 = lane & 7, q4 = lane >> 3;
+    const int r = threadIdx.x / QUADS, q = threadIdx.x % QUADS;
 #pragma unroll
     for (int i = 0; i < PASSES; i++) {
-      const int task = i * kBandWorkWarps + warp;
-      const int rg = task / QG, core = (task % QG) * 4 + q4;
-      const int row = row0 + rg * 8 + r8;
+      const int row = row0 + i * STEP + r;
       v[i] = (row >= 0 && row < limit)
-                 ? __ldg(reinterpret_cast<const float4*>(src + (size_t)((unsigned long long)(unsigned)row * ld) + core * 4))
+                 ? __ldg(reinterpret_cast<const float4*>(src + (size_t)((unsigned long long)(unsigned)row * ld) + q * 4))
                  : make_float4(0.f, 0.f, 0.f, 0.f);
     }
   }
   __device__ __forceinline__ void store(float* __restrict__ hi, float* __restrict__ lo) const {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int r8 = lane & 7, q4 = lane >> 3;
+    const int r = threadIdx.x / QUADS, q = threadIdx.x % QUADS;
 #pragma unroll
     for (int i = 0; i < PASSES; i++) {
-      const int task = i * kBandWorkWarps + warp;
-      const int rg = task / QG, core = (task % QG) * 4 + q4;
-      const int off = rg * 8 * D + core * 32 + r8 * 4;
+      const int row = i * STEP + r;
+      const int off = (q >> 3) * (ROWS * 32) + row * 32 + ((q ^ row) & 7) * 4;
       uint4 h, l;
       attn_split(v[i].x, h.x, l.x); attn_split(v[i].y, h.y, l.y);
       attn_split(v[i].z, h.z, l.z); attn_split(v[i].w, h.w, l.w);
@@ -208,9 +204,9 @@ struct BandPiece {
 };
 
 // 64 rows [row0, row0 + 64) of V (row pitch ld floats, rows outside [0, limit) read as zeros) ->
-// hi / lo parts of their transpose in the same canonical layout: "rows" are now the D features,
-// the 64 window columns are the contiguous (K) direction, so an 8-feature group holds 16 cores of
-// 128 bytes.  (The B operand of O += P V has to be K-major: with the descriptor's B-major bit set
+// hi / lo parts of their transpose in the K-major layout without swizzle (core matrix = 8 rows x 16
+// bytes): "rows" are now the D features, the 64 window columns are the contiguous (K) direction, so an
+// 8-feature group holds 16 cores of 128 bytes.  (The B operand of O += P V has to be K-major: with the descriptor's B-major bit set
 // the tf32 instruction left the accumulator untouched on this hardware.)  A thread gathers four
 // consecutive window columns of one feature with scalar loads (a warp reads 128 contiguous bytes
 // per load) and stores them as one 16-byte piece; the 8 lanes of a feature group fill one core
@@ -251,10 +247,9 @@ struct BandPieceT {
 template <int D>
 __global__ void __launch_bounds__(kBandThreads, 1)
 attn_band_kernel(AttnArgs a, BandArgs b) {
-  extern __shared__ __align__(128) unsigned char band_smem[];
+  extern __shared__ __align__(1024) unsigned char band_smem[];   // (the swizzle counts from 1024-byte boundaries)
   constexpr int TILE_FLOATS = kBandRows * D;           // one 128 x D operand part (hi or lo)
   constexpr int VT_FLOATS = 64 * D;                    // one part of a transposed 64-row piece of V
-  constexpr uint32_t GROUP_BYTES = 8 * D * 4;          // an 8-row group: stride between row groups
   constexpr uint32_t VT_GROUP_BYTES = (64 / 4) * 128;  // 8 features x 64 window columns of V^T
   constexpr uint32_t CORE_BYTES = 128;                 // a core matrix: stride between neighbouring cores
   constexpr int KSTEPS = D / 8;                        // tcgen05.mma steps over the head dimension
@@ -307,23 +302,23 @@ attn_band_kernel(AttnArgs a, BandArgs b) {
   constexpr uint32_t IDESC_S = umma_idesc_tf32(kBandRows, 128, 0);
   constexpr uint32_t IDESC_O = umma_idesc_tf32(kBandRows, D, 0);
 
-  // Descriptors of the operand parts, built once; a k-step moves the start address by two cores
-  // (2 * 128 bytes = 16 units of 16 bytes), which is a plain addition on the descriptor.
-  const uint64_t dq_hi = umma_desc(smem_u32(q_hi), CORE_BYTES, GROUP_BYTES);
-  const uint64_t dq_lo = umma_desc(smem_u32(q_lo), CORE_BYTES, GROUP_BYTES);
+  // Descriptors of the operand parts, built once; a k-step (8 features) moves the start address: by two
+  // cores in V^T, by 32 bytes in a block of 32 features of Q and K, then to the next block.  In units of
+  // 16 bytes these are plain additions on the descriptor.
+  const uint64_t dq_hi = umma_desc_sw128(smem_u32(q_hi)), dq_lo = umma_desc_sw128(smem_u32(q_lo));
   constexpr uint64_t KSTEP = (2 * CORE_BYTES) >> 4;
+  auto k_step = [](int ks) { return (uint64_t)((ks & 3) * 2 + (ks >> 2) * (128 * 128 >> 4)); };
   // S[:, 128 c .. 128 c + 127] = Q K_c^T from K piece buffer `buf` (one thread; three passes of the split)
   auto issue_scores = [&](int c, int buf, uint32_t bar) {
     tc_fence_after();
-    const uint64_t dk_hi = umma_desc(smem_u32(k_hi(buf)), CORE_BYTES, GROUP_BYTES);
-    const uint64_t dk_lo = umma_desc(smem_u32(k_lo(buf)), CORE_BYTES, GROUP_BYTES);
+    const uint64_t dk_hi = umma_desc_sw128(smem_u32(k_hi(buf))), dk_lo = umma_desc_sw128(smem_u32(k_lo(buf)));
     const uint32_t d_tmem = tmem + (uint32_t)(c * 128);
 #pragma unroll
     for (int pass = 0; pass < 3; pass++) {
       const uint64_t aa = pass == 0 ? dq_lo : dq_hi, bb = pass == 1 ? dk_lo : dk_hi;
 #pragma unroll
       for (int ks = 0; ks < KSTEPS; ks++)
-        umma_ss(d_tmem, aa + ks * KSTEP, bb + ks * KSTEP, IDESC_S, (pass | ks) != 0 ? 1u : 0u);
+        umma_ss(d_tmem, aa + k_step(ks), bb + k_step(ks), IDESC_S, (pass | ks) != 0 ? 1u : 0u);
     }
     umma_commit(bar);
   };
@@ -347,6 +342,14 @@ attn_band_kernel(AttnArgs a, BandArgs b) {
   const float scale = a.scale * 1.4426950408889634f;   // scores in log2 units
   float M_s = -INFINITY, L_s = 0.f, ms = 0.f, sum = 0.f;
   bool failed = false;
+  // The epilogue turns a warp's 32 rows x D / 2 columns over in shared memory, so that O is read and
+  // written a whole line at a time (a thread per row took 6,400 cycles): rows 4 i + out_r, columns out_c.
+  constexpr int HALF = D / 2, OUT_PASSES = HALF / 4;
+  static_assert(HALF == 32, "a quarter warp covers half a row");
+  const int out_r = lane >> 3, out_c = h * HALF + (lane & 7) * 4;
+  float4 scat[OUT_PASSES];   // the scattered entries' part
+#pragma unroll
+  for (int i = 0; i < OUT_PASSES; i++) scat[i] = make_float4(0.f, 0.f, 0.f, 0.f);
 
   do {
     // ---- S = Q K^T: K pieces of 128 window columns through two buffers; pieces are loaded into
@@ -378,6 +381,11 @@ attn_band_kernel(AttnArgs a, BandArgs b) {
     for (int w = 0; w < kBandWords; w++)
       words[w] = !live ? 0u : b.bits ? __ldg(b.bits + (size_t)row * kBandWords + w) : 0xffffffffu;  // (probe: all stored)
     const float* mask_val = (a.mask_val && !__ldg(a.mask_is_ones)) ? a.mask_val : nullptr;
+    if (a.has_rem && live) {
+      const float2 st = __ldg(a.stats + bz * a.m + row);
+      M_s = st.x;
+      L_s = st.y;
+    }
     const int ent0 = (live && b.ent0) ? __ldg(b.ent0 + row) : 0;
     // scores of a 32-column chunk: scaled, times the mask value, -inf where nothing is stored.
     // Without branches: lanes differ in which columns are stored.  `ep` walks the row's entries
@@ -457,11 +465,6 @@ attn_band_kernel(AttnArgs a, BandArgs b) {
 
     if (worker) s_red[h * kBandRows + r] = mx;
     __syncthreads();
-    if (a.has_rem && live) {
-      const float2 st = __ldg(a.stats + bz * a.m + row);
-      M_s = st.x;
-      L_s = st.y;
-    }
     if (worker) {
       const float mt = fmaxf(fmaxf(s_red[r], s_red[kBandRows + r]), M_s);
       ms = (mt == -INFINITY) ? 0.f : mt;
@@ -528,6 +531,13 @@ attn_band_kernel(AttnArgs a, BandArgs b) {
       mark();   // 13 + 4 g
     }
     if (failed) break;
+    if (a.has_rem && worker) {
+#pragma unroll
+      for (int i = 0; i < OUT_PASSES; i++) {
+        const int orow = i0 + lane_base + 4 * i + out_r;
+        if (orow < a.m) scat[i] = *reinterpret_cast<const float4*>(O + (long long)orow * a.ldo + out_c);
+      }
+    }
     if ((failed = wait_all(bar_pv, (uint32_t)((ROUNDS - 1) & 1)))) break;
     mark();   // 34
   } while (false);
@@ -537,25 +547,25 @@ attn_band_kernel(AttnArgs a, BandArgs b) {
   if (worker) s_red[h * kBandRows + r] = sum;
   __syncthreads();
   if (!failed && !b.raw_scores && worker) {
-    constexpr int HALF = D / 2;
     const float alpha = attn_exp2(M_s - ms);             // 0 for a row without scattered entries
     const float den = s_red[r] + s_red[kBandRows + r] + alpha * L_s;
     const float inv = den > 0.f ? 1.f / den : 0.f;
     float v[32];
-    tmem_ld32(t_row + (uint32_t)(kTmemO + h * HALF), v);   // (reads 32 columns; HALF of them are used)
-    if (live) {
-      float* orow = O + (long long)row * a.ldo + h * HALF;
+    tmem_ld32(t_row + (uint32_t)(kTmemO + h * HALF), v);
+    constexpr int PITCH = HALF + 4;                      // an odd number of 16-byte pieces: no bank conflicts
+    float* turn = kbuf + warp * (32 * PITCH);            // (the tensor cores are done with the operands)
 #pragma unroll
-      for (int j = 0; j < HALF; j += 4) {
-        float4 x = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-        if (a.has_rem) {
-          const float4 s = *reinterpret_cast<const float4*>(orow + j);
-          x.x = fmaf(alpha, s.x, x.x); x.y = fmaf(alpha, s.y, x.y);
-          x.z = fmaf(alpha, s.z, x.z); x.w = fmaf(alpha, s.w, x.w);
-        }
-        x.x *= inv; x.y *= inv; x.z *= inv; x.w *= inv;
-        *reinterpret_cast<float4*>(orow + j) = x;
-      }
+    for (int j = 0; j < HALF; j += 4)
+      *reinterpret_cast<float4*>(turn + lane * PITCH + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < OUT_PASSES; i++) {
+      const int rr = 4 * i + out_r, orow = i0 + lane_base + rr;
+      const float al = __shfl_sync(FULL, alpha, rr), in = __shfl_sync(FULL, inv, rr);
+      float4 x = *reinterpret_cast<const float4*>(turn + rr * PITCH + (lane & 7) * 4);
+      x.x = fmaf(al, scat[i].x, x.x) * in; x.y = fmaf(al, scat[i].y, x.y) * in;
+      x.z = fmaf(al, scat[i].z, x.z) * in; x.w = fmaf(al, scat[i].w, x.w) * in;
+      if (orow < a.m) *reinterpret_cast<float4*>(O + (long long)orow * a.ldo + out_c) = x;
     }
   }
   mark_i = 35;

@@ -17,6 +17,11 @@ __device__ __forceinline__ uint64_t umma_desc(uint32_t saddr, uint32_t lbo_bytes
   return (uint64_t)((saddr >> 4) & 0x3fffu) | ((uint64_t)((lbo_bytes >> 4) & 0x3fffu) << 16) |
          ((uint64_t)((sbo_bytes >> 4) & 0x3fffu) << 32) | (1ull << 46);
 }
+// The same for a K-major operand with the 128-byte swizzle: groups of 8 rows x 128 bytes one after the
+// other (stride 1024 bytes, each group on a 1024-byte boundary), swizzle mode 2 in bits 61-63.
+__device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t saddr) {
+  return umma_desc(saddr, 16, 1024) | (2ull << 61);
+}
 // Instruction descriptor of kind::tf32 with fp32 accumulation: D format F32 (bits 4-5 = 1), A and B
 // format TF32 (bits 7-9, 10-12 = 2), B major (bit 16: 1 = MN-major), N / 8 (bits 17-22), M / 16 (24-28).
 __host__ __device__ constexpr uint32_t umma_idesc_tf32(int M, int N, int b_mn_major) {
