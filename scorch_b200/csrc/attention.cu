@@ -306,6 +306,7 @@ __device__ __forceinline__ void attn_scatter_range(const AttnArgs& a, const floa
 template <int L>
 __global__ void __launch_bounds__(kScatWarps * 32, 4)
 attn_scattered_kernel(const __grid_constant__ AttnArgs a) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // (attn_band_kernel waits where it needs these results)
   constexpr int G = 32 / L;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane / L, l = lane % L;

@@ -19,11 +19,11 @@
 //   3. every thread of the eight warps owns one row and half of the columns: it reads its scores
 //      with tcgen05.ld, masks the entries that are not stored (without branches), applies scale
 //      and mask values, takes the row maxima piece by piece while the next piece's products run,
-//      and then writes P = exp2(S - max) back as hi (in place) and lo (64 spare columns);
+//      and then writes P = exp2(S - max) back as hi (in place) and lo (64 columns that are free);
 //   4. O += P V  is issued with P read from TMEM as the A operand and V^T (transposed while it is
 //      staged, so that it is K-major like K) as the B operand, 64 window columns at a time;
 //   5. the epilogue reads O from TMEM, merges the scattered entries' (max, sum, O) and writes O / sum.
-// TMEM: columns [0,384) S / P_hi, [384,448) O, [448,512) P_lo.  Every mbarrier wait is bounded by
+// TMEM: columns [0,384) S / P_hi (the first 128 also P_lo), [384,512) O.  Every mbarrier wait is bounded by
 // a clock limit; a wait that runs out sets a status word (sb_attn_band_status), the CTA frees its
 // TMEM and returns.  No TMA, no multicast, no cluster: every operand goes through registers for
 // the hi / lo split anyway.
@@ -42,7 +42,7 @@ constexpr int kBandWorkWarps = 8;              // warps that stage operands and 
 constexpr int kBandThreads = (kBandWorkWarps + 1) * 32;   // + one warp whose lane 0 issues the tensor-core work
 constexpr int kTmemCols = 512;
 constexpr int kTmemO = 384;                     // first TMEM column of the output accumulator
-constexpr int kTmemPlo = 448;                   // first TMEM column of the lo parts of P
+constexpr int kTmemO2 = 448;                    // first TMEM column of its second half (products with V lo)
 
 __device__ int g_band_status = 0;  // 0 ok; 1 a wait for the tensor cores ran out
 
@@ -155,7 +155,7 @@ struct BandArgs {
   const int* ent0;
   const unsigned* bits;
   float* raw_scores;   // probe only: the tile's 128 x 384 products Q K^T, unscaled and unmasked
-  float* tmem_image;   // probe only: the tile's 128 x 512 tensor-memory cells after the last O += P V
+  float* tmem_image;   // probe only, 128 x 512: P hi (as its round read it), P V, lo parts of P's last 64 columns
   int probe_tile;
   long long* clocks;   // probe only: clock64() of thread 0 at the kernel's phase boundaries
   int last_entry;      // nnz - 1 (bound of the mask-value reads)
@@ -234,7 +234,7 @@ struct BandPieceT {
 #pragma unroll
     for (int it = 0; it < ITEMS; it++) {
       const int f = (it % HALVES) * 32 + lane, jb = warp * 2 + it / HALVES;
-      const int off = (f >> 3) * (16 * 32) + jb * 32 + (f & 7) * 4;   // floats
+      const int off = (jb >> 3) * (2 * D * 32) + f * 32 + ((jb ^ f) & 7) * 4;   // floats
       uint4 h, l;
       attn_split(v[it][0], h.x, l.x); attn_split(v[it][1], h.y, l.y);
       attn_split(v[it][2], h.z, l.z); attn_split(v[it][3], h.w, l.w);
@@ -250,8 +250,7 @@ attn_band_kernel(AttnArgs a, BandArgs b) {
   extern __shared__ __align__(1024) unsigned char band_smem[];   // (the swizzle counts from 1024-byte boundaries)
   constexpr int TILE_FLOATS = kBandRows * D;           // one 128 x D operand part (hi or lo)
   constexpr int VT_FLOATS = 64 * D;                    // one part of a transposed 64-row piece of V
-  constexpr uint32_t VT_GROUP_BYTES = (64 / 4) * 128;  // 8 features x 64 window columns of V^T
-  constexpr uint32_t CORE_BYTES = 128;                 // a core matrix: stride between neighbouring cores
+  constexpr int VT_LO = D * 32;                        // its lo part, from the hi part on (64 x 32 columns later)
   constexpr int KSTEPS = D / 8;                        // tcgen05.mma steps over the head dimension
   constexpr int ROUNDS = kBandCols / 64;               // O += P V, 64 window columns per round
   float* q_hi = reinterpret_cast<float*>(band_smem);
@@ -259,11 +258,11 @@ attn_band_kernel(AttnArgs a, BandArgs b) {
   float* kbuf = q_lo + TILE_FLOATS;                    // two K pieces (hi, lo each) = four V^T pieces
   float* s_red = kbuf + 4 * TILE_FLOATS;               // [2][128] row maxima, then row sums
   unsigned long long* bars = reinterpret_cast<unsigned long long*>(s_red + 2 * kBandRows);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 3);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 4);
   auto k_hi = [&](int i) { return kbuf + i * 2 * TILE_FLOATS; };
   auto k_lo = [&](int i) { return kbuf + i * 2 * TILE_FLOATS + TILE_FLOATS; };
   auto v_hi = [&](int i) { return kbuf + i * 2 * VT_FLOATS; };
-  auto v_lo = [&](int i) { return kbuf + i * 2 * VT_FLOATS + VT_FLOATS; };
+  auto v_lo = [&](int i) { return kbuf + i * 2 * VT_FLOATS + VT_LO; };
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tile = b.raw_scores ? b.probe_tile : (int)blockIdx.x;
@@ -274,13 +273,15 @@ attn_band_kernel(AttnArgs a, BandArgs b) {
   const float* K = a.K + bz * a.stride_k;
   const float* V = a.V + bz * a.stride_v;
   float* O = a.O + bz * a.stride_o;
-  // mbarriers: [0], [1] = the tensor cores are done with K piece buffer 0 / 1; [2] = with a round of O += P V
+  // mbarriers: [0], [1] = the tensor cores are done with K piece buffer 0 / 1; [2], [3] = with an even / odd
+  // round of O += P V
   const uint32_t bar_k0 = smem_u32(bars), bar_k1 = smem_u32(bars + 1), bar_pv = smem_u32(bars + 2);
 
   if (threadIdx.x == 0) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar_k0) : "memory");
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar_k1) : "memory");
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar_pv) : "memory");
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar_pv + 8) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) {
@@ -300,13 +301,12 @@ attn_band_kernel(AttnArgs a, BandArgs b) {
   mark();   // 0
 
   constexpr uint32_t IDESC_S = umma_idesc_tf32(kBandRows, 128, 0);
-  constexpr uint32_t IDESC_O = umma_idesc_tf32(kBandRows, D, 0);
+  constexpr uint32_t IDESC_O = umma_idesc_tf32(kBandRows, D, 0), IDESC_O2 = umma_idesc_tf32(kBandRows, 2 * D, 0);
 
   // Descriptors of the operand parts, built once; a k-step (8 features) moves the start address: by two
   // cores in V^T, by 32 bytes in a block of 32 features of Q and K, then to the next block.  In units of
   // 16 bytes these are plain additions on the descriptor.
   const uint64_t dq_hi = umma_desc_sw128(smem_u32(q_hi)), dq_lo = umma_desc_sw128(smem_u32(q_lo));
-  constexpr uint64_t KSTEP = (2 * CORE_BYTES) >> 4;
   auto k_step = [](int ks) { return (uint64_t)((ks & 3) * 2 + (ks >> 2) * (128 * 128 >> 4)); };
   // S[:, 128 c .. 128 c + 127] = Q K_c^T from K piece buffer `buf` (one thread; three passes of the split)
   auto issue_scores = [&](int c, int buf, uint32_t bar) {
@@ -381,8 +381,11 @@ attn_band_kernel(AttnArgs a, BandArgs b) {
     for (int w = 0; w < kBandWords; w++)
       words[w] = !live ? 0u : b.bits ? __ldg(b.bits + (size_t)row * kBandWords + w) : 0xffffffffu;  // (probe: all stored)
     const float* mask_val = (a.mask_val && !__ldg(a.mask_is_ones)) ? a.mask_val : nullptr;
+    // (up to here nothing was read that the scattered-entry kernel writes: the first CTAs may begin
+    // beside its last)
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     if (a.has_rem && live) {
-      const float2 st = __ldg(a.stats + bz * a.m + row);
+      const float2 st = a.stats[bz * a.m + row];
       M_s = st.x;
       L_s = st.y;
     }
@@ -472,6 +475,13 @@ attn_band_kernel(AttnArgs a, BandArgs b) {
     mark();   // 9: row maxima
 
     // ---- O += P V, 64 window columns per round; V^T piece g sits in buffer (g + 2) % 4 -------------------
+    // V^T hi and lo are one operand of 2 D rows for P hi (8 instructions of N = 128, 135 cycles each, instead of
+    // 16 of N = 64, 79 cycles each), so O has D columns for the products with V hi and D for those with V lo.
+    // Round 0's lo parts of P sit in the latter, whose sums begin with round 1; the later rounds' take turns
+    // in the columns of rounds 0 and 1.  So rounds 1 and 2 wait for the round before, the others for the one
+    // before that: the tensor cores have the next round's products at hand when they end one.  (Rounds of 1,790
+    // cycles instead of 2,190; what is left is the workers' arithmetic, about 14 operations per probability.
+    // 16 worker warps took as long, and a CTA that goes on to further tiles spills to an L1 of 30 KB: slower.)
     int ep = ent0;
 #pragma unroll 1
     for (int g = 0; g < ROUNDS; g++) {
@@ -493,17 +503,28 @@ attn_band_kernel(AttnArgs a, BandArgs b) {
           attn_split(p, ph[j], pl[j]);
         }
         if (h == 0) ep += __popc(w1);
-        // piece g + 3 goes to the buffer that round g - 1 releases below
-        if (g >= 1 && g + 3 < ROUNDS) pv0.load(V, a.ldv, c0 + (g + 3) * 64, b.n);
+        // piece g + 2 goes to the buffer of piece g - 2, whose round is done below
+        if (g >= 2 && g + 2 < ROUNDS) pv0.load(V, a.ldv, c0 + (g + 2) * 64, b.n);
       }
       mark();   // 10 + 4 g: probabilities of the round in registers
-      // the round before must be done with the lo columns and with the V^T buffer that is refilled
-      if (g > 0 && (failed = wait_all(bar_pv, (uint32_t)((g - 1) & 1)))) break;
-      mark();   // 11 + 4 g: the round before is done
+      // the lo columns and the V^T buffer that is refilled must be free
+      const int before = g <= 2 ? g - 1 : g - 2;
+      if (before >= 0 && (failed = wait_all(bar_pv + 8 * (before & 1), (uint32_t)(before >> 1) & 1u))) break;
+      mark();   // 11 + 4 g: that round is done
+      const uint32_t lo_col = g == 0 ? kTmemO2 : (uint32_t)(((g - 1) & 1) * 64);
       if (worker) {
+        if (b.tmem_image && g < 2) {   // (whose cells change later)
+#pragma unroll
+          for (int j = 0; j < 32; j++) b.tmem_image[(size_t)r * kTmemCols + cb + j] = __uint_as_float(ph[j]);
+        }
         tmem_st32(t_row + (uint32_t)cb, ph);
-        tmem_st32(t_row + (uint32_t)(kTmemPlo + h * 32), pl);
-        if (g >= 1 && g + 3 < ROUNDS) pv0.store(v_hi((g + 1) & 3), v_lo((g + 1) & 3));
+        tmem_st32(t_row + lo_col + (uint32_t)(h * 32), pl);
+        if (g == 1) {
+#pragma unroll
+          for (int j = 0; j < 32; j++) pl[j] = 0u;
+          tmem_st32(t_row + (uint32_t)(kTmemO2 + h * 32), pl);
+        }
+        if (g >= 2 && g + 2 < ROUNDS) pv0.store(v_hi(g & 3), v_lo(g & 3));
         tmem_st_wait();
       }
       async_proxy_fence();
@@ -513,20 +534,24 @@ attn_band_kernel(AttnArgs a, BandArgs b) {
       if (issuer) {
         tc_fence_after();
         const int vb = (g + 2) & 3;
-        const uint64_t dv_hi = umma_desc(smem_u32(v_hi(vb)), CORE_BYTES, VT_GROUP_BYTES);
-        const uint64_t dv_lo = umma_desc(smem_u32(v_lo(vb)), CORE_BYTES, VT_GROUP_BYTES);
+        const uint64_t dv_hi = umma_desc_sw128(smem_u32(v_hi(vb)));   // V^T lo follows
         const uint32_t d_tmem = tmem + (uint32_t)kTmemO;
-        const uint32_t p_hi = tmem + (uint32_t)(g * 64), p_lo = tmem + (uint32_t)kTmemPlo;
+        const uint32_t p_hi = tmem + (uint32_t)(g * 64), p_lo = tmem + lo_col;
         const uint32_t later = g != 0 ? 1u : 0u;
 #pragma unroll
-        for (int pass = 0; pass < 3; pass++) {
-          const uint32_t a_tmem = pass == 0 ? p_lo : p_hi;
-          const uint64_t bb = pass == 1 ? dv_lo : dv_hi;
+        for (int ks = 0; ks < 8; ks++)
+          umma_ts(d_tmem, p_lo + (uint32_t)(ks * 8), dv_hi + k_step(ks), IDESC_O, ks != 0 ? 1u : later);
+        if (g == 0) {
+          const uint64_t dv_lo = umma_desc_sw128(smem_u32(v_lo(vb)));
 #pragma unroll
-          for (int ks = 0; ks < 8; ks++)
-            umma_ts(d_tmem, a_tmem + (uint32_t)(ks * 8), bb + ks * KSTEP, IDESC_O, (pass | ks) != 0 ? 1u : later);
+          for (int ks = 0; ks < 8; ks++) umma_ts(d_tmem, p_hi + (uint32_t)(ks * 8), dv_lo + k_step(ks), IDESC_O, 1u);
+#pragma unroll
+          for (int ks = 0; ks < 8; ks++) umma_ts(d_tmem, p_hi + (uint32_t)(ks * 8), dv_hi + k_step(ks), IDESC_O, 1u);
+        } else {
+#pragma unroll
+          for (int ks = 0; ks < 8; ks++) umma_ts(d_tmem, p_hi + (uint32_t)(ks * 8), dv_hi + k_step(ks), IDESC_O2, 1u);
         }
-        umma_commit(bar_pv);
+        umma_commit(bar_pv + 8 * (g & 1));
       }
       mark();   // 13 + 4 g
     }
@@ -538,7 +563,7 @@ attn_band_kernel(AttnArgs a, BandArgs b) {
         if (orow < a.m) scat[i] = *reinterpret_cast<const float4*>(O + (long long)orow * a.ldo + out_c);
       }
     }
-    if ((failed = wait_all(bar_pv, (uint32_t)((ROUNDS - 1) & 1)))) break;
+    if ((failed = wait_all(bar_pv + 8 * ((ROUNDS - 1) & 1), (uint32_t)((ROUNDS - 1) >> 1) & 1u))) break;
     mark();   // 34
   } while (false);
 
@@ -552,6 +577,12 @@ attn_band_kernel(AttnArgs a, BandArgs b) {
     const float inv = den > 0.f ? 1.f / den : 0.f;
     float v[32];
     tmem_ld32(t_row + (uint32_t)(kTmemO + h * HALF), v);
+    {
+      float v2[32];
+      tmem_ld32(t_row + (uint32_t)(kTmemO2 + h * HALF), v2);
+#pragma unroll
+      for (int j = 0; j < 32; j++) v[j] += v2[j];
+    }
     constexpr int PITCH = HALF + 4;                      // an odd number of 16-byte pieces: no bank conflicts
     float* turn = kbuf + warp * (32 * PITCH);            // (the tensor cores are done with the operands)
 #pragma unroll
@@ -572,11 +603,12 @@ attn_band_kernel(AttnArgs a, BandArgs b) {
   mark();     // 35: output written
   if (!failed && b.tmem_image && worker) {
 #pragma unroll 1
-    for (int c = 0; c < kTmemCols / 64; c++) {
-      float v[32];
-      tmem_ld32(t_row + (uint32_t)(c * 64 + h * 32), v);
+    for (int c = 2; c < kTmemCols / 64; c++) {   // P hi of rounds 2 to 5, O, P lo of round 5
+      float v[32], v2[32];
+      tmem_ld32(t_row + (uint32_t)((c == 7 ? 0 : c * 64) + h * 32), v);
+      tmem_ld32(t_row + (uint32_t)(kTmemO2 + h * 32), v2);
 #pragma unroll
-      for (int j = 0; j < 32; j++) b.tmem_image[(size_t)r * kTmemCols + c * 64 + h * 32 + j] = v[j];
+      for (int j = 0; j < 32; j++) b.tmem_image[(size_t)r * kTmemCols + c * 64 + h * 32 + j] = c == 6 ? v[j] + v2[j] : v[j];
     }
   }
   if (failed && threadIdx.x == 0) atomicExch(&g_band_status, 1);
@@ -592,11 +624,17 @@ static size_t band_smem_bytes() {
 }
 
 template <int D>
-static int band_launch(const AttnArgs& a, const BandArgs& b, unsigned tiles, unsigned batch, cudaStream_t st) {
+// `after_scattered`: the launch just before on the stream is attn_scattered_kernel's
+static int band_launch(const AttnArgs& a, const BandArgs& b, unsigned tiles, unsigned batch, bool after_scattered,
+                       cudaStream_t st) {
   const size_t smem = band_smem_bytes<D>();
   // (set on every call: the attribute belongs to the current device's copy of the function, and a
   // process may drive more than one device)
   SB_CUDA(cudaFuncSetAttribute(attn_band_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (after_scattered) {
+    SB_CUDA(launch_early(attn_band_kernel<D>, dim3(tiles, batch), kBandThreads, smem, st, a, b));
+    return SB_OK;
+  }
   attn_band_kernel<D><<<dim3(tiles, batch), kBandThreads, smem, st>>>(a, b);
   SB_LAUNCH_CHECK("attn_band_kernel");
   return SB_OK;
@@ -712,7 +750,8 @@ int sb_sparse_attention_band_f32(int64_t m, int64_t n, int64_t d, int64_t nnz, c
   }
   if (stages & SB_ATTN_STAGE_BLOCKS) {
     BandArgs b = {(int)n, p.ent0, p.bits, nullptr, nullptr, 0, nullptr, (int)std::max<int64_t>(nnz - 1, 0)};
-    rc = band_launch<64>(a, b, (unsigned)ceil_div(m, kBandRows), (unsigned)batch, st);
+    rc = band_launch<64>(a, b, (unsigned)ceil_div(m, kBandRows), (unsigned)batch,
+                         (stages & SB_ATTN_STAGE_SCATTERED) && rem_nnz > 0, st);
     if (rc != SB_OK) return rc;
   }
   return SB_OK;
@@ -731,7 +770,7 @@ int sb_attn_band_probe(int64_t m, int64_t n, int64_t d, int64_t tile, const floa
   a.scale = 1.f;
   // (no plan: every window column counts as stored; O is not written)
   BandArgs b = {(int)n, nullptr, nullptr, raw_scores, tmem_image, (int)tile, phase_clocks, 0};
-  return band_launch<64>(a, b, 1u, 1u, (cudaStream_t)stream);
+  return band_launch<64>(a, b, 1u, 1u, false, (cudaStream_t)stream);
 }
 
 int sb_attn_band_status(void) {
