@@ -31,6 +31,8 @@
 #include <algorithm>
 #include <vector>
 
+#include <cooperative_groups.h>
+
 #include "spgemm_rows.cuh"
 
 namespace sb {
@@ -825,8 +827,11 @@ int exclusive_scan_i32(int n, const int* cnt, int* out, long long* block_sum, lo
 // Bitmap and accumulators of all n columns in shared memory (n up to kSmemColumns): one CTA per row,
 // no plan, no read-back, one launch instead of the bucket path's ten (20,011 columns, ten rows of
 // 8,200 to 80,000 products: 190 us there, 92 us here, beside the other bins' kernels).
+// Few such rows leave most of the GPU to the others, so up to eight CTAs - a cluster - share a row: each
+// takes its part of the products into a bitmap and accumulators of its own, then emits a slice of the
+// columns, adding the others' sums out of their shared memory (CLUSTERED).
 constexpr int kSmemColumns = 24576, kSmemThreads = 1024;
-template <typename T, bool NUMERIC>
+template <typename T, bool NUMERIC, bool CLUSTERED>
 __global__ void __launch_bounds__(kSmemThreads)
 spgemm_smem_kernel(const int* __restrict__ rows, CsrIn in, int n, const unsigned long long* __restrict__ max_b,
                    RowsOut out) {
@@ -837,8 +842,12 @@ spgemm_smem_kernel(const int* __restrict__ rows, CsrIn in, int n, const unsigned
   __shared__ ExpandSmem<T, NT> s_expand;
   __shared__ double s_abs[NW];
   __shared__ int s_part[NW], s_at[kSmemColumns / 32];
+  __shared__ int s_total;
   let_next_begin();
-  const int i = __ldg(rows + blockIdx.x), tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  namespace cg = cooperative_groups;
+  const int parts = CLUSTERED ? (int)cg::this_cluster().num_blocks() : 1;
+  const int part = CLUSTERED ? (int)cg::this_cluster().block_rank() : 0;
+  const int i = __ldg(rows + blockIdx.x / parts), tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int ab = __ldg(in.Apos + i), ae = __ldg(in.Apos + i + 1);
   for (int x = tid; x < kSmemColumns / 32; x += NT) bits[x] = 0;
   if (NUMERIC)
@@ -863,10 +872,20 @@ spgemm_smem_kernel(const int* __restrict__ rows, CsrIn in, int n, const unsigned
     const unsigned bit = 1u << (c & 31);
     if (!(bits[c >> 5] & bit)) atomicOr(&bits[c >> 5], bit);
     if (NUMERIC) acc_add_smem<T>(&acc[c], product_bits<T>(a, __ldg(Bval + pb)), scale, fixed);
-  });
-  __syncthreads();
-  // kSmemColumns / 32 = 768 words: one per thread, in column order
-  unsigned m = tid < kSmemColumns / 32 ? bits[tid] : 0;
+  }, part, parts);
+  // this CTA's words of the bitmap (kSmemColumns / 32 = 768 in all), one per thread, in column order
+  const int words = kSmemColumns / 32 / parts, w0 = part * words;
+  unsigned m = 0;
+  if constexpr (CLUSTERED) {
+    cg::this_cluster().sync();
+    if (tid < words) {
+      for (int p = 0; p < parts; p++) m |= cg::this_cluster().map_shared_rank(bits, p)[w0 + tid];
+      bits[w0 + tid] = m;      // (a part's words are read by that part alone)
+    }
+  } else {
+    __syncthreads();
+    if (tid < words) m = bits[tid];
+  }
   const int c = __popc(m);
   int incl = c;
 #pragma unroll
@@ -883,25 +902,48 @@ spgemm_smem_kernel(const int* __restrict__ rows, CsrIn in, int n, const unsigned
     if (w < warp) before += v;
     total += v;
   }
-  if (out.row_cnt && tid == 0) out.row_cnt[i] = total;
+  int before_parts = 0;
+  if constexpr (CLUSTERED) {
+    if (tid == 0) s_total = total;
+    cg::this_cluster().sync();
+    total = 0;
+    for (int p = 0; p < parts; p++) {
+      const int v = *cg::this_cluster().map_shared_rank(&s_total, p);
+      if (p < part) before_parts += v;
+      total += v;
+    }
+  }
+  if (out.row_cnt && tid == 0 && part == 0) out.row_cnt[i] = total;
   if (NUMERIC) {
     // a warp per word, a lane per column
-    if (tid < kSmemColumns / 32) s_at[tid] = before + incl - c;
+    if (tid < words) s_at[tid] = before + incl - c;
     __syncthreads();
-    const long long base = __ldg(out.off + i);
+    const long long base = __ldg(out.off + i) + before_parts;
     const double inv = 1.0 / scale;
-    for (int w = warp; w < kSmemColumns / 32; w += NW) {
-      const unsigned word = bits[w];
+    for (int w = warp; w < words; w += NW) {
+      const unsigned word = bits[w0 + w];
       if (!(word >> lane & 1)) continue;
       const long long at = base + s_at[w] + __popc(word & ((1u << lane) - 1u));
-      const Slot v = acc[w * 32 + lane];
-      out.crd[at] = w * 32 + lane;
+      const int col = (w0 + w) * 32 + lane;
+      Slot v = acc[col];
+      if constexpr (CLUSTERED) {
+        v = *cg::this_cluster().map_shared_rank(acc + col, 0);
+        for (int p = 1; p < parts; p++) {
+          const Slot x = *cg::this_cluster().map_shared_rank(acc + col, p);
+          if (kIsFloat<T> && !fixed)
+            v = (Slot)__double_as_longlong(__longlong_as_double((long long)v) + __longlong_as_double((long long)x));
+          else
+            v += x;
+        }
+      }
+      out.crd[at] = col;
       T value;
       if constexpr (kIsFloat<T>) value = fixed ? (T)((double)(long long)v * inv) : (T)__longlong_as_double((long long)v);
       else value = (T)v;
       static_cast<T*>(out.val)[at] = value;
     }
   }
+  if constexpr (CLUSTERED) cg::this_cluster().sync();   // (the others read this CTA's sums)
   end_after_previous();
 }
 
@@ -1051,10 +1093,32 @@ static int max_abs(const WsLayout& w, const CsrIn& in, int64_t kb, cudaStream_t 
 template <typename T, bool NUMERIC>
 static int launch_smem_bin(const int* rows, int64_t count, const WsLayout& w, int64_t n, const CsrIn& in,
                            const RowsOut& out, cudaStream_t st) {
-  auto k = spgemm_smem_kernel<T, NUMERIC>;
   const int smem = kSmemColumns / 8 + (NUMERIC ? (int)n * 8 : 0);
+  // CTAs per row: as many as keep all of them (one per SM) on the GPU at a time
+  unsigned parts = 8;
+  while (parts > 1 && (int64_t)parts * count > sm_count()) parts /= 2;
+  if (parts == 1) {
+    auto k = spgemm_smem_kernel<T, NUMERIC, false>;
+    SB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    SB_CUDA(launch_early(k, dim3((unsigned)count), kSmemThreads, smem, st, rows, in, (int)n, w.max_b, out));
+    return SB_OK;
+  }
+  auto k = spgemm_smem_kernel<T, NUMERIC, true>;
   SB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  SB_CUDA(launch_early(k, dim3((unsigned)count), kSmemThreads, smem, st, rows, in, (int)n, w.max_b, out));
+  cudaLaunchAttribute attr[2] = {};
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = parts;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)count * parts);
+  cfg.blockDim = dim3(kSmemThreads);
+  cfg.dynamicSmemBytes = (size_t)smem;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  SB_CUDA(cudaLaunchKernelEx(&cfg, k, rows, in, (int)n, (const unsigned long long*)w.max_b, out));
   return SB_OK;
 }
 

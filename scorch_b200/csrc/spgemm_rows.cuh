@@ -261,7 +261,8 @@ __device__ __forceinline__ int expand_products(const CsrIn& in, int pa0, int pa1
 // The same for a CTA of NT threads, NT entries at a time: product q goes to thread q % NT whatever the
 // lengths of the B rows are, the search runs over the scanned lengths in shared memory.  (With a
 // warp per 32 entries, a row whose products come mostly from one long B row - the usual long row of
-// a power-law matrix - kept one warp busy and the rest waiting.)
+// a power-law matrix - kept one warp busy and the rest waiting.)  `part` of `parts` CTAs takes every
+// parts-th NT products.
 template <typename T, int NT>
 struct ExpandSmem {
   int excl[NT], off[NT];
@@ -269,7 +270,8 @@ struct ExpandSmem {
   int part[NT / 32];
 };
 template <typename T, bool NUMERIC, int NT, typename F>
-__device__ __forceinline__ void expand_cta(const CsrIn& in, int ab, int ae, ExpandSmem<T, NT>& sm, int tid, F&& emit) {
+__device__ __forceinline__ void expand_cta(const CsrIn& in, int ab, int ae, ExpandSmem<T, NT>& sm, int tid, F&& emit,
+                                           int part = 0, int parts = 1) {
   const int warp = tid >> 5, lane = tid & 31;
   int first = 0;
   for (int p0 = ab; p0 < ae; p0 += NT) {
@@ -300,7 +302,7 @@ __device__ __forceinline__ void expand_cta(const CsrIn& in, int ab, int ae, Expa
     sm.off[tid] = bb - excl;
     __syncthreads();
 #pragma unroll 4
-    for (int q = tid; q < total; q += NT) {
+    for (int q = part * NT + tid; q < total; q += parts * NT) {
       int e = 0;   // largest e with excl[e] <= q
 #pragma unroll
       for (int step = NT / 2; step > 0; step >>= 1)

@@ -75,3 +75,12 @@ def test_row_beyond_the_area():
     rng = np.random.default_rng(3)
     B = _csr([900] * 1300, 1000, rng, np.float32)
     _check(_csr([1300, 2, 700], 1300, rng, np.float32), B, 1000, np.float32)
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64, np.int32])
+@pytest.mark.parametrize("rows,n", [(1, 24576), (18, 45), (19, 5000), (38, 24575), (75, 1000)])
+def test_long_rows_shared_by_clusters(rows, n, dtype):
+    # over 8192 products a row: 8, 8, 4, 2 and 1 CTAs per row on 148 SMs; 45 columns leave most CTAs none
+    rng = np.random.default_rng(rows)
+    B = _csr([40] * 299 + [min(n, 3000)], n, rng, dtype)
+    _check(_csr([250] * rows + [0, 7], 300, rng, dtype), B, n, dtype)
