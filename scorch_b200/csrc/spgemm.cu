@@ -756,21 +756,23 @@ scan_write_kernel(int m, const int* __restrict__ cnt, const long long* __restric
   }
 }
 
-// All of it by one CTA, for short arrays: a warp per contiguous part, 32 counts at a time.
+// All of it by one CTA, for short arrays: a warp per contiguous part, 128 counts at a time, four per lane
+// (one per lane made a chain of 20 scans for 20,000 counts: 9.2 us).
 constexpr int kScanSmall = 32768;
 __global__ void __launch_bounds__(1024)
 scan_small_kernel(int m, const int* __restrict__ cnt, int* __restrict__ out, long long* __restrict__ total) {
-  constexpr int STEPS = kScanSmall / 1024;
+  constexpr int STEPS = kScanSmall / 4096;
   __shared__ long long s[32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int steps = (m + 1023) / 1024, b = warp * steps * 32;
-  int c[STEPS];
+  const int steps = (m + 4095) / 4096, b = warp * steps * 128;
   long long mine = 0;
 #pragma unroll
   for (int i = 0; i < STEPS; i++) {
-    const int x = b + i * 32 + lane;
-    c[i] = i < steps && x < m ? cnt[x] : 0;
-    mine += c[i];
+    const int x = b + i * 128 + lane * 4;
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      if (i < steps && x + q < m) mine += cnt[x + q];
+    }
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(FULL, mine, o);
@@ -787,14 +789,23 @@ scan_small_kernel(int m, const int* __restrict__ cnt, int* __restrict__ out, lon
 #pragma unroll
   for (int i = 0; i < STEPS; i++) {
     if (i >= steps) break;
-    long long incl = c[i];
+    const int x = b + i * 128 + lane * 4;
+    int c[4];   // (read again: kept, they would spill)
+#pragma unroll
+    for (int q = 0; q < 4; q++) c[q] = x + q < m ? cnt[x + q] : 0;
+    const long long four = (long long)c[0] + c[1] + c[2] + c[3];
+    long long incl = four;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const long long y = __shfl_up_sync(FULL, incl, o);
       if (lane >= o) incl += y;
     }
-    const int x = b + i * 32 + lane;
-    if (x < m) out[x + 1] = (int)(run + incl);
+    long long at = run + incl - four;
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      at += c[q];
+      if (x + q < m) out[x + q + 1] = (int)at;
+    }
     run += __shfl_sync(FULL, incl, 31);
   }
 }
