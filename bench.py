@@ -720,8 +720,13 @@ class GcnSharded(Workload):
 
     @property
     def launches_per_step(self):
-        # per layer one SpMM launch per row chunk (rows and heavy-row segments share the launch)
-        return self.shard.splits[0].chunks + self.shard.splits[-1].chunks
+        # per layer one SpMM launch per row chunk (rows and heavy-row segments share the launch), or two per
+        # column chunk and panel of a matrix that is cut by columns
+        def launches(split, k):
+            cut = [b.columns[1] if b.columns else None for b in split.blocks]
+            return sum(2 * len(c.counts) * -(-k // K.SPLIT_PANEL) if c is not None else 1 for c in cut)
+        from scorch_b200 import kernels as K
+        return launches(self.shard.splits[0], self.K1) + launches(self.shard.splits[-1], self.K2)
 
     def begin_block(self):
         self.timeline = self.S.Timeline()

@@ -465,18 +465,21 @@ DENSE_MATMUL_MIN_ROWS = 32768
 DENSE_MATMUL_MAX_K = 256
 
 
-def dense_matmul(X: torch.Tensor, W: torch.Tensor) -> torch.Tensor:
+def dense_matmul(X: torch.Tensor, W: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """X @ W in fp32 for a tall X: on the tensor cores in fp32 accuracy (``sb_dense_matmul_f32``) where
     the operands have the layout it takes, else ``torch.matmul``."""
     if (X.dim() != 2 or W.dim() != 2 or X.shape[0] < DENSE_MATMUL_MIN_ROWS or X.dtype != torch.float32
             or W.dtype != torch.float32 or not X.is_cuda or W.device != X.device or X.shape[1] != W.shape[0]
             or not X.is_contiguous() or not W.is_contiguous() or not 0 < X.shape[1] <= DENSE_MATMUL_MAX_K or X.shape[1] % 4
-            or W.shape[1] == 0 or W.shape[1] % 8 or X.data_ptr() % 16):
-        return torch.matmul(X, W)
+            or W.shape[1] == 0 or W.shape[1] % 8 or X.data_ptr() % 16
+            or (out is not None and (out.shape != (X.shape[0], W.shape[1]) or out.dtype != torch.float32
+                                     or out.device != X.device or not out.is_contiguous() or out.data_ptr() % 32))):
+        return torch.matmul(X, W, out=out)
     (m, k), n = X.shape, W.shape[1]
     L = _lib.lib()
     with torch.cuda.device(X.device):
-        out = torch.empty((m, n), dtype=torch.float32, device=X.device)
+        if out is None:
+            out = torch.empty((m, n), dtype=torch.float32, device=X.device)
         wbytes = L.sb_dense_matmul_workspace_bytes(n, k)
         ws = torch.empty(wbytes, dtype=torch.uint8, device=X.device)
         check(L.sb_dense_matmul_f32(m, n, k, X.data_ptr(), k, W.data_ptr(), n, out.data_ptr(), n, ws.data_ptr(),
@@ -534,9 +537,11 @@ class ColumnSplit:
                 raise
             return None
 
-    def matmul(self, B: torch.Tensor, relu: bool = False) -> torch.Tensor:
+    def matmul(self, B: torch.Tensor, relu: bool = False, out: Optional[torch.Tensor] = None,
+               accumulate: bool = False) -> torch.Tensor:
         k = B.shape[1]
-        out = torch.empty((self.m, k), dtype=torch.float32, device=B.device)
+        if out is None:
+            out = torch.empty((self.m, k), dtype=torch.float32, device=B.device)
         L, last = _lib.lib(), len(self.counts) - 1
         with torch.cuda.device(B.device):
             wbytes = max(L.sb_spmm_csr_once_workspace_bytes(SB_F32, min(k, SPLIT_PANEL), c) for c in self.counts)
@@ -548,7 +553,7 @@ class ColumnSplit:
                     check(L.sb_spmm_csr_once(SB_F32, self.m, self.n, min(SPLIT_PANEL, k - k0), count,
                                              self.pos[c].data_ptr(), self.crd.data_ptr() + 4 * first,
                                              self.val.data_ptr() + 4 * first, B.data_ptr() + 4 * k0, k, None,
-                                             int(relu and c == last), int(c > 0), out.data_ptr() + 4 * k0, k,
+                                             int(relu and c == last), int(accumulate or c > 0), out.data_ptr() + 4 * k0, k,
                                              ws.data_ptr(), wbytes, stream))
                     first += count
         return out

@@ -239,7 +239,7 @@ class HostGcnForward:
         # for chunk c + 2 to arrive)
         H = S.gcn_forward_sharded(shard, self.x, self.W1, self.W2, x_ready=ready, first_layer_only=True,
                                   lookahead=0)
-        torch.matmul(H, self.W2, out=self.t2)
+        K.dense_matmul(H, self.W2, out=self.t2)
         for r0, r1, blk in self.out_blocks:
             if r1 == r0:
                 continue

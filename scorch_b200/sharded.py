@@ -70,6 +70,7 @@ class CsrBlock:
     crd: torch.Tensor          # int32 [nnz]
     val: torch.Tensor
     plan: object = None
+    columns: object = None     # (chunks, kernels.ColumnSplit or None) for operands much larger than L2
 
     @property
     def rows(self) -> int:
@@ -244,6 +245,15 @@ def _split_by_chunk(local: CsrBlock, bounds: List[int], offsets: List[int]) -> L
 def _default_spmm(block: CsrBlock, B: torch.Tensor, out: torch.Tensor, relu: bool,
                   accumulate: bool = False) -> None:
     from . import kernels as K
+    # (an operand that L2 nearly holds whole is multiplied in one pass)
+    if B.is_contiguous() and out.is_contiguous() and 4 * B.numel() > 1.3 * K.SPLIT_CHUNK_BYTES:
+        chunks = K.split_chunks(block.rows, B.shape[0], block.nnz, B.shape[1])
+        if chunks:
+            if block.columns is None or block.columns[0] != chunks:
+                block.columns = chunks, K.ColumnSplit.of(block.pos, block.crd, block.val, B.shape[0], B.shape[1])
+            if block.columns[1] is not None:
+                block.columns[1].matmul(B, relu, out=out, accumulate=accumulate)
+                return
     if block.plan is None:
         block.plan = K.CsrPlan(block.pos, block.nnz)
     K.spmm_csr(block.pos, block.crd, block.val, B, relu=relu, plan=block.plan, out=out,
@@ -355,6 +365,7 @@ def _pipelined_layer(shard: ShardedCsr, split: Split, g: _Gatherer, name: str, x
     """out = act(A (x_local W)) over this rank's rows, chunk by chunk (W = None: act(A x)).
     ``x_ready``: one CUDA event per chunk after which that chunk's rows of ``x_local`` are valid
     (rows that are still arriving, e.g. by a host-to-device copy on another stream)."""
+    from .kernels import dense_matmul
     S, dev = split.chunks, x_local.device
     k = out.shape[1]
     send = shard.buffer(name + "send", (shard.max_rows, k), dev)
@@ -382,7 +393,7 @@ def _pipelined_layer(shard: ShardedCsr, split: Split, g: _Gatherer, name: str, x
             if hi > lo:
                 with _span(tlg, "dense_transform", side):
                     if weight is not None:
-                        torch.matmul(x_local[lo:hi], weight, out=send[lo:hi])
+                        dense_matmul(x_local[lo:hi], weight, out=send[lo:hi])
                     else:
                         send[lo:hi].copy_(x_local[lo:hi])
             if side is not None:
@@ -430,11 +441,12 @@ def gcn_forward_sharded(shard: ShardedCsr, x_local: torch.Tensor, W1: torch.Tens
     """This rank's rows of  A_hat ReLU(A_hat X W1) W2  (reference caller: bench/bench_gcn.py:314-329;
     transform first, then the sparse product, as there).
 
-    Per layer the local transform of row chunk c (cuBLAS through torch) is all-gathered while the
+    Per layer the local transform of row chunk c is all-gathered while the
     sub-matrices of earlier chunks are multiplied; transforms run ``lookahead`` chunks ahead of
     the SpMMs on the main stream so that the communication stream always has a gather queued.
     Exposed communication is one chunk's transform + gather at the start of each layer.  With one
-    rank and one chunk every layer is a single full-width SpMM.
+    rank and one chunk every layer is a single SpMM, by column chunks where the graph is large
+    (``kernels.split_chunks``; the cut matrix stays with the block).
     ``x_ready``: per first-layer chunk, the event after which that chunk's rows of ``x_local`` are
     valid; ``first_layer_only``: return the hidden layer ReLU(A_hat X W1) (this rank's rows)."""
     spmm_fn = spmm_fn or _default_spmm

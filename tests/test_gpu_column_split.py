@@ -59,3 +59,21 @@ def test_columns_that_do_not_ascend_are_not_split(monkeypatch):
     want = A @ (torch.relu(A @ (X.double() @ W1.double())) @ W2.double())
     for got in (out, back):
         assert ((got.double() - want).norm() / want.norm()).item() < 1e-6
+
+
+@pytest.mark.parametrize("chunks", [1, 2])
+def test_sharded_forward_by_column_chunks(monkeypatch, chunks):
+    # one rank; row chunks of the operand accumulate, each cut by columns on its own
+    from scorch_b200 import kernels as K, sharded as S
+    monkeypatch.setattr(K, "SPLIT_CHUNK_BYTES", 1e5)
+    pos, crd, val = _csr([60] * 2000, 2000, seed=4)
+    g = torch.Generator().manual_seed(1)
+    X, W1, W2 = (torch.randn(s, generator=g).cuda() for s in ((2000, 64), (64, 72), (72, 40)))
+    p, c, v = (torch.from_numpy(a).cuda() for a in (pos, crd, val))
+    shard = S.ShardedCsr.from_global(p, c, v, 0, 1, chunks=chunks)
+    A = torch.sparse_csr_tensor(p, c, v, size=(2000, 2000)).to_dense().double()
+    want = A @ (torch.relu(A @ (X.double() @ W1.double())) @ W2.double())
+    for _ in range(2):
+        got = S.gcn_forward_sharded(shard, X, W1, W2)
+        assert ((got.double() - want).norm() / want.norm()).item() < 1e-6
+    assert all(b.columns[1] is not None for b in shard.blocks)
