@@ -288,7 +288,7 @@ topk_rows_kernel(int m, int n, int k, const float* __restrict__ X, long long ldx
     s_n = 0;
   }
   if (k <= kTopkFastK) {
-    // (fmaxf passes over NaNs: the bound only gets lower)
+    // (fmaxf passes over NaNs: a thread that saw nothing else counts as -inf)
     float mx = -INFINITY;
     const int n4 = VEC ? n / 4 : 0;
 #pragma unroll 4
@@ -327,7 +327,7 @@ topk_rows_kernel(int m, int n, int k, const float* __restrict__ X, long long ldx
     }
     __syncthreads();
     const int c = s_n;
-    if (c <= kTopkCands) {
+    if (k <= c && c <= kTopkCands) {
       for (int i = tid; i < c; i += kTopkThreads) {
         const unsigned key = s_key[i];
         const int col = s_col[i];
