@@ -87,11 +87,13 @@ int spmm_wide_launch(int64_t m, int64_t k, const int* pos, const int* crd, const
                      int64_t ldb, const float* bias, int relu, float* C, int64_t ldc, cudaStream_t st);
 
 #ifdef __CUDACC__
-// Launch of a kernel that waits for the kernel before it on the stream itself (griddepcontrol.wait):
-// its CTAs may be set up while that one still runs (a follow-up launch costs about a microsecond less).
+// Launch of a kernel; `early`: its CTAs may be set up while the kernel before it on the stream still
+// runs (a follow-up launch costs about a microsecond less).  An early kernel waits by itself
+// (griddepcontrol.wait) before it touches what that kernel, or one that kernel did not wait for, has
+// written: without the wait nothing orders its reads behind their writes.
 template <typename... P, typename... A>
-inline cudaError_t launch_early(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st,
-                                A... args) {
+inline cudaError_t launch_kernel(bool early, void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem,
+                                 cudaStream_t st, A... args) {
   cudaLaunchAttribute attr{};
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
@@ -101,8 +103,13 @@ inline cudaError_t launch_early(void (*kernel)(P...), dim3 grid, unsigned thread
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cfg.attrs = &attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = early ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+template <typename... P, typename... A>
+inline cudaError_t launch_early(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st,
+                                A... args) {
+  return launch_kernel(true, kernel, grid, threads, smem, st, args...);
 }
 #endif
 

@@ -1103,7 +1103,7 @@ static int max_abs(const WsLayout& w, const CsrIn& in, int64_t kb, cudaStream_t 
 
 template <typename T, bool NUMERIC>
 static int launch_smem_bin(const int* rows, int64_t count, const WsLayout& w, int64_t n, const CsrIn& in,
-                           const RowsOut& out, cudaStream_t st) {
+                           const RowsOut& out, bool early, cudaStream_t st) {
   const int smem = kSmemColumns / 8 + (NUMERIC ? (int)n * 8 : 0);
   // CTAs per row: as many as keep all of them (one per SM) on the GPU at a time
   unsigned parts = 8;
@@ -1111,24 +1111,24 @@ static int launch_smem_bin(const int* rows, int64_t count, const WsLayout& w, in
   if (parts == 1) {
     auto k = spgemm_smem_kernel<T, NUMERIC, false>;
     SB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    SB_CUDA(launch_early(k, dim3((unsigned)count), kSmemThreads, smem, st, rows, in, (int)n, w.max_b, out));
+    SB_CUDA(launch_kernel(early, k, dim3((unsigned)count), kSmemThreads, smem, st, rows, in, (int)n, w.max_b, out));
     return SB_OK;
   }
   auto k = spgemm_smem_kernel<T, NUMERIC, true>;
   SB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   cudaLaunchAttribute attr[2] = {};
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = parts;
-  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = parts;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)count * parts);
   cfg.blockDim = dim3(kSmemThreads);
   cfg.dynamicSmemBytes = (size_t)smem;
   cfg.stream = st;
   cfg.attrs = attr;
-  cfg.numAttrs = 2;
+  cfg.numAttrs = early ? 2 : 1;
   SB_CUDA(cudaLaunchKernelEx(&cfg, k, rows, in, (int)n, (const unsigned long long*)w.max_b, out));
   return SB_OK;
 }
@@ -1189,20 +1189,20 @@ static int big_rows(const WsLayout& w, int64_t count, int64_t m, int64_t n, cons
 
 template <typename T, bool NUMERIC, typename KEY>
 static int launch_warp_bin(const int* rows, int64_t count, const WsLayout& w, const CsrIn& in, int shift,
-                           const RowsOut& out, cudaStream_t st) {
+                           const RowsOut& out, bool early, cudaStream_t st) {
   constexpr int WARPS = 4;
-  SB_CUDA(launch_early(spgemm_warp_kernel<T, NUMERIC, KEY, WARPS>, dim3((unsigned)ceil_div(count, WARPS)), 32 * WARPS,
-                       0, st, rows, (int)count, w.upper, in, shift, out));
+  SB_CUDA(launch_kernel(early, spgemm_warp_kernel<T, NUMERIC, KEY, WARPS>, dim3((unsigned)ceil_div(count, WARPS)),
+                        32 * WARPS, 0, st, rows, (int)count, w.upper, in, shift, out));
   return SB_OK;
 }
 
 template <typename T, bool NUMERIC, typename KEY, int NT, int RMAX>
 static int launch_cta_bin(const int* rows, int64_t count, const WsLayout& w, const CsrIn& in, int shift,
-                          const RowsOut& out, cudaStream_t st) {
+                          const RowsOut& out, bool early, cudaStream_t st) {
   auto k = spgemm_cta_kernel<T, NUMERIC, KEY, NT, RMAX>;
   const int smem = RMAX * NT * (int)(sizeof(KEY) + (NUMERIC ? sizeof(Slot) : 0));
   SB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  SB_CUDA(launch_early(k, dim3((unsigned)count), NT, smem, st, rows, w.upper, in, shift, out));
+  SB_CUDA(launch_kernel(early, k, dim3((unsigned)count), NT, smem, st, rows, w.upper, in, shift, out));
   return SB_OK;
 }
 
@@ -1219,8 +1219,9 @@ static int launch_split_bin(const int* rows, int64_t count, const WsLayout& w, c
 
 // All rows; the longest first, so that the short ones fill in behind them: a bin's kernel lets the
 // next one start as soon as its own CTAs have (they do not depend on one another) and ends after the
-// one before it.  A key holds the column
-// above the product's ordinal: 32 bits where both fit.
+// one before it.  The first of them is an ordinary launch: it begins behind the completed work of the
+// stream (max |b|, the operands), and so do all that begin after it, which read these without a wait
+// of their own.  A key holds the column above the product's ordinal: 32 bits where both fit.
 template <typename T, bool NUMERIC>
 static int launch_bins(const WsLayout& w, const long long* counts, int64_t m, int64_t kb, int64_t n,
                        const CsrIn& in, const RowsOut& out, cudaStream_t st) {
@@ -1236,29 +1237,34 @@ static int launch_bins(const WsLayout& w, const long long* counts, int64_t m, in
   typedef unsigned K32;
   typedef unsigned long long K64;
   const int* rows = w.bin_rows;
+  bool early = false;
   if (counts[3] > 0) {
     // (a segment's part of the column and 13 bits of ordinal fit one key up to 2^24 columns)
     rc = nbits <= 24 ? launch_split_bin<T, NUMERIC>(rows + 3 * m, counts[3], w, in, nbits, out, st)
-                     : launch_cta_bin<T, NUMERIC, K64, 512, 16>(rows + 3 * m, counts[3], w, in, 13, out, st);
+                     : launch_cta_bin<T, NUMERIC, K64, 512, 16>(rows + 3 * m, counts[3], w, in, 13, out, early, st);
     if (rc != SB_OK) return rc;
+    early = true;
   }
   if (counts[2] > 0) {
-    rc = nbits <= 21 ? launch_cta_bin<T, NUMERIC, K32, 128, 16>(rows + 2 * m, counts[2], w, in, 11, out, st)
-                     : launch_cta_bin<T, NUMERIC, K64, 128, 16>(rows + 2 * m, counts[2], w, in, 11, out, st);
+    rc = nbits <= 21 ? launch_cta_bin<T, NUMERIC, K32, 128, 16>(rows + 2 * m, counts[2], w, in, 11, out, early, st)
+                     : launch_cta_bin<T, NUMERIC, K64, 128, 16>(rows + 2 * m, counts[2], w, in, 11, out, early, st);
     if (rc != SB_OK) return rc;
+    early = true;
   }
   if (counts[1] > 0) {
-    rc = nbits <= 23 ? launch_cta_bin<T, NUMERIC, K32, 64, 8>(rows + m, counts[1], w, in, 9, out, st)
-                     : launch_cta_bin<T, NUMERIC, K64, 64, 8>(rows + m, counts[1], w, in, 9, out, st);
+    rc = nbits <= 23 ? launch_cta_bin<T, NUMERIC, K32, 64, 8>(rows + m, counts[1], w, in, 9, out, early, st)
+                     : launch_cta_bin<T, NUMERIC, K64, 64, 8>(rows + m, counts[1], w, in, 9, out, early, st);
     if (rc != SB_OK) return rc;
+    early = true;
   }
   if (counts[0] > 0) {
-    rc = nbits <= 25 ? launch_warp_bin<T, NUMERIC, K32>(rows, counts[0], w, in, 7, out, st)
-                     : launch_warp_bin<T, NUMERIC, K64>(rows, counts[0], w, in, 7, out, st);
+    rc = nbits <= 25 ? launch_warp_bin<T, NUMERIC, K32>(rows, counts[0], w, in, 7, out, early, st)
+                     : launch_warp_bin<T, NUMERIC, K64>(rows, counts[0], w, in, 7, out, early, st);
     if (rc != SB_OK) return rc;
+    early = true;
   }
   if (counts[4] > 0 && in_smem)
-    rc = launch_smem_bin<T, NUMERIC>(rows + 4 * m, counts[4], w, n, in, out, st);
+    rc = launch_smem_bin<T, NUMERIC>(rows + 4 * m, counts[4], w, n, in, out, early, st);
   return rc;
 }
 

@@ -1,0 +1,71 @@
+"""Which launches may begin before the one ahead of them has completed: the library's host code runs over a
+stand-in for the CUDA runtime (launch_recorder.cpp) that notes its launches.  A kernel that reads what an
+earlier kernel wrote without waiting by itself has to come behind an ordinary launch."""
+from __future__ import annotations
+
+import ctypes as C
+import glob
+import itertools
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+from conftest import ROOT
+
+
+@pytest.fixture(scope="module")
+def recorded(tmp_path_factory):
+    from torch.utils import cpp_extension as ext
+
+    from scorch_b200 import _lib, build
+    build.build()
+    path = str(tmp_path_factory.mktemp("recorder") / "librecorded.so")
+    include = [f"-I{d}" for d in ext.include_paths("cuda") + ["/usr/local/cuda/include"]]
+    subprocess.check_call([build._host_cxx(), "-O1", "-std=c++17", "-shared", "-fPIC", "-Wl,-Bsymbolic", *include,
+                           os.path.join(ROOT, "tests", "launch_recorder.cpp"),
+                           *sorted(glob.glob(os.path.join(build.OBJDIR, "*.o"))), "-o", path])
+    lib = C.CDLL(path)
+    for name, (res, args) in _lib.SIGNATURES.items():
+        getattr(lib, name).restype, getattr(lib, name).argtypes = res, args
+    lib.recorder_kernel.restype = C.c_char_p
+
+    class Recorded:
+        abi = lib
+
+        @staticmethod
+        def call(fn, *args):
+            """(kernel name, begins early, CTAs per cluster) of the call's launches."""
+            lib.recorder_reset()
+            assert fn(*args) == 0, lib.sb_last_error()
+            return [(lib.recorder_kernel(i).decode(), bool(lib.recorder_early(i)), lib.recorder_cluster(i))
+                    for i in range(lib.recorder_count())]
+    return Recorded
+
+
+def _ptr(a):
+    return a.ctypes.data
+
+
+@pytest.mark.parametrize("dtype", [0, 1, 2, 3])
+@pytest.mark.parametrize("n", [1000, 30000])
+def test_spgemm_rows_begin_behind_max_abs(recorded, dtype, n):
+    # the first kernel of the bins, whichever it is, is an ordinary launch: it and those that begin beside it
+    # read max |b| and the operands without a wait
+    m = 64
+    i32, i64 = (lambda k: np.zeros(k, np.int32)), (lambda k: np.zeros(k, np.int64))
+    ws = np.zeros(recorded.abi.sb_spgemm_workspace_bytes(m, n, dtype) + 16, np.uint8)
+    pos, crd, val, off, tcrd, tval, cpos = i32(m + 1), i32(4), i64(4), i32(m + 1), i32(4), i64(4), i32(m + 1)
+    for bins in itertools.product((0, 7), repeat=5):
+        if not any(bins) or (n > 24576 and bins[4]):        # (the bucket path reads its rows back)
+            continue
+        got = recorded.call(recorded.abi.sb_spgemm_rows, dtype, m, m, n, _ptr(pos), _ptr(crd), _ptr(val), _ptr(pos),
+                            _ptr(crd), _ptr(val), _ptr(off), (C.c_int64 * 5)(*bins), _ptr(tcrd), _ptr(tval),
+                            _ptr(cpos), C.byref(C.c_int64(0)), (_ptr(ws) + 15) // 16 * 16, ws.size - 16, None)
+        rows = [g for g in got if any(k in g[0] for k in ("warp_kernel", "cta_kernel", "split_kernel", "smem_kernel"))]
+        assert len(rows) == sum(b > 0 for b in bins)
+        assert [early for _, early, _ in rows] == [False] + [True] * (len(rows) - 1), rows
+        assert ("max_abs" in got[0][0]) == (bins[4] > 0 and dtype < 2) and not got[0][1]
+        assert ("smem_kernel" in rows[-1][0]) == (bins[4] > 0) and rows[-1][2] == (8 if bins[4] else 1)
+        assert "scan" in got[-1][0] and not got[-1][1]       # behind all of them
