@@ -383,10 +383,12 @@ static int launch_tiles(const SpmmArgs<T>& a, int64_t nnz, void* ws, cudaStream_
     const bool resident = !in_l2 && t.tiles <= 148 * tile_ctas(L);
     SB_CUDA(launch_early(kernel, dim3((unsigned)t.tiles, resident ? 1 : panels), kTileThreadsMm, sizeof(Smem), st, a, t));
   }
-  // (may be set up while the tiles still run: it waits for them itself)
-  SB_CUDA(launch_early(spmm_tile_rows_kernel<T>,
-                       dim3((unsigned)ceil_div(a.m, kTileThreadsMm), (unsigned)std::min<int64_t>(ceil_div(a.k, 32), 64)),
-                       kTileThreadsMm, 0, st, a, t));
+  // (may be set up while the tiles still run: it waits for them itself.  It reads the row pointers before
+  // that, which is sound behind the tile kernel, whose CTAs have waited for whatever made them; a
+  // matrix without entries has no tile kernel, and an ordinary launch)
+  SB_CUDA(launch_kernel(t.tiles > 0, spmm_tile_rows_kernel<T>,
+                        dim3((unsigned)ceil_div(a.m, kTileThreadsMm), (unsigned)std::min<int64_t>(ceil_div(a.k, 32), 64)),
+                        kTileThreadsMm, 0, st, a, t));
   return SB_OK;
 }
 

@@ -69,3 +69,19 @@ def test_spgemm_rows_begin_behind_max_abs(recorded, dtype, n):
         assert ("max_abs" in got[0][0]) == (bins[4] > 0 and dtype < 2) and not got[0][1]
         assert ("smem_kernel" in rows[-1][0]) == (bins[4] > 0) and rows[-1][2] == (8 if bins[4] else 1)
         assert "scan" in got[-1][0] and not got[-1][1]       # behind all of them
+
+
+@pytest.mark.parametrize("dtype", [0, 1, 2, 3])
+@pytest.mark.parametrize("k", [1, 16, 77, 600])
+@pytest.mark.parametrize("accumulate", [0, 1])
+def test_spmm_without_entries_begins_behind_its_operands(recorded, dtype, k, accumulate):
+    # the second kernel reads the row pointers before its wait: behind the tile kernel that is sound, alone it
+    # has to be an ordinary launch
+    pos, val, out = np.zeros(10, np.int32), np.zeros(4, np.int64), np.zeros(9 * k, np.int64)
+    ws = np.zeros(recorded.abi.sb_spmm_csr_once_workspace_bytes(dtype, k, 4) + 16, np.uint8)
+    for nnz in (0, 4):
+        got = recorded.call(recorded.abi.sb_spmm_csr_once, dtype, 9, 4, k, nnz, _ptr(pos), _ptr(pos), _ptr(val),
+                            _ptr(out), k, None, 0, accumulate, _ptr(out), k, (_ptr(ws) + 15) // 16 * 16, ws.size - 16,
+                            None)
+        assert "spmm_tile_rows_kernel" in got[-1][0]
+        assert [early for _, early, _ in got] == ([True, True] if nnz else [False]), got
