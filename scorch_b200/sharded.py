@@ -70,7 +70,7 @@ class CsrBlock:
     crd: torch.Tensor          # int32 [nnz]
     val: torch.Tensor
     plan: object = None
-    columns: object = None     # (chunks, kernels.ColumnSplit or None) for operands much larger than L2
+    columns: object = None     # (key, kernels.ColumnSplit or None) for operands much larger than L2: columns_for
 
     @property
     def rows(self) -> int:
@@ -79,6 +79,27 @@ class CsrBlock:
     @property
     def nnz(self) -> int:
         return int(self.crd.numel())
+
+    def columns_for(self, n: int, k: int):
+        """The block cut by columns (``kernels.ColumnSplit``) for products with an (n x k) operand, or None
+        where that does not pay.  The split holds a copy of the block's indices and values (8 bytes per
+        entry).  It is kept until one of the block's tensors is written in place (as its version counter
+        tells) or replaced; tensors that do not count their writes (inference mode) are cut on every call."""
+        from . import kernels as K
+        chunks = K.split_chunks(self.rows, n, self.nnz, k)
+        if not chunks:
+            return None
+        sources = (self.pos, self.crd, self.val)
+        counted = not any(t.is_inference() for t in sources)
+        # (the key holds the tensors: another tensor cannot take their place in memory meanwhile)
+        key = (chunks, n, [(t._version, t.data_ptr()) for t in sources] if counted else None, sources)
+        kept = self.columns
+        if (counted and kept is not None and kept[0][:3] == key[:3]
+                and all(a is b for a, b in zip(kept[0][3], sources))):
+            return kept[1]
+        split = K.ColumnSplit.of(self.pos, self.crd, self.val, n, k)
+        self.columns = (key, split)
+        return split
 
 
 def row_block(pos: torch.Tensor, crd: torch.Tensor, val: torch.Tensor, rank: int, world: int,
@@ -247,13 +268,10 @@ def _default_spmm(block: CsrBlock, B: torch.Tensor, out: torch.Tensor, relu: boo
     from . import kernels as K
     # (an operand that L2 nearly holds whole is multiplied in one pass)
     if B.is_contiguous() and out.is_contiguous() and 4 * B.numel() > 1.3 * K.SPLIT_CHUNK_BYTES:
-        chunks = K.split_chunks(block.rows, B.shape[0], block.nnz, B.shape[1])
-        if chunks:
-            if block.columns is None or block.columns[0] != chunks:
-                block.columns = chunks, K.ColumnSplit.of(block.pos, block.crd, block.val, B.shape[0], B.shape[1])
-            if block.columns[1] is not None:
-                block.columns[1].matmul(B, relu, out=out, accumulate=accumulate)
-                return
+        split = block.columns_for(B.shape[0], B.shape[1])
+        if split is not None:
+            split.matmul(B, relu, out=out, accumulate=accumulate)
+            return
     if block.plan is None:
         block.plan = K.CsrPlan(block.pos, block.nnz)
     K.spmm_csr(block.pos, block.crd, block.val, B, relu=relu, plan=block.plan, out=out,

@@ -77,3 +77,62 @@ def test_sharded_forward_by_column_chunks(monkeypatch, chunks):
         got = S.gcn_forward_sharded(shard, X, W1, W2)
         assert ((got.double() - want).norm() / want.norm()).item() < 1e-6
     assert all(b.columns[1] is not None for b in shard.blocks)
+
+
+@pytest.mark.parametrize("chunks", [1, 2])
+def test_sharded_forward_sees_values_written_in_place(monkeypatch, chunks):
+    # with one row chunk the block's arrays are the caller's own: the kept split has to follow them
+    from scorch_b200 import kernels as K, sharded as S
+    monkeypatch.setattr(K, "SPLIT_CHUNK_BYTES", 1e5)
+    pos, crd, val = _csr([60] * 2000, 2000, seed=5)
+    g = torch.Generator().manual_seed(2)
+    X, W1, W2 = (torch.randn(s, generator=g).cuda() for s in ((2000, 64), (64, 72), (72, 64)))
+    p, c, v = (torch.from_numpy(a).cuda() for a in (pos, crd, val))
+    shard = S.ShardedCsr.from_global(p, c, v, 0, 1, chunks=chunks)
+    blocks = shard.blocks
+
+    def check():
+        # (the pieces' columns are numbered from 0)
+        A = torch.cat([torch.sparse_csr_tensor(b.pos, b.crd, b.val, size=(2000, 2000 // chunks)).to_dense()
+                       for b in blocks], 1).double()
+        want = A @ (torch.relu(A @ (X.double() @ W1.double())) @ W2.double())
+        got = S.gcn_forward_sharded(shard, X, W1, W2)
+        assert ((got.double() - want).norm() / want.norm()).item() < 1e-6
+
+    check()
+    assert all(b.columns[1] is not None for b in blocks)
+    kept = [b.columns[1] for b in blocks]
+    check()
+    assert all(b.columns[1] is k for b, k in zip(blocks, kept))          # nothing was written: cut once
+    for b in blocks:
+        b.val.mul_(torch.linspace(0.5, 2.0, b.nnz, device="cuda"))
+    check()
+    if chunks == 1:
+        v[::3] = 0.25                                                    # through the caller's tensor
+        check()
+    for b in blocks:
+        last = torch.full_like(b.crd, 2000 // chunks - 1)
+        b.crd.copy_(last - torch.flip(b.crd, (0,)))                      # other columns, ascending in a row again
+        b.pos.copy_(b.nnz - torch.flip(b.pos, (0,)))
+    check()
+    for b in blocks:
+        b.val = torch.ones_like(b.val)                                   # another tensor
+    check()
+
+
+def test_sharded_forward_in_inference_mode(monkeypatch):
+    # tensors made there count no writes
+    from scorch_b200 import kernels as K, sharded as S
+    monkeypatch.setattr(K, "SPLIT_CHUNK_BYTES", 1e5)
+    pos, crd, val = _csr([60] * 2000, 2000, seed=6)
+    with torch.inference_mode():
+        g = torch.Generator().manual_seed(3)
+        X, W1, W2 = (torch.randn(s, generator=g).cuda() for s in ((2000, 64), (64, 72), (72, 64)))
+        p, c, v = (torch.from_numpy(a).cuda() for a in (pos, crd, val))
+        shard = S.ShardedCsr.from_global(p, c, v, 0, 1)
+        for _ in range(2):
+            A = torch.sparse_csr_tensor(p, c, v, size=(2000, 2000)).to_dense().double()
+            want = A @ (torch.relu(A @ (X.double() @ W1.double())) @ W2.double())
+            got = S.gcn_forward_sharded(shard, X, W1, W2)
+            assert ((got.double() - want).norm() / want.norm()).item() < 1e-6
+            v.mul_(-0.5)
