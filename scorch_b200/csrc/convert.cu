@@ -170,14 +170,19 @@ __global__ void transpose_gather_kernel(long long nnz, const int* __restrict__ p
 }
 
 // ---- per-row top-k -> CSR ----------------------------------------------------------------------
-// Keys order like the floats: larger float <-> larger unsigned key (NaN above +inf, as torch.topk).
-__device__ __forceinline__ unsigned topk_key(float x) {
-  const unsigned u = __float_as_uint(x);
-  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+// Keys order like the floats: larger float <-> larger unsigned key (NaN above +inf, as torch.topk; one
+// with the sign bit set below -inf).  Whole-number arithmetic on the loaded bits: a sign bit set by `or` on a
+// float's bits was compiled to a float operation, which turns every NaN into one pattern (0x7fc00000
+// then ordered as -0, and came back as -0).
+__device__ __forceinline__ unsigned topk_key(unsigned u) { return u ^ ((unsigned)((int)u >> 31) | 0x80000000u); }
+// ... and back.
+__device__ __forceinline__ unsigned topk_bits(unsigned key) {
+  return key ^ (~(unsigned)((int)key >> 31) | 0x80000000u);
 }
+__device__ __forceinline__ bool topk_positive(unsigned u) { return u - 1u < 0x7f800000u; }   // (false for NaN)
 
-__device__ __forceinline__ float topk_value(unsigned key) {
-  return __uint_as_float((key & 0x80000000u) ? (key & 0x7fffffffu) : ~key);
+__device__ __forceinline__ unsigned ld_stream_u32(const unsigned* p) {
+  return (unsigned)ld_stream(reinterpret_cast<const int*>(p));
 }
 
 constexpr int kTopkThreads = 512;
@@ -187,8 +192,8 @@ constexpr int kTopkFastK = kTopkThreads / 2;
 // Any input: four 8-bit radix passes find the key T of the k-th largest element and how many elements
 // equal to T are still needed; a last pass keeps, in column order, every element above T and the
 // first `need` elements equal to T (ties go to the lower column).  The whole CTA, one row.
-__device__ __noinline__ void topk_row_radix(int n, int k, const float* __restrict__ x, int relu, long long out0,
-                                            int* __restrict__ crd, float* __restrict__ val) {
+__device__ __noinline__ void topk_row_radix(int n, int k, const unsigned* __restrict__ x, int relu, long long out0,
+                                            int* __restrict__ crd, unsigned* __restrict__ val) {
   __shared__ int hist[256];
   __shared__ unsigned s_prefix;
   __shared__ int s_need;
@@ -201,7 +206,7 @@ __device__ __noinline__ void topk_row_radix(int n, int k, const float* __restric
     if (tid < 256) hist[tid] = 0;
     __syncthreads();
     for (int j = tid; j < n; j += kTopkThreads) {
-      const unsigned key = topk_key(ld_stream(x + j));
+      const unsigned key = topk_key(ld_stream_u32(x + j));
       if ((key & mask) == prefix) atomicAdd(&hist[(key >> shift) & 255u], 1);
     }
     __syncthreads();
@@ -225,10 +230,10 @@ __device__ __noinline__ void topk_row_radix(int n, int k, const float* __restric
   __syncthreads();
   for (int j0 = 0; j0 < n; j0 += kTopkThreads) {
     const int j = j0 + tid;
-    float v = 0.f;
+    unsigned v = 0;
     bool gt = false, eq = false;
     if (j < n) {
-      v = ld_stream(x + j);
+      v = ld_stream_u32(x + j);
       const unsigned key = topk_key(v);
       gt = key > prefix;
       eq = key == prefix;
@@ -246,7 +251,7 @@ __device__ __noinline__ void topk_row_radix(int n, int k, const float* __restric
     const int slot = s_out + gt_before + __popc(m_gt & below) + eq_kept_before;
     if (keep) {
       crd[out0 + slot] = j;
-      val[out0 + slot] = (relu && !(v > 0.f)) ? 0.f : v;
+      val[out0 + slot] = (relu && !topk_positive(v)) ? 0u : v;
     }
     __syncthreads();
     if (tid == 0) {
@@ -273,14 +278,14 @@ __device__ __noinline__ void topk_row_radix(int n, int k, const float* __restric
 // elements).
 template <bool VEC>
 __global__ void __launch_bounds__(kTopkThreads, 4)
-topk_rows_kernel(int m, int n, int k, const float* __restrict__ X, long long ldx, int relu,
-                 int* __restrict__ pos, int* __restrict__ crd, float* __restrict__ val) {
+topk_rows_kernel(int m, int n, int k, const unsigned* __restrict__ X, long long ldx, int relu,
+                 int* __restrict__ pos, int* __restrict__ crd, unsigned* __restrict__ val) {
   __shared__ unsigned s_key[kTopkCands];
   __shared__ int s_col[kTopkCands];
   __shared__ unsigned char s_keep[kTopkCands];
   __shared__ int s_n;
   const int tid = threadIdx.x;
-  const float* x = X + (long long)blockIdx.x * ldx;
+  const unsigned* x = X + (long long)blockIdx.x * ldx;   // bits of the floats
   const long long out0 = (long long)blockIdx.x * k;
   if (tid == 0) {
     pos[blockIdx.x] = (int)out0;
@@ -289,41 +294,42 @@ topk_rows_kernel(int m, int n, int k, const float* __restrict__ X, long long ldx
   }
   if (k <= kTopkFastK) {
     // (fmaxf passes over NaNs: a thread that saw nothing else counts as -inf)
+    auto value = [](unsigned u) { return __uint_as_float(u); };
     float mx = -INFINITY;
     const int n4 = VEC ? n / 4 : 0;
 #pragma unroll 4
     for (int q = tid; q < n4; q += kTopkThreads) {
-      const float4 v = __ldg(reinterpret_cast<const float4*>(x) + q);
-      mx = fmaxf(mx, fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)));
+      const uint4 v = __ldg(reinterpret_cast<const uint4*>(x) + q);
+      mx = fmaxf(mx, fmaxf(fmaxf(value(v.x), value(v.y)), fmaxf(value(v.z), value(v.w))));
     }
 #pragma unroll 4
-    for (int j = 4 * n4 + tid; j < n; j += kTopkThreads) mx = fmaxf(mx, __ldg(x + j));
+    for (int j = 4 * n4 + tid; j < n; j += kTopkThreads) mx = fmaxf(mx, value(__ldg(x + j)));
     // largest v such that k threads have (upper half of the key of) their maximum >= v
-    const unsigned top = topk_key(mx) >> 16;
+    const unsigned top = topk_key(__float_as_uint(mx)) >> 16;
     unsigned v = 0;
     for (unsigned bit = 1u << 15; bit; bit >>= 1)
       if (__syncthreads_count(top >= (v | bit)) >= k) v |= bit;
     const unsigned bound = v << 16;
     // the elements that reach the bound
-    auto take = [&](float f, int j) {
-      const unsigned key = topk_key(f);
+    auto take = [&](unsigned u, int j) {
+      const unsigned key = topk_key(u);
       if (key < bound) return;
       const int i = atomicAdd(&s_n, 1);
       if (i < kTopkCands) { s_key[i] = key; s_col[i] = j; }
     };
-    const float fb = topk_value(bound);
+    const float fb = value(topk_bits(bound));
 #pragma unroll 4
     for (int q = tid; q < n4; q += kTopkThreads) {
-      const float4 f = __ldg(reinterpret_cast<const float4*>(x) + q);
+      const uint4 f = __ldg(reinterpret_cast<const uint4*>(x) + q);
       // (!(f < fb) lets NaNs through, as the key order wants)
-      if (!(f.x < fb) || !(f.y < fb) || !(f.z < fb) || !(f.w < fb)) {
+      if (!(value(f.x) < fb) || !(value(f.y) < fb) || !(value(f.z) < fb) || !(value(f.w) < fb)) {
         take(f.x, 4 * q); take(f.y, 4 * q + 1); take(f.z, 4 * q + 2); take(f.w, 4 * q + 3);
       }
     }
 #pragma unroll 4
     for (int j = 4 * n4 + tid; j < n; j += kTopkThreads) {
-      const float f = __ldg(x + j);
-      if (!(f < fb)) take(f, j);
+      const unsigned f = __ldg(x + j);
+      if (!(value(f) < fb)) take(f, j);
     }
     __syncthreads();
     const int c = s_n;
@@ -341,9 +347,9 @@ topk_rows_kernel(int m, int n, int k, const float* __restrict__ X, long long ldx
         const int col = s_col[i];
         int slot = 0;
         for (int j = 0; j < c; j++) slot += s_keep[j] && s_col[j] < col;
-        const float f = topk_value(s_key[i]);
+        const unsigned u = topk_bits(s_key[i]);
         crd[out0 + slot] = col;
-        val[out0 + slot] = (relu && !(f > 0.f)) ? 0.f : f;
+        val[out0 + slot] = (relu && !topk_positive(u)) ? 0u : u;
       }
       return;
     }
@@ -438,10 +444,13 @@ int sb_topk_rows_to_csr_f32(int64_t m, int64_t n, int64_t k, const float* X, int
     return SB_OK;
   }
   SB_CHECK_ARG(X && crd && val, "topk_rows: null pointer");
+  const unsigned* bits = reinterpret_cast<const unsigned*>(X);
   if (ldx % 4 == 0 && aligned16(X))
-    topk_rows_kernel<true><<<(unsigned)m, kTopkThreads, 0, st>>>((int)m, (int)n, (int)k, X, ldx, relu, pos, crd, val);
+    topk_rows_kernel<true><<<(unsigned)m, kTopkThreads, 0, st>>>((int)m, (int)n, (int)k, bits, ldx, relu, pos, crd,
+                                                                       (unsigned*)val);
   else
-    topk_rows_kernel<false><<<(unsigned)m, kTopkThreads, 0, st>>>((int)m, (int)n, (int)k, X, ldx, relu, pos, crd, val);
+    topk_rows_kernel<false><<<(unsigned)m, kTopkThreads, 0, st>>>((int)m, (int)n, (int)k, bits, ldx, relu, pos, crd,
+                                                                       (unsigned*)val);
   SB_LAUNCH_CHECK("topk_rows_kernel");
   return SB_OK;
 }

@@ -42,10 +42,10 @@ def test_topk_rows_of_a_wider_buffer():
     assert all(np.array_equal(g.cpu().numpy(), w) for g, w in zip(got, want))
 
 
-@pytest.mark.parametrize("n,k", [(33, 32), (512, 8), (1000, 256), (3000, 2), (4096, 32), (32768, 64)])
-@pytest.mark.parametrize("numbers", [0, 1, 5])
+@pytest.mark.parametrize("n,k", [(33, 32), (512, 8), (1000, 256), (1000, 300), (3000, 2), (4096, 32), (32768, 64)])
+@pytest.mark.parametrize("numbers", [0, 1, 5, 400])
 def test_topk_rows_of_nans(n, k, numbers):
-    # Rows that hold fewer than k numbers.  A NaN with the sign bit set (0xffc00000, what x86 arithmetic
+    # Rows of few numbers, many of them fewer than k.  A NaN with the sign bit set (0xffc00000, what x86 arithmetic
     # yields) orders below -inf, one without above +inf; equal bits go to the lower column.
     from scorch_b200 import kernels as K
     rng = np.random.default_rng(n + k + numbers)
@@ -54,10 +54,13 @@ def test_topk_rows_of_nans(n, k, numbers):
     bits[2, rng.choice(n, 3, replace=False)] = 0x7FC00000
     bits[3, rng.choice(n, 3, replace=False)] = 0xFF800000              # -inf
     for row in bits:
-        row[rng.choice(n, numbers, replace=False)] = rng.standard_normal(numbers).astype(np.float32).view(np.uint32)
+        at = rng.choice(np.flatnonzero(row >= 0xFFC00000), min(numbers, n // 2), replace=False)
+        row[at] = rng.standard_normal(at.size).astype(np.float32).view(np.uint32)
     pos, crd, val = K.topk_rows_to_csr(torch.from_numpy(bits.view(np.float32)).cuda(), k)
     key = np.where(bits >> 31, ~bits, bits | np.uint32(0x80000000)).astype(np.int64)
     want = np.sort(np.argsort(-key, axis=1, kind="stable")[:, :k], axis=1)
     assert np.array_equal(pos.cpu().numpy(), np.arange(5) * k)
     assert np.array_equal(crd.cpu().numpy().reshape(4, k), want)
     assert np.array_equal(val.cpu().numpy().view(np.uint32).reshape(4, k), np.take_along_axis(bits, want, 1))
+    relu = K.topk_rows_to_csr(torch.from_numpy(bits.view(np.float32)).cuda(), k, relu=True)
+    assert torch.equal(relu[1], crd) and torch.equal(relu[2], torch.where(val > 0, val, torch.zeros_like(val)))
