@@ -170,8 +170,13 @@ SB_API int sb_spmm_csr_typed(int dtype, int64_t m, int64_t n, int64_t k, int64_t
  * feature transforms of a graph layer, A tall (m x k, row pitch lda), W small (k x n).  k <= 32768 and
  * lda multiples of 4, A 16-byte aligned; ldc a multiple of 8, C 32-byte aligned (SB_ERR_UNSUPPORTED
  * otherwise); ws: sb_dense_matmul_workspace_bytes(n, k) bytes, 16-byte aligned.
- * sb_dense_matmul_status() (synchronises): 0, or 1 when a wait inside the kernel ever ran out, or -1
- * when it could not be read.
+ * Any values: rows of A with values of 2^127 and above, Inf or NaN, and every row where W holds one, take
+ * fp32 FMAs instead of the tensor cores, as do the rows behind a wait inside the kernel that ran out.
+ * sb_dense_matmul_status() (synchronises): 0, or 1 when such a wait ever ran out, or -1 when it could not
+ * be read.
+ * sb_dense_matmul_probe: self-test.  The tensor cores' issuing thread of every CTA stops at its 32-row
+ * chunk of K number `stop` (>= 0, counted over the CTA's tiles), so that the others' waits run out; returns,
+ * synchronised, the status of that call and leaves sb_dense_matmul_status() as it was.
  * Replaces: the torch.matmul(X, W) of the reference's caller, bench/bench_gcn.py:314-329.
  * -------------------------------------------------------------------------------------------- */
 SB_API size_t sb_dense_matmul_workspace_bytes(int64_t n, int64_t k);
@@ -179,6 +184,9 @@ SB_API int sb_dense_matmul_f32(int64_t m, int64_t n, int64_t k, const float* A, 
                                const float* W, int64_t ldw, float* C, int64_t ldc, void* ws,
                                size_t ws_bytes, void* stream);
 SB_API int sb_dense_matmul_status(void);
+SB_API int sb_dense_matmul_probe(int64_t m, int64_t n, int64_t k, const float* A, int64_t lda,
+                                 const float* W, int64_t ldw, float* C, int64_t ldc, void* ws,
+                                 size_t ws_bytes, int stop, int* status_host, void* stream);
 
 /* --------------------------------------------------------------------------------------------
  * CSR SpMV: y[i] = sum_p val[p] * x[crd[p]].  Every y[i] is written.

@@ -48,6 +48,8 @@ SIGNATURES = {
     "sb_dense_matmul_workspace_bytes": (_sz, [_i64, _i64]),
     "sb_dense_matmul_f32": (_int, [_i64, _i64, _i64, _ptr, _i64, _ptr, _i64, _ptr, _i64, _ptr, _sz, _ptr]),
     "sb_dense_matmul_status": (_int, []),
+    "sb_dense_matmul_probe": (_int, [_i64, _i64, _i64, _ptr, _i64, _ptr, _i64, _ptr, _i64, _ptr, _sz, _int,
+                                     C.POINTER(_int), _ptr]),
     "sb_spmv_csr_scratch_bytes": (_sz, [_i64]),
     "sb_spmv_csr_f32": (_int, [_i64, _i64, _i64, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _sz, _ptr]),
     "sb_spmv_csr_typed": (_int, [_int, _i64, _i64, _i64, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr]),

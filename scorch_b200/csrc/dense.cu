@@ -21,8 +21,10 @@
 //   * one thread issues the 12 tcgen05.mma (M 128, N up to 128, K 16) of a chunk into one of two pairs
 //     of accumulators in tensor memory;
 //   * four warps write the other pair to C, so that the stores overlap the next tile's products.
-// Every wait is bounded; one that runs out sets a status word and ends the CTA.
-// Tiles that hold a value too large for the split (2^127 and above, Inf, NaN) are done again with fp32 FMAs.
+// Every wait is bounded; one that runs out sets a status word and ends the CTA's pipeline.
+// The CTA's tiles that the pipeline left - behind a wait that ran out, or with a value too large for the
+// split (2^127 and above, Inf, NaN) in the rows of A, or all of them with one in W - it does with fp32
+// FMAs at its end, so C is complete whatever happened.
 #include <algorithm>
 
 #include "tensor_core.cuh"
@@ -32,6 +34,7 @@ namespace sb {
 constexpr int kGemmRows = 128, kGemmK = 32;
 constexpr int kGemmProducers = 256, kGemmThreads = kGemmProducers + 128 + 32;
 constexpr int kRaw = 4;                       // chunks of A on their way
+constexpr int kRedoWords = 512;               // tiles of a CTA that are noted one by one (14,170 at most on 148 SMs)
 constexpr unsigned kSplitMax = 0x7f000000u;   // bits of 2^127: values from here on, Inf and NaN are not split
 
 __device__ int g_gemm_status = 0;  // 0 ok; 1 a wait ran out
@@ -49,6 +52,7 @@ struct GemmArgs {
   long long ldc;
   int tiles, chunks;   // row tiles x column panels; 32-column chunks of K
   int panels;
+  int stop;            // self-test: the issuing thread gives up at this chunk of every CTA (-1: never)
 };
 
 // Two values as three packed pairs of bf16 parts.
@@ -123,11 +127,59 @@ struct GemmSmem {
   // the tile (its number mod 8) holds a value the split cannot take; the producers are at most
   // 2 + STAGES tiles ahead of the epilogue, so a place is free again before it is used again
   int odd[8];
+  int done;                   // tiles the epilogue has finished ...
+  unsigned redo[kRedoWords];  // ... and those among them that it has left out (odd), a bit each
 };
+
+// One tile by fp32 FMAs, in the order of K: 256 threads, 4 rows x NMAX / 16 columns each at a time,
+// operands through L1 (2 M x 256 x 256: 18.3 ms against cuBLAS's 4.6; one thread per row, which the epilogue
+// used to fall back on, took 474).
+template <int NMAX>
+__device__ __forceinline__ void gemm_redo_tile(const GemmArgs& g, long long row0, int n0) {
+  constexpr int RT = 4, CT = NMAX / 16;
+  if (threadIdx.x >= 256) return;
+  const int cols = min(NMAX, g.n - n0), cl = threadIdx.x & 15, rl = threadIdx.x >> 4;
+#pragma unroll 1
+  for (int r0 = rl; r0 < kGemmRows; r0 += 16 * RT) {
+    const float* a[RT];
+#pragma unroll
+    for (int i = 0; i < RT; i++) a[i] = g.A + min(row0 + r0 + 16 * i, g.m - 1) * g.lda;
+    float acc[RT][CT];
+#pragma unroll
+    for (int i = 0; i < RT; i++) {
+#pragma unroll
+      for (int j = 0; j < CT; j++) acc[i][j] = 0.f;
+    }
+#pragma unroll 1
+    for (int k = 0; k < g.k; k += 4) {
+      float4 x[RT];
+#pragma unroll
+      for (int i = 0; i < RT; i++) x[i] = ldg4(a[i] + k);
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        const float* w = g.W + (k + q) * g.ldw + n0 + cl;
+#pragma unroll
+        for (int j = 0; j < CT; j++) {
+          const float y = cl + 16 * j < cols ? __ldg(w + 16 * j) : 0.f;
+#pragma unroll
+          for (int i = 0; i < RT; i++)
+            acc[i][j] = fmaf(q == 0 ? x[i].x : q == 1 ? x[i].y : q == 2 ? x[i].z : x[i].w, y, acc[i][j]);
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < RT; i++) {
+      const long long row = row0 + r0 + 16 * i;
+#pragma unroll
+      for (int j = 0; j < CT; j++)
+        if (row < g.m && cl + 16 * j < cols) g.C[row * g.ldc + n0 + cl + 16 * j] = acc[i][j];
+    }
+  }
+}
 
 template <int NMAX, int STAGES>
 __global__ void __launch_bounds__(kGemmThreads, 1)
-gemm_f32_kernel(GemmArgs g) {
+gemm_f32_kernel(const __grid_constant__ GemmArgs g) {
   using Smem = GemmSmem<NMAX, STAGES>;
   constexpr uint32_t TMEM_COLS = 4 * NMAX;       // two pairs of accumulators
   constexpr uint32_t GROUP = 8 * kGemmK * 2;     // bytes of an 8-row group: 4 core matrices of 128 bytes
@@ -144,8 +196,10 @@ gemm_f32_kernel(GemmArgs g) {
       mbar_init(smem_u32(&sm.acc_empty[i]), 128);
     }
     for (int i = 0; i < 8; i++) sm.odd[i] = 0;
+    sm.done = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  for (int i = threadIdx.x; i < kRedoWords; i += kGemmThreads) sm.redo[i] = 0;
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
                  ::"r"(smem_u32(&sm.tmem)), "r"(TMEM_COLS) : "memory");
@@ -157,7 +211,8 @@ gemm_f32_kernel(GemmArgs g) {
   asm volatile("griddepcontrol.wait;" ::: "memory");   // the parts of W
   const uint32_t tmem = sm.tmem;
   const int my_tiles = ((int)blockIdx.x < g.tiles) ? (g.tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
-  const int steps = my_tiles * g.chunks;
+  // (a value of W that cannot be split: no tile takes the tensor cores)
+  const int run_tiles = *g.w_flag ? 0 : my_tiles, steps = run_tiles * g.chunks;
   auto tile_of = [&](int i) { return (int)blockIdx.x + i * (int)gridDim.x; };
   auto give_up = [&]() { atomicExch(&g_gemm_status, 1); };
 
@@ -244,6 +299,7 @@ gemm_f32_kernel(GemmArgs g) {
       int i = 0, c = 0, stage = 0, use = 0;
       uint32_t acc = 0, idesc = 0;
       for (int step = 0; step < steps; step++) {
+        if (step == g.stop) { give_up(); break; }
         if (c == 0) {
           acc = tmem + (uint32_t)((i & 1) * 2 * NMAX);
           const int cols = min(NMAX, g.n - (tile_of(i) % g.panels) * NMAX);
@@ -281,8 +337,7 @@ gemm_f32_kernel(GemmArgs g) {
     // ---- epilogue: warps 8..11, a row per thread ----
     const int r = (warp & 3) * 32 + lane;
     const uint32_t t_row = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-    const bool w_odd = *g.w_flag != 0;
-    for (int i = 0; i < my_tiles; i++) {
+    for (int i = 0; i < run_tiles; i++) {
       const int work = tile_of(i), n0 = (work % g.panels) * NMAX, cols = min(NMAX, g.n - n0);
       const long long row = (long long)(work / g.panels) * kGemmRows + r;
       // (the four warps agree on the outcome: they meet at a barrier below)
@@ -291,7 +346,7 @@ gemm_f32_kernel(GemmArgs g) {
                    "barrier.cta.red.and.pred q, 1, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "+r"(ok)::"memory");
       if (!ok) { give_up(); break; }
       tc_fence_after();
-      const bool odd_a = *(volatile int*)&sm.odd[i & 7] != 0, odd = odd_a || w_odd;
+      const bool odd = *(volatile int*)&sm.odd[i & 7] != 0;
       float* crow = g.C + row * g.ldc + n0;
       for (int c0 = 0; c0 < cols; c0 += 32) {
         float v[32], small[32];
@@ -314,16 +369,15 @@ gemm_f32_kernel(GemmArgs g) {
           }
         }
       }
-      if (odd && row < g.m) {
-        for (int c = 0; c < cols; c++) {
-          float s = 0.f;
-          for (int k = 0; k < g.k; k++) s = fmaf(g.A[row * g.lda + k], g.W[(long long)k * g.ldw + n0 + c], s);
-          crow[c] = s;
-        }
-      }
       tc_fence_before();
       asm volatile("barrier.cta.sync 1, 128;" ::: "memory");   // all four warps have read `odd`
-      if (odd_a && r == 0) *(volatile int*)&sm.odd[i & 7] = 0;
+      if (r == 0) {
+        if (odd) {
+          *(volatile int*)&sm.odd[i & 7] = 0;
+          sm.redo[min(i >> 5, kRedoWords - 1)] |= 1u << (i & 31);
+        }
+        sm.done = i + 1;
+      }
       mbar_arrive(smem_u32(&sm.acc_empty[i & 1]));
     }
   }
@@ -331,6 +385,14 @@ gemm_f32_kernel(GemmArgs g) {
   __syncthreads();
   if (warp == 0)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
+  // What the pipeline left.  (Behind a wait that ran out nothing of it is in flight any more: the last
+  // copies and products were issued before that wait, a second ago.)  Tiles from the last word on share
+  // its bits: some are then done a second time.
+  for (int i = 0; i < my_tiles; i++) {
+    if (i < sm.done && !(sm.redo[min(i >> 5, kRedoWords - 1)] >> (i & 31) & 1)) continue;
+    const int work = tile_of(i);
+    gemm_redo_tile<NMAX>(g, (long long)(work / g.panels) * kGemmRows, (work % g.panels) * NMAX);
+  }
 }
 
 template <int NMAX, int STAGES>
@@ -366,8 +428,8 @@ size_t sb_dense_matmul_workspace_bytes(int64_t n, int64_t k) {
   return 256 + (size_t)(ceil_div(n, panel) * panel) * (size_t)(ceil_div(k, kGemmK) * kGemmK) * 6;
 }
 
-int sb_dense_matmul_f32(int64_t m, int64_t n, int64_t k, const float* A, int64_t lda, const float* W, int64_t ldw,
-                        float* C, int64_t ldc, void* ws, size_t ws_bytes, void* stream) {
+static int dense_matmul(int64_t m, int64_t n, int64_t k, const float* A, int64_t lda, const float* W, int64_t ldw,
+                        float* C, int64_t ldc, void* ws, size_t ws_bytes, int stop, void* stream) {
   SB_CHECK_ARG(m >= 0 && n >= 0 && k >= 0 && n < INT32_MAX / 2 && k < INT32_MAX / 2 && m < INT32_MAX &&
                ceil_div(m, 128) * ceil_div(n, 64) < INT32_MAX / 1024, "dense_matmul: bad size");
   SB_CHECK_ARG(lda >= k && ldw >= n && ldc >= n, "dense_matmul: leading dimension smaller than the row");
@@ -383,9 +445,28 @@ int sb_dense_matmul_f32(int64_t m, int64_t n, int64_t k, const float* A, int64_t
   GemmArgs g;
   g.m = m; g.n = (int)n; g.k = (int)k; g.A = A; g.lda = lda; g.W = W; g.ldw = ldw; g.C = C; g.ldc = ldc;
   g.tiles = (int)ceil_div(m, kGemmRows);
+  g.stop = stop;
   g.chunks = (int)ceil_div(k, kGemmK);
   if (n <= 64) return launch_gemm<64, 4>(g, ws, st);
   return launch_gemm<128, 3>(g, ws, st);
+}
+
+int sb_dense_matmul_f32(int64_t m, int64_t n, int64_t k, const float* A, int64_t lda, const float* W, int64_t ldw,
+                        float* C, int64_t ldc, void* ws, size_t ws_bytes, void* stream) {
+  return dense_matmul(m, n, k, A, lda, W, ldw, C, ldc, ws, ws_bytes, -1, stream);
+}
+
+int sb_dense_matmul_probe(int64_t m, int64_t n, int64_t k, const float* A, int64_t lda, const float* W, int64_t ldw,
+                          float* C, int64_t ldc, void* ws, size_t ws_bytes, int stop, int* status_host, void* stream) {
+  SB_CHECK_ARG(status_host && stop >= 0, "dense_matmul_probe: null status or negative chunk");
+  const int before = sb_dense_matmul_status();
+  const int rc = dense_matmul(m, n, k, A, lda, W, ldw, C, ldc, ws, ws_bytes, stop, stream);
+  if (rc != SB_OK) return rc;
+  SB_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
+  *status_host = sb_dense_matmul_status();
+  // (what the probe has set on purpose is no finding of a later reader)
+  SB_CUDA(cudaMemcpyToSymbol(g_gemm_status, &before, sizeof(int)));
+  return SB_OK;
 }
 
 int sb_dense_matmul_status(void) {

@@ -45,3 +45,49 @@ def test_values_beyond_the_split():
     W[3, 7] = float("nan")
     got = _run(X, W)
     assert torch.isnan(got[:, 7]).all() and torch.isfinite(got[0, :7]).all()
+
+
+@pytest.mark.parametrize("m,n,k,stop", [(128, 64, 64, 0), (5000, 72, 100, 0), (60000, 128, 64, 1), (60000, 64, 256, 11),
+                                        (60000, 136, 128, 10 ** 6)])
+def test_result_is_whole_behind_a_wait_that_ran_out(m, n, k, stop):
+    # the issuing thread of every CTA stops: the other waits run out after a second, the rest of the rows is
+    # done without the tensor cores
+    import ctypes as C
+    from scorch_b200 import _lib
+    L = _lib.lib()
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    X = torch.randn((m, k), generator=g, device="cuda")
+    W = torch.randn((k, n), generator=g, device="cuda") * k ** -0.5
+    out = torch.full((m + 1, n), 7.0, device="cuda")
+    ws = torch.empty(L.sb_dense_matmul_workspace_bytes(n, k), dtype=torch.uint8, device="cuda")
+    status = C.c_int(-1)
+    _lib.check(L.sb_dense_matmul_probe(m, n, k, X.data_ptr(), k, W.data_ptr(), n, out.data_ptr(), n, ws.data_ptr(),
+                                       ws.numel(), stop, C.byref(status), torch.cuda.current_stream().cuda_stream))
+    assert status.value == (1 if stop < 10 ** 6 else 0)
+    assert L.sb_dense_matmul_status() == 0 and (out[m] == 7.0).all()
+    want = X.double() @ W.double()
+    assert ((out[:m].double() - want).norm() / want.norm()).item() <= 1.2e-7 + 1.7e-7 * (k / 256) ** 0.5
+    assert torch.equal(_run(X, W), _run(X, W))
+
+
+def test_values_beyond_the_split_take_no_longer_than_other_kernels_do():
+    # one NaN in W sends every tile to the FMA form: 4 times the library product at this size (measured);
+    # a thread per row, walking K for every column, took 100 times that
+    X = torch.randn((200_000, 256), device="cuda")
+    W = torch.randn((256, 256), device="cuda")
+
+    def ms(f):
+        f()
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        for _ in range(5):
+            f()
+        b.record()
+        b.synchronize()
+        return a.elapsed_time(b) / 5
+    from scorch_b200 import kernels as K
+    library = ms(lambda: torch.matmul(X, W))
+    W[5, 7] = float("nan")
+    mine = ms(lambda: K.dense_matmul(X, W))
+    print(f"library {library:.3f} ms, FMA form {mine:.3f} ms")
+    assert mine < 8 * library
