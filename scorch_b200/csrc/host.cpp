@@ -99,6 +99,18 @@ PyObject* guarded(F&& f) {
   return nullptr;
 }
 
+// The interpreter is free for other threads while one of these lives: around calls that wait for the
+// device.  Nothing of Python is touched meanwhile.
+class Unlocked {
+  PyThreadState* const state = PyEval_SaveThread();
+
+ public:
+  Unlocked() = default;
+  Unlocked(const Unlocked&) = delete;
+  Unlocked& operator=(const Unlocked&) = delete;
+  ~Unlocked() { PyEval_RestoreThread(state); }
+};
+
 // pos, crd, val of a matrix times B (rows x k): the common part of the entry points below.
 PyObject* spmm(const at::Tensor& pos, const at::Tensor& crd, const at::Tensor& val, const at::Tensor& B,
                const at::Tensor* bias, bool relu, int64_t n) {
@@ -284,10 +296,53 @@ PyObject* py_attention(PyObject*, PyObject* const* a, Py_ssize_t count) {
   });
 }
 
+// C = A B in one pass; kTwoPhases where the products need more memory than that form may take.
+constexpr int64_t kOnePassBytes = (int64_t)16 << 30;
+constexpr int kTwoPhases = -1;
+
+int spgemm(int code, const at::Tensor& apos, const at::Tensor& acrd, const at::Tensor& aval, const at::Tensor& bpos,
+           const at::Tensor& bcrd, const at::Tensor& bval, int64_t n, at::Tensor& cpos, at::Tensor& ccrd,
+           at::Tensor& cval) {
+  const int64_t m = apos.numel() - 1, kb = bpos.numel() - 1, size = aval.element_size();
+  const c10::cuda::CUDAGuard device(aval.device());
+  void* stream = stream_of(aval);
+  const size_t bytes = abi.spgemm_bytes(m, n, code);
+  at::Tensor ws = workspace(bytes, aval), off = at::empty({m + 1}, apos.options());
+  int64_t counts[5], products = 0, total = 0;
+  const int *ap = apos.const_data_ptr<int>(), *ac = acrd.const_data_ptr<int>();
+  const int *bp = bpos.const_data_ptr<int>(), *bc = bcrd.const_data_ptr<int>();
+  int rc = abi.spgemm_begin(m, kb, n, ap, ac, bp, off.data_ptr<int>(), counts, &products, ws.data_ptr(), bytes, stream);
+  if (rc != SB_OK) return rc;
+  if (products > INT32_MAX || products * (4 + size) > kOnePassBytes) return kTwoPhases;
+  cpos = at::empty({m + 1}, apos.options());
+  at::Tensor tcrd, tval;
+  try {
+    tcrd = at::empty({products}, apos.options());
+    tval = at::empty({products}, aval.options());
+  } catch (const c10::OutOfMemoryError&) {
+    return kTwoPhases;
+  }
+  rc = abi.spgemm_rows(code, m, kb, n, ap, ac, aval.const_data_ptr(), bp, bc, bval.const_data_ptr(),
+                       off.data_ptr<int>(), counts, tcrd.data_ptr<int>(), tval.data_ptr(), cpos.data_ptr<int>(), &total,
+                       ws.data_ptr(), bytes, stream);
+  if (rc != SB_OK) return rc;
+  if (total == products) {     // no two products met: the rows are in place already
+    ccrd = tcrd;
+    cval = tval;
+    return SB_OK;
+  }
+  try {
+    ccrd = at::empty({total}, apos.options());
+    cval = at::empty({total}, aval.options());
+  } catch (const c10::OutOfMemoryError&) {
+    return kTwoPhases;
+  }
+  return abi.spgemm_finish(code, m, total, off.data_ptr<int>(), tcrd.data_ptr<int>(), tval.data_ptr(),
+                           cpos.data_ptr<int>(), ccrd.data_ptr<int>(), cval.data_ptr(), stream);
+}
+
 // spgemm(Apos, Acrd, Aval, Bpos, Bcrd, Bval, n) -> (Cpos, Ccrd, Cval), or None: not in the plain
 // form, or more products than the one-pass form has memory for
-constexpr int64_t kOnePassBytes = (int64_t)16 << 30;
-
 PyObject* py_spgemm(PyObject*, PyObject* const* a, Py_ssize_t count) {
   return guarded([&]() -> PyObject* {
     if (count != 7) Py_RETURN_NONE;
@@ -296,53 +351,22 @@ PyObject* py_spgemm(PyObject*, PyObject* const* a, Py_ssize_t count) {
       if (!(t[i] = tensor(a[i]))) Py_RETURN_NONE;
     const long long n = PyLong_AsLongLong(a[6]);
     if (n == -1 && PyErr_Occurred()) return nullptr;
-    const at::Tensor &apos = *t[0], &acrd = *t[1], &aval = *t[2], &bpos = *t[3], &bcrd = *t[4], &bval = *t[5];
+    // (copies: the wait for the device lets other threads run)
+    const at::Tensor apos = *t[0], acrd = *t[1], aval = *t[2], bpos = *t[3], bcrd = *t[4], bval = *t[5];
     const int code = dtype_code(aval.scalar_type());
     if (code < 0 || !indices(apos) || !indices(acrd) || !indices(bpos) || !indices(bcrd) ||
         !plain(aval, aval.scalar_type()) || !plain(bval, aval.scalar_type()) || aval.dim() != 1 || bval.dim() != 1 ||
         aval.numel() != acrd.numel() || bval.numel() != bcrd.numel() || apos.numel() < 1 || bpos.numel() < 1 ||
         checking())
       Py_RETURN_NONE;
-    const int64_t m = apos.numel() - 1, kb = bpos.numel() - 1, size = aval.element_size();
-    const c10::cuda::CUDAGuard device(aval.device());
-    void* stream = stream_of(aval);
-    const size_t bytes = abi.spgemm_bytes(m, n, code);
-    at::Tensor ws = workspace(bytes, aval), off = at::empty({m + 1}, apos.options());
-    int64_t counts[5], products = 0, total = 0;
-    const int *ap = apos.const_data_ptr<int>(), *ac = acrd.const_data_ptr<int>();
-    const int *bp = bpos.const_data_ptr<int>(), *bc = bcrd.const_data_ptr<int>();
-    int rc = abi.spgemm_begin(m, kb, n, ap, ac, bp, off.data_ptr<int>(), counts, &products, ws.data_ptr(), bytes,
-                              stream);
-    if (rc != SB_OK) return fail(rc);
-    if (products > INT32_MAX || products * (4 + size) > kOnePassBytes) Py_RETURN_NONE;
-    at::Tensor cpos = at::empty({m + 1}, apos.options()), ccrd, cval;
+    at::Tensor cpos, ccrd, cval;
+    int rc;
     {
-      at::Tensor tcrd, tval;
-      try {
-        tcrd = at::empty({products}, apos.options());
-        tval = at::empty({products}, aval.options());
-      } catch (const c10::OutOfMemoryError&) {
-        Py_RETURN_NONE;
-      }
-      rc = abi.spgemm_rows(code, m, kb, n, ap, ac, aval.const_data_ptr(), bp, bc, bval.const_data_ptr(),
-                           off.data_ptr<int>(), counts, tcrd.data_ptr<int>(), tval.data_ptr(), cpos.data_ptr<int>(),
-                           &total, ws.data_ptr(), bytes, stream);
-      if (rc != SB_OK) return fail(rc);
-      if (total == products) {     // no two products met: the rows are in place already
-        ccrd = tcrd;
-        cval = tval;
-      } else {
-        try {
-          ccrd = at::empty({total}, apos.options());
-          cval = at::empty({total}, aval.options());
-        } catch (const c10::OutOfMemoryError&) {
-          Py_RETURN_NONE;
-        }
-        rc = abi.spgemm_finish(code, m, total, off.data_ptr<int>(), tcrd.data_ptr<int>(), tval.data_ptr(),
-                               cpos.data_ptr<int>(), ccrd.data_ptr<int>(), cval.data_ptr(), stream);
-        if (rc != SB_OK) return fail(rc);
-      }
+      const Unlocked unlocked;
+      rc = spgemm(code, apos, acrd, aval, bpos, bcrd, bval, n, cpos, ccrd, cval);
     }
+    if (rc == kTwoPhases) Py_RETURN_NONE;
+    if (rc != SB_OK) return fail(rc);
     return Py_BuildValue("(NNN)", THPVariable_Wrap(std::move(cpos)), THPVariable_Wrap(std::move(ccrd)),
                          THPVariable_Wrap(std::move(cval)));
   });
