@@ -519,17 +519,19 @@ class ColumnSplit:
                                              self.pos.data_ptr(), self.crd.data_ptr(), self.val.data_ptr(), counts,
                                              ws.data_ptr(), wbytes, _stream()))
         self.counts = list(counts)
+        self.first = [sum(self.counts[:c]) for c in range(chunks)]     # first entry of every chunk
 
     @staticmethod
     def of(pos, crd, val, n: int, k: int) -> Optional["ColumnSplit"]:
         """The split for products with operands of up to ``k`` columns, or None where it does not pay, or
         the columns do not ascend."""
-        if not (val.dtype == torch.float32 and val.is_cuda and pos.is_contiguous() and crd.is_contiguous()
-                and val.is_contiguous() and pos.dtype == crd.dtype == torch.int32 and val.numel() == crd.numel()):
+        if not (val.dtype == torch.float32 and pos.dtype == crd.dtype == torch.int32 and val.numel() == crd.numel()
+                and all(t.is_cuda and t.is_contiguous() for t in (pos, crd, val))):
             return None
         chunks = split_chunks(pos.numel() - 1, n, crd.numel(), k)
         if not chunks:
             return None
+        _validated(pos, crd, n, "ColumnSplit")
         try:
             return ColumnSplit(pos, crd, val, n, chunks)
         except _lib.ScorchB200Error as e:
@@ -539,7 +541,10 @@ class ColumnSplit:
 
     def matmul(self, B: torch.Tensor, relu: bool = False, out: Optional[torch.Tensor] = None,
                accumulate: bool = False) -> torch.Tensor:
+        """act(out + A B), ``out`` only with ``accumulate``; B (n, k) and ``out`` (rows, k) contiguous."""
         k = B.shape[1]
+        for c, first in enumerate(self.first):
+            _validated(self.pos[c], self.crd[first:first + self.counts[c]], B.shape[0], "ColumnSplit.matmul")
         if out is None:
             out = torch.empty((self.m, k), dtype=torch.float32, device=B.device)
         L, last = _lib.lib(), len(self.counts) - 1
@@ -548,14 +553,12 @@ class ColumnSplit:
             ws = torch.empty(wbytes, dtype=torch.uint8, device=B.device)
             stream = _stream()
             for k0 in range(0, k, SPLIT_PANEL):
-                first = 0
-                for c, count in enumerate(self.counts):
+                for c, (first, count) in enumerate(zip(self.first, self.counts)):
                     check(L.sb_spmm_csr_once(SB_F32, self.m, self.n, min(SPLIT_PANEL, k - k0), count,
                                              self.pos[c].data_ptr(), self.crd.data_ptr() + 4 * first,
                                              self.val.data_ptr() + 4 * first, B.data_ptr() + 4 * k0, k, None,
                                              int(relu and c == last), int(accumulate or c > 0), out.data_ptr() + 4 * k0, k,
                                              ws.data_ptr(), wbytes, stream))
-                    first += count
         return out
 
 

@@ -72,7 +72,7 @@ def test_result_is_whole_behind_a_wait_that_ran_out(m, n, k, stop):
 
 def test_values_beyond_the_split_take_no_longer_than_other_kernels_do():
     # one NaN in W sends every tile to the FMA form: 4 times the library product at this size (measured);
-    # a thread per row, walking K for every column, took 100 times that
+    # a thread per row, walking K for every column, took 100 times the library's
     X = torch.randn((200_000, 256), device="cuda")
     W = torch.randn((256, 256), device="cuda")
 

@@ -64,3 +64,42 @@ def test_front_end_refuses_invalid_operands_when_asked(monkeypatch):
     with pytest.raises(ValueError, match="not strictly ascending"):
         K.spgemm_csr(dev(POS), dev([4, 1, 0, 2, 3, 4]), val, dev([0, 1, 2, 3, 4, 5]), dev([0, 1, 2, 3, 4]),
                      torch.ones(5, device="cuda"), 5)
+
+
+def test_column_split_refuses_invalid_operands_when_asked(monkeypatch):
+    # the products of large graphs go through the column split, not through spmm_csr
+    from scorch_b200 import kernels as K, pipelines as P, sharded as S
+    monkeypatch.setattr(K, "SPLIT_CHUNK_BYTES", 2e5)
+    n, per = 2000, 40
+    pos = np.arange(n + 1, dtype=np.int32) * per
+    crd = np.tile(np.arange(per, dtype=np.int32) * 50, n)
+    val = torch.ones(n * per, device="cuda")
+    X, W1, W2 = (torch.ones(s, device="cuda") for s in ((n, 64), (64, 64), (64, 40)))
+    monkeypatch.setenv("SCORCH_B200_VALIDATE", "1")
+    good = P.gcn_forward(dev(pos), dev(crd), val, X, W1, W2)
+    assert K.ColumnSplit.of(dev(pos), dev(crd), val, n, 64) is not None and torch.isfinite(good).all()
+    far = crd.copy()
+    far[-1] = n
+    down = pos.copy()
+    down[7] = down[9]
+    for p, c, message in ((pos, far, "column index out of range"), (down, crd, "row pointers decrease")):
+        with pytest.raises(ValueError, match=message):
+            P.gcn_forward(dev(p), dev(c), val, X, W1, W2)                 # never reaches the kernels
+        block = S.CsrBlock(dev(p), dev(c), val)
+        with pytest.raises(ValueError, match=message):
+            S._default_spmm(block, X, torch.empty((n, 64), device="cuda"), False)
+    split = K.ColumnSplit(dev(pos), dev(crd), val, n, 4)
+    split.crd[3] = n + 5                                                  # a split is an operand of its own
+    with pytest.raises(ValueError, match="column index out of range"):
+        split.matmul(X)
+
+
+def test_column_split_leaves_host_tensors_to_spmm(monkeypatch):
+    from scorch_b200 import kernels as K, pipelines as P
+    monkeypatch.setattr(K, "SPLIT_CHUNK_BYTES", 2e5)
+    n, per = 2000, 40
+    pos, crd = dev(np.arange(n + 1) * per), dev(np.tile(np.arange(per) * 50, n))
+    val, X, W1, W2 = (torch.ones(s, device="cuda") for s in ((n * per,), (n, 64), (64, 64), (64, 40)))
+    for args in ((pos.cpu(), crd, val), (pos, crd.cpu(), val), (pos, crd, val.cpu())):
+        with pytest.raises(TypeError, match="CUDA tensor"):
+            P.gcn_forward(*args, X, W1, W2)
