@@ -499,7 +499,7 @@ def split_chunks(m: int, n: int, nnz: int, k: int) -> int:
     per row and chunk on.  2 M rows, 100 entries each, 256 columns: 24.0 ms in one pass, 21.0 in six."""
     row = 4 * min(k, SPLIT_PANEL)
     chunks = -(-n * row // int(SPLIT_CHUNK_BYTES))
-    return chunks if 1 < chunks <= 64 and nnz >= SPLIT_MIN_ENTRIES * chunks * m and m * chunks < 2 ** 31 - 4096 else 0
+    return chunks if 1 < chunks <= 64 and m > 0 and nnz >= SPLIT_MIN_ENTRIES * chunks * m and m * chunks < 2 ** 31 - 4096 else 0
 
 
 class ColumnSplit:
@@ -541,8 +541,16 @@ class ColumnSplit:
 
     def matmul(self, B: torch.Tensor, relu: bool = False, out: Optional[torch.Tensor] = None,
                accumulate: bool = False) -> torch.Tensor:
-        """act(out + A B), ``out`` only with ``accumulate``; B (n, k) and ``out`` (rows, k) contiguous."""
+        """act(A B), or act(out + A B) with ``accumulate``; B (n, k), ``out`` (rows, k) contiguous."""
+        B = _dev(B, torch.float32, "B")
+        if B.dim() != 2 or B.shape[0] < self.n:
+            raise ValueError(f"B must be a matrix of {self.n} rows")
         k = B.shape[1]
+        if accumulate and out is None:
+            raise ValueError("accumulate needs the tensor to add to (out=)")
+        if out is not None and not (out.is_cuda and out.dtype == torch.float32 and out.is_contiguous()
+                                    and tuple(out.shape) == (self.m, k)):
+            raise ValueError(f"out must be a contiguous float32 CUDA tensor of shape {(self.m, k)}")
         for c, first in enumerate(self.first):
             _validated(self.pos[c], self.crd[first:first + self.counts[c]], B.shape[0], "ColumnSplit.matmul")
         if out is None:

@@ -136,3 +136,33 @@ def test_sharded_forward_in_inference_mode(monkeypatch):
             got = S.gcn_forward_sharded(shard, X, W1, W2)
             assert ((got.double() - want).norm() / want.norm()).item() < 1e-6
             v.mul_(-0.5)
+
+
+def test_split_product_refuses_what_spmm_refuses():
+    from scorch_b200 import kernels as K
+    pos, crd, val = (torch.from_numpy(a).cuda() for a in _csr([5] * 30, 40, seed=7))
+    split = K.ColumnSplit(pos, crd, val, 40, 3)
+    B = torch.randn((40, 12), device="cuda")
+    want = K.spmm_csr(pos, crd, val, B)
+    got = split.matmul(B.t().contiguous().t())
+    assert torch.allclose(got, want, rtol=1e-4, atol=1e-5)               # other strides: copied, as there
+    for bad in (B.double(), B.cpu()):
+        with pytest.raises(TypeError):
+            split.matmul(bad)
+    for bad in (B[:39], B[:, 0]):
+        with pytest.raises(ValueError):
+            split.matmul(bad)
+    for out in (torch.empty((30, 11), device="cuda"), torch.empty((30, 12), device="cuda").double(),
+                torch.empty((12, 30), device="cuda").t()):
+        with pytest.raises(ValueError):
+            split.matmul(B, out=out)
+    with pytest.raises(ValueError):
+        split.matmul(B, accumulate=True)
+
+
+def test_graph_without_rows_is_not_split():
+    from scorch_b200 import kernels as K
+    assert K.split_chunks(0, 1_000_000, 0, 64) == 0
+    none = torch.empty(0, dtype=torch.int32, device="cuda")
+    A = torch.zeros(1, dtype=torch.int32, device="cuda"), none, none.float()
+    assert K.ColumnSplit.of(*A, 1_000_000, 64) is None
