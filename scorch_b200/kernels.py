@@ -484,7 +484,7 @@ def dense_matmul(X: torch.Tensor, W: torch.Tensor, out: Optional[torch.Tensor] =
         ws = torch.empty(wbytes, dtype=torch.uint8, device=X.device)
         check(L.sb_dense_matmul_f32(m, n, k, X.data_ptr(), k, W.data_ptr(), n, out.data_ptr(), n, ws.data_ptr(),
                                     wbytes, _stream()))
-    return out
+    return _wrote(out)
 
 
 SPLIT_PANEL = 64                  # operand columns multiplied at a time (256 bytes of each operand row)
@@ -567,7 +567,7 @@ class ColumnSplit:
                                              self.val.data_ptr() + 4 * first, B.data_ptr() + 4 * k0, k, None,
                                              int(relu and c == last), int(accumulate or c > 0), out.data_ptr() + 4 * k0, k,
                                              ws.data_ptr(), wbytes, stream))
-        return out
+        return _wrote(out)
 
 
 def spmv_csr(pos, crd, val, x, plan: Optional[CsrPlan] = None) -> torch.Tensor:
