@@ -46,6 +46,8 @@ constexpr int64_t kBigProductsMax = (int64_t)1 << 26;
 constexpr int64_t kBucketProducts = 1024;      // buckets per row: U / this, rounded up to a power of two
 constexpr int kBucketSort = 2048;              // products a bucket's sorting kernel takes
 constexpr int kBigTasks = 1 << 17;
+// Columns up to which long rows are summed in shared memory (spgemm_smem_kernel) and need no area.
+constexpr int kSmemColumns = 24576;
 
 static int64_t big_products(int64_t m, int64_t n) {
   return std::min<int64_t>(kBigProductsMax, std::max<int64_t>((int64_t)1 << 20, 64 * (m + n)));
@@ -60,7 +62,7 @@ struct WsLayout {
   int* row_cnt;         // m ints
   unsigned long long* max_b;  // bit pattern of max |b| over the right operand
   long long* block_sum; // scan temporaries
-  char* area;           // long rows
+  char* area;           // long rows (empty up to kSmemColumns columns)
   int64_t products;     // its capacity
   size_t area_bytes;
   size_t total;
@@ -121,7 +123,7 @@ static WsLayout ws_layout(void* base, int64_t m, int64_t n) {
   w.max_b = (unsigned long long*)take(8);
   w.block_sum = (long long*)take((size_t)(ceil_div(m > 0 ? m : 1, 4096) + 1) * 8);
   w.products = big_products(m, n);
-  w.area_bytes = std::max(big_area(nullptr, w.products).bytes, dense_bytes(n));
+  w.area_bytes = n <= kSmemColumns ? 0 : std::max(big_area(nullptr, w.products).bytes, dense_bytes(n));
   w.area = take(w.area_bytes);
   w.total = off;
   return w;
@@ -841,7 +843,7 @@ int exclusive_scan_i32(int n, const int* cnt, int* out, long long* block_sum, lo
 // Few such rows leave most of the GPU to the others, so up to eight CTAs - a cluster - share a row: each
 // takes its part of the products into a bitmap and accumulators of its own, then emits a slice of the
 // columns, adding the others' sums out of their shared memory (CLUSTERED).
-constexpr int kSmemColumns = 24576, kSmemThreads = 1024;
+constexpr int kSmemThreads = 1024;
 template <typename T, bool NUMERIC, bool CLUSTERED>
 __global__ void __launch_bounds__(kSmemThreads)
 spgemm_smem_kernel(const int* __restrict__ rows, CsrIn in, int n, const unsigned long long* __restrict__ max_b,

@@ -43,6 +43,10 @@ def test_size_queries_are_pure_host_functions(sb_lib):
     small = sb_lib.sb_spgemm_workspace_bytes(100, 100, 0)
     big = sb_lib.sb_spgemm_workspace_bytes(100, 1 << 20, 0)
     assert 0 < small < big
+    # long rows of up to 24,576 columns are summed in shared memory: no area for them, whatever the rows
+    assert sb_lib.sb_spgemm_workspace_bytes(2_000_000, 24576, 0) < 2_000_000 * 40
+    assert sb_lib.sb_spgemm_workspace_bytes(20011, 20011, 0) < (1 << 20)
+    assert sb_lib.sb_spgemm_workspace_bytes(20011, 24577, 0) > 64 * (20011 + 24577) * 32
     # the dense-row area is capped, so a huge column count cannot ask for unbounded memory
     assert sb_lib.sb_spgemm_workspace_bytes(1000, 1 << 30, 1) < (20 << 30)
 
