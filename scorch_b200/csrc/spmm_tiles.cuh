@@ -46,9 +46,9 @@ static_assert(tile_window(8) / kWarpRow + tile_window(8) / kUnit + 4 <= kTileLis
 constexpr int tile_ctas(int L) { return L == 32 ? 4 : 3; }
 // Entries per window, a multiple of 32: as few full waves of CTAs over the chip as windows of at
 // most tile_window(L) allow (a last wave that is half empty costs as much as a full one), at least 64
-// and at least four per lane group. 
+// and at least four per lane group.
 inline int tile_entries(int64_t nnz, int L) {
-  const int64_t slots = 148 * tile_ctas(L);
+  const int64_t slots = (int64_t)sm_count() * tile_ctas(L);
   const int64_t waves = std::max<int64_t>(1, ceil_div(nnz, slots * tile_window(L)));
   const int64_t te = ceil_div(ceil_div(nnz, slots * waves), 32) * 32;
   return (int)std::min<int64_t>(std::max<int64_t>(te, std::max(64, 1024 / L)), tile_window(L));
@@ -380,7 +380,7 @@ static int launch_tiles(const SpmmArgs<T>& a, int64_t nnz, void* ws, cudaStream_
       SB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem)));
       if (dev >= 0 && dev < 64) sized[dev] = true;
     }
-    const bool resident = !in_l2 && t.tiles <= 148 * tile_ctas(L);
+    const bool resident = !in_l2 && t.tiles <= sm_count() * tile_ctas(L);
     SB_CUDA(launch_early(kernel, dim3((unsigned)t.tiles, resident ? 1 : panels), kTileThreadsMm, sizeof(Smem), st, a, t));
   }
   // (may be set up while the tiles still run: it waits for them itself.  It reads the row pointers before

@@ -13,13 +13,14 @@ namespace {
 struct Launch {
   std::string kernel;
   bool early;
-  unsigned cluster;
+  unsigned cluster, grid;
 };
 std::map<const void*, std::string>& names() {
   static std::map<const void*, std::string> m;
   return m;
 }
 std::vector<Launch> launches;
+int device = 0;
 struct { dim3 grid, block; size_t smem; void* stream; } pushed;
 }  // namespace
 
@@ -28,6 +29,8 @@ void recorder_reset() { launches.clear(); }
 int recorder_count() { return (int)launches.size(); }
 const char* recorder_kernel(int i) { return launches[i].kernel.c_str(); }
 int recorder_early(int i) { return launches[i].early; }
+int recorder_grid(int i) { return (int)launches[i].grid; }
+void recorder_device(int d) { device = d; }   // 0: 148 SMs, 1: 60
 int recorder_cluster(int i) { return (int)launches[i].cluster; }
 
 void** __cudaRegisterFatBinary(void*) { static void* handle; return &handle; }
@@ -48,12 +51,12 @@ cudaError_t __cudaPopCallConfiguration(dim3* grid, dim3* block, size_t* smem, vo
   *static_cast<void**>(stream) = pushed.stream;
   return cudaSuccess;
 }
-cudaError_t cudaLaunchKernel(const void* f, dim3, dim3, void**, size_t, cudaStream_t) {
-  launches.push_back({names()[f], false, 1});
+cudaError_t cudaLaunchKernel(const void* f, dim3 grid, dim3, void**, size_t, cudaStream_t) {
+  launches.push_back({names()[f], false, 1, grid.x});
   return cudaSuccess;
 }
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void**) {
-  Launch l{names()[f], false, 1};
+  Launch l{names()[f], false, 1, c->gridDim.x};
   for (unsigned i = 0; i < c->numAttrs; i++) {
     if (c->attrs[i].id == cudaLaunchAttributeProgrammaticStreamSerialization)
       l.early = c->attrs[i].val.programmaticStreamSerializationAllowed != 0;
@@ -73,7 +76,7 @@ cudaError_t cudaMemsetAsync(void* p, int v, size_t n, cudaStream_t) {
 cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaGetLastError() { return cudaSuccess; }
 const char* cudaGetErrorString(cudaError_t) { return "none"; }
-cudaError_t cudaGetDevice(int* d) { *d = 0; return cudaSuccess; }
-cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr, int) { *v = 148; return cudaSuccess; }
+cudaError_t cudaGetDevice(int* d) { *d = device; return cudaSuccess; }
+cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr, int d) { *v = d == 0 ? 148 : 60; return cudaSuccess; }
 cudaError_t cudaFuncSetAttribute(const void*, cudaFuncAttribute, int) { return cudaSuccess; }
 }

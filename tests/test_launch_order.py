@@ -85,3 +85,19 @@ def test_spmm_without_entries_begins_behind_its_operands(recorded, dtype, k, acc
                             None)
         assert "spmm_tile_rows_kernel" in got[-1][0]
         assert [early for _, early, _ in got] == ([True, True] if nnz else [False]), got
+
+
+@pytest.mark.parametrize("k,per_sm", [(64, 3), (256, 4)])
+def test_spmm_windows_fill_the_device_at_hand(recorded, k, per_sm):
+    # one wave of windows for a matrix that does not need more, on 148 SMs and on 60
+    nnz = 100_000
+    pos, x = np.zeros(10, np.int32), np.zeros(64, np.float32)
+    ws = np.zeros(recorded.abi.sb_spmm_csr_once_workspace_bytes(0, k, nnz) + 16, np.uint8)
+    for device, sms in ((0, 148), (1, 60)):
+        recorded.abi.recorder_device(device)
+        try:
+            recorded.call(recorded.abi.sb_spmm_csr_once, 0, 9, 4, k, nnz, _ptr(pos), _ptr(pos), _ptr(x), _ptr(x) // 32 * 32,
+                          k, None, 0, 0, _ptr(x) // 32 * 32, k, (_ptr(ws) + 15) // 16 * 16, ws.size - 16, None)
+            assert sms * per_sm * 0.8 < recorded.abi.recorder_grid(0) <= sms * per_sm
+        finally:
+            recorded.abi.recorder_device(0)
