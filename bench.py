@@ -408,7 +408,6 @@ class SpmmWorkload(Workload):
         self.pos, self.crd = A.pos.cuda(), A.crd.cuda()
         self.val, self.B = (t.cuda() for t in self.host)
         self.stage = [torch.empty_like(t, device="cuda") for t in self.host]
-        self.plan = K.CsrPlan(self.pos, self.nnz)
         self.out = torch.empty((self.m, self.k), dtype=torch.float32, device="cuda")
         self.host_out = torch.empty((self.m, self.k), dtype=torch.float32).pin_memory()
         # small problems stay in L2 between iterations: flush it with a 256 MiB write
@@ -437,7 +436,7 @@ class SpmmWorkload(Workload):
             self.flush.zero_()
         if ev is not None:
             ev[0].record()
-        self.K.spmm_csr(self.pos, self.crd, self.val, self.B, plan=self.plan, out=self.out)
+        self.K.spmm_csr(self.pos, self.crd, self.val, self.B, out=self.out)
         if ev is not None:
             ev[1].record()
 
@@ -483,8 +482,8 @@ class SpmmWorkload(Workload):
             for name, mode in (("gather kernel (ld.global.nc.v8 through L1)", 0),
                                ("bulk-copy kernel (cp.async.bulk through shared memory)", 1)):
                 L.sb_spmm_wide_select(mode)
-                t = timed(lambda: self.K.spmm_csr(self.pos, self.crd, self.val, self.B, plan=self.plan,
-                                                  out=self.out), reps=10)
+                t = timed(lambda: self.K.spmm_csr(self.pos, self.crd, self.val, self.B, out=self.out),
+                          reps=10)
                 per_kernel[name] = {"ms": t, "l2_to_sm_GBps": volume / (t * 1e-3) / 1e9,
                                     "frac_of_probe": volume / (t * 1e-3) / 1e9 / peak}
         finally:
@@ -497,7 +496,7 @@ class SpmmWorkload(Workload):
     def e2e_step(self):
         for dst, src in zip(self.stage, self.host):
             dst.copy_(src, non_blocking=True)
-        self.K.spmm_csr(self.pos, self.crd, self.stage[0], self.stage[1], plan=self.plan, out=self.out)
+        self.K.spmm_csr(self.pos, self.crd, self.stage[0], self.stage[1], out=self.out)
         self.host_out.copy_(self.out, non_blocking=True)
         torch.cuda.current_stream().synchronize()
 
@@ -706,10 +705,10 @@ class GcnSharded(Workload):
 
     def run_info(self):
         sp = self.shard.splits
-        segs = [b.plan.segments if b.plan is not None else None for b in sp[0].blocks]
+        cut = [b.columns[1] if b.columns else None for b in sp[0].blocks]
         return {"rows_this_rank": self.shard.rows, "nnz_this_rank": self.shard.nnz,
                 "row_chunk_offsets_layer1": sp[0].offsets, "row_chunk_offsets_layer2": sp[-1].offsets,
-                "heavy_segments_per_chunk_layer1": segs}
+                "column_chunks_per_row_chunk_layer1": [len(c.counts) if c is not None else 1 for c in cut]}
 
     def alg_bytes(self):
         rows, nnz, n = self.shard.rows, self.shard.nnz, self.n

@@ -357,8 +357,8 @@ def spmm_csr(pos, crd, val, B, bias=None, relu: bool = False, plan: Optional[Csr
     shared by all batch items — or (batch, nnz).  Returns (m, k) or (batch, m, k).
     2-D ``B`` / ``out`` may be column slices of wider row-major buffers (row pitch > k).
     ``accumulate``: act(bias + out + A @ B), ``out`` required.
-    One matrix runs over equal tiles of its entries and needs no ``plan``; a batch uses the plan of
-    its long rows (``plan_for(pos)`` when none is given)."""
+    One matrix runs over equal tiles of its entries and needs no ``plan`` (one that is given is not
+    used); a batch uses the plan of its long rows (``plan_for(pos)`` when none is given)."""
     if out is None and block_plan is None and not accumulate:
         r = _lib.host().spmm(pos, crd, val, B, bias, relu, -1 if n is None else n)
         if r is not None:

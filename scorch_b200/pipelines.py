@@ -77,12 +77,13 @@ def sparse_attention(pos: torch.Tensor, crd: torch.Tensor, mask_val: Optional[to
 
 def gcn_forward(pos, crd, val, X, W1, W2, plan: Optional[K.CsrPlan] = None) -> torch.Tensor:
     """Large graphs: the matrix is cut by columns once per call, and the products run chunk by chunk
-    with the operand in L2 (``kernels.split_chunks``)."""
+    with the operand in L2 (``kernels.split_chunks``).  ``plan`` is accepted and not needed: products of one
+    matrix run over equal tiles of its entries."""
     n, hidden, width = X.shape[0], W1.shape[1], W2.shape[1]
     split = K.ColumnSplit.of(pos, crd, val, n, max(hidden, width)) if W1.is_cuda and X.dtype == torch.float32 else None
     # (an operand that L2 nearly holds whole is multiplied in one pass)
     product = lambda B, relu: (split.matmul(B, relu) if split is not None and 4 * n * B.shape[1] > 1.3 * K.SPLIT_CHUNK_BYTES
-                               else K.spmm_csr(pos, crd, val, B, relu=relu, plan=plan))
+                               else K.spmm_csr(pos, crd, val, B, relu=relu))
     return product(K.dense_matmul(product(K.dense_matmul(X, W1), True), W2), False)
 
 

@@ -65,11 +65,10 @@ def row_bounds(pos: torch.Tensor, parts: int) -> List[int]:
 
 @dataclass
 class CsrBlock:
-    """A CSR matrix with the state the SpMM wrapper caches for it."""
+    """A CSR matrix with what is kept for products with it."""
     pos: torch.Tensor          # int32 [rows + 1]
     crd: torch.Tensor          # int32 [nnz]
     val: torch.Tensor
-    plan: object = None
     columns: object = None     # (key, kernels.ColumnSplit or None) for operands much larger than L2: columns_for
 
     @property
@@ -79,6 +78,13 @@ class CsrBlock:
     @property
     def nnz(self) -> int:
         return int(self.crd.numel())
+
+    @property
+    def plan(self):
+        """The block's long rows (``kernels.plan_for``), for callers of batched products; those of one
+        matrix need none."""
+        from . import kernels as K
+        return K.plan_for(self.pos, self.nnz)
 
     def columns_for(self, n: int, k: int):
         """The block cut by columns (``kernels.ColumnSplit``) for products with an (n x k) operand, or None
@@ -272,10 +278,7 @@ def _default_spmm(block: CsrBlock, B: torch.Tensor, out: torch.Tensor, relu: boo
         if split is not None:
             split.matmul(B, relu, out=out, accumulate=accumulate)
             return
-    if block.plan is None:
-        block.plan = K.CsrPlan(block.pos, block.nnz)
-    K.spmm_csr(block.pos, block.crd, block.val, B, relu=relu, plan=block.plan, out=out,
-               accumulate=accumulate)
+    K.spmm_csr(block.pos, block.crd, block.val, B, relu=relu, out=out, accumulate=accumulate)
 
 
 def sharded_spmm_replicated(block: CsrBlock, B: torch.Tensor, bias=None, relu: bool = False,
@@ -283,9 +286,7 @@ def sharded_spmm_replicated(block: CsrBlock, B: torch.Tensor, bias=None, relu: b
     """This rank's rows of act(bias + A B) for a dense operand every rank holds (a weight matrix,
     a replicated feature matrix): no communication, any matrix shape."""
     from . import kernels as K
-    if block.plan is None:
-        block.plan = K.CsrPlan(block.pos, block.nnz)
-    return K.spmm_csr(block.pos, block.crd, block.val, B, bias=bias, relu=relu, plan=block.plan, out=out)
+    return K.spmm_csr(block.pos, block.crd, block.val, B, bias=bias, relu=relu, out=out)
 
 
 class Timeline:

@@ -193,3 +193,19 @@ def test_sharded_spgemm_single_process_has_no_offset(oracle):
     assert offset == 0 and total == ccrd.numel() and bounds == [0, 4000]
     wpos, wcrd, _ = oracle.spgemm(*(t.cpu().numpy() for t in (A.pos, A.crd, A.val, A.pos, A.crd, A.val)), 4000)
     assert np.array_equal(cpos.cpu().numpy(), wpos) and np.array_equal(ccrd.cpu().numpy(), wcrd)
+
+
+def test_layers_build_no_row_plans(monkeypatch):
+    # products of one matrix take no plan, and building one reads sizes back from the device
+    from scorch_b200 import kernels as K, sharded as S, workloads as W
+    g = W.gcn_graph(5000, mean_deg=10.0, max_deg=2000, seed=1).to("cuda")
+    shard = S.ShardedCsr.from_global(g.pos, g.crd, g.val, 0, 1, chunks=3)
+    X = torch.randn((5000, 64), device="cuda")
+
+    def refuse(*args, **kwargs):
+        raise AssertionError("a row plan was built")
+    with monkeypatch.context() as patch:
+        patch.setattr(K, "CsrPlan", refuse)
+        S.gcn_forward_sharded(shard, X, torch.randn((64, 64), device="cuda"), torch.randn((64, 16), device="cuda"))
+        S.sharded_spmm_replicated(S.row_block(g.pos, g.crd, g.val, 0, 2)[0], X)
+    assert all(b.plan is b.plan and b.plan.nnz == b.nnz for b in shard.blocks)
