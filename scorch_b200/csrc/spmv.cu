@@ -14,23 +14,18 @@ __device__ __forceinline__ T shfl_xor_t(T v, int o) { return __shfl_xor_sync(FUL
 template <typename T, int G>
 __global__ void __launch_bounds__(256)
 spmv_rows_kernel(int m, const int* __restrict__ pos, const int* __restrict__ crd,
-                 const T* __restrict__ val, const T* __restrict__ x, T* __restrict__ y,
-                 int skip_heavy) {
+                 const T* __restrict__ val, const T* __restrict__ x, T* __restrict__ y) {
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long row = t / G;
   const int l = (int)(t % G);
   T acc = T(0);
-  bool write = false;
   if (row < m) {
     const int b = __ldg(pos + row), e = __ldg(pos + row + 1);
-    if (!(skip_heavy && e - b > SB_HEAVY_ROW_NNZ)) {
-      write = true;
-      for (int p = b + l; p < e; p += G) acc += val[p] * __ldg(x + crd[p]);
-    }
+    for (int p = b + l; p < e; p += G) acc += val[p] * __ldg(x + crd[p]);
   }
 #pragma unroll
   for (int o = G / 2; o > 0; o >>= 1) acc += shfl_xor_t(acc, o);
-  if (write && l == 0) y[row] = acc;
+  if (row < m && l == 0) y[row] = acc;
 }
 
 // ---- entry-tiled kernel --------------------------------------------------------------------------
@@ -174,12 +169,12 @@ static int launch_tiles(int64_t m, int64_t nnz, const int32_t* pos, const int32_
 
 template <typename T>
 static int launch_rows(int64_t m, int64_t nnz, const int32_t* pos, const int32_t* crd,
-                       const T* val, const T* x, T* y, int skip_heavy, cudaStream_t st) {
+                       const T* val, const T* x, T* y, cudaStream_t st) {
   const double mean = m > 0 ? (double)nnz / (double)m : 0.0;
   const int threads = 256;
 #define SB_SPMV_LAUNCH(G)                                                                    \
   spmv_rows_kernel<T, G><<<(unsigned)ceil_div(m * (int64_t)G, threads), threads, 0, st>>>(   \
-      (int)m, pos, crd, val, x, y, skip_heavy)
+      (int)m, pos, crd, val, x, y)
   if (mean <= 3.0) SB_SPMV_LAUNCH(2);
   else if (mean <= 6.0) SB_SPMV_LAUNCH(4);
   else if (mean <= 12.0) SB_SPMV_LAUNCH(8);
@@ -265,15 +260,15 @@ int sb_spmv_csr_typed(int dtype, int64_t m, int64_t n, int64_t nnz, const int32_
   cudaStream_t st = (cudaStream_t)stream;
   switch (dtype) {
     case SB_F32:  // without scratch: the lanes-per-row kernel
-      return launch_rows<float>(m, nnz, pos, crd, (const float*)val, (const float*)x, (float*)y, 0, st);
+      return launch_rows<float>(m, nnz, pos, crd, (const float*)val, (const float*)x, (float*)y, st);
     case SB_F64:
-      return launch_rows<double>(m, nnz, pos, crd, (const double*)val, (const double*)x, (double*)y, 0, st);
+      return launch_rows<double>(m, nnz, pos, crd, (const double*)val, (const double*)x, (double*)y, st);
     case SB_I32:  // unsigned arithmetic: same bits as the reference's wrapping int32 math
       return launch_rows<unsigned int>(m, nnz, pos, crd, (const unsigned int*)val,
-                                       (const unsigned int*)x, (unsigned int*)y, 0, st);
+                                       (const unsigned int*)x, (unsigned int*)y, st);
     case SB_I64:
       return launch_rows<unsigned long long>(m, nnz, pos, crd, (const unsigned long long*)val,
-                                             (const unsigned long long*)x, (unsigned long long*)y, 0, st);
+                                             (const unsigned long long*)x, (unsigned long long*)y, st);
     default:
       return fail(SB_ERR_UNSUPPORTED, "spmv_typed: unknown dtype %d", dtype);
   }
