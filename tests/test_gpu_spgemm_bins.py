@@ -84,3 +84,14 @@ def test_long_rows_shared_by_clusters(rows, n, dtype):
     rng = np.random.default_rng(rows)
     B = _csr([40] * 299 + [min(n, 3000)], n, rng, dtype)
     _check(_csr([250] * rows + [0, 7], 300, rng, dtype), B, n, dtype)
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64, np.int32])
+def test_row_beyond_the_area_of_a_wide_matrix(dtype):
+    # as test_row_beyond_the_area, with more columns than shared memory holds sums of: there the rows of more
+    # products than the workspace's area takes (64 (m + n) here) go to the dense kernel one by one
+    rng = np.random.default_rng(4)
+    n = 30000
+    B = _csr([1500] * 1400, n, rng, dtype)
+    assert 1400 * 1500 > 64 * (3 + n) > 700 * 1500 > 8192
+    _check(_csr([1400, 2, 700], 1400, rng, dtype), B, n, dtype)
