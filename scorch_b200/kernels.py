@@ -524,12 +524,13 @@ class ColumnSplit:
     @staticmethod
     def of(pos, crd, val, n: int, k: int) -> Optional["ColumnSplit"]:
         """The split for products with operands of up to ``k`` columns, or None where it does not pay, or
-        the columns do not ascend."""
+        the columns do not ascend.  None too while the stream is captured into a graph: the split waits for
+        the device, and a graph would go on reading a copy of the matrix as it was."""
         if not (val.dtype == torch.float32 and pos.dtype == crd.dtype == torch.int32 and val.numel() == crd.numel()
                 and all(t.is_cuda and t.is_contiguous() for t in (pos, crd, val))):
             return None
         chunks = split_chunks(pos.numel() - 1, n, crd.numel(), k)
-        if not chunks:
+        if not chunks or torch.cuda.is_current_stream_capturing():
             return None
         _validated(pos, crd, n, "ColumnSplit")
         try:

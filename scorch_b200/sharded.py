@@ -93,8 +93,8 @@ class CsrBlock:
         tells) or replaced; tensors that do not count their writes (inference mode) are cut on every call."""
         from . import kernels as K
         chunks = K.split_chunks(self.rows, n, self.nnz, k)
-        if not chunks:
-            return None
+        if not chunks or torch.cuda.is_current_stream_capturing():
+            return None           # (a graph would read the copy after it has been replaced)
         sources = (self.pos, self.crd, self.val)
         counted = not any(t.is_inference() for t in sources)
         # (the key holds the tensors: another tensor cannot take their place in memory meanwhile)

@@ -166,3 +166,34 @@ def test_graph_without_rows_is_not_split():
     none = torch.empty(0, dtype=torch.int32, device="cuda")
     A = torch.zeros(1, dtype=torch.int32, device="cuda"), none, none.float()
     assert K.ColumnSplit.of(*A, 1_000_000, 64) is None
+
+
+@pytest.mark.parametrize("sharded", [False, True])
+def test_captured_forward_reads_the_matrix_itself(monkeypatch, sharded):
+    # no wait for the device while a graph is captured, and a replay sees values written since
+    from scorch_b200 import kernels as K, pipelines as P, sharded as S
+    monkeypatch.setattr(K, "SPLIT_CHUNK_BYTES", 1e5)
+    pos, crd, val = _csr([60] * 2000, 2000, seed=8)
+    g = torch.Generator().manual_seed(4)
+    X, W1, W2 = (torch.randn(s, generator=g).cuda() for s in ((2000, 64), (64, 72), (72, 64)))
+    p, c, v = (torch.from_numpy(a).cuda() for a in (pos, crd, val))
+    shard = S.ShardedCsr.from_global(p, c, v, 0, 1)
+    forward = (lambda: S.gcn_forward_sharded(shard, X, W1, W2)) if sharded else (lambda: P.gcn_forward(p, c, v, X, W1, W2))
+    forward()                                    # buffers, kept split
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        forward()
+    torch.cuda.current_stream().wait_stream(side)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = forward()
+    for _ in range(2):
+        v.mul_(-0.5)
+        forward()                                # another split takes the kept one's place
+        junk = [torch.full((1 << 20,), 1 << 30, dtype=torch.int32, device="cuda") for _ in range(4)]
+        graph.replay()
+        del junk
+        A = torch.sparse_csr_tensor(p, c, v, size=(2000, 2000)).to_dense().double()
+        want = A @ (torch.relu(A @ (X.double() @ W1.double())) @ W2.double())
+        assert ((out.double() - want).norm() / want.norm()).item() < 1e-6
