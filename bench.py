@@ -427,9 +427,10 @@ class SpmmWorkload(Workload):
         return {"rows_this_rank": self.m, "nnz_this_rank": self.nnz}
 
     def alg_bytes(self):
-        return {"spmm_rows_kernel": (self.m + 1) * 4 + self.nnz * 8 + self.n * self.k * 4 + self.m * self.k * 4}
+        return {"spmm_tile_kernel": (self.m + 1) * 4 + self.nnz * 8 + self.n * self.k * 4 + self.m * self.k * 4}
 
-    kernels = ("spmm_rows_kernel",)
+    kernels = ("spmm_tile_kernel",)
+    launches_per_step = 2    # the tiles; empty rows and sums of rows in several units
 
     def step(self, ev=None):
         if self.flush is not None:
@@ -441,7 +442,7 @@ class SpmmWorkload(Workload):
             ev[1].record()
 
     def extras(self, stage_ms):
-        ms = stage_ms["spmm_rows_kernel"]
+        ms = stage_ms["spmm_tile_kernel"]
         gm_bytes = self.nnz * (8 + self.k * 4) + self.m * self.k * 4
         out = {"gather_model": {"bytes": gm_bytes, "GBps": gm_bytes / (ms * 1e-3) / 1e9,
                                 "what": "every stored entry counted as one operand-row read"}}
@@ -532,8 +533,8 @@ class SpmmWorkload(Workload):
 
 
 class SpgemmSpmv(Workload):
-    """Config 5: SpMV sweep and SpGEMM C = A A on a 2M power-law matrix; symbolic and numeric
-    phases timed separately.  Metric here: products (2 flops each) + SpMV flops per second."""
+    """Config 5: SpMV sweep and SpGEMM C = A A on a 2M power-law matrix, in the one-pass form that ``matmul``
+    takes.  Metric here: products (2 flops each) + SpMV flops per second."""
     name = "c5_spmspm_spmv_2M_powerlaw"
     SPMV_SWEEP = 10  # back-to-back SpMV calls per step: keeps the GPU busy between launches
 
@@ -554,7 +555,6 @@ class SpgemmSpmv(Workload):
         self.mv, _ = S.row_block(A.pos, A.crd, A.val, rank, self.world)
         self.mm, _ = S.row_block(A.pos, A.crd, A.val, rank, self.world,
                                  bounds=S.product_bounds(A.pos, A.crd, A.pos, self.world))
-        self.timings = []
 
     @property
     def flops_total(self):
@@ -577,15 +577,11 @@ class SpgemmSpmv(Workload):
         mv, mm = self.mv, self.mm
         # per rank: its rows of the left operand, the replicated operand read once, its outputs
         return {"spmv": (mv.rows + 1) * 4 + mv.nnz * 8 + n * 4 + mv.rows * 4,
-                "spgemm_symbolic": (mm.rows + 1) * 4 + mm.nnz * 4 + (n + 1) * 4 + nnz * 4 + (mm.rows + 1) * 4,
-                "spgemm_numeric": (mm.rows + 1) * 4 + mm.nnz * 8 + (n + 1) * 4 + nnz * 8 + (mm.rows + 1) * 4
-                                  + nnzc * 8}
+                "spgemm": (mm.rows + 1) * 4 + mm.nnz * 8 + (n + 1) * 4 + nnz * 8 + (mm.rows + 1) * 4 + nnzc * 8}
 
-    kernels = ("spmv", "spgemm_symbolic", "spgemm_numeric")
-    launches_per_step = 12
-
-    def begin_block(self):
-        self.timings = []
+    kernels = ("spmv", "spgemm")
+    # SpMV: tiles' rows, tiles, rows cut by tiles; SpGEMM: the launch list in profiles/c5_spgemm_spmv_kernels.md
+    launches_per_step = 3 * SPMV_SWEEP + 38
 
     def step(self, ev=None):
         A, mv, mm = self.A, self.mv, self.mm
@@ -595,20 +591,23 @@ class SpgemmSpmv(Workload):
             self.y = self.K.spmv_csr(mv.pos, mv.crd, mv.val, self.x)
         if ev is not None:
             ev[1].record()
-        t = {}
-        cpos, ccrd, cval = self.K.spgemm_csr(mm.pos, mm.crd, mm.val, A.pos, A.crd, A.val, self.n, timings=t)
-        self.nnzc = int(ccrd.numel())
+        cpos, ccrd, cval = self.K.spgemm_csr(mm.pos, mm.crd, mm.val, A.pos, A.crd, A.val, self.n)
         if ev is not None:
-            self.timings.append(t)
+            ev[2].record()
+        self.nnzc = int(ccrd.numel())
         del cpos, ccrd, cval
 
     def stage_times(self, evs):
-        return {"spmv": statistics.mean(e[0].elapsed_time(e[1]) for e in evs) / self.SPMV_SWEEP,
-                "spgemm_symbolic": statistics.mean(t["symbolic_ms"] for t in self.timings),
-                "spgemm_numeric": statistics.mean(t["numeric_ms"] for t in self.timings)}
+        ms = super().stage_times(evs)
+        return {"spmv": ms["spmv"] / self.SPMV_SWEEP, "spgemm": ms["spgemm"]}
 
     def extras(self, stage_ms):
-        return {"products_per_second": self.products / (stage_ms["spgemm_numeric"] * 1e-3)}
+        A, mm, phases = self.A, self.mm, {}
+        for _ in range(2):       # (the second call's times)
+            self.K.spgemm_csr(mm.pos, mm.crd, mm.val, A.pos, A.crd, A.val, self.n, timings=phases)
+        return {"products_per_second": self.products / (stage_ms["spgemm"] * 1e-3),
+                "two_phase_calls": {"what": "the same product through the symbolic and numeric calls, not part "
+                                            "of the step", **phases}}
 
     def traffic_key(self):
         return self.name
@@ -719,12 +718,17 @@ class GcnSharded(Workload):
 
     @property
     def launches_per_step(self):
-        # per layer one SpMM launch per row chunk (rows and heavy-row segments share the launch), or two per
-        # column chunk and panel of a matrix that is cut by columns
+        # two per product (the tiles, then empty rows and sums of rows in several units), a product per row
+        # chunk, or per column chunk and panel of a matrix that is cut by columns; two per dense transform
+        # that runs on the tensor cores (the split of W, the product)
+        from scorch_b200 import kernels as K
+
         def launches(split, k):
             cut = [b.columns[1] if b.columns else None for b in split.blocks]
-            return sum(2 * len(c.counts) * -(-k // K.SPLIT_PANEL) if c is not None else 1 for c in cut)
-        from scorch_b200 import kernels as K
+            products = sum(len(c.counts) * -(-k // K.SPLIT_PANEL) if c is not None else 1 for c in cut)
+            ends = [min(o, self.shard.rows) for o in split.offsets]
+            transforms = sum(b - a >= K.DENSE_MATMUL_MIN_ROWS for a, b in zip(ends, ends[1:]))
+            return 2 * products + 2 * transforms
         return launches(self.shard.splits[0], self.K1) + launches(self.shard.splits[-1], self.K2)
 
     def begin_block(self):
