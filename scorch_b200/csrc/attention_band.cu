@@ -23,8 +23,8 @@
 //   4. O += P V  is issued with P read from TMEM as the A operand and V^T (transposed while it is
 //      staged, so that it is K-major like K) as the B operand, 64 window columns at a time;
 //   5. the epilogue reads O from TMEM, merges the scattered entries' (max, sum, O) and writes O / sum.
-// TMEM: columns [0,384) S / P_hi (the first 128 also P_lo), [384,512) O.  Every mbarrier wait is bounded by
-// a clock limit; a wait that runs out sets a status word (sb_attn_band_status), the CTA frees its
+// TMEM: columns [0,384) S / P_hi (the first 128 also P_lo, in turns), [384,448) O by V hi, [448,512) O by V lo
+// (round 0's P_lo before that).  Every mbarrier wait is bounded by a clock limit; a wait that runs out sets a status word (sb_attn_band_status), the CTA frees its
 // TMEM and returns.  No TMA, no multicast, no cluster: every operand goes through registers for
 // the hi / lo split anyway.
 #include <algorithm>
@@ -204,13 +204,13 @@ struct BandPiece {
 };
 
 // 64 rows [row0, row0 + 64) of V (row pitch ld floats, rows outside [0, limit) read as zeros) ->
-// hi / lo parts of their transpose in the K-major layout without swizzle (core matrix = 8 rows x 16
-// bytes): "rows" are now the D features, the 64 window columns are the contiguous (K) direction, so an
-// 8-feature group holds 16 cores of 128 bytes.  (The B operand of O += P V has to be K-major: with the descriptor's B-major bit set
-// the tf32 instruction left the accumulator untouched on this hardware.)  A thread gathers four
-// consecutive window columns of one feature with scalar loads (a warp reads 128 contiguous bytes
-// per load) and stores them as one 16-byte piece; the 8 lanes of a feature group fill one core
-// matrix, so the stores are free of bank conflicts.
+// hi / lo parts of their transpose in the K-major layout with the 128-byte swizzle: "rows" are now the D
+// features, the 64 window columns are the contiguous (K) direction, in two halves of 32 columns = 128
+// bytes per feature; a half holds the D rows of the hi part, then those of the lo part.  (The B operand of
+// O += P V has to be K-major: with the descriptor's B-major bit set the tf32 instruction left the
+// accumulator untouched on this hardware.)  A thread gathers four consecutive window columns of one feature
+// with scalar loads (a warp reads 128 contiguous bytes per load) and stores them as one 16-byte piece;
+// the swizzle puts the pieces of 8 consecutive features into different banks.
 template <int D>
 struct BandPieceT {
   static constexpr int HALVES = D / 32;

@@ -837,12 +837,12 @@ int exclusive_scan_i32(int n, const int* cnt, int* out, long long* block_sum, lo
 }
 
 // ---- long rows of a matrix of few columns ---------------------------------------------------------
-// Bitmap and accumulators of all n columns in shared memory (n up to kSmemColumns): one CTA per row,
-// no plan, no read-back, one launch instead of the bucket path's ten (20,011 columns, ten rows of
-// 8,200 to 80,000 products: 190 us there, 92 us here, beside the other bins' kernels).
-// Few such rows leave most of the GPU to the others, so up to eight CTAs - a cluster - share a row: each
-// takes its part of the products into a bitmap and accumulators of its own, then emits a slice of the
-// columns, adding the others' sums out of their shared memory (CLUSTERED).
+// Bitmap and accumulators of all n columns in shared memory (n up to kSmemColumns): no plan, no read-back,
+// one launch instead of the bucket path's ten.  Few such rows leave most of the GPU to the others, so up to
+// eight CTAs - a cluster - share a row: each takes its part of the products into a bitmap and accumulators
+// of its own, then emits a slice of the columns, adding the others' sums out of their shared memory
+// (CLUSTERED).  20,011 columns, ten rows of 8,200 to 80,000 products: 190 us by buckets, 92 by one CTA per
+// row (beside the other bins' kernels), 49 by clusters of eight.
 constexpr int kSmemThreads = 1024;
 template <typename T, bool NUMERIC, bool CLUSTERED>
 __global__ void __launch_bounds__(kSmemThreads)
