@@ -24,9 +24,9 @@
 //      staged, so that it is K-major like K) as the B operand, 64 window columns at a time;
 //   5. the epilogue reads O from TMEM, merges the scattered entries' (max, sum, O) and writes O / sum.
 // TMEM: columns [0,384) S / P_hi (the first 128 also P_lo, in turns), [384,448) O by V hi, [448,512) O by V lo
-// (round 0's P_lo before that).  Every mbarrier wait is bounded by a clock limit; a wait that runs out sets a status word (sb_attn_band_status), the CTA frees its
-// TMEM and returns.  No TMA, no multicast, no cluster: every operand goes through registers for
-// the hi / lo split anyway.
+// (round 0's P_lo before that).  Every mbarrier wait is bounded by a clock limit; a wait that runs out sets
+// a status word (sb_attn_band_status), the CTA frees its TMEM and returns.  No TMA, no multicast, no
+// cluster: every operand goes through registers for the hi / lo split anyway.
 #include <algorithm>
 
 #include "attention.cuh"

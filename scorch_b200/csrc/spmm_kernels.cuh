@@ -743,7 +743,8 @@ static int launch_vec2(const SpmmArgs<T>& a, int64_t batch, const void* plan, in
 // (entry tiles when the caller gave their workspace; they have one variant for both)
 #define SB_GO(L, VEC, W, EXACT)                                                                \
   do {                                                                                         \
-    if (tile_ws && a.ldb * (long long)sizeof(T) < (1ll << 32)) return launch_tiles<T, L, VEC, W>(a, nnz, tile_ws, st);                       \
+    if (tile_ws && a.ldb * (long long)sizeof(T) < (1ll << 32))                                 \
+      return launch_tiles<T, L, VEC, W>(a, nnz, tile_ws, st);                                  \
     return launch_vec2<T, L, VEC, W, EXACT>(a, batch, plan, nnz, plan_segments, scratch, st);  \
   } while (0)
 #define SB_GO_FIT(L, VEC, W)                                  \
