@@ -581,7 +581,7 @@ class SpgemmSpmv(Workload):
 
     kernels = ("spmv", "spgemm")
     # SpMV: tiles' rows, tiles, rows cut by tiles; SpGEMM: the launch list in profiles/c5_spgemm_spmv_kernels.md
-    launches_per_step = 3 * SPMV_SWEEP + 38
+    launches_per_step = 3 * SPMV_SWEEP + 28
 
     def step(self, ev=None):
         A, mv, mm = self.A, self.mv, self.mm
