@@ -29,6 +29,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <exception>
 #include <vector>
 
 #include <cooperative_groups.h>
@@ -1320,6 +1321,16 @@ static int row_pointers(const WsLayout& w, int64_t m, int32_t* Cpos, int64_t* to
   return SB_OK;
 }
 
+// No C++ exception leaves a C entry point: the long rows' plans are vectors in host memory.
+template <typename F>
+static int caught(const char* name, F&& f) {
+  try {
+    return f();
+  } catch (const std::exception& e) {
+    return fail(SB_ERR_CUDA, "%s: out of host memory (%s)", name, e.what());
+  }
+}
+
 }  // namespace sb
 
 using namespace sb;
@@ -1354,7 +1365,9 @@ int sb_spgemm_symbolic(int64_t m, int64_t kb, int64_t n, const int32_t* Apos, co
   long long counts[kBins];
   for (int b = 0; b < kBins; b++) counts[b] = cursors[b];
   const CsrIn in{Apos, Acrd, nullptr, Bpos, Bcrd, nullptr};
-  rc = launch_bins<float, false>(w, counts, m, kb, n, in, RowsOut{w.row_cnt, nullptr, nullptr, nullptr}, st);
+  rc = caught("spgemm_symbolic", [&] {
+    return launch_bins<float, false>(w, counts, m, kb, n, in, RowsOut{w.row_cnt, nullptr, nullptr, nullptr}, st);
+  });
   if (rc != SB_OK) return rc;
   // keep the bin sizes in the workspace header for the numeric phase
   SB_CUDA(cudaMemcpyAsync(w.hdr, counts, sizeof(counts), cudaMemcpyHostToDevice, st));
@@ -1385,7 +1398,9 @@ int sb_spgemm_numeric(int dtype, int64_t m, int64_t kb, int64_t n, const int32_t
   if (binned == 0) return SB_OK;
   SB_CHECK_ARG(Ccrd && Cval && Aval && Bval, "spgemm_numeric: null pointer");
   const CsrIn in{Apos, Acrd, Aval, Bpos, Bcrd, Bval};
-  return launch_bins_typed<true>(dtype, w, counts, m, kb, n, in, RowsOut{nullptr, Cpos, Ccrd, Cval}, st);
+  return caught("spgemm_numeric", [&] {
+    return launch_bins_typed<true>(dtype, w, counts, m, kb, n, in, RowsOut{nullptr, Cpos, Ccrd, Cval}, st);
+  });
 }
 
 int sb_spgemm_begin(int64_t m, int64_t kb, int64_t n, const int32_t* Apos, const int32_t* Acrd,
@@ -1436,7 +1451,9 @@ int sb_spgemm_rows(int dtype, int64_t m, int64_t kb, int64_t n, const int32_t* A
   SB_CHECK_ARG(binned <= m, "spgemm_rows: counts are not those of sb_spgemm_begin");
   SB_CHECK_ARG(binned == 0 || (tcrd && tval && Aval && Bval), "spgemm_rows: null pointer");
   const CsrIn in{Apos, Acrd, Aval, Bpos, Bcrd, Bval};
-  rc = launch_bins_typed<true>(dtype, w, counts, m, kb, n, in, RowsOut{w.row_cnt, off, tcrd, tval}, st);
+  rc = caught("spgemm_rows", [&] {
+    return launch_bins_typed<true>(dtype, w, counts, m, kb, n, in, RowsOut{w.row_cnt, off, tcrd, tval}, st);
+  });
   if (rc != SB_OK) return rc;
   return row_pointers(w, m, Cpos, total_nnz_host, st);
 }

@@ -33,6 +33,7 @@ def recorded(tmp_path_factory):
 
     class Recorded:
         abi = lib
+        file = path
 
         @staticmethod
         def call(fn, *args):
@@ -101,3 +102,30 @@ def test_spmm_windows_fill_the_device_at_hand(recorded, k, per_sm):
             assert sms * per_sm * 0.8 < recorded.abi.recorder_grid(0) <= sms * per_sm
         finally:
             recorded.abi.recorder_device(0)
+
+
+def test_spgemm_reports_missing_host_memory(recorded):
+    # the list of the long rows (2 GB for 2^27 of them) does not fit the process: a status, not an exception
+    # through the C entry point, which would end the process
+    import sys
+
+    from scorch_b200._lib import SIGNATURES
+    m = 1 << 27
+    script = f"""
+import ctypes as C, resource
+L = C.CDLL({recorded.file!r})
+L.sb_spgemm_workspace_bytes.restype, L.sb_spgemm_workspace_bytes.argtypes = C.c_size_t, [C.c_int64, C.c_int64, C.c_int]
+L.sb_last_error.restype = C.c_char_p
+need = L.sb_spgemm_workspace_bytes({m}, 30000, 2)
+resource.setrlimit(resource.RLIMIT_AS, (1 << 30, 1 << 30))
+p = [C.c_void_p(16)] * 9                  # never dereferenced: the list comes first
+counts, total = (C.c_int64 * 5)(0, 0, 0, 0, {m}), C.c_int64(0)
+I = C.c_int64
+rc = L.sb_spgemm_rows(C.c_int(2), I({m}), I({m}), I(30000), *p[:7], counts, p[7], p[8], p[0], C.byref(total),
+                      p[1], C.c_size_t(need), None)
+print(rc, L.sb_last_error().decode())
+"""
+    assert len(SIGNATURES["sb_spgemm_rows"][1]) == 19
+    r = subprocess.run([sys.executable, "-c", script], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stderr
+    assert r.stdout.startswith("2 ") and "host memory" in r.stdout
