@@ -170,8 +170,9 @@ SB_API int sb_spmm_csr_typed(int dtype, int64_t m, int64_t n, int64_t k, int64_t
  * feature transforms of a graph layer, A tall (m x k, row pitch lda), W small (k x n).  k <= 32768 and
  * lda multiples of 4, A 16-byte aligned; ldc a multiple of 8, C 32-byte aligned (SB_ERR_UNSUPPORTED
  * otherwise); ws: sb_dense_matmul_workspace_bytes(n, k) bytes, 16-byte aligned.
- * Any values: rows of A with values of 2^127 and above, Inf or NaN, and every row where W holds one, take
- * fp32 FMAs instead of the tensor cores, as do the rows behind a wait inside the kernel that ran out.
+ * Any values: rows of A with values of 2^127 and above, Inf or NaN, every row where W holds one, and rows
+ * with results that are not finite or below 2^-100 (but not 0) take fp32 FMAs instead of the tensor cores,
+ * as do the rows behind a wait inside the kernel that ran out.  Denormal operands may count as 0.
  * sb_dense_matmul_status() (synchronises): 0, or 1 when such a wait ever ran out, or -1 when it could not
  * be read.
  * sb_dense_matmul_probe: self-test.  The tensor cores' issuing thread of every CTA stops at its 32-row

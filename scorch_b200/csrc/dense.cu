@@ -24,7 +24,9 @@
 // Every wait is bounded; one that runs out sets a status word and ends the CTA's pipeline.
 // The CTA's tiles that the pipeline left - behind a wait that ran out, or with a value too large for the
 // split (2^127 and above, Inf, NaN) in the rows of A, or all of them with one in W - it does with fp32
-// FMAs at its end, so C is complete whatever happened.
+// FMAs at its end, so C is complete whatever happened; and so the tiles with a result that is not finite
+// (the parts' products overflow to opposite infinities) or below 2^-100 and not 0 (the parts are denormal
+// and short of bits: 3e-5 off at 1e-36).
 #include <algorithm>
 
 #include "tensor_core.cuh"
@@ -36,6 +38,7 @@ constexpr int kGemmProducers = 256, kGemmThreads = kGemmProducers + 128 + 32;
 constexpr int kRaw = 4;                       // chunks of A on their way
 constexpr int kRedoWords = 512;               // tiles of a CTA that are noted one by one (14,170 at most on 148 SMs)
 constexpr unsigned kSplitMax = 0x7f000000u;   // bits of 2^127: values from here on, Inf and NaN are not split
+constexpr unsigned kResultMin = 0x0d800000u;  // bits of 2^-100: results from here to the largest float are kept
 
 __device__ int g_gemm_status = 0;  // 0 ok; 1 a wait ran out
 
@@ -128,7 +131,7 @@ struct GemmSmem {
   // 2 + STAGES tiles ahead of the epilogue, so a place is free again before it is used again
   int odd[8];
   int done;                   // tiles the epilogue has finished ...
-  unsigned redo[kRedoWords];  // ... and those among them that it has left out (odd), a bit each
+  unsigned redo[kRedoWords];  // ... and those among them that are to be done again, a bit each
 };
 
 // One tile by fp32 FMAs, in the order of K: 256 threads, 4 rows x NMAX / 16 columns each at a time,
@@ -348,12 +351,18 @@ gemm_f32_kernel(const __grid_constant__ GemmArgs g) {
       tc_fence_after();
       const bool odd = *(volatile int*)&sm.odd[i & 7] != 0;
       float* crow = g.C + row * g.ldc + n0;
+      float finite = 0.f;          // (NaN once a result is not)
+      unsigned least = ~0u;        // 2 x (bits of the smallest magnitude but 0) - 2
       for (int c0 = 0; c0 < cols; c0 += 32) {
         float v[32], small[32];
         tmem_ld32(t_row + (uint32_t)((i & 1) * 2 * NMAX + c0), v);
         tmem_ld32(t_row + (uint32_t)((i & 1) * 2 * NMAX + NMAX + c0), small);
 #pragma unroll
-        for (int j = 0; j < 32; j++) v[j] += small[j];
+        for (int j = 0; j < 32; j++) {
+          v[j] += small[j];
+          finite = fmaf(v[j], 0.f, finite);
+          least = min(least, 2u * __float_as_uint(v[j]) - 2u);
+        }
         if (row < g.m && !odd) {
           if (c0 + 32 <= cols) {
 #pragma unroll
@@ -371,11 +380,10 @@ gemm_f32_kernel(const __grid_constant__ GemmArgs g) {
       }
       tc_fence_before();
       asm volatile("barrier.cta.sync 1, 128;" ::: "memory");   // all four warps have read `odd`
+      if (odd || finite != 0.f || least < 2u * kResultMin - 2u)
+        atomicOr(&sm.redo[min(i >> 5, kRedoWords - 1)], 1u << (i & 31));
       if (r == 0) {
-        if (odd) {
-          *(volatile int*)&sm.odd[i & 7] = 0;
-          sm.redo[min(i >> 5, kRedoWords - 1)] |= 1u << (i & 31);
-        }
+        if (odd) *(volatile int*)&sm.odd[i & 7] = 0;
         sm.done = i + 1;
       }
       mbar_arrive(smem_u32(&sm.acc_empty[i & 1]));

@@ -91,3 +91,40 @@ def test_values_beyond_the_split_take_no_longer_than_other_kernels_do():
     mine = ms(lambda: K.dense_matmul(X, W))
     print(f"library {library:.3f} ms, FMA form {mine:.3f} ms")
     assert mine < 8 * library
+
+
+def test_results_that_overflow():
+    # the library's answer to sums beyond the largest float: infinities, not what the parts of the split add up to
+    g = torch.Generator(device="cuda").manual_seed(0)
+    X, W = torch.randn((40000, 64), generator=g, device="cuda"), torch.randn((64, 72), generator=g, device="cuda")
+    X[5], X[6, 0], X[39999, 3] = 1.6e38, 1.6e38, -1.6e38
+    W[0], W[3] = 1414.2135, 141.42135
+    got, want = _run(X, W), X.double() @ W.double()
+    for row, sign in ((6, 1), (39999, -1)):
+        assert (got[row] == sign * float("inf")).all()
+    assert not torch.isnan(got[torch.arange(40000, device="cuda") != 5]).any()
+    fine = want.abs().amax(1) < 1e30
+    assert fine.sum() == 40000 - 3
+    assert ((got[fine].double() - want[fine]).norm() / want[fine].norm()).item() < 2e-7
+
+
+@pytest.mark.parametrize("scale", [1e-38, 1e-36, 1e-33, 1e-30, 1e30, 1e36])
+@pytest.mark.parametrize("of", ["X", "W", "one row", "one column"])
+def test_results_far_from_one(scale, of):
+    g = torch.Generator(device="cuda").manual_seed(1)
+    X, W = torch.randn((40000, 64), generator=g, device="cuda"), torch.randn((64, 72), generator=g, device="cuda")
+    rows, cols = slice(None), slice(None)
+    if of == "X":
+        X *= scale
+    elif of == "W":
+        W *= scale
+    elif of == "one row":
+        rows = slice(777, 778)
+        X[rows] *= scale
+    else:
+        cols = slice(70, 71)
+        W[:, cols] *= scale
+    got, want, library = (c[rows, cols].double() for c in (_run(X, W), X.double() @ W.double(), torch.matmul(X, W)))
+    err = lambda c: ((c - want).norm() / want.norm()).item()
+    # (one denormal step of 2^-149 per product where operands of 1e-38 lose bits of their own)
+    assert err(got) <= max(2e-7, 1.5 * err(library))
