@@ -101,9 +101,9 @@ def test_spmm_vs_oracle_all_column_widths(oracle, k):
 
 @pytest.mark.parametrize("k", [8, 16, 20, 32, 64, 72, 128, 256, 300])
 def test_spmm_many_short_rows(oracle, k):
-    """Mean row length below the short-row threshold: a row per lane group (narrow tiles) or
-    several rows per warp; rows too long for a lane group, empty rows and heavy rows mixed in,
-    plain and accumulating, with and without the heavy-row plan."""
+    """Short rows with rows too long for a lane group, empty rows and rows of several units mixed in, plain and
+    accumulating; a plan that is given makes no difference (one matrix runs over tiles of its entries; the row
+    kernels of the same shapes are in test_gpu_row_kernels.py)."""
     from scorch_b200 import kernels as K
     from scorch_b200._lib import HEAVY_ROW_NNZ as T
     rng = np.random.default_rng(100 + k)
@@ -133,7 +133,8 @@ def test_spmm_many_short_rows(oracle, k):
 
 @pytest.mark.parametrize("k", [64, 256, 520])
 def test_spmm_heavy_rows_and_plan(oracle, k):
-    """Rows around and far above the heavy threshold go through the segment kernels."""
+    """Rows around and far above the plan's threshold, in units of the tile kernel (the segment kernels of the
+    same shapes are in test_gpu_row_kernels.py)."""
     from scorch_b200 import kernels as K
     from scorch_b200._lib import HEAVY_ROW_NNZ as T
     m, n = 40, 6000
@@ -151,14 +152,15 @@ def test_spmm_heavy_rows_and_plan(oracle, k):
     bias = np.random.default_rng(13).standard_normal(k).astype(np.float32)
     got = K.spmm_csr(dpos, dev(crd), dev(val), dev(B), bias=dev(bias), relu=False, plan=plan)
     assert_close(oracle, got, oracle.spmm_csr_acc64(pos, crd, val, B, bias, False), "heavy rows")
-    # bitwise reproducible: partial sums are combined in a fixed order
+    # bitwise reproducible: unit sums are combined in a fixed order
     again = K.spmm_csr(dpos, dev(crd), dev(val), dev(B), bias=dev(bias), relu=False, plan=plan)
     assert torch.equal(got, again)
 
 
 @pytest.mark.parametrize("k", [64, 256])
 def test_spmm_accumulating_form(oracle, k):
-    """sb_spmm_csr_acc_f32: act(bias + C + A B) with short, empty and multi-segment heavy rows."""
+    """act(bias + C + A B) with short and empty rows and rows of several units (sb_spmm_csr_acc_f32:
+    test_gpu_row_kernels.py)."""
     from scorch_b200 import kernels as K
     from scorch_b200._lib import HEAVY_ROW_NNZ as T
     m, n = 50, 5000
@@ -208,7 +210,7 @@ def test_spmm_degenerate_shapes(oracle):
 
 
 def test_c1_config_full_size(oracle):
-    """4096x4096, 1 % uniform, k = 64, through scorch.matmul on host tensors."""
+    """Benchmark configuration 1: 4096x4096, 1 % uniform, k = 64, through scorch.matmul on host tensors."""
     import scorch_b200 as scorch
     from scorch_b200 import workloads as W
     A = W.csr_uniform(4096, 4096, 0.01, seed=0)
@@ -321,7 +323,7 @@ def test_softmax_golden_and_edge_rows(oracle, golden):
 
 
 def test_c2_sparse_attention_reduced_and_batched(oracle):
-    """BASELINE config 2 at seq 1024 (band 32 + 1 % random), 2x3 heads: whole pipeline vs fp64."""
+    """Benchmark configuration 2 at seq 1024 (band 32 + 1 % random), 2x3 heads: whole pipeline vs fp64."""
     from scorch_b200 import kernels as K, pipelines as P, workloads as W
     mask = W.attention_mask(1024, window=32, density=0.01, seed=0)
     Q, Km, V = W.attention_qkv(2, 3, 1024, 64, seed=1)

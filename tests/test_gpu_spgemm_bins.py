@@ -71,7 +71,7 @@ def test_buckets_with_many_equal_columns(dtype):
 
 
 def test_row_beyond_the_area():
-    # more products in one row than the workspace holds (1 M for a small matrix): dense kernel
+    # more products in one row than the area of a wider matrix holds (1 M): summed in shared memory here
     rng = np.random.default_rng(3)
     B = _csr([900] * 1300, 1000, rng, np.float32)
     _check(_csr([1300, 2, 700], 1300, rng, np.float32), B, 1000, np.float32)
