@@ -524,8 +524,9 @@ class ColumnSplit:
     @staticmethod
     def of(pos, crd, val, n: int, k: int) -> Optional["ColumnSplit"]:
         """The split for products with operands of up to ``k`` columns, or None where it does not pay, or
-        the columns do not ascend.  None too while the stream is captured into a graph: the split waits for
-        the device, and a graph would go on reading a copy of the matrix as it was."""
+        the columns do not ascend, or memory for the copy is not there.  None too while the stream is
+        captured into a graph: the split waits for the device, and a graph would go on reading a copy of the
+        matrix as it was."""
         if not (val.dtype == torch.float32 and pos.dtype == crd.dtype == torch.int32 and val.numel() == crd.numel()
                 and all(t.is_cuda and t.is_contiguous() for t in (pos, crd, val))):
             return None
@@ -538,6 +539,8 @@ class ColumnSplit:
         except _lib.ScorchB200Error as e:
             if e.status != 5:
                 raise
+            return None
+        except torch.OutOfMemoryError:
             return None
 
     def matmul(self, B: torch.Tensor, relu: bool = False, out: Optional[torch.Tensor] = None,

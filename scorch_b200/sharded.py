@@ -103,6 +103,7 @@ class CsrBlock:
         if (counted and kept is not None and kept[0][:3] == key[:3]
                 and all(a is b for a, b in zip(kept[0][3], sources))):
             return kept[1]
+        self.columns = kept = None           # (its memory is free for the next one)
         split = K.ColumnSplit.of(self.pos, self.crd, self.val, n, k)
         self.columns = (key, split)
         return split

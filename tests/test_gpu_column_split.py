@@ -197,3 +197,25 @@ def test_captured_forward_reads_the_matrix_itself(monkeypatch, sharded):
         A = torch.sparse_csr_tensor(p, c, v, size=(2000, 2000)).to_dense().double()
         want = A @ (torch.relu(A @ (X.double() @ W1.double())) @ W2.double())
         assert ((out.double() - want).norm() / want.norm()).item() < 1e-6
+
+
+@pytest.mark.parametrize("sharded", [False, True])
+def test_forward_without_memory_for_the_copy(monkeypatch, sharded):
+    # the products of the matrix itself need none
+    from scorch_b200 import kernels as K, pipelines as P, sharded as S
+    monkeypatch.setattr(K, "SPLIT_CHUNK_BYTES", 1e5)
+    pos, crd, val = _csr([60] * 2000, 2000, seed=9)
+    g = torch.Generator().manual_seed(5)
+    X, W1, W2 = (torch.randn(s, generator=g).cuda() for s in ((2000, 64), (64, 72), (72, 64)))
+    p, c, v = (torch.from_numpy(a).cuda() for a in (pos, crd, val))
+    tried = []
+
+    def no_memory(self, *args):
+        tried.append(args)
+        raise torch.OutOfMemoryError("no memory")
+    monkeypatch.setattr(K.ColumnSplit, "__init__", no_memory)
+    got = (S.gcn_forward_sharded(S.ShardedCsr.from_global(p, c, v, 0, 1), X, W1, W2) if sharded
+           else P.gcn_forward(p, c, v, X, W1, W2))
+    A = torch.sparse_csr_tensor(p, c, v, size=(2000, 2000)).to_dense().double()
+    want = A @ (torch.relu(A @ (X.double() @ W1.double())) @ W2.double())
+    assert tried and ((got.double() - want).norm() / want.norm()).item() < 1e-6
