@@ -357,24 +357,30 @@ gemm_f32_kernel(const __grid_constant__ GemmArgs g) {
         float v[32], small[32];
         tmem_ld32(t_row + (uint32_t)((i & 1) * 2 * NMAX + c0), v);
         tmem_ld32(t_row + (uint32_t)((i & 1) * 2 * NMAX + NMAX + c0), small);
+        // (columns from `cols` on hold what an earlier kernel left there)
+        auto look = [&](float x) {
+          finite = fmaf(x, 0.f, finite);
+          least = min(least, 2u * __float_as_uint(x) - 2u);
+        };
 #pragma unroll
-        for (int j = 0; j < 32; j++) {
-          v[j] += small[j];
-          finite = fmaf(v[j], 0.f, finite);
-          least = min(least, 2u * __float_as_uint(v[j]) - 2u);
-        }
-        if (row < g.m && !odd) {
-          if (c0 + 32 <= cols) {
+        for (int j = 0; j < 32; j++) v[j] += small[j];
+        if (c0 + 32 <= cols) {
+#pragma unroll
+          for (int j = 0; j < 32; j++) look(v[j]);
+          if (row < g.m && !odd) {
 #pragma unroll
             for (int j = 0; j < 32; j += 8)
               asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(crow + c0 + j), "f"(v[j]),
                            "f"(v[j + 1]), "f"(v[j + 2]), "f"(v[j + 3]), "f"(v[j + 4]), "f"(v[j + 5]), "f"(v[j + 6]),
                            "f"(v[j + 7])
                            : "memory");
-          } else {
+          }
+        } else {
 #pragma unroll
-            for (int j = 0; j < 32; j++)
-              if (c0 + j < cols) crow[c0 + j] = v[j];
+          for (int j = 0; j < 32; j++) {
+            if (c0 + j >= cols) continue;
+            look(v[j]);
+            if (row < g.m && !odd) crow[c0 + j] = v[j];
           }
         }
       }

@@ -128,3 +128,18 @@ def test_results_far_from_one(scale, of):
     err = lambda c: ((c - want).norm() / want.norm()).item()
     # (one denormal step of 2^-149 per product where operands of 1e-38 lose bits of their own)
     assert err(got) <= max(2e-7, 1.5 * err(library))
+
+
+@pytest.mark.parametrize("n", [8, 16, 40, 72, 136])
+def test_bits_do_not_depend_on_what_ran_before(n):
+    # tensor-memory columns behind the last one of C hold what an earlier product left: NaNs here
+    g = torch.Generator(device="cuda").manual_seed(n)
+    X, W = torch.randn((40000, 64), generator=g, device="cuda"), torch.randn((64, n), generator=g, device="cuda")
+    wide = torch.randn((64, 64 if n <= 64 else 128), generator=g, device="cuda")
+    bad = X.clone()
+    bad[:, 5] = float("nan")
+    results = []
+    for before in (bad, X, X * 1e-36):
+        _run(before, wide)
+        results.append(_run(X, W))
+    assert torch.equal(results[0], results[1]) and torch.equal(results[0], results[2])
