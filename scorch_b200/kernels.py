@@ -520,6 +520,7 @@ class ColumnSplit:
                                              ws.data_ptr(), wbytes, _stream()))
         self.counts = list(counts)
         self.first = [sum(self.counts[:c]) for c in range(chunks)]     # first entry of every chunk
+        self.stream = torch.cuda.current_stream(dev)
 
     @staticmethod
     def of(pos, crd, val, n: int, k: int) -> Optional["ColumnSplit"]:
@@ -559,6 +560,10 @@ class ColumnSplit:
             _validated(self.pos[c], self.crd[first:first + self.counts[c]], B.shape[0], "ColumnSplit.matmul")
         if out is None:
             out = torch.empty((self.m, k), dtype=torch.float32, device=B.device)
+        here = torch.cuda.current_stream(B.device)
+        if here != self.stream:          # (memory of a split that is dropped waits for its last product)
+            for t in (self.pos, self.crd, self.val):
+                t.record_stream(here)
         L, last = _lib.lib(), len(self.counts) - 1
         with torch.cuda.device(B.device):
             wbytes = max(L.sb_spmm_csr_once_workspace_bytes(SB_F32, min(k, SPLIT_PANEL), c) for c in self.counts)

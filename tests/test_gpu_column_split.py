@@ -219,3 +219,22 @@ def test_forward_without_memory_for_the_copy(monkeypatch, sharded):
     A = torch.sparse_csr_tensor(p, c, v, size=(2000, 2000)).to_dense().double()
     want = A @ (torch.relu(A @ (X.double() @ W1.double())) @ W2.double())
     assert tried and ((got.double() - want).norm() / want.norm()).item() < 1e-6
+
+
+def test_split_dropped_while_another_stream_multiplies_it():
+    from scorch_b200 import kernels as K
+    pos, crd, val = (torch.from_numpy(a).cuda() for a in _csr([60] * 20000, 20000, seed=10))
+    B = torch.randn((20000, 64), device="cuda")
+    want = K.spmm_csr(pos, crd, val, B)
+    out = torch.empty_like(want)
+    split, side = K.ColumnSplit(pos, crd, val, 20000, 5), torch.cuda.Stream()
+    sizes = [(t.numel(), t.dtype) for t in (split.pos, split.crd, split.val)]
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(200_000_000)           # a tenth of a second: the product is still to come
+        split.matmul(B, out=out)
+    del split
+    fresh = [torch.zeros(n, dtype=t, device="cuda") for n, t in sizes]      # would take the split's memory
+    torch.cuda.synchronize()
+    assert all((t == 0).all() for t in fresh)
+    assert torch.allclose(out, want, rtol=1e-4, atol=1e-4)
