@@ -4,7 +4,8 @@
 // or lane group per row, most of the GPU waits for the few that got long rows.  Here a CTA takes
 // the rows that begin in a window of TE consecutive entries, so every CTA has about the same number
 // of entries, and inside it a row is taken by whatever suits its length:
-//   up to kGroupRow entries    one lane group (L lanes across the operand's columns)
+//   up to kGroupRow entries    one lane group (L lanes across the operand's columns), rows of similar
+//                              length side by side in a warp
 //   up to kWarpRow             the lane groups of a warp, a slice each
 //   longer                     all lane groups of the CTA, in units of kUnit entries; the unit sums
 //                              of a row of several units are added in order by a second launch
@@ -28,18 +29,28 @@ constexpr int kUnit = 512;             // a window's last row or unit reaches up
 // Largest window.  Wide rows (L = 32) have work enough in 1536 entries and lose residency to more
 // (6 M entries, 256 columns: 371 us, 415 with 3072); narrow ones gain by having their start-up
 // spread over twice as many (0.8 M entries in rows of 8, 64 columns: 27.0 us, 22.9 with 3072).
-constexpr int tile_window(int L) { return L == 32 ? 1536 : 3072; }
+// 8-byte types, whose entries take 16 bytes: as much as lets three CTAs stay within 196 KB of shared memory.
+// Beyond that 23 KB are left to L1 in place of 55 and the gathers wait for it (120,000 rows of 27 entries, 16
+// float64 columns: 47.9 us with 3072, 43.2 with this).
+constexpr int tile_window(int L, int size = 4) { return L == 32 ? 1536 : size == 8 ? 2560 : 3072; }
 // Rows of up to this length go to a lane group.  32 lets the warp's other groups help with a row of
 // a power-law graph (2 M rows, 64 columns: 6.10 ms with 64, 5.66 with 32); the 8 groups of four
-// lanes have too little of a 33-entry row each (27 entries per row, 16 float64 columns: 53.6 us
-// with 32, 49.6 with 64).
+// lanes have too little of a 33-entry row each (27 entries per row, 16 float64 columns: 51.4 us
+// with 32, 47.9 with 40 and with 64; power law of mean 20, 8 columns: 29.0, 29.6, 31.7).
 template <int L>
-constexpr int kGroupRow = L == 4 ? 64 : 32;
+constexpr int kGroupRow = L == 4 ? 40 : 32;
 constexpr int kWarpRow = 192;
 constexpr int kTileRowCap = 1024;      // row pointers kept in shared memory at a time
 constexpr int kTileLists = 96;         // rows of the window that a warp / the CTA takes
-static_assert(tile_window(8) / 33 + 2 <= kTileLists && tile_window(4) / 65 + 2 <= kTileLists &&
-              tile_window(32) / 33 + 2 <= kTileLists, "rows longer than kGroupRow of a window");
+// Classes of similar length among the rows that a lane group takes.  A warp's groups take rows of one class,
+// the longest first: in the order of the matrix they waited for the longest of their 2 to 8 rows.  (GCN
+// layer of 2 M rows, 202 M entries, 64-column panels: 20.4 ms in the matrix's order, 19.1 by class; power law
+// of mean 12, 32 columns: 46.8 us, 39.8.  Taken as one stream of entries per group across the rows' ends,
+// without a wait at any of them, the same rows were slower by 2: 505 us in place of 250 with 256 columns.)
+constexpr int kShortClasses = 4;
+static_assert(tile_window(8) / (kGroupRow<8> + 1) + 2 <= kTileLists &&
+              tile_window(4) / (kGroupRow<4> + 1) + 2 <= kTileLists &&
+              tile_window(32) / (kGroupRow<32> + 1) + 2 <= kTileLists, "rows longer than kGroupRow of a window");
 static_assert(tile_window(8) / kWarpRow + tile_window(8) / kUnit + 4 <= kTileLists, "units of a window");
 
 // Resident CTAs per SM the kernels are compiled for (64 / 80 registers; measured per lane count).
@@ -47,11 +58,11 @@ constexpr int tile_ctas(int L) { return L == 32 ? 4 : 3; }
 // Entries per window, a multiple of 32: as few full waves of CTAs over the chip as windows of at
 // most tile_window(L) allow (a last wave that is half empty costs as much as a full one), at least 64
 // and at least four per lane group.
-inline int tile_entries(int64_t nnz, int L) {
+inline int tile_entries(int64_t nnz, int L, int size) {
   const int64_t slots = (int64_t)sm_count() * tile_ctas(L);
-  const int64_t waves = std::max<int64_t>(1, ceil_div(nnz, slots * tile_window(L)));
+  const int64_t waves = std::max<int64_t>(1, ceil_div(nnz, slots * tile_window(L, size)));
   const int64_t te = ceil_div(ceil_div(nnz, slots * waves), 32) * 32;
-  return (int)std::min<int64_t>(std::max<int64_t>(te, std::max(64, 1024 / L)), tile_window(L));
+  return (int)std::min<int64_t>(std::max<int64_t>(te, std::max(64, 1024 / L)), tile_window(L, size));
 }
 
 template <typename T>
@@ -75,9 +86,13 @@ struct TileUnit {
 template <typename T, int L, int VEC, int W>
 struct TileSmem {
   Pack<T, W> part[kTileWarps][VEC][L];
-  Entry<T> entry[tile_window(L) + kUnit];
+  Entry<T> entry[tile_window(L, sizeof(T)) + kUnit];
   int pos[kTileRowCap + 2];
   TileUnit by_warp[kTileLists], by_cta[kTileLists];
+  // rows of a turn that a lane group takes, by length (where a warp has several groups)
+  // (two classes share an array, one from each end)
+  unsigned short short_row[L == 32 ? 1 : kShortClasses / 2][kTileRowCap];
+  int n_short[kShortClasses];
   int n_warp, n_cta, next_warp, next_row;
   int count[kTileWarps];
 };
@@ -199,7 +214,8 @@ spmm_tile_kernel(SpmmArgs<T> a, TileArgs<T> t) {
   for (int next = e0; next < e1;) {
     const int r0 = cta_row_of<kTileThreadsMm>(a.pos, a.m, next, sm.count);
     for (int i = tid; i < kTileRowCap + 1; i += kTileThreadsMm) sm.pos[i] = __ldg(a.pos + min(a.m, r0 + i));
-    if (tid == 0) { sm.n_warp = sm.n_cta = sm.next_warp = sm.next_row = 0; }
+    if (tid < kShortClasses) sm.n_short[tid] = 0;
+    if (tid == 0) sm.n_warp = sm.n_cta = sm.next_warp = sm.next_row = 0;
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
     // rows and units too long for a lane group, as far as they begin in the window
@@ -208,6 +224,22 @@ spmm_tile_kernel(SpmmArgs<T> a, TileArgs<T> t) {
       const int b = sm.pos[i], len = sm.pos[i + 1] - b;
       const bool here = b < e1 && r0 + i < a.m;
       rows += here;
+      if constexpr (G > 1) {
+        if (!__any_sync(FULL, here)) break;
+        const int c = here && b >= next && len > 0 && len <= kGroupRow<L>
+                          ? kShortClasses - 1 - (len - 1) / (kGroupRow<L> / kShortClasses) : -1;
+        unsigned mine = 0, lanes = 0;    // lanes of this lane's class, of class `lane`
+#pragma unroll
+        for (int q = 0; q < kShortClasses; q++) {
+          const unsigned x = __ballot_sync(FULL, c == q);
+          mine = c == q ? x : mine;
+          lanes = lane == q ? x : lanes;
+        }
+        int at = 0;
+        if (lane < kShortClasses) at = atomicAdd(&sm.n_short[lane], __popc(lanes));
+        at = __shfl_sync(FULL, at, c & (kShortClasses - 1)) + __popc(mine & ((1u << lane) - 1u));
+        if (c >= 0) sm.short_row[c >> 1][c & 1 ? kTileRowCap - 1 - at : at] = (unsigned short)i;
+      }
       if (!here || len <= kGroupRow<L>) continue;
       if (len <= kWarpRow) {
         if (b >= next) sm.by_warp[atomicAdd(&sm.n_warp, 1)] = TileUnit{r0 + i, b, len, 1};
@@ -219,12 +251,20 @@ spmm_tile_kernel(SpmmArgs<T> a, TileArgs<T> t) {
           sm.by_cta[atomicAdd(&sm.n_cta, 1)] = TileUnit{r0 + i, b + u * kUnit, min(kUnit, len - u * kUnit), len <= kUnit};
       }
     }
-    rows = __reduce_add_sync(FULL, rows);
-    if (lane == 0) sm.count[warp] = rows;
-    __syncthreads();
-    rows = 0;
+    int n_short[kShortClasses];          // (rows up to the class's end)
+    if constexpr (G > 1) {
+      __syncthreads();
+      rows = 0;
 #pragma unroll
-    for (int w = 0; w < kTileWarps; w++) rows += sm.count[w];
+      for (int c = 0; c < kShortClasses; c++) n_short[c] = rows += sm.n_short[c];
+    } else {
+      rows = __reduce_add_sync(FULL, rows);
+      if (lane == 0) sm.count[warp] = rows;
+      __syncthreads();
+      rows = 0;
+#pragma unroll
+      for (int w = 0; w < kTileWarps; w++) rows += sm.count[w];
+    }
     const int n_cta = sm.n_cta, n_warp = sm.n_warp;
 
     for (int panel = blockIdx.y; panel < t.panels; panel += gridDim.y) {
@@ -295,8 +335,18 @@ spmm_tile_kernel(SpmmArgs<T> a, TileArgs<T> t) {
       i = __shfl_sync(FULL, i, 0);
       if (i >= rows) break;
       i += g;
-      const int b = sm.pos[i < rows ? i : 0], len = i < rows ? sm.pos[i + 1] - b : 0;
-      if (b < next || len == 0 || len > kGroupRow<L>) continue;
+      if constexpr (G > 1) {
+        if (i >= rows) continue;
+        int c = 0, before = 0;
+#pragma unroll
+        for (int q = 0; q + 1 < kShortClasses; q++) {
+          c += i >= n_short[q];
+          before = i >= n_short[q] ? n_short[q] : before;
+        }
+        i = sm.short_row[c >> 1][c & 1 ? kTileRowCap - 1 - (i - before) : i - before];
+      }
+      const int b = sm.pos[i], len = sm.pos[i + 1] - b;
+      if (G == 1 && (b < next || len == 0 || len > kGroupRow<L>)) continue;
       Pack<T, W> s[VEC];
       tile_begin_row<T, L, VEC, W>(s, a, r0 + i, col0, col_ok, true);
       tile_add<T, VEC, W, U>(s, sm.entry, b - e0, b - e0 + len, Bcol, pitch);
@@ -367,7 +417,7 @@ static int launch_tiles(const SpmmArgs<T>& a, int64_t nnz, void* ws, cudaStream_
   // which L2 holds (262,144 entries, 16 panels of 32 MB: 286 us panel by panel, 249 this way).
   // Otherwise panel after panel on grid.y.
   const bool in_l2 = (double)a.n * a.ldb * sizeof(T) <= 64e6;
-  t.entries = tile_entries(in_l2 ? nnz * panels : nnz, L);
+  t.entries = tile_entries(in_l2 ? nnz * panels : nnz, L, sizeof(T));
   t.tiles = (int)ceil_div(nnz, t.entries);
   t.first = static_cast<T*>(ws);
   t.rest = t.first + (size_t)(nnz / kUnit + 1) * a.k;
