@@ -47,6 +47,7 @@ constexpr int64_t kBigProductsMax = (int64_t)1 << 26;
 constexpr int64_t kBucketProducts = 1024;      // buckets per row: U / this, rounded up to a power of two
 constexpr int kBucketSort = 2048;              // products a bucket's sorting kernel takes
 constexpr int kBigTasks = 1 << 17;
+constexpr int kTurnProducts = 8192;            // products of 256 entries of A that a task takes; the rest is dealt out anew
 // Columns up to which long rows are summed in shared memory (spgemm_smem_kernel) and need no area.
 constexpr int kSmemColumns = 24576;
 
@@ -81,7 +82,9 @@ struct BigArea {
   int* row;             // [rows] row id
   int* p0;              // [rows + 1] first bucket
   int* shift;           // [rows] bucket of a column = first bucket + (column >> shift)
-  int* tasks;           // [tasks][3] row index, first and last + 1 entry of A
+  int4* tasks;          // row index, first and last + 1 entry of A, part << 16 | parts (0: see big_expand)
+  int* nrest;           // number of ...
+  int4* rest;           // ... products left over: row index, first and last + 1 entry of A, first product
   double* scale;        // [rows] fixed-point scale
   int *cnt, *off, *cursor, *bucket_row, *ucnt, *uoff;   // per bucket
   long long* block_sum;
@@ -95,7 +98,9 @@ static BigArea big_area(char* p, int64_t products) {
   size_t off = 0;
   auto take = [&](size_t bytes) { char* q = p + off; off += align_up(bytes); return q; };
   b.row = (int*)take(nb * 4); b.p0 = (int*)take(nb * 4); b.shift = (int*)take(nb * 4);
-  b.tasks = (int*)take((size_t)kBigTasks * 12);
+  b.tasks = (int4*)take((size_t)kBigTasks * sizeof(int4));
+  b.nrest = (int*)take(4);
+  b.rest = (int4*)take((size_t)(products / kTurnProducts + 1) * sizeof(int4));
   b.scale = (double*)take(nb * 8);
   b.cnt = (int*)take(nb * 4); b.off = (int*)take(nb * 4); b.cursor = (int*)take(nb * 4);
   b.bucket_row = (int*)take(nb * 4); b.ucnt = (int*)take(nb * 4); b.uoff = (int*)take(nb * 4);
@@ -333,40 +338,141 @@ big_scale_kernel(BigArea b, const int* __restrict__ Apos, const T* __restrict__ 
   }
 }
 
-// One task = some entries of one long row of A.  SCATTER false: products per bucket; true: every
-// product's column (and value) to the next free place of its bucket.
+// One task = some entries of one long row of A, or, of a row of up to 512 entries, a part of the products.  SCATTER false: products per bucket; true: every
+// product's column (and value) to the next free place of its bucket.  A task of the first kind takes
+// up to kTurnProducts products per 256 entries; what is beyond that - an entry of A can bring 400,000 - is noted by the
+// counting kernel in equal parts, which REST launches of both take: the CTA that had such an entry kept the GPU waiting.
 // (One 16-byte record per product: a column and a value array cost a third scattered access.)
+// Bound: the latency of a batch (B's entries in short pieces, places, stores).  A CTA counts kScatter products a
+// thread per bucket, takes their places together, one atomic per bucket, and writes them in the buckets' order.
+// Rows of more buckets than are counted in shared memory take a place per product.  67 M products of 2,350 rows:
+// counted in 0.27 ms (0.56 with a task per 512 entries), scattered in 1.0 (1.47).
+constexpr int kScatter = 8, kScatterCta = 256 * kScatter;
 template <typename T, bool NUMERIC, bool SCATTER>
-__global__ void __launch_bounds__(256)
-big_expand_kernel(BigArea b, CsrIn in) {
-  __shared__ int s_hist[SCATTER ? 1 : kHistBuckets];
-  __shared__ ExpandSmem<T, 256> s_expand;
-  const int tid = threadIdx.x;
-  const int r = b.tasks[3 * blockIdx.x], ab = b.tasks[3 * blockIdx.x + 1], ae = b.tasks[3 * blockIdx.x + 2];
-  const int p0 = b.p0[r], buckets = b.p0[r + 1] - p0, shift = b.shift[r];
-  const bool in_smem = !SCATTER && buckets <= kHistBuckets;
+struct BigExpandSmem {
+  int hist[kHistBuckets], to[SCATTER ? kHistBuckets : 1], warp[8];
+  unsigned col[SCATTER ? kScatterCta : 1];
+  Slot val[SCATTER && NUMERIC ? kScatterCta : 1];
+  ExpandSmem<T, 256> expand;
+};
+template <typename T, bool NUMERIC, bool SCATTER, bool REST>
+__device__ __forceinline__ void big_expand(const BigArea& b, const CsrIn& in, BigExpandSmem<T, NUMERIC, SCATTER>& sm,
+                                           int r, int ab, int ae, int begin, int step, int end) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int p0 = b.p0[r], buckets = b.p0[r + 1] - p0, shift = b.shift[r], per = (buckets + 255) / 256;
+  const bool in_smem = buckets <= kHistBuckets;
   if (in_smem) {
-    for (int p = tid; p < buckets; p += 256) s_hist[p] = 0;
+    for (int p = tid; p < buckets; p += 256) sm.hist[p] = 0;
     __syncthreads();
   }
   const T* Bval = static_cast<const T*>(in.Bval);
-  expand_cta<T, NUMERIC, 256>(in, ab, ae, s_expand, tid, [&](int, T a, int pb) {
-    const int c = __ldg(in.Bcrd + pb), p = c >> shift;
-    if (!SCATTER) {
-      atomicAdd(in_smem ? &s_hist[p] : &b.cnt[p0 + p], 1);
-    } else {
-      const Slot v = NUMERIC ? product_bits<T>(a, __ldg(Bval + pb)) : 0;
-      const int slot = atomicAdd(&b.cursor[p0 + p], 1);
-      if (NUMERIC) b.rec[slot] = BigRecord{(unsigned)c, 0u, v};
-      else b.key[slot] = (unsigned)c;
+  auto put = [&](int slot, unsigned c, Slot v) {
+    if (NUMERIC) b.rec[slot] = BigRecord{c, 0u, v};
+    else b.key[slot] = c;
+  };
+  int turn0 = ab;
+  expand_turns<T, NUMERIC, 256>(in, ab, ae, sm.expand, tid, [&](int, int total, auto&& find) {
+    if (!REST && !SCATTER && total > end) {
+      __shared__ int s_rest;
+      const int n = (total - 1) / kTurnProducts;
+      if (tid == 0) s_rest = atomicAdd(b.nrest, n);
+      __syncthreads();
+      for (int x = tid; x < n; x += 256)
+        b.rest[s_rest + x] = make_int4(r, turn0, min(turn0 + 256, ae), (x + 1) * kTurnProducts);
+      __syncthreads();
+    }
+    turn0 += 256;
+    total = min(total, end);
+    for (int q0 = begin; q0 < total; q0 += step) {
+      unsigned c[kScatter];
+      Slot v[kScatter];
+      int rank[kScatter];
+#pragma unroll
+      for (int k = 0; k < kScatter; k++) {
+        const int q = q0 + k * 256 + tid;
+        if (q >= total) continue;
+        const int e = find(q), pb = sm.expand.off[e] + q;
+        c[k] = (unsigned)__ldg(in.Bcrd + pb);
+        if (SCATTER) v[k] = NUMERIC ? product_bits<T>(sm.expand.a[e], __ldg(Bval + pb)) : 0;
+      }
+      if (!in_smem) {
+#pragma unroll
+        for (int k = 0; k < kScatter; k++) {
+          if (q0 + k * 256 + tid >= total) continue;
+          const int p = p0 + (int)(c[k] >> shift);
+          if (SCATTER) put(atomicAdd(&b.cursor[p], 1), c[k], v[k]);
+          else atomicAdd(&b.cnt[p], 1);
+        }
+        continue;
+      }
+#pragma unroll
+      for (int k = 0; k < kScatter; k++)
+        if (q0 + k * 256 + tid < total) rank[k] = atomicAdd(&sm.hist[c[k] >> shift], 1);
+      if constexpr (SCATTER) {
+        __syncthreads();
+        // counts to places of the buckets in the batch (hist) and, less these, in the area (to)
+        int sum = 0;
+        for (int p = tid * per; p < min(buckets, tid * per + per); p++) sum += sm.hist[p];
+        int incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int y = __shfl_up_sync(FULL, incl, o);
+          if (lane >= o) incl += y;
+        }
+        if (lane == 31) sm.warp[warp] = incl;
+        __syncthreads();
+        int at = incl - sum;
+#pragma unroll
+        for (int w = 0; w < 8; w++) at += w < warp ? sm.warp[w] : 0;
+        for (int p = tid * per; p < min(buckets, tid * per + per); p++) {
+          const int n = sm.hist[p];
+          if (n) sm.to[p] = atomicAdd(&b.cursor[p0 + p], n) - at;
+          sm.hist[p] = at;
+          at += n;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < kScatter; k++) {
+          if (q0 + k * 256 + tid < total) {
+            const int x = sm.hist[c[k] >> shift] + rank[k];
+            sm.col[x] = c[k];
+            if (NUMERIC) sm.val[x] = v[k];
+          }
+        }
+        __syncthreads();
+        for (int x = tid; x < min(total - q0, kScatterCta); x += 256)
+          put(sm.to[sm.col[x] >> shift] + x, sm.col[x], NUMERIC ? sm.val[x] : 0);
+        for (int p = tid; p < buckets; p += 256) sm.hist[p] = 0;
+        __syncthreads();
+      }
     }
   });
-  if (in_smem) {
+  if (!SCATTER && in_smem) {
     __syncthreads();
     for (int p = tid; p < buckets; p += 256) {
-      const int c = s_hist[p];
+      const int c = sm.hist[p];
       if (c) atomicAdd(&b.cnt[p0 + p], c);
     }
+    __syncthreads();
+  }
+}
+
+template <typename T, bool NUMERIC, bool SCATTER, bool REST>
+__global__ void __launch_bounds__(256)
+big_expand_kernel(BigArea b, CsrIn in) {
+  __shared__ BigExpandSmem<T, NUMERIC, SCATTER> sm;
+  if (REST) {
+    const int n = *b.nrest;
+    for (int i = blockIdx.x; i < n; i += gridDim.x) {
+      const int4 x = b.rest[i];
+      big_expand<T, NUMERIC, SCATTER, true>(b, in, sm, x.x, x.y, x.z, x.w, kScatterCta, x.w + kTurnProducts);
+      __syncthreads();
+    }
+  } else {
+    const int4 x = b.tasks[blockIdx.x];
+    const int part = x.w >> 16, parts = x.w & 0xffff;
+    big_expand<T, NUMERIC, SCATTER, false>(b, in, sm, x.x, x.y, x.z, part * kScatterCta, max(parts, 1) * kScatterCta,
+                                           parts ? INT_MAX : kTurnProducts);
   }
 }
 
@@ -759,58 +865,35 @@ scan_write_kernel(int m, const int* __restrict__ cnt, const long long* __restric
   }
 }
 
-// All of it by one CTA, for short arrays: a warp per contiguous part, 128 counts at a time, four per lane
-// (one per lane made a chain of 20 scans for 20,000 counts: 9.2 us).
+// Short arrays in one launch: a CTA scans 1024 counts and adds up all that lie before them, so that no CTA
+// waits for another.  (By one CTA: 7.3 us for 20,000 counts, 4.0 this way.)
 constexpr int kScanSmall = 32768;
 __global__ void __launch_bounds__(1024)
 scan_small_kernel(int m, const int* __restrict__ cnt, int* __restrict__ out, long long* __restrict__ total) {
-  constexpr int STEPS = kScanSmall / 4096;
-  __shared__ long long s[32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int steps = (m + 4095) / 4096, b = warp * steps * 128;
-  long long mine = 0;
+  __shared__ long long s_before[32], s_sum[32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, b0 = blockIdx.x * 1024;
+  long long before = 0;
+#pragma unroll 8
+  for (int x = tid; x < b0; x += 1024) before += __ldg(cnt + x);
+  const int i = b0 + tid, c = i < m ? __ldg(cnt + i) : 0;
+  long long incl = c;
 #pragma unroll
-  for (int i = 0; i < STEPS; i++) {
-    const int x = b + i * 128 + lane * 4;
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      if (i < steps && x + q < m) mine += cnt[x + q];
-    }
+  for (int o = 1; o < 32; o <<= 1) {
+    const long long y = __shfl_up_sync(FULL, incl, o);
+    if (lane >= o) incl += y;
   }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(FULL, mine, o);
-  if (lane == 0) s[warp] = mine;
+  for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(FULL, before, o);
+  if (lane == 0) s_before[warp] = before;
+  if (lane == 31) s_sum[warp] = incl;
   __syncthreads();
-  long long run = 0, all = 0;
+  long long at = s_before[lane] + (lane < warp ? s_sum[lane] : 0);
 #pragma unroll
-  for (int w = 0; w < 32; w++) {
-    const long long v = s[w];
-    if (w < warp) run += v;
-    all += v;
-  }
-  if (threadIdx.x == 0) { out[0] = 0; *total = all; }
-#pragma unroll
-  for (int i = 0; i < STEPS; i++) {
-    if (i >= steps) break;
-    const int x = b + i * 128 + lane * 4;
-    int c[4];   // (read again: kept, they would spill)
-#pragma unroll
-    for (int q = 0; q < 4; q++) c[q] = x + q < m ? cnt[x + q] : 0;
-    const long long four = (long long)c[0] + c[1] + c[2] + c[3];
-    long long incl = four;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const long long y = __shfl_up_sync(FULL, incl, o);
-      if (lane >= o) incl += y;
-    }
-    long long at = run + incl - four;
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      at += c[q];
-      if (x + q < m) out[x + q + 1] = (int)at;
-    }
-    run += __shfl_sync(FULL, incl, 31);
-  }
+  for (int o = 16; o > 0; o >>= 1) at += __shfl_xor_sync(FULL, at, o);
+  at += incl;
+  if (i < m) out[i + 1] = (int)at;
+  if (i == 0) out[0] = 0;
+  if (i == m - 1) *total = at;
 }
 
 // Exclusive scan of n int counts into out[0..n] (int32), running total in int64 at *total_dev.
@@ -823,7 +906,7 @@ int exclusive_scan_i32(int n, const int* cnt, int* out, long long* block_sum, lo
     return SB_OK;
   }
   if (n <= kScanSmall) {
-    scan_small_kernel<<<1, 1024, 0, st>>>(n, cnt, out, total_dev);
+    scan_small_kernel<<<(unsigned)ceil_div(n, 1024), 1024, 0, st>>>(n, cnt, out, total_dev);
     SB_LAUNCH_CHECK("scan_small_kernel");
     return SB_OK;
   }
@@ -844,7 +927,7 @@ int exclusive_scan_i32(int n, const int* cnt, int* out, long long* block_sum, lo
 // of its own, then emits a slice of the columns, adding the others' sums out of their shared memory
 // (CLUSTERED).  20,011 columns, ten rows of 8,200 to 80,000 products: 190 us by buckets, 92 by one CTA per
 // row (beside the other bins' kernels), 49 by clusters of eight.
-constexpr int kSmemThreads = 1024;
+constexpr int kSmemThreads = 1024, kSmemParts = 8;
 template <typename T, bool NUMERIC, bool CLUSTERED>
 __global__ void __launch_bounds__(kSmemThreads)
 spgemm_smem_kernel(const int* __restrict__ rows, CsrIn in, int n, const unsigned long long* __restrict__ max_b,
@@ -856,6 +939,7 @@ spgemm_smem_kernel(const int* __restrict__ rows, CsrIn in, int n, const unsigned
   __shared__ ExpandSmem<T, NT> s_expand;
   __shared__ double s_abs[NW];
   __shared__ int s_part[NW], s_at[kSmemColumns / 32];
+  __shared__ unsigned s_words[CLUSTERED ? kSmemColumns / 32 : 1];   // the parts' words of this CTA's columns
   __shared__ int s_total;
   let_next_begin();
   namespace cg = cooperative_groups;
@@ -865,7 +949,7 @@ spgemm_smem_kernel(const int* __restrict__ rows, CsrIn in, int n, const unsigned
   const int ab = __ldg(in.Apos + i), ae = __ldg(in.Apos + i + 1);
   for (int x = tid; x < kSmemColumns / 32; x += NT) bits[x] = 0;
   if (NUMERIC)
-    for (int x = tid; x < n; x += NT) acc[x] = 0;
+    for (int x = tid; x < (n + 1) / 2; x += NT) reinterpret_cast<ulonglong2*>(acc)[x] = ulonglong2{0, 0};
   double scale = 1.0;
   if constexpr (NUMERIC && kIsFloat<T>) {
     double s = 0.0;
@@ -881,19 +965,30 @@ spgemm_smem_kernel(const int* __restrict__ rows, CsrIn in, int n, const unsigned
   const bool fixed = scale == scale;
   __syncthreads();
   const T* Bval = static_cast<const T*>(in.Bval);
-  expand_cta<T, NUMERIC, NT>(in, ab, ae, s_expand, tid, [&](int, T a, int pb) {
+  // a row of many entries is cut by entries (every part looking all of them up took 51,000 cycles for 10,014 of
+  // them, 23,000 to 43,000 this way), one of few by products: a single entry can bring most of them
+  const bool by_entries = parts > 1 && ae - ab >= 2 * NT;
+  const int share = by_entries ? (ae - ab + parts - 1) / parts : ae - ab;
+  const int eb = by_entries ? min(ae, ab + part * share) : ab, ee = by_entries ? min(ae, eb + share) : ae;
+  expand_cta<T, NUMERIC, NT>(in, eb, ee, s_expand, tid, [&](int, T a, int pb) {
     const int c = __ldg(in.Bcrd + pb);
     const unsigned bit = 1u << (c & 31);
     if (!(bits[c >> 5] & bit)) atomicOr(&bits[c >> 5], bit);
     if (NUMERIC) acc_add_smem<T>(&acc[c], product_bits<T>(a, __ldg(Bval + pb)), scale, fixed);
-  }, part, parts);
+  }, by_entries ? 0 : part, by_entries ? 1 : parts);
   // this CTA's words of the bitmap (kSmemColumns / 32 = 768 in all), one per thread, in column order
   const int words = kSmemColumns / 32 / parts, w0 = part * words;
   unsigned m = 0;
   if constexpr (CLUSTERED) {
     cg::this_cluster().sync();
     if (tid < words) {
-      for (int p = 0; p < parts; p++) m |= cg::this_cluster().map_shared_rank(bits, p)[w0 + tid];
+#pragma unroll
+      for (int p = 0; p < kSmemParts; p++) {
+        if (p >= parts) break;
+        const unsigned x = cg::this_cluster().map_shared_rank(bits, p)[w0 + tid];
+        s_words[p * words + tid] = x;
+        m |= x;
+      }
       bits[w0 + tid] = m;      // (a part's words are read by that part alone)
     }
   } else {
@@ -921,8 +1016,9 @@ spgemm_smem_kernel(const int* __restrict__ rows, CsrIn in, int n, const unsigned
     if (tid == 0) s_total = total;
     cg::this_cluster().sync();
     total = 0;
-    for (int p = 0; p < parts; p++) {
-      const int v = *cg::this_cluster().map_shared_rank(&s_total, p);
+#pragma unroll
+    for (int p = 0; p < kSmemParts; p++) {
+      const int v = p < parts ? *cg::this_cluster().map_shared_rank(&s_total, p) : 0;
       if (p < part) before_parts += v;
       total += v;
     }
@@ -941,13 +1037,19 @@ spgemm_smem_kernel(const int* __restrict__ rows, CsrIn in, int n, const unsigned
       const int col = (w0 + w) * 32 + lane;
       Slot v = acc[col];
       if constexpr (CLUSTERED) {
-        v = *cg::this_cluster().map_shared_rank(acc + col, 0);
-        for (int p = 1; p < parts; p++) {
-          const Slot x = *cg::this_cluster().map_shared_rank(acc + col, p);
+        Slot x[kSmemParts];
+#pragma unroll
+        for (int p = 0; p < kSmemParts; p++) {   // (only what a part has: 140 KB a CTA otherwise)
+          const bool has = p < parts && s_words[p * words + w] >> lane & 1;
+          x[p] = has ? *cg::this_cluster().map_shared_rank(acc + col, p) : 0;
+        }
+        v = x[0];
+#pragma unroll
+        for (int p = 1; p < kSmemParts; p++) {
           if (kIsFloat<T> && !fixed)
-            v = (Slot)__double_as_longlong(__longlong_as_double((long long)v) + __longlong_as_double((long long)x));
+            v = (Slot)__double_as_longlong(__longlong_as_double((long long)v) + __longlong_as_double((long long)x[p]));
           else
-            v += x;
+            v += x[p];
         }
       }
       out.crd[at] = col;
@@ -962,39 +1064,47 @@ spgemm_smem_kernel(const int* __restrict__ rows, CsrIn in, int n, const unsigned
 }
 
 // ---- one-pass form: the rows' entries from their product offsets to their place ------------------
-// A CTA moves kMoveTile consecutive entries of the result, whatever the rows' lengths (a warp per row
+// A CTA moves `tile` consecutive entries of the result, whatever the rows' lengths (a warp per row
 // left the hub rows to a warp each: 4.7 ms for 272 M entries); a thread finds the row of its entry
-// among the tile's row pointers in shared memory.
+// among the tile's row pointers in shared memory.  Tiles of kMoveTile entries, smaller where that leaves SMs idle
+// (1.1 M entries: 15.3 us in 136 tiles of 8192, 9.4 in 542 of 2048).
 constexpr int kMoveTile = 8192, kMoveRows = 1024;
 template <typename T>
 __global__ void __launch_bounds__(256)
-spgemm_move_kernel(int m, int nnz, const int* __restrict__ off, const int* __restrict__ Cpos,
+spgemm_move_kernel(int m, int nnz, int tile, const int* __restrict__ off, const int* __restrict__ Cpos,
                    const int* __restrict__ tcrd, const T* __restrict__ tval, int* __restrict__ Ccrd,
                    T* __restrict__ Cval) {
   __shared__ int s_pos[kMoveRows + 1], s_shift[kMoveRows];
-  __shared__ int s_count[8];
-  const int tid = threadIdx.x;
-  const int e1 = min((long long)nnz, ((long long)blockIdx.x + 1) * kMoveTile);
-  for (int e = blockIdx.x * kMoveTile; e < e1;) {
+  __shared__ int s_first[kMoveRows / 32], s_count[8];
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int e1 = min((long long)nnz, ((long long)blockIdx.x + 1) * tile);
+  for (int e = blockIdx.x * tile; e < e1;) {
     const int r0 = cta_row_of<256>(Cpos, m, e, s_count);
     for (int x = tid; x < kMoveRows + 1; x += 256) {
       const int r = min(m, r0 + x), p = __ldg(Cpos + r);
       s_pos[x] = p;
+      if (x % 32 == 0 && x < kMoveRows) s_first[x / 32] = p;
       if (x < kMoveRows && r < m) s_shift[x] = __ldg(off + r) - p;
     }
     __syncthreads();
     const int stop = min(e1, s_pos[kMoveRows]);
 #pragma unroll 4
-    for (int o = e + tid; o < stop; o += 256) {
-      int lo = 0, hi = kMoveRows;
-#pragma unroll
-      for (int step = 0; step < 10; step++) {
-        const int mid = (lo + hi) >> 1;
-        const bool right = s_pos[mid] <= o;
-        lo = right ? mid : lo;
-        hi = right ? hi : mid;
+    for (int o0 = e + (tid & ~31); o0 < stop; o0 += 256) {
+      // the row of the warp's first entry by two rounds of 32 looks, this lane's a few rows behind it
+      const int c = __popc(__ballot_sync(FULL, s_first[lane] <= o0)) - 1;
+      int r = 32 * c + __popc(__ballot_sync(FULL, s_pos[32 * c + lane] <= o0)) - 1;
+      const int o = o0 + lane;
+      if (o >= stop) continue;
+#pragma unroll 1
+      for (int step = 0; step < 6 && s_pos[r + 1] <= o; step++) r++;
+      if (s_pos[r + 1] <= o) {           // many short or empty rows
+        int hi = kMoveRows;
+        while (hi - r > 1) {
+          const int mid = (r + hi) >> 1;
+          if (s_pos[mid] <= o) r = mid; else hi = mid;
+        }
       }
-      const int src = o + s_shift[lo];
+      const int src = o + s_shift[r];
       Ccrd[o] = __ldg(tcrd + src);
       Cval[o] = __ldg(tval + src);
     }
@@ -1051,28 +1161,40 @@ static int dense_row(const WsLayout& w, int row, int64_t n, const CsrIn& in, con
 // One batch of long rows whose plan (rows, first buckets, shifts, tasks) is in host memory.
 template <typename T, bool NUMERIC>
 static int big_batch(const WsLayout& w, const std::vector<int>& row, const std::vector<int>& p0,
-                     const std::vector<int>& shift, const std::vector<int>& tasks, int64_t n, const CsrIn& in,
+                     const std::vector<int>& shift, const std::vector<int4>& tasks, int64_t n, const CsrIn& in,
                      const RowsOut& out, cudaStream_t st) {
   const BigArea b = big_area(w.area, w.products);
   const int rows = (int)row.size(), buckets = p0.back();
   SB_CUDA(cudaMemcpyAsync(b.row, row.data(), row.size() * 4, cudaMemcpyHostToDevice, st));
   SB_CUDA(cudaMemcpyAsync(b.p0, p0.data(), p0.size() * 4, cudaMemcpyHostToDevice, st));
   SB_CUDA(cudaMemcpyAsync(b.shift, shift.data(), shift.size() * 4, cudaMemcpyHostToDevice, st));
-  SB_CUDA(cudaMemcpyAsync(b.tasks, tasks.data(), tasks.size() * 4, cudaMemcpyHostToDevice, st));
-  const unsigned ntasks = (unsigned)(tasks.size() / 3);
+  SB_CUDA(cudaMemcpyAsync(b.tasks, tasks.data(), tasks.size() * sizeof(int4), cudaMemcpyHostToDevice, st));
+  // products may be left over where a row is cut by entries
+  bool left = false;
+  for (const int4& x : tasks) left = left || !x.w;
+  if (left) SB_CUDA(cudaMemsetAsync(b.nrest, 0, 4, st));
+  const unsigned ntasks = (unsigned)tasks.size(), nrest = 4u * sm_count();
   big_setup_kernel<<<rows, 128, 0, st>>>(b, rows);
   SB_LAUNCH_CHECK("big_setup_kernel");
   if constexpr (NUMERIC && kIsFloat<T>) {
     big_scale_kernel<T><<<rows, 256, 0, st>>>(b, in.Apos, static_cast<const T*>(in.Aval), w.max_b);
     SB_LAUNCH_CHECK("big_scale_kernel");
   }
-  big_expand_kernel<T, false, false><<<ntasks, 256, 0, st>>>(b, in);
+  big_expand_kernel<T, false, false, false><<<ntasks, 256, 0, st>>>(b, in);
   SB_LAUNCH_CHECK("big_expand_kernel");
+  if (left) {
+    big_expand_kernel<T, false, false, true><<<nrest, 256, 0, st>>>(b, in);
+    SB_LAUNCH_CHECK("big_expand_kernel");
+  }
   int rc = exclusive_scan_i32(buckets, b.cnt, b.off, b.block_sum, w.hdr + 8, st);
   if (rc != SB_OK) return rc;
   SB_CUDA(cudaMemcpyAsync(b.cursor, b.off, (size_t)buckets * 4, cudaMemcpyDeviceToDevice, st));
-  big_expand_kernel<T, NUMERIC, true><<<ntasks, 256, 0, st>>>(b, in);
+  big_expand_kernel<T, NUMERIC, true, false><<<ntasks, 256, 0, st>>>(b, in);
   SB_LAUNCH_CHECK("big_expand_kernel");
+  if (left) {
+    big_expand_kernel<T, NUMERIC, true, true><<<nrest, 256, 0, st>>>(b, in);
+    SB_LAUNCH_CHECK("big_expand_kernel");
+  }
   const int widest = *std::max_element(shift.begin(), shift.end());
   if (widest + 11 <= 32) big_sort_kernel<T, NUMERIC, unsigned><<<buckets, 128, 0, st>>>(b);
   else big_sort_kernel<T, NUMERIC, unsigned long long><<<buckets, 128, 0, st>>>(b);
@@ -1107,9 +1229,9 @@ static int max_abs(const WsLayout& w, const CsrIn& in, int64_t kb, cudaStream_t 
 template <typename T, bool NUMERIC>
 static int launch_smem_bin(const int* rows, int64_t count, const WsLayout& w, int64_t n, const CsrIn& in,
                            const RowsOut& out, bool early, cudaStream_t st) {
-  const int smem = kSmemColumns / 8 + (NUMERIC ? (int)n * 8 : 0);
+  const int smem = kSmemColumns / 8 + (NUMERIC ? (int)(n + 1) / 2 * 16 : 0);
   // CTAs per row: as many as keep all of them (one per SM) on the GPU at a time
-  unsigned parts = 8;
+  unsigned parts = kSmemParts;
   while (parts > 1 && (int64_t)parts * count > sm_count()) parts /= 2;
   if (parts == 1) {
     auto k = spgemm_smem_kernel<T, NUMERIC, false>;
@@ -1150,8 +1272,15 @@ static int big_rows(const WsLayout& w, int64_t count, int64_t m, int64_t n, cons
     SB_CUDA(cudaStreamSynchronize(st));
   }
   const int nbits = ceil_log2(std::max<int64_t>(n, 1));
-  std::vector<int> row, p0{0}, shift, tasks;
-  int64_t products = 0;
+  std::vector<int> row, p0{0}, shift;
+  std::vector<int4> tasks;
+  // batches of about equal size, as few as the area allows
+  int64_t products = 0, total = 0;
+  for (const int4& x : info) total += x.y > w.products ? 0 : x.y;
+  const int64_t target = total / std::max<int64_t>(1, ceil_div(total, w.products));
+  // products per task: small enough to give every SM a few tasks
+  const int64_t task_products =
+      std::min<int64_t>(kTurnProducts, std::max<int64_t>(kScatterCta, total / (4 * sm_count()) / kScatterCta * kScatterCta));
   auto flush = [&]() -> int {
     if (row.empty()) return SB_OK;
     const int rc = big_batch<T, NUMERIC>(w, row, p0, shift, tasks, n, in, out, st);
@@ -1170,18 +1299,19 @@ static int big_rows(const WsLayout& w, int64_t count, int64_t m, int64_t n, cons
     const int s = std::max(0, nbits - ceil_log2(ceil_div(x.y, kBucketProducts)));
     const int buckets = (int)((n - 1) >> s) + 1;
     const int len = x.w - x.z;
-    int chunk = 512;                     // A entries per task
+    int chunk = 512;                     // A entries per task; the products of up to that many are cut evenly
     while (ceil_div(len, chunk) > kBigTasks / 4) chunk *= 2;
-    if (products + x.y > w.products || p0.back() + buckets > big_buckets(w.products) ||
-        (int64_t)tasks.size() / 3 + ceil_div(len, chunk) > kBigTasks) {
+    const int parts = len <= chunk ? (int)std::min<int64_t>(kBigTasks / 4, ceil_div(x.y, task_products)) : 0;
+    const int64_t more = std::max<int64_t>(parts, ceil_div(len, chunk));
+    if (products >= target || products + x.y > w.products || p0.back() + buckets > big_buckets(w.products) ||
+        (int64_t)tasks.size() + more > kBigTasks) {
       const int rc = flush();
       if (rc != SB_OK) return rc;
     }
-    for (int b = x.z; b < x.w; b += chunk) {
-      tasks.push_back((int)row.size());
-      tasks.push_back(b);
-      tasks.push_back((int)std::min<int64_t>((int64_t)b + chunk, x.w));
-    }
+    for (int part = 0; part < parts; part++) tasks.push_back(make_int4((int)row.size(), x.z, x.w, part << 16 | parts));
+    if (!parts)
+      for (int b = x.z; b < x.w; b += chunk)
+        tasks.push_back(make_int4((int)row.size(), b, (int)std::min<int64_t>((int64_t)b + chunk, x.w), 0));
     row.push_back(x.x);
     shift.push_back(s);
     p0.push_back(p0.back() + buckets);
@@ -1209,15 +1339,24 @@ static int launch_cta_bin(const int* rows, int64_t count, const WsLayout& w, con
   return SB_OK;
 }
 
-template <typename T, bool NUMERIC>
-static int launch_split_bin(const int* rows, int64_t count, const WsLayout& w, const CsrIn& in, int nbits,
-                            const RowsOut& out, cudaStream_t st) {
-  auto k = spgemm_split_kernel<T, NUMERIC>;
+template <typename T, bool NUMERIC, int NT>
+static int launch_split_rows(const int* rows, int64_t count, const WsLayout& w, const CsrIn& in, int64_t n,
+                             const RowsOut& out, cudaStream_t st) {
+  auto k = spgemm_split_kernel<T, NUMERIC, NT>;
   const int smem = kSplitCap * (int)(sizeof(unsigned) + (NUMERIC ? sizeof(Slot) : 0));
   SB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  k<<<(unsigned)count, kSplitThreads, smem, st>>>(rows, w.upper, in, std::max(0, nbits - 5), out);
+  const unsigned width = (unsigned)std::max<int64_t>(1, ceil_div(n, kSplitSegments<NT>));
+  k<<<(unsigned)count, NT, smem, st>>>(rows, w.upper, in, (int)width,
+                                       (unsigned)(((1ull << 32) + width - 1) / width), out);
   SB_LAUNCH_CHECK("spgemm_split_kernel");
   return SB_OK;
+}
+// (a CTA per SM while all rows fit so, with twice the threads; beyond that two per SM)
+template <typename T, bool NUMERIC>
+static int launch_split_bin(const int* rows, int64_t count, const WsLayout& w, const CsrIn& in, int64_t n,
+                            const RowsOut& out, cudaStream_t st) {
+  return count <= sm_count() ? launch_split_rows<T, NUMERIC, 1024>(rows, count, w, in, n, out, st)
+                             : launch_split_rows<T, NUMERIC, 512>(rows, count, w, in, n, out, st);
 }
 
 // All rows; the longest first, so that the short ones fill in behind them: a bin's kernel lets the
@@ -1243,7 +1382,7 @@ static int launch_bins(const WsLayout& w, const long long* counts, int64_t m, in
   bool early = false;
   if (counts[3] > 0) {
     // (a segment's part of the column and 13 bits of ordinal fit one key up to 2^24 columns)
-    rc = nbits <= 24 ? launch_split_bin<T, NUMERIC>(rows + 3 * m, counts[3], w, in, nbits, out, st)
+    rc = nbits <= 24 ? launch_split_bin<T, NUMERIC>(rows + 3 * m, counts[3], w, in, n, out, st)
                      : launch_cta_bin<T, NUMERIC, K64, 512, 16>(rows + 3 * m, counts[3], w, in, 13, out, early, st);
     if (rc != SB_OK) return rc;
     early = true;
@@ -1298,8 +1437,7 @@ static int check_spgemm(int64_t m, int64_t kb, int64_t n, const void* Apos, cons
 // Product bounds and bins of the rows.
 static int bin_rows(const WsLayout& w, int64_t m, const int32_t* Apos, const int32_t* Acrd, const int32_t* Bpos,
                     cudaStream_t st) {
-  SB_CUDA(cudaMemsetAsync(w.hdr, 0, 16 * 8, st));
-  SB_CUDA(cudaMemsetAsync(w.bin_cursor, 0, 16 * 4, st));
+  SB_CUDA(cudaMemsetAsync(w.hdr, 0, 256 + 16 * 4, st));   // header and cursors are neighbours
   const int rows = (int)std::min<int64_t>(kBinRows, std::max<int64_t>(32, ceil_div(m, 2 * sm_count() * 32) * 32));
   spgemm_bin_kernel<<<(unsigned)ceil_div(m, rows), kBinThreads, 0, st>>>((int)m, rows, Apos, Acrd, Bpos, w.upper,
                                                                          w.bin_rows, w.bin_cursor, w.row_cnt);
@@ -1465,13 +1603,14 @@ int sb_spgemm_finish(int dtype, int64_t m, int64_t nnz, const int32_t* off, cons
   if (m == 0 || nnz == 0) return SB_OK;
   SB_CHECK_ARG(off && tcrd && tval && Cpos && Ccrd && Cval, "spgemm_finish: null pointer");
   cudaStream_t st = (cudaStream_t)stream;
-  const unsigned grid = (unsigned)ceil_div(nnz, kMoveTile);
+  const int tile = (int)std::min<int64_t>(kMoveTile, std::max<int64_t>(512, ceil_div(ceil_div(nnz, 4 * sm_count()), 256) * 256));
+  const unsigned grid = (unsigned)ceil_div(nnz, tile);
   if (dtype == SB_F32 || dtype == SB_I32)
-    spgemm_move_kernel<unsigned><<<grid, 256, 0, st>>>((int)m, (int)nnz, off, Cpos, tcrd, (const unsigned*)tval, Ccrd,
+    spgemm_move_kernel<unsigned><<<grid, 256, 0, st>>>((int)m, (int)nnz, tile, off, Cpos, tcrd, (const unsigned*)tval, Ccrd,
                                                        (unsigned*)Cval);
   else
     spgemm_move_kernel<unsigned long long><<<grid, 256, 0, st>>>(
-        (int)m, (int)nnz, off, Cpos, tcrd, (const unsigned long long*)tval, Ccrd, (unsigned long long*)Cval);
+        (int)m, (int)nnz, tile, off, Cpos, tcrd, (const unsigned long long*)tval, Ccrd, (unsigned long long*)Cval);
   SB_LAUNCH_CHECK("spgemm_move_kernel");
   return SB_OK;
 }

@@ -269,19 +269,42 @@ struct ExpandSmem {
   T a[NT];
   int part[NT / 32];
 };
+// `turn(first, total, find)` is called per NT entries, with the number of the first product and of products; find(q)
+// = entry of the turn's product q.
 template <typename T, bool NUMERIC, int NT, typename F>
-__device__ __forceinline__ void expand_cta(const CsrIn& in, int ab, int ae, ExpandSmem<T, NT>& sm, int tid, F&& emit,
-                                           int part = 0, int parts = 1) {
+__device__ __forceinline__ void expand_turns(const CsrIn& in, int ab, int ae, ExpandSmem<T, NT>& sm, int tid, F&& turn) {
   const int warp = tid >> 5, lane = tid & 31;
   int first = 0;
-  for (int p0 = ab; p0 < ae; p0 += NT) {
-    const int pa = p0 + tid;
-    int bb = 0, len = 0;
+  // (groups of 512 threads and more, which rows of several NT entries come to: the row pointers of the next NT
+  // entries and the columns of the NT after those are on their way meanwhile; the others mostly take one turn)
+  constexpr bool AHEAD = NT >= 512;
+  int next_bb = 0, next_len = 0, next_j = 0;
+  T next_a = T(0);
+  auto fetch_row = [&](int pa, int j) {
+    next_bb = next_len = 0;
     if (pa < ae) {
-      const int j = __ldg(in.Acrd + pa);
-      bb = __ldg(in.Bpos + j);
-      len = __ldg(in.Bpos + j + 1) - bb;
-      if (NUMERIC) sm.a[tid] = static_cast<const T*>(in.Aval)[pa];
+      if (!AHEAD) j = __ldg(in.Acrd + pa);
+      next_bb = __ldg(in.Bpos + j);
+      next_len = __ldg(in.Bpos + j + 1) - next_bb;
+      if (NUMERIC) next_a = static_cast<const T*>(in.Aval)[pa];
+    }
+  };
+  auto fetch_column = [&](int pa) {
+    if (pa < ae) next_j = __ldg(in.Acrd + pa);
+  };
+  if constexpr (AHEAD) {
+    fetch_column(ab + tid);
+    const int j = next_j;
+    fetch_column(ab + NT + tid);
+    fetch_row(ab + tid, j);
+  }
+  for (int p0 = ab; p0 < ae; p0 += NT) {
+    if (!AHEAD) fetch_row(p0 + tid, 0);
+    const int bb = next_bb, len = next_len;
+    if (NUMERIC) sm.a[tid] = next_a;
+    if (AHEAD && p0 + NT < ae) {
+      fetch_row(p0 + NT + tid, next_j);
+      fetch_column(p0 + 2 * NT + tid);
     }
     int incl = len;
 #pragma unroll
@@ -301,17 +324,28 @@ __device__ __forceinline__ void expand_cta(const CsrIn& in, int ab, int ae, Expa
     sm.excl[tid] = excl;
     sm.off[tid] = bb - excl;
     __syncthreads();
-#pragma unroll 4
-    for (int q = part * NT + tid; q < total; q += parts * NT) {
+    turn(first, total, [&](int q) {
       int e = 0;   // largest e with excl[e] <= q
 #pragma unroll
       for (int step = NT / 2; step > 0; step >>= 1)
         if (sm.excl[e + step] <= q) e += step;
-      emit(first + q, NUMERIC ? sm.a[e] : T(0), sm.off[e] + q);
-    }
+      return e;
+    });
     first += total;
     __syncthreads();
   }
+}
+
+template <typename T, bool NUMERIC, int NT, typename F>
+__device__ __forceinline__ void expand_cta(const CsrIn& in, int ab, int ae, ExpandSmem<T, NT>& sm, int tid, F&& emit,
+                                           int part = 0, int parts = 1) {
+  expand_turns<T, NUMERIC, NT>(in, ab, ae, sm, tid, [&](int first, int total, auto&& find) {
+#pragma unroll 4
+    for (int q = part * NT + tid; q < total; q += parts * NT) {
+      const int e = find(q);
+      emit(first + q, NUMERIC ? sm.a[e] : T(0), sm.off[e] + q);
+    }
+  });
 }
 
 // All products of A row [ab, ae) to shared memory: keys[o] = column << shift | o, prods[o]; their
@@ -423,12 +457,18 @@ spgemm_cta_kernel(const int* __restrict__ rows, const int* __restrict__ upper, C
   end_after_previous();
 }
 
-// Rows of 2049 to 8192 products: a CTA each, the row's columns cut into up to 32 segments that a warp
-// sorts each.  The network over the whole row would need 64-bit keys (21 bits of column and 13 of
+// Rows of 2049 to 8192 products: a CTA each, the row's columns cut into segments of equal width that a
+// warp sorts each.  The network over the whole row would need 64-bit keys (21 bits of column and 13 of
 // ordinal on a 2 M-column matrix), 128 KB of shared memory and ten exchanges through it: 4.6 ms
-// for 10,562 rows where the segments take 1.9 ms.  Segments of more than 512 products (columns
+// for 10,562 rows where the segments take 1.0 ms.  Segments of more than 512 products (columns
 // crowded together) are sorted by the CTA in shared memory.
-constexpr int kSplitThreads = 512, kSplitCap = 8192, kSegments = 32, kSegmentSort = 512, kSplitOrd = 13;
+// Bound: the network's issue rate and the emission's chains.  16 warps and 32 segments a row, two rows per SM; where
+// there are no more rows than SMs 32 warps and 64 segments (a row of 7,700 products and 1,500 entries: 50 us, 31 so).
+// (Ranks by counting within some 4,000 buckets in place of the networks of all the CTA kernels took fewer
+// instructions in ALU and more waiting: 1.15 ms to 1.44 for the 56,789 rows of 513 to 2048 products.)
+constexpr int kSplitCap = 8192, kSegmentSort = 512, kSplitOrd = 13;
+template <int NT>
+constexpr int kSplitSegments = NT / 16;
 
 // Ascending sort of any number of keys in shared memory by NT threads: the bitonic network in the form
 // in which every comparison puts the smaller key first, so that places behind the end need no key.
@@ -451,17 +491,46 @@ __device__ __noinline__ void sort_in_smem(KEY* keys, int count, int tid) {
   __syncthreads();
 }
 
-template <typename T, bool NUMERIC>
-__global__ void __launch_bounds__(kSplitThreads, 2)
-spgemm_split_kernel(const int* __restrict__ rows, const int* __restrict__ upper, CsrIn in, int seg_shift,
+// Segment of a column: column / width (width = columns / segments, rounded up; scale = 2^32 / width, rounded up:
+// at most one too many).
+__device__ __forceinline__ int segment_of(unsigned col, int width, unsigned scale) {
+  const int seg = width > 1 ? (int)__umulhi(col, scale) : (int)col;
+  return seg - ((unsigned)seg * (unsigned)width > col);
+}
+// Exclusive sums of the segments' counts by a warp, the total behind them (known to lane 31).
+template <int SEGMENTS>
+__device__ __forceinline__ int exclusive_segments(const int* cnt, int* start, int lane) {
+  constexpr int PER = SEGMENTS / 32;
+  int c[PER], incl = 0;
+#pragma unroll
+  for (int q = 0; q < PER; q++) incl += c[q] = cnt[PER * lane + q];
+  int at = -incl;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(FULL, incl, o);
+    if (lane >= o) incl += y;
+  }
+  at += incl;
+#pragma unroll
+  for (int q = 0; q < PER; q++) {
+    start[PER * lane + q] = at;
+    at += c[q];
+  }
+  if (lane == 31) start[SEGMENTS] = incl;
+  return incl;
+}
+
+template <typename T, bool NUMERIC, int NT>
+__global__ void __launch_bounds__(NT, 1024 / NT)
+spgemm_split_kernel(const int* __restrict__ rows, const int* __restrict__ upper, CsrIn in, int width, unsigned scale,
                     RowsOut out) {
-  constexpr int NT = kSplitThreads, NW = NT / 32, R = kSplitCap / NT;
+  constexpr int NW = NT / 32, R = kSplitCap / NT, kSegments = kSplitSegments<NT>;
   typedef unsigned KEY;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Slot* prods = reinterpret_cast<Slot*>(smem_raw);
   KEY* keys = reinterpret_cast<KEY*>(smem_raw + (NUMERIC ? sizeof(Slot) * kSplitCap : 0));
   __shared__ ExpandSmem<T, NT> s_expand;
-  __shared__ int s_cnt[kSegments], s_start[kSegments + 1], s_u[kSegments];
+  __shared__ int s_cnt[kSegments + 1], s_start[kSegments + 1], s_u[kSegments];
   const int i = __ldg(rows + blockIdx.x), tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int count = __ldg(upper + i), ab = __ldg(in.Apos + i), ae = __ldg(in.Apos + i + 1);
   const long long base = NUMERIC ? __ldg(out.off + i) : 0;
@@ -470,35 +539,23 @@ spgemm_split_kernel(const int* __restrict__ rows, const int* __restrict__ upper,
   expand_row<T, NUMERIC, KEY, NT, true>(in, ab, ae, 0, keys, prods, tid, &s_expand);
   // columns to their segments (in any order: the sort brings it), the ordinal below the column
   KEY c[R];
-  int rank[R];
+  int place[R];                // segment << 16 | place in it
 #pragma unroll
   for (int q = 0; q < R; q++) {
     const int x = tid + q * NT;
     if (x < count) {
-      c[q] = keys[x];
-      rank[q] = atomicAdd(&s_cnt[c[q] >> seg_shift], 1);
+      const int seg = segment_of(keys[x], width, scale);
+      c[q] = keys[x] - (unsigned)(seg * width);
+      place[q] = seg << 16 | atomicAdd(&s_cnt[seg], 1);
     }
   }
   __syncthreads();
-  if (warp == 0) {
-    const int v = s_cnt[lane];
-    int incl = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(FULL, incl, o);
-      if (lane >= o) incl += y;
-    }
-    s_start[lane + 1] = incl;
-    if (lane == 0) s_start[0] = 0;
-  }
+  if (warp == 0) exclusive_segments<kSegments>(s_cnt, s_start, lane);
   __syncthreads();
 #pragma unroll
   for (int q = 0; q < R; q++) {
     const int x = tid + q * NT;
-    if (x < count) {
-      const int seg = c[q] >> seg_shift;
-      keys[s_start[seg] + rank[q]] = ((c[q] & (((KEY)1 << seg_shift) - 1)) << kSplitOrd) | (KEY)x;
-    }
+    if (x < count) keys[s_start[place[q] >> 16] + (place[q] & 0xffff)] = c[q] << kSplitOrd | (KEY)x;
   }
   __syncthreads();
   for (int seg = 0; seg < kSegments; seg++) {
@@ -510,23 +567,25 @@ spgemm_split_kernel(const int* __restrict__ rows, const int* __restrict__ upper,
     if (n <= kSegmentSort) {
       if (n > 256) sort_keys<KEY, 16, 32>(keys + b, n, lane);
       else if (n > 128) sort_keys<KEY, 8, 32>(keys + b, n, lane);
-      else if (n > 1) sort_keys<KEY, 4, 32>(keys + b, n, lane);
+      else if (n > 64) sort_keys<KEY, 4, 32>(keys + b, n, lane);
+      else if (n > 32) sort_keys<KEY, 2, 32>(keys + b, n, lane);
+      else if (n > 1) sort_keys<KEY, 1, 32>(keys + b, n, lane);
     }
     const int u = count_runs<KEY>(keys + b, 0, n, kSplitOrd, lane);
     if (lane == 0) s_u[seg] = u;
   }
   __syncthreads();
-  if (out.row_cnt && warp == 0) {
-    const int u = __reduce_add_sync(FULL, s_u[lane]);
-    if (lane == 0) out.row_cnt[i] = u;
+  if (warp == 0) {
+    const int u = exclusive_segments<kSegments>(s_u, s_cnt, lane);
+    if (out.row_cnt && lane == 31) out.row_cnt[i] = u;
   }
   if (NUMERIC) {
+    __syncthreads();
     T* val = static_cast<T*>(out.val);
     for (int seg = warp; seg < kSegments; seg += NW) {
       const int b = s_start[seg], n = s_start[seg + 1] - b;
-      const int before = __reduce_add_sync(FULL, lane < seg ? s_u[lane] : 0);
       const KEY* k = keys + b;
-      write_runs<KEY>(k, 0, n, n, kSplitOrd, lane, seg << seg_shift, base + before,
+      write_runs<KEY>(k, 0, n, n, kSplitOrd, lane, seg * width, base + s_cnt[seg],
                       [&](long long o, int col, int x, int last) {
         out.crd[o] = col;
         RunSum<T> s;
