@@ -460,6 +460,9 @@ def _spmm_typed(pos, crd, val, B, n):
 # Rows from which the tensor-core transform is the faster one (9,220 x 256 x 64: 17.5 us against cuBLAS's
 # 12.5; 40,000 x 100 x 128: 25.9 against 35.9): two 128-row tiles per SM keep its pipeline full.
 DENSE_MATMUL_MIN_ROWS = 32768
+# ... or, from 4096 rows (32 tiles) on, multiplications, where its rate counts for more than what a launch of it takes (30,000 x 100 x 128:
+# 22.1 us, cuBLAS 26.9; 12,000 x 256 x 256: 27.6, 40.2; but 20,000 x 100 x 128: 22.3, 20.7; 20,000 x 256 x 64: 25.0, 22.7).
+DENSE_MATMUL_MIN_WORK = 350_000_000
 # Width up to which its result is as close to float64 as a chain of fp32 FMAs (2.3e-7 against 2.9e-7 at 256):
 # its error grows with the number of truncating additions, faster than the FMA chain's.
 DENSE_MATMUL_MAX_K = 256
@@ -468,7 +471,9 @@ DENSE_MATMUL_MAX_K = 256
 def dense_matmul(X: torch.Tensor, W: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """X @ W in fp32 for a tall X: on the tensor cores in fp32 accuracy (``sb_dense_matmul_f32``) where
     the operands have the layout it takes, else ``torch.matmul``."""
-    if (X.dim() != 2 or W.dim() != 2 or X.shape[0] < DENSE_MATMUL_MIN_ROWS or X.dtype != torch.float32
+    if (X.dim() != 2 or W.dim() != 2
+            or (X.shape[0] < DENSE_MATMUL_MIN_ROWS
+                and (X.shape[0] < 4096 or X.numel() * W.shape[1] < DENSE_MATMUL_MIN_WORK)) or X.dtype != torch.float32
             or W.dtype != torch.float32 or not X.is_cuda or W.device != X.device or X.shape[1] != W.shape[0]
             or not X.is_contiguous() or not W.is_contiguous() or not 0 < X.shape[1] <= DENSE_MATMUL_MAX_K or X.shape[1] % 4
             or W.shape[1] == 0 or W.shape[1] % 8 or X.data_ptr() % 16
@@ -488,7 +493,10 @@ def dense_matmul(X: torch.Tensor, W: torch.Tensor, out: Optional[torch.Tensor] =
 
 
 SPLIT_PANEL = 64                  # operand columns multiplied at a time (256 bytes of each operand row)
-SPLIT_CHUNK_BYTES = 96e6          # operand bytes of one chunk and panel: they stay in the 126 MB L2
+# Operand bytes of one chunk and panel.  They stay in the 126 MB L2, better the fewer they are, but every chunk reads and
+# writes the result once more (700,000 rows: two chunks of 90 MB 6.89 ms, three of 60 MB 6.42; 1.4 M: four of 90 MB
+# 17.4 ms, five of 72 MB 17.1; 2 M: five of 102 MB 26.5 ms, six of 85 MB 26.1, seven of 73 MB 26.7; 1 M: three of 85 MB 7.8).
+SPLIT_CHUNK_BYTES = 86e6
 SPLIT_MIN_ENTRIES = 6             # mean entries per row and chunk
 
 
