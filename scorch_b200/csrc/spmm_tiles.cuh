@@ -361,36 +361,84 @@ spmm_tile_kernel(SpmmArgs<T> a, TileArgs<T> t) {
   }
 }
 
-// Rows without entries (zeros, or act(bias)), and rows of several units: their unit sums in order.
-// A warp looks at 32 rows and takes those that need something, a lane per column.
-template <typename T>
+// Rows without entries (zeros, or act(bias)), and rows of several units: their unit sums, every eighth one added in
+// order, then these eight sums.  A warp looks at 32 rows and takes those that need something, a lane per column.
+// SHARED: rows of more than eight units are taken by the CTA, a warp per eighth: by one warp the rows of 90,000
+// entries of a power-law matrix kept the product waiting (150,000 rows, 128 columns: 186 us, 172 so).  Products of
+// fewer than kSharedSums entries have few units and go without the barriers (layer of 2,500 rows: 8.2 us with, 7.9).
+constexpr int kWarpUnits = 8;
+static_assert(kWarpUnits == kTileWarps, "a warp per part");
+constexpr int64_t kSharedSums = 1 << 17;
+template <typename T, bool SHARED>
 __global__ void __launch_bounds__(kTileThreadsMm)
 spmm_tile_rows_kernel(SpmmArgs<T> a, TileArgs<T> t) {
-  const int lane = threadIdx.x & 31;
+  __shared__ int s_rows[SHARED ? kTileThreadsMm : 1], s_n;
+  __shared__ T s_part[SHARED ? kTileWarps : 1][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // (what follows waits for this kernel's end)
-  const long long r0 = ((long long)blockIdx.x * kTileWarps + (threadIdx.x >> 5)) * 32;
+  const long long r0 = ((long long)blockIdx.x * kTileWarps + warp) * 32;
   int b = 0, len = 1;
   if (r0 + lane < a.m) {
     b = __ldg(a.pos + r0 + lane);
     len = __ldg(a.pos + r0 + lane + 1) - b;
   }
   // (an empty row of an accumulating product without bias or ReLU stays what it is)
-  const bool keep_empty = a.accumulate && !a.bias && !a.relu;
-  unsigned todo = __ballot_sync(FULL, (len == 0 && !keep_empty) || len > kUnit);
+  const bool keep_empty = a.accumulate && !a.bias && !a.relu, by_cta = SHARED && len > kWarpUnits * kUnit;
+  unsigned todo = __ballot_sync(FULL, (len == 0 && !keep_empty) || (len > kUnit && !by_cta));
+  bool some = false;
+  if constexpr (SHARED) {
+    if (threadIdx.x == 0) s_n = 0;
+    some = __syncthreads_or(by_cta);
+  }
+  if (by_cta) s_rows[atomicAdd(&s_n, 1)] = (int)(r0 + lane);
   asm volatile("griddepcontrol.wait;" ::: "memory");   // the tile kernel's results
+  auto unit_sum = [&](int rb, int u, int col) { return (u ? t.rest : t.first)[((long long)(rb / kUnit) + u) * a.k + col]; };
+  auto store = [&](T* c, int col, T s) {
+    Pack<T, 1> x;
+    x.v[0] = s + (a.accumulate ? *c : T(0));
+    st_stream<T, 1>(c, epilogue<T, 1>(x, a.bias, col, a.relu));
+  };
   while (todo) {
     const int i = __ffs(todo) - 1;
     todo &= todo - 1;
     const int rb = __shfl_sync(FULL, b, i), units = (__shfl_sync(FULL, len, i) + kUnit - 1) / kUnit;
     T* crow = a.C + (r0 + i) * a.ldc;
     for (int col = blockIdx.y * 32 + lane; col < a.k; col += gridDim.y * 32) {
-      T s = T(0);
-      if (units > 0) s = t.first[(long long)(rb / kUnit) * a.k + col];
+      T s[kWarpUnits];
+#pragma unroll
+      for (int w = 0; w < kWarpUnits; w++) s[w] = w < units ? unit_sum(rb, w, col) : T(0);
+      for (int u = kWarpUnits; u < units; u += kWarpUnits) {
+#pragma unroll
+        for (int w = 0; w < kWarpUnits; w++)
+          if (u + w < units) s[w] += unit_sum(rb, u + w, col);
+      }
+      T sum = s[0];
+#pragma unroll
+      for (int w = 1; w < kWarpUnits; w++)
+        if (w < units) sum += s[w];
+      store(crow + col, col, sum);
+    }
+  }
+  if (!SHARED || !some) return;
+  __syncthreads();
+  for (int i = 0; i < s_n; i++) {
+    const int r = s_rows[i], rb = __ldg(a.pos + r), units = (__ldg(a.pos + r + 1) - rb + kUnit - 1) / kUnit;
+    for (int col0 = blockIdx.y * 32; col0 < a.k; col0 += gridDim.y * 32) {
+      const int col = col0 + lane;
+      if (col < a.k) {
+        T s = unit_sum(rb, warp, col);
 #pragma unroll 8
-      for (int u = 1; u < units; u++) s += t.rest[((long long)(rb / kUnit) + u) * a.k + col];
-      Pack<T, 1> x;
-      x.v[0] = s + (a.accumulate ? crow[col] : T(0));
-      st_stream<T, 1>(crow + col, epilogue<T, 1>(x, a.bias, col, a.relu));
+        for (int u = warp + kWarpUnits; u < units; u += kWarpUnits) s += unit_sum(rb, u, col);
+        s_part[SHARED ? warp : 0][lane] = s;
+      }
+      __syncthreads();
+      if (warp == 0 && col < a.k) {
+        T s = s_part[0][lane];
+#pragma unroll
+        for (int w = 1; w < (SHARED ? kTileWarps : 1); w++) s += s_part[w][lane];
+        store(a.C + (long long)r * a.ldc + col, col, s);
+      }
+      __syncthreads();
     }
   }
 }
@@ -436,9 +484,9 @@ static int launch_tiles(const SpmmArgs<T>& a, int64_t nnz, void* ws, cudaStream_
   // (may be set up while the tiles still run: it waits for them itself.  It reads the row pointers before
   // that, which is sound behind the tile kernel, whose CTAs have waited for whatever made them; a
   // matrix without entries has no tile kernel, and an ordinary launch)
-  SB_CUDA(launch_kernel(t.tiles > 0, spmm_tile_rows_kernel<T>,
-                        dim3((unsigned)ceil_div(a.m, kTileThreadsMm), (unsigned)std::min<int64_t>(ceil_div(a.k, 32), 64)),
-                        kTileThreadsMm, 0, st, a, t));
+  const dim3 grid((unsigned)ceil_div(a.m, kTileThreadsMm), (unsigned)std::min<int64_t>(ceil_div(a.k, 32), 64));
+  SB_CUDA(launch_kernel(t.tiles > 0, nnz >= kSharedSums ? spmm_tile_rows_kernel<T, true> : spmm_tile_rows_kernel<T, false>,
+                        grid, kTileThreadsMm, 0, st, a, t));
   return SB_OK;
 }
 

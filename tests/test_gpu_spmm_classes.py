@@ -37,3 +37,36 @@ def test_rows_by_length(lens, dtype, k):
     r0, r1 = len(lens) // 3, len(lens) - 5
     part = K.spmm_csr(d(pos[r0:r1 + 1] - pos[r0]), dcrd[pos[r0]:pos[r1]].clone(), dval[pos[r0]:pos[r1]].clone(), dB)
     assert torch.equal(part, got[r0:r1])
+
+
+@pytest.mark.parametrize("units", [1, 2, 7, 8, 9, 16, 17, 200])
+@pytest.mark.parametrize("dtype,k", [("f32", 8), ("f32", 77), ("f64", 40)])
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_rows_of_several_units(units, dtype, k, accumulate):
+    # alone (few entries) and among more than 2^17 entries, where the CTA adds the unit sums: the same bits
+    from scorch_b200 import kernels as K
+    t = np.float32 if dtype == "f32" else np.float64
+    if accumulate and dtype == "f64":
+        pytest.skip("accumulation is float32")
+    n, rng = 3000, np.random.default_rng(units)
+    lens = [3, 512 * units - 511, 0, 512 * units] + [40] * 3300
+    pos = np.zeros(len(lens) + 1, np.int32)
+    np.cumsum(lens, out=pos[1:])
+    assert pos[-1] > 1 << 17
+    crd = rng.integers(0, n, pos[-1]).astype(np.int32)
+    val, B = rng.standard_normal(pos[-1]).astype(t), rng.standard_normal((n, k)).astype(t)
+    d = lambda a: torch.from_numpy(a).cuda()
+    dB, base = d(B), torch.full((len(lens), k), 2.0, device="cuda")
+    run = (lambda p, c, v, out: K.spmm_csr(p, c, v, dB, accumulate=True, out=out)) if accumulate else (
+        lambda p, c, v, out: K.spmm_csr(p, c, v, dB))
+    got = run(d(pos), d(crd), d(val), base.clone())
+    e = pos[4]
+    part = run(d(pos[:5]), d(crd[:e]), d(val[:e]), base[:4].clone())
+    assert torch.equal(part, got[:4])
+    rows = np.repeat(np.arange(4), lens[:4])
+    term = val[:e, None].astype(np.float64) * B[crd[:e]]
+    want, size = np.full((4, k), 2.0 * accumulate), np.full((4, k), 2.0 * accumulate)
+    np.add.at(want, rows, term)
+    np.add.at(size, rows, np.abs(term))
+    eps = 2.0 ** -24 if dtype == "f32" else 2.0 ** -53
+    assert np.all(np.abs(part.cpu().numpy() - want) <= 128 * eps * size)     # (at most some 100 additions one after another)
