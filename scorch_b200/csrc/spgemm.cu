@@ -1068,7 +1068,8 @@ spgemm_smem_kernel(const int* __restrict__ rows, CsrIn in, int n, const unsigned
 // left the hub rows to a warp each: 4.7 ms for 272 M entries); a thread finds the row of its entry
 // among the tile's row pointers in shared memory.  Tiles of kMoveTile entries, smaller where that leaves SMs idle
 // (1.1 M entries: 15.3 us in 136 tiles of 8192, 9.4 in 542 of 2048).
-constexpr int kMoveTile = 8192, kMoveRows = 1024;
+// The places of kMoveAhead entries are found before the first is loaded: 284 M entries 1.06 ms one by one, 0.76 so = 6.0 TB/s.
+constexpr int kMoveTile = 8192, kMoveRows = 1024, kMoveAhead = 4;
 template <typename T>
 __global__ void __launch_bounds__(256)
 spgemm_move_kernel(int m, int nnz, int tile, const int* __restrict__ off, const int* __restrict__ Cpos,
@@ -1088,25 +1089,40 @@ spgemm_move_kernel(int m, int nnz, int tile, const int* __restrict__ off, const 
     }
     __syncthreads();
     const int stop = min(e1, s_pos[kMoveRows]);
-#pragma unroll 4
-    for (int o0 = e + (tid & ~31); o0 < stop; o0 += 256) {
-      // the row of the warp's first entry by two rounds of 32 looks, this lane's a few rows behind it
-      const int c = __popc(__ballot_sync(FULL, s_first[lane] <= o0)) - 1;
-      int r = 32 * c + __popc(__ballot_sync(FULL, s_pos[32 * c + lane] <= o0)) - 1;
-      const int o = o0 + lane;
-      if (o >= stop) continue;
+    for (int o0 = e + (tid & ~31); o0 < stop; o0 += 256 * kMoveAhead) {
+      int src[kMoveAhead];
+#pragma unroll
+      for (int q = 0; q < kMoveAhead; q++) {
+        // the row of the warp's first entry by two rounds of 32 looks, this lane's a few rows behind it
+        const int first = min(o0 + q * 256, stop - 1), o = min(first + lane, stop - 1);
+        const int c = __popc(__ballot_sync(FULL, s_first[lane] <= first)) - 1;
+        int r = 32 * c + __popc(__ballot_sync(FULL, s_pos[32 * c + lane] <= first)) - 1;
 #pragma unroll 1
-      for (int step = 0; step < 6 && s_pos[r + 1] <= o; step++) r++;
-      if (s_pos[r + 1] <= o) {           // many short or empty rows
-        int hi = kMoveRows;
-        while (hi - r > 1) {
-          const int mid = (r + hi) >> 1;
-          if (s_pos[mid] <= o) r = mid; else hi = mid;
+        for (int step = 0; step < 6 && s_pos[r + 1] <= o; step++) r++;
+        if (s_pos[r + 1] <= o) {           // many short or empty rows
+          int hi = kMoveRows;
+          while (hi - r > 1) {
+            const int mid = (r + hi) >> 1;
+            if (s_pos[mid] <= o) r = mid; else hi = mid;
+          }
         }
+        src[q] = o + s_shift[r];
       }
-      const int src = o + s_shift[r];
-      Ccrd[o] = __ldg(tcrd + src);
-      Cval[o] = __ldg(tval + src);
+      int crd[kMoveAhead];
+      T val[kMoveAhead];
+#pragma unroll
+      for (int q = 0; q < kMoveAhead; q++) {
+        if (o0 + q * 256 + lane >= stop) continue;
+        crd[q] = __ldg(tcrd + src[q]);
+        val[q] = __ldg(tval + src[q]);
+      }
+#pragma unroll
+      for (int q = 0; q < kMoveAhead; q++) {
+        const int o = o0 + q * 256 + lane;
+        if (o >= stop) continue;
+        Ccrd[o] = crd[q];
+        Cval[o] = val[q];
+      }
     }
     e = stop;
     __syncthreads();
@@ -1258,10 +1274,10 @@ static int launch_smem_bin(const int* rows, int64_t count, const WsLayout& w, in
   return SB_OK;
 }
 
-template <typename T, bool NUMERIC>
-static int big_rows(const WsLayout& w, int64_t count, int64_t m, int64_t n, const CsrIn& in,
-                    const RowsOut& out, cudaStream_t st) {
-  std::vector<int4> info((size_t)count);
+// The long rows' numbers, products and entries, to the host.
+static int big_list(const WsLayout& w, int64_t count, int64_t m, const CsrIn& in, std::vector<int4>& info,
+                    cudaStream_t st) {
+  info.resize((size_t)count);
   const int64_t room = (int64_t)(w.area_bytes / sizeof(int4));
   for (int64_t x0 = 0; x0 < count; x0 += room) {
     const int part = (int)std::min<int64_t>(room, count - x0);
@@ -1271,6 +1287,12 @@ static int big_rows(const WsLayout& w, int64_t count, int64_t m, int64_t n, cons
     SB_CUDA(cudaMemcpyAsync(info.data() + x0, w.area, (size_t)part * sizeof(int4), cudaMemcpyDeviceToHost, st));
     SB_CUDA(cudaStreamSynchronize(st));
   }
+  return SB_OK;
+}
+
+template <typename T, bool NUMERIC>
+static int big_rows(const WsLayout& w, const std::vector<int4>& info, int64_t n, const CsrIn& in, const RowsOut& out,
+                    cudaStream_t st) {
   const int nbits = ceil_log2(std::max<int64_t>(n, 1));
   std::vector<int> row, p0{0}, shift;
   std::vector<int4> tasks;
@@ -1374,7 +1396,9 @@ static int launch_bins(const WsLayout& w, const long long* counts, int64_t m, in
     if (counts[4] > 0) rc = max_abs<T>(w, in, kb, st);
     if (rc != SB_OK) return rc;
   }
-  if (counts[4] > 0 && !in_smem) rc = big_rows<T, NUMERIC>(w, counts[4], m, n, in, out, st);
+  // (the long rows' list is read back ahead of the other bins, which run while the host plans the long rows' tasks)
+  std::vector<int4> info;
+  if (counts[4] > 0 && !in_smem) rc = big_list(w, counts[4], m, in, info, st);
   if (rc != SB_OK) return rc;
   typedef unsigned K32;
   typedef unsigned long long K64;
@@ -1405,8 +1429,9 @@ static int launch_bins(const WsLayout& w, const long long* counts, int64_t m, in
     if (rc != SB_OK) return rc;
     early = true;
   }
-  if (counts[4] > 0 && in_smem)
-    rc = launch_smem_bin<T, NUMERIC>(rows + 4 * m, counts[4], w, n, in, out, early, st);
+  if (counts[4] > 0)
+    rc = in_smem ? launch_smem_bin<T, NUMERIC>(rows + 4 * m, counts[4], w, n, in, out, early, st)
+                 : big_rows<T, NUMERIC>(w, info, n, in, out, st);
   return rc;
 }
 
@@ -1603,7 +1628,7 @@ int sb_spgemm_finish(int dtype, int64_t m, int64_t nnz, const int32_t* off, cons
   if (m == 0 || nnz == 0) return SB_OK;
   SB_CHECK_ARG(off && tcrd && tval && Cpos && Ccrd && Cval, "spgemm_finish: null pointer");
   cudaStream_t st = (cudaStream_t)stream;
-  const int tile = (int)std::min<int64_t>(kMoveTile, std::max<int64_t>(512, ceil_div(ceil_div(nnz, 4 * sm_count()), 256) * 256));
+  const int tile = (int)std::min<int64_t>(kMoveTile, std::max<int64_t>(256 * kMoveAhead, ceil_div(ceil_div(nnz, 4 * sm_count()), 256) * 256));
   const unsigned grid = (unsigned)ceil_div(nnz, tile);
   if (dtype == SB_F32 || dtype == SB_I32)
     spgemm_move_kernel<unsigned><<<grid, 256, 0, st>>>((int)m, (int)nnz, tile, off, Cpos, tcrd, (const unsigned*)tval, Ccrd,

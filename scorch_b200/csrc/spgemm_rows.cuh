@@ -164,23 +164,27 @@ __device__ __forceinline__ int count_runs(const KEY* keys, int b, int e, int shi
   return heads;
 }
 // ... and for each one write(o, column, first, last): o = at, at + 1, ..., [first, last) its run of
-// sorted keys (which may end behind e, at most at `count`).
+// sorted keys (which may end behind e, at most at `count`).  Returns their number.
 template <typename KEY, typename F>
-__device__ __forceinline__ void write_runs(const KEY* keys, int b, int e, int count, int shift, int lane, int col0,
-                                           long long at, F&& write) {
+__device__ __forceinline__ int write_runs(const KEY* keys, int b, int e, int count, int shift, int lane, int col0,
+                                          long long at, F&& write) {
+  int n = 0;
   for (int x0 = b; x0 < e; x0 += 32) {
     const int x = x0 + lane;
     const KEY col = x < e ? keys[x] >> shift : KEY(0);
     const bool head = x < e && (x == 0 || col != (keys[x - 1] >> shift));
     const unsigned heads = __ballot_sync(FULL, head);
     if (head) {
-      int last = x + 1;
-      while (last < count && (keys[last] >> shift) == col) last++;
-      const long long o = at + __popc(heads & ((1u << lane) - 1u));
-      write(o, col0 + (int)col, x, last);
+      // up to the next head, or, from the last one of the 32, as far as the column goes
+      const unsigned next = heads >> lane >> 1;
+      int last = next ? x + __ffs(next) : min(e, x0 + 32);
+      if (!next)
+        while (last < count && (keys[last] >> shift) == col) last++;
+      write(at + n + __popc(heads & ((1u << lane) - 1u)), col0 + (int)col, x, last);
     }
-    at += __popc(heads);
+    n += __popc(heads);
   }
+  return n;
 }
 // Both for a group of NT threads, every warp a contiguous part (s_part: one int per warp); returns
 // the number of distinct columns.
@@ -207,8 +211,8 @@ __device__ __forceinline__ int emit_runs(const KEY* keys, int count, int shift, 
     }
   }
   if (EMIT) {
-    if (NW == 1) total = count_runs<KEY>(keys, b, e, shift, lane);
-    write_runs<KEY>(keys, b, e, count, shift, lane, col0, base + before, write);
+    const int n = write_runs<KEY>(keys, b, e, count, shift, lane, col0, base + before, write);
+    if (NW == 1) total = n;
   }
   return total;
 }
