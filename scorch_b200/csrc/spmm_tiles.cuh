@@ -41,17 +41,17 @@ template <int L>
 constexpr int kGroupRow = L == 4 ? 40 : 32;
 constexpr int kWarpRow = 192;
 constexpr int kTileRowCap = 1024;      // row pointers kept in shared memory at a time
-constexpr int kTileLists = 96;         // rows of the window that a warp / the CTA takes
+// Rows of a window that a warp takes, and units that the CTA takes, at most.
+template <int L, int SIZE>
+constexpr int kWarpList = tile_window(L, SIZE) / (kGroupRow<L> + 1) + 2;
+template <int L, int SIZE>
+constexpr int kUnitList = tile_window(L, SIZE) / kWarpRow + tile_window(L, SIZE) / kUnit + 4;
 // Classes of similar length among the rows that a lane group takes.  A warp's groups take rows of one class,
 // the longest first: in the order of the matrix they waited for the longest of their 2 to 8 rows.  (GCN
 // layer of 2 M rows, 202 M entries, 64-column panels: 20.4 ms in the matrix's order, 19.1 by class; power law
-// of mean 12, 32 columns: 46.8 us, 39.8.  Taken as one stream of entries per group across the rows' ends,
-// without a wait at any of them, the same rows were slower by 2: 505 us in place of 250 with 256 columns.)
+// of mean 12, 32 columns: 46.8 us, 39.8; 60,000 rows of 16, 7 columns: 15.0, 13.1.  Taken as one stream of entries per group across the rows' ends,
+// an operand row fetched for every one added, the same rows took 1.7 to 2 times as long.)
 constexpr int kShortClasses = 4;
-static_assert(tile_window(8) / (kGroupRow<8> + 1) + 2 <= kTileLists &&
-              tile_window(4) / (kGroupRow<4> + 1) + 2 <= kTileLists &&
-              tile_window(32) / (kGroupRow<32> + 1) + 2 <= kTileLists, "rows longer than kGroupRow of a window");
-static_assert(tile_window(8) / kWarpRow + tile_window(8) / kUnit + 4 <= kTileLists, "units of a window");
 
 // Resident CTAs per SM the kernels are compiled for (64 / 80 registers; measured per lane count).
 constexpr int tile_ctas(int L) { return L == 32 ? 4 : 3; }
@@ -88,10 +88,10 @@ struct TileSmem {
   Pack<T, W> part[kTileWarps][VEC][L];
   Entry<T> entry[tile_window(L, sizeof(T)) + kUnit];
   int pos[kTileRowCap + 2];
-  TileUnit by_warp[kTileLists], by_cta[kTileLists];
+  TileUnit by_warp[kWarpList<L, sizeof(T)>], by_cta[kUnitList<L, sizeof(T)>];
   // rows of a turn that a lane group takes, by length (where a warp has several groups)
   // (two classes share an array, one from each end)
-  unsigned short short_row[L == 32 ? 1 : kShortClasses / 2][kTileRowCap];
+  unsigned short short_row[kShortClasses / 2][L == 32 ? 1 : kTileRowCap];
   int n_short[kShortClasses];
   int n_warp, n_cta, next_warp, next_row;
   int count[kTileWarps];
