@@ -27,8 +27,10 @@ constexpr int kTileThreadsMm = 256;
 constexpr int kTileWarps = kTileThreadsMm / 32;
 constexpr int kUnit = 512;             // a window's last row or unit reaches up to this far behind it
 // Largest window.  Wide rows (L = 32) have work enough in 1536 entries and lose residency to more
-// (6 M entries, 256 columns: 371 us, 415 with 3072); narrow ones gain by having their start-up
-// spread over twice as many (0.8 M entries in rows of 8, 64 columns: 27.0 us, 22.9 with 3072).
+// (6 M entries, 256 columns: 371 us, 415 with 3072; 2048 saves uniform matrices of 0.9 to 1.2 M entries a second
+// wave, 64.4 us to 60.7 with 256 columns, but leaves a power law's windows uneven, 64.8 to 67.5 with 77); narrow
+// ones gain by having their start-up spread over twice as many (0.8 M entries in rows of 8, 64 columns: 27.0 us, 22.9
+// with 3072).
 // 8-byte types, whose entries take 16 bytes: as much as lets three CTAs stay within 196 KB of shared memory.
 // Beyond that 23 KB are left to L1 in place of 55 and the gathers wait for it (120,000 rows of 27 entries, 16
 // float64 columns: 47.9 us with 3072, 43.2 with this).
