@@ -1088,13 +1088,14 @@ spgemm_move_kernel(int m, int nnz, int tile, const int* __restrict__ off, const 
       if (x < kMoveRows && r < m) s_shift[x] = __ldg(off + r) - p;
     }
     __syncthreads();
-    const int stop = min(e1, s_pos[kMoveRows]);
-    for (int o0 = e + (tid & ~31); o0 < stop; o0 += 256 * kMoveAhead) {
+    const int stop = min(e1, s_pos[kMoveRows]), count = stop - e;
+    // (counted from the first entry: entry numbers themselves may end at 2^31 - 1, a step beyond it wraps)
+    for (int t0 = tid & ~31; t0 < count; t0 += 256 * kMoveAhead) {
       int src[kMoveAhead];
 #pragma unroll
       for (int q = 0; q < kMoveAhead; q++) {
         // the row of the warp's first entry by two rounds of 32 looks, this lane's a few rows behind it
-        const int first = min(o0 + q * 256, stop - 1), o = min(first + lane, stop - 1);
+        const int t = t0 + q * 256, first = e + min(t, count - 1), o = e + min(t + lane, count - 1);
         const int c = __popc(__ballot_sync(FULL, s_first[lane] <= first)) - 1;
         int r = 32 * c + __popc(__ballot_sync(FULL, s_pos[32 * c + lane] <= first)) - 1;
 #pragma unroll 1
@@ -1112,16 +1113,16 @@ spgemm_move_kernel(int m, int nnz, int tile, const int* __restrict__ off, const 
       T val[kMoveAhead];
 #pragma unroll
       for (int q = 0; q < kMoveAhead; q++) {
-        if (o0 + q * 256 + lane >= stop) continue;
+        if (t0 + q * 256 + lane >= count) continue;
         crd[q] = __ldg(tcrd + src[q]);
         val[q] = __ldg(tval + src[q]);
       }
 #pragma unroll
       for (int q = 0; q < kMoveAhead; q++) {
-        const int o = o0 + q * 256 + lane;
-        if (o >= stop) continue;
-        Ccrd[o] = crd[q];
-        Cval[o] = val[q];
+        const int t = t0 + q * 256 + lane;
+        if (t >= count) continue;
+        Ccrd[e + t] = crd[q];
+        Cval[e + t] = val[q];
       }
     }
     e = stop;
