@@ -143,12 +143,13 @@ static WsLayout ws_layout(void* base, int64_t m, int64_t n) {
 // bin is 0.4 ms there: five addresses for everybody).  Rows with U = 0 get row_cnt = 0 and join no bin.
 constexpr int kBinThreads = 1024, kBinRows = 1024, kBinLaneRow = 64, kBinWarpRow = 2048;
 
+// (Numbers of entries of A are stepped through unsigned: they may end at 2^31 - 1, and the step behind wraps an int.)
 // Products of the entries b + x, b + x + step, ... before e.
 __device__ __forceinline__ long long count_products(const int* __restrict__ Acrd, const int* __restrict__ Bpos,
                                                     int b, int e, int x, int step) {
   long long u = 0;
 #pragma unroll 4
-  for (int p = b + x; p < e; p += step) {
+  for (unsigned p = (unsigned)b + x; p < (unsigned)e; p += step) {
     const int j = ld_stream(Acrd + p);
     u += __ldg(Bpos + j + 1) - __ldg(Bpos + j);
   }
@@ -325,9 +326,10 @@ __global__ void __launch_bounds__(256)
 big_scale_kernel(BigArea b, const int* __restrict__ Apos, const T* __restrict__ Aval,
                  const unsigned long long* __restrict__ max_b) {
   __shared__ double s_part[8];
-  const int row = b.row[blockIdx.x], e = __ldg(Apos + row + 1);
+  const int row = b.row[blockIdx.x];
+  const unsigned e = __ldg(Apos + row + 1);
   double s = 0.0;
-  for (int p = __ldg(Apos + row) + threadIdx.x; p < e; p += 256) s += fabs((double)Aval[p]);
+  for (unsigned p = __ldg(Apos + row) + threadIdx.x; p < e; p += 256) s += fabs((double)Aval[p]);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(FULL, s, o);
   if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = s;
@@ -370,7 +372,7 @@ __device__ __forceinline__ void big_expand(const BigArea& b, const CsrIn& in, Bi
     if (NUMERIC) b.rec[slot] = BigRecord{c, 0u, v};
     else b.key[slot] = c;
   };
-  int turn0 = ab;
+  unsigned turn0 = ab;
   expand_turns<T, NUMERIC, 256>(in, ab, ae, sm.expand, tid, [&](int, int total, auto&& find) {
     if (!REST && !SCATTER && total > end) {
       __shared__ int s_rest;
@@ -378,7 +380,7 @@ __device__ __forceinline__ void big_expand(const BigArea& b, const CsrIn& in, Bi
       if (tid == 0) s_rest = atomicAdd(b.nrest, n);
       __syncthreads();
       for (int x = tid; x < n; x += 256)
-        b.rest[s_rest + x] = make_int4(r, turn0, min(turn0 + 256, ae), (x + 1) * kTurnProducts);
+        b.rest[s_rest + x] = make_int4(r, (int)turn0, (int)min(turn0 + 256, (unsigned)ae), (x + 1) * kTurnProducts);
       __syncthreads();
     }
     turn0 += 256;
@@ -657,7 +659,7 @@ __global__ void dense_batch_setup_kernel(const int* __restrict__ rows, int r0, i
       ctl.task_pref[k] = run;
       const int i = rows[r0 + k];
       const int len = Apos[i + 1] - Apos[i];
-      run += max(1, (len + kDenseChunk - 1) / kDenseChunk);
+      run += len > 0 ? (len - 1) / kDenseChunk + 1 : 1;
       ctl.done[k] = 0;
     }
     ctl.task_pref[nb] = run;
@@ -700,7 +702,7 @@ spgemm_dense_kernel(const int* __restrict__ rows, int r0, int nb, CsrIn in, long
     if (NUMERIC && kIsFloat<T>) scale = row_scale[k];
     const bool fixed = scale == scale;
     const int ab = __ldg(in.Apos + i) + chunk * kDenseChunk;
-    const int ae = min(__ldg(in.Apos + i + 1), ab + kDenseChunk);
+    const int ae = ab + min(__ldg(in.Apos + i + 1) - ab, kDenseChunk);
     auto add = [&](T av, int pb) {
       const int c = __ldg(in.Bcrd + pb);
       if (NUMERIC) acc_add<T>(acc + c, product_bits<T>(av, static_cast<const T*>(in.Bval)[pb]), scale, fixed);
@@ -953,7 +955,7 @@ spgemm_smem_kernel(const int* __restrict__ rows, CsrIn in, int n, const unsigned
   double scale = 1.0;
   if constexpr (NUMERIC && kIsFloat<T>) {
     double s = 0.0;
-    for (int p = ab + tid; p < ae; p += NT) s += fabs((double)static_cast<const T*>(in.Aval)[p]);
+    for (unsigned p = (unsigned)ab + tid; p < (unsigned)ae; p += NT) s += fabs((double)static_cast<const T*>(in.Aval)[p]);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(FULL, s, o);
     if (lane == 0) s_abs[warp] = s;
@@ -968,8 +970,8 @@ spgemm_smem_kernel(const int* __restrict__ rows, CsrIn in, int n, const unsigned
   // a row of many entries is cut by entries (every part looking all of them up took 51,000 cycles for 10,014 of
   // them, 23,000 to 43,000 this way), one of few by products: a single entry can bring most of them
   const bool by_entries = parts > 1 && ae - ab >= 2 * NT;
-  const int share = by_entries ? (ae - ab + parts - 1) / parts : ae - ab;
-  const int eb = by_entries ? min(ae, ab + part * share) : ab, ee = by_entries ? min(ae, eb + share) : ae;
+  const int share = by_entries ? (ae - ab - 1) / parts + 1 : ae - ab;
+  const int eb = by_entries ? ab + part * share : ab, ee = by_entries ? eb + min(ae - eb, share) : ae;
   expand_cta<T, NUMERIC, NT>(in, eb, ee, s_expand, tid, [&](int, T a, int pb) {
     const int c = __ldg(in.Bcrd + pb);
     const unsigned bit = 1u << (c & 31);
@@ -1333,8 +1335,8 @@ static int big_rows(const WsLayout& w, const std::vector<int4>& info, int64_t n,
     }
     for (int part = 0; part < parts; part++) tasks.push_back(make_int4((int)row.size(), x.z, x.w, part << 16 | parts));
     if (!parts)
-      for (int b = x.z; b < x.w; b += chunk)
-        tasks.push_back(make_int4((int)row.size(), b, (int)std::min<int64_t>((int64_t)b + chunk, x.w), 0));
+      for (int64_t b = x.z; b < x.w; b += chunk)
+        tasks.push_back(make_int4((int)row.size(), (int)b, (int)std::min<int64_t>(b + chunk, x.w), 0));
     row.push_back(x.x);
     shift.push_back(s);
     p0.push_back(p0.back() + buckets);

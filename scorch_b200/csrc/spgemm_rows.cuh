@@ -218,7 +218,7 @@ __device__ __forceinline__ int emit_runs(const KEY* keys, int count, int shift, 
 }
 
 // ---- expansion ------------------------------------------------------------------------------------
-// The products of A entries [pa0, pa1) (at most 32, one per lane) spread evenly over the lanes
+// The products of `entries` A entries from pa0 on (at most 32, one per lane) spread evenly over the lanes
 // of a warp: lane l looks up the B row of entry pa0 + l, a warp scan of the row lengths numbers
 // the products, and every lane then takes products lane, lane + 32, ... — a 5-step search over
 // the scanned lengths tells which entry a product belongs to.  No lane idles on a short B row and
@@ -227,11 +227,11 @@ __device__ __forceinline__ int emit_runs(const KEY* keys, int count, int shift, 
 // per product with its number in this group, the value of its A entry (T(0) in the symbolic phase)
 // and its position in B; the number of products is returned.
 template <typename T, bool NUMERIC, typename F>
-__device__ __forceinline__ int expand_products(const CsrIn& in, int pa0, int pa1, int lane, F&& emit) {
-  const int pa = pa0 + lane;
+__device__ __forceinline__ int expand_products(const CsrIn& in, int pa0, int entries, int lane, F&& emit) {
   int bb = 0, len = 0;
   T a = T(0);
-  if (pa < pa1) {
+  if (lane < entries) {
+    const int pa = pa0 + lane;
     const int j = __ldg(in.Acrd + pa);
     bb = __ldg(in.Bpos + j);
     len = __ldg(in.Bpos + j + 1) - bb;
@@ -278,35 +278,37 @@ struct ExpandSmem {
 template <typename T, bool NUMERIC, int NT, typename F>
 __device__ __forceinline__ void expand_turns(const CsrIn& in, int ab, int ae, ExpandSmem<T, NT>& sm, int tid, F&& turn) {
   const int warp = tid >> 5, lane = tid & 31;
+  // (unsigned: what is looked at ahead of A's last entries, up to 2^31 - 1 of them, lies beyond an int)
+  const unsigned a0 = ab, a1 = ae;
   int first = 0;
   // (groups of 512 threads and more, which rows of several NT entries come to: the row pointers of the next NT
   // entries and the columns of the NT after those are on their way meanwhile; the others mostly take one turn)
   constexpr bool AHEAD = NT >= 512;
   int next_bb = 0, next_len = 0, next_j = 0;
   T next_a = T(0);
-  auto fetch_row = [&](int pa, int j) {
+  auto fetch_row = [&](unsigned pa, int j) {
     next_bb = next_len = 0;
-    if (pa < ae) {
+    if (pa < a1) {
       if (!AHEAD) j = __ldg(in.Acrd + pa);
       next_bb = __ldg(in.Bpos + j);
       next_len = __ldg(in.Bpos + j + 1) - next_bb;
       if (NUMERIC) next_a = static_cast<const T*>(in.Aval)[pa];
     }
   };
-  auto fetch_column = [&](int pa) {
-    if (pa < ae) next_j = __ldg(in.Acrd + pa);
+  auto fetch_column = [&](unsigned pa) {
+    if (pa < a1) next_j = __ldg(in.Acrd + pa);
   };
   if constexpr (AHEAD) {
-    fetch_column(ab + tid);
+    fetch_column(a0 + tid);
     const int j = next_j;
-    fetch_column(ab + NT + tid);
-    fetch_row(ab + tid, j);
+    fetch_column(a0 + NT + tid);
+    fetch_row(a0 + tid, j);
   }
-  for (int p0 = ab; p0 < ae; p0 += NT) {
+  for (unsigned p0 = a0; p0 < a1; p0 += NT) {
     if (!AHEAD) fetch_row(p0 + tid, 0);
     const int bb = next_bb, len = next_len;
     if (NUMERIC) sm.a[tid] = next_a;
-    if (AHEAD && p0 + NT < ae) {
+    if (AHEAD && p0 + NT < a1) {
       fetch_row(p0 + NT + tid, next_j);
       fetch_column(p0 + 2 * NT + tid);
     }
@@ -345,8 +347,8 @@ __device__ __forceinline__ void expand_cta(const CsrIn& in, int ab, int ae, Expa
                                            int part = 0, int parts = 1) {
   expand_turns<T, NUMERIC, NT>(in, ab, ae, sm, tid, [&](int first, int total, auto&& find) {
 #pragma unroll 4
-    for (int q = part * NT + tid; q < total; q += parts * NT) {
-      const int e = find(q);
+    for (unsigned u = part * NT + tid; u < (unsigned)total; u += parts * NT) {
+      const int q = (int)u, e = find(q);
       emit(first + q, NUMERIC ? sm.a[e] : T(0), sm.off[e] + q);
     }
   });
@@ -365,8 +367,8 @@ __device__ __forceinline__ void expand_row(const CsrIn& in, int ab, int ae, int 
   };
   if constexpr (NT == 32) {
     int first = 0;
-    for (int p0 = ab; p0 < ae; p0 += 32)
-      first += expand_products<T, NUMERIC>(in, p0, min(ae, p0 + 32), tid, [&](int o, T a, int pb) {
+    for (int left = ae - ab; left > 0; left -= 32)
+      first += expand_products<T, NUMERIC>(in, ae - left, min(left, 32), tid, [&](int o, T a, int pb) {
         put(first + o, a, pb);
       });
     __syncwarp();
