@@ -7,6 +7,7 @@ path lives in ``scorch_ops``).
 from __future__ import annotations
 
 import ctypes as C
+import math
 import os
 from typing import Optional, Tuple, Union
 
@@ -493,21 +494,30 @@ def dense_matmul(X: torch.Tensor, W: torch.Tensor, out: Optional[torch.Tensor] =
 
 
 SPLIT_PANEL = 64                  # operand columns multiplied at a time (256 bytes of each operand row)
-# Operand bytes of one chunk and panel.  They stay in the 126 MB L2, better the fewer they are, but every chunk reads and
-# writes the result once more (700,000 rows: two chunks of 90 MB 6.89 ms, three of 60 MB 6.42; 1.4 M: four of 90 MB
-# 17.4 ms, five of 72 MB 17.1; 2 M: five of 102 MB 26.5 ms, six of 85 MB 26.1, seven of 73 MB 26.7; 1 M: three of 85 MB 7.8).
+# Column chunks for an operand of n rows, a panel of `row` bytes of each, and a matrix of d entries per row.  Every chunk
+# reads and writes the result once more: m * row * chunks.  The larger a chunk, the more operand rows L2 (126 MB) loses
+# between two uses: of the m * d gathers a share that grows with n * row / chunks.  Their sum is least at
+# sqrt(n * row * d) times a constant, here 1 / sqrt(86 MB * 17.5), from products of 0.4 to 4 M rows by 2 to 25 chunks (ms
+# of 256 + 64 columns, d = 101 | best count | this one): 0.4 M 3 | 3.73 | 3; 0.7 M 3 | 7.07 | 3; 1 M 5 | 10.87 | 4: 10.99;
+# 1.4 M 5 | 16.0 | 5; 2 M 6 | 25.07 | 6 (7: 25.84); 2.02 M 6 | 25.37 | 6; 3 M 7 | 41.8 | 7; 4 M 8 | 60.2 | one pass.
+# d = 51: 1 M 2 | 6.22 | 3: 6.40; 1.4 M 2 | 9.36 | 3: 9.58; 2 M 2 | 14.27 | one pass: 15.38.
 SPLIT_CHUNK_BYTES = 86e6
-SPLIT_MIN_ENTRIES = 6             # mean entries per row and chunk
+SPLIT_CHUNK_ENTRIES = 17.5
+# Mean entries per row and chunk from which a split pays for itself and the cut (5.7 ns per 1000 entries; d = 25, 0.7 M
+# rows: two chunks 2.61 ms, one pass 2.47; 1 M: 3.81, 3.67; d = 51, 0.7 M: 4.24, 4.88; 3 M: seven chunks 27.9, 23.8).  By
+# the rule above it says as well that a chunk fits L2: 17.5 / 13 * 86 = 116 MB.
+SPLIT_MIN_ENTRIES = 13
 
 
 def split_chunks(m: int, n: int, nnz: int, k: int) -> int:
-    """Column chunks for the product of an (m x n) matrix with an (n x k) operand, 0 for none.  A chunk's
-    pass costs reading and writing the result once more (8 bytes per value at DRAM rate), every entry
-    of it gains its operand row from L2 (17 TB/s) instead of DRAM (7): worth it from some six entries
-    per row and chunk on.  2 M rows, 100 entries each, 256 columns: 24.0 ms in one pass, 21.0 in six."""
+    """Column chunks for the product of an (m x n) matrix with an (n x k) operand, 0 for none: as many as cost
+    least, for operands larger than L2 holds.  2 M rows, 100 entries each, 256 columns: 25.0 ms in one pass,
+    20.0 in six."""
     row = 4 * min(k, SPLIT_PANEL)
-    chunks = -(-n * row // int(SPLIT_CHUNK_BYTES))
-    return chunks if 1 < chunks <= 64 and m > 0 and nnz >= SPLIT_MIN_ENTRIES * chunks * m and m * chunks < 2 ** 31 - 4096 else 0
+    if m <= 0 or n * row <= SPLIT_CHUNK_BYTES or 4 * n * k <= 1.3 * SPLIT_CHUNK_BYTES:
+        return 0
+    chunks = round(math.sqrt(n * row / SPLIT_CHUNK_BYTES * nnz / m / SPLIT_CHUNK_ENTRIES))
+    return chunks if 1 < chunks <= 64 and nnz >= SPLIT_MIN_ENTRIES * chunks * m and m * chunks < 2 ** 31 - 4096 else 0
 
 
 class ColumnSplit:
