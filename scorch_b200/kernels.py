@@ -461,10 +461,19 @@ def _spmm_typed(pos, crd, val, B, n):
 # Rows from which the tensor-core transform is the faster one (9,220 x 256 x 64: 17.5 us against cuBLAS's
 # 12.5; 40,000 x 100 x 128: 25.9 against 35.9): two 128-row tiles per SM keep its pipeline full.
 DENSE_MATMUL_MIN_ROWS = 32768
-# ... or, from 4096 rows (32 tiles) on, multiplications, where its rate counts for more than what a launch of it takes (30,000 x 100 x 128:
-# 22.1 us, cuBLAS 26.9; 12,000 x 256 x 256: 27.6, 40.2; but 20,000 x 100 x 128: 22.3, 20.7; 20,000 x 256 x 64: 25.0, 22.7).
+# ... or from 4096 rows (32 tiles) and so many multiplications on, where its rate counts for more than what a launch
+# of it takes. Kernel alone, us, own | cuBLAS (as called, launch gaps included, own is another 1 to 2 ahead): 4096 x
+# 256 x 256 (268 M) 18.6 | 14.4; 5342 x 256 x 256 (350 M) 18.6 | 21.0; 4096 x 256 x 336 19.1 | 21.4; 8000 x 256 x
+# 256 20.2 | 24.3; 12,000 x 256 x 256 28.7 | 40.2; 22,000 x 128 x 128 (360 M) 20.6 | 20.2; 30,000 x 100 x 128 20.5 |
+# 24.8; 20,000 x 100 x 128 (256 M) 18.5 | 18.1. Where the tiles are few more than the SMs cuBLAS can be ahead
+# (10,938 x 200 x 192: 24.8 | 21.5).
 DENSE_MATMUL_MIN_WORK = 350_000_000
-# Width up to which its result is as close to float64 as a chain of fp32 FMAs (2.3e-7 against 2.9e-7 at 256):
+# Not for results of up to 64 columns, of which cuBLAS computes up to 28,416 rows in one wave (28,000 x 256 x 64:
+# 24.9 | 21.4; 30,000: 25.1 | 27.8), nor for rows of few values, where writing the result and the padded K step
+# decide (21,363 x 16 x 1024: 39.1 | 32.5; 14,242 x 24 x 1024: 29.1 | 27.6; 12,208 x 28 x 1024: 28.3 | 29.3).
+DENSE_MATMUL_WORK_COLUMNS, DENSE_MATMUL_WORK_K = 65, 28
+# Width up to which its result is as close to float64 as a chain of fp32 FMAs (2.3e-7 against 2.9e-7 at 256, 1.2e-7
+# against 2.0e-7 at 128, 0.7e-7 against 1.4e-7 at 64, the same from 4096 rows to 40,000):
 # its error grows with the number of truncating additions, faster than the FMA chain's.
 DENSE_MATMUL_MAX_K = 256
 
@@ -474,9 +483,12 @@ def dense_matmul(X: torch.Tensor, W: torch.Tensor, out: Optional[torch.Tensor] =
     the operands have the layout it takes, else ``torch.matmul``."""
     if (X.dim() != 2 or W.dim() != 2
             or (X.shape[0] < DENSE_MATMUL_MIN_ROWS
-                and (X.shape[0] < 4096 or X.numel() * W.shape[1] < DENSE_MATMUL_MIN_WORK)) or X.dtype != torch.float32
+                and (X.shape[0] < 4096 or X.numel() * W.shape[1] < DENSE_MATMUL_MIN_WORK
+                     or W.shape[1] < DENSE_MATMUL_WORK_COLUMNS or X.shape[1] < DENSE_MATMUL_WORK_K))
+            or X.dtype != torch.float32
             or W.dtype != torch.float32 or not X.is_cuda or W.device != X.device or X.shape[1] != W.shape[0]
-            or not X.is_contiguous() or not W.is_contiguous() or not 0 < X.shape[1] <= DENSE_MATMUL_MAX_K or X.shape[1] % 4
+            or not X.is_contiguous() or not W.is_contiguous() or not 0 < X.shape[1] <= DENSE_MATMUL_MAX_K
+            or X.shape[1] % 4
             or W.shape[1] == 0 or W.shape[1] % 8 or X.data_ptr() % 16
             or (out is not None and (out.shape != (X.shape[0], W.shape[1]) or out.dtype != torch.float32
                                      or out.device != X.device or not out.is_contiguous() or out.data_ptr() % 32))):
@@ -494,18 +506,20 @@ def dense_matmul(X: torch.Tensor, W: torch.Tensor, out: Optional[torch.Tensor] =
 
 
 SPLIT_PANEL = 64                  # operand columns multiplied at a time (256 bytes of each operand row)
-# Column chunks for an operand of n rows, a panel of `row` bytes of each, and a matrix of d entries per row.  Every chunk
-# reads and writes the result once more: m * row * chunks.  The larger a chunk, the more operand rows L2 (126 MB) loses
-# between two uses: of the m * d gathers a share that grows with n * row / chunks.  Their sum is least at
-# sqrt(n * row * d) times a constant, here 1 / sqrt(86 MB * 17.5), from products of 0.4 to 4 M rows by 2 to 25 chunks (ms
-# of 256 + 64 columns, d = 101 | best count | this one): 0.4 M 3 | 3.73 | 3; 0.7 M 3 | 7.07 | 3; 1 M 5 | 10.87 | 4: 10.99;
-# 1.4 M 5 | 16.0 | 5; 2 M 6 | 25.07 | 6 (7: 25.84); 2.02 M 6 | 25.37 | 6; 3 M 7 | 41.8 | 7; 4 M 8 | 60.2 | one pass.
-# d = 51: 1 M 2 | 6.22 | 3: 6.40; 1.4 M 2 | 9.36 | 3: 9.58; 2 M 2 | 14.27 | one pass: 15.38.
+# Column chunks for an operand of n rows, a panel of `row` bytes of each, and a matrix of m rows with d entries
+# each. Every chunk reads and writes the result once more: chunks * m * row bytes. The larger a chunk, the more
+# operand rows L2 (126 MB) loses between two uses: of the m * d gathers a share that grows with n * row / chunks.
+# The sum of both is least at a constant times sqrt(n * row * d); the constant, 1 / sqrt(86 MB * 17.5), comes from
+# products of 0.4 to 4 M rows in 2 to 25 chunks. d = 101, ms of a product with 256 and one with 64 columns, best
+# count measured | this one: 0.4 M rows 3 | 3: 3.73; 0.7 M 3 | 3: 7.07; 1 M 5: 10.87 | 4: 10.99; 1.4 M 5 | 5: 16.0;
+# 2 M 6 | 6: 25.1 (7: 25.8); 2.02 M 6 | 6: 25.4; 3 M 7 | 7: 41.8. d = 51: 1 M 2: 6.22 | 3: 6.40; 1.4 M 2: 9.36 | 3:
+# 9.58.
 SPLIT_CHUNK_BYTES = 86e6
 SPLIT_CHUNK_ENTRIES = 17.5
-# Mean entries per row and chunk from which a split pays for itself and the cut (5.7 ns per 1000 entries; d = 25, 0.7 M
-# rows: two chunks 2.61 ms, one pass 2.47; 1 M: 3.81, 3.67; d = 51, 0.7 M: 4.24, 4.88; 3 M: seven chunks 27.9, 23.8).  By
-# the rule above it says as well that a chunk fits L2: 17.5 / 13 * 86 = 116 MB.
+# Mean entries per row and chunk from which a split pays for itself and the cut (5.7 ns per 1000 entries). Chunks
+# with the cut | one pass, ms: d = 25, 0.7 M rows 2: 2.61 | 2.47; 1 M 2: 3.81 | 3.67; d = 51, 0.7 M 2: 4.24 | 4.88;
+# 2 M 4: 15.1 | 15.4 and as whole forwards alike; 3 M 5: 26.4 | 23.8; d = 101, 4 M 8: 62.5 | 64.3. By the rule above
+# it says as well that a chunk fits L2: 17.5 / 13 * 86 MB = 116 MB.
 SPLIT_MIN_ENTRIES = 13
 
 
