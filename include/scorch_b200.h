@@ -387,9 +387,9 @@ SB_API int sb_csr_validate(int64_t m, int64_t n, int64_t nnz, const int32_t* pos
  *                          tensor-memory cells at the end: columns [0,384) the hi parts of
  *                          P = exp2(log2(e) S - row max), [384,448) the unnormalised O = P V,
  *                          [448,512) the lo parts of P's last 64 columns; `phase_clocks` (may be
- *                          null, 36 values; the scores are then not copied out) the SM clock at the kernel's phase boundaries (scores
- *                          staged and issued piece by piece, row maxima, the six rounds of
- *                          O += P V, end).  O is not written.
+ *                          null, 36 values; the scores are then not copied out) the SM clock at
+ *                          the kernel's phase boundaries (scores staged and issued piece by
+ *                          piece, row maxima, the six rounds of O += P V, end).  O is not written.
  * -------------------------------------------------------------------------------------------- */
 #define SB_ATTN_BAND_ROWS 128
 #define SB_ATTN_BAND_COLS 384
@@ -422,7 +422,7 @@ SB_API int sb_attn_band_status(void);
  *             stream (the caller must size Ccrd/Cval).  SB_ERR_OVERFLOW when total >= 2^31.
  *   numeric : fills Ccrd/Cval for the Cpos of the symbolic call; `ws` must be the SAME,
  *             unmodified workspace (it carries the row bins).
- * A has m rows; B has `kb` rows and n columns.
+ * A has m rows; B has `kb` rows and n columns.  A, B and the result may hold up to INT32_MAX entries.
  * -------------------------------------------------------------------------------------------- */
 SB_API size_t sb_spgemm_workspace_bytes(int64_t m, int64_t n, int dtype);
 SB_API int sb_spgemm_symbolic(int64_t m, int64_t kb, int64_t n, const int32_t* Apos,

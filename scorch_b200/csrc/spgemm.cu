@@ -5,7 +5,8 @@
 //   bin 0  U <= 128     one warp per row, products sorted by (column, ordinal) in registers
 //   bin 1  U <= 512     one 64-thread CTA per row, the same network across its warps
 //   bin 2  U <= 2048    one 128-thread CTA per row
-//   bin 3  U <= 8192    one 512-thread CTA per row, its columns in segments of a warp each
+//   bin 3  U <= 8192    one CTA per row, 512 threads (1024 where there are no more such rows than SMs), its columns in
+//                       segments of a warp each
 //   bin 4  U  > 8192    the row's columns are cut into buckets of some 700 products, the products
 //                       scattered to their buckets in global memory and every bucket sorted by a CTA
 // (spgemm_rows.cuh: the sorting kernels of bins 0-3.)  Columns come out ascending like the
@@ -47,7 +48,7 @@ constexpr int64_t kBigProductsMax = (int64_t)1 << 26;
 constexpr int64_t kBucketProducts = 1024;      // buckets per row: U / this, rounded up to a power of two
 constexpr int kBucketSort = 2048;              // products a bucket's sorting kernel takes
 constexpr int kBigTasks = 1 << 17;
-constexpr int kTurnProducts = 8192;            // products of 256 entries of A that a task takes; the rest is dealt out anew
+constexpr int kTurnProducts = 8192;            // products of 256 entries of A that a task takes; the rest is dealt out
 // Columns up to which long rows are summed in shared memory (spgemm_smem_kernel) and need no area.
 constexpr int kSmemColumns = 24576;
 
@@ -291,7 +292,8 @@ __device__ __forceinline__ T acc_value(Slot v, double scale, bool fixed) {
 }
 
 template <typename T>
-__global__ void spgemm_max_abs_kernel(const int* __restrict__ nnz_ptr, const T* __restrict__ val, unsigned long long* out) {
+__global__ void spgemm_max_abs_kernel(const int* __restrict__ nnz_ptr, const T* __restrict__ val,
+                                      unsigned long long* out) {
   const long long nnz = *nnz_ptr;
   double mx = 0.0;
   bool bad = false;
@@ -340,10 +342,11 @@ big_scale_kernel(BigArea b, const int* __restrict__ Apos, const T* __restrict__ 
   }
 }
 
-// One task = some entries of one long row of A, or, of a row of up to 512 entries, a part of the products.  SCATTER false: products per bucket; true: every
-// product's column (and value) to the next free place of its bucket.  A task of the first kind takes
-// up to kTurnProducts products per 256 entries; what is beyond that - an entry of A can bring 400,000 - is noted by the
-// counting kernel in equal parts, which REST launches of both take: the CTA that had such an entry kept the GPU waiting.
+// One task = some entries of one long row of A, or, of a row of up to 512 entries, a part of the products.  SCATTER
+// false: products per bucket; true: every product's column (and value) to the next free place of its bucket.  A task of
+// the first kind takes up to kTurnProducts products per 256 entries; what is beyond that - an entry of A can bring
+// 400,000 - is noted by the counting kernel in equal parts, which REST launches of both take: the CTA that had such an
+// entry kept the GPU waiting.
 // (One 16-byte record per product: a column and a value array cost a third scattered access.)
 // Bound: the latency of a batch (B's entries in short pieces, places, stores).  A CTA counts kScatter products a
 // thread per bucket, takes their places together, one atomic per bucket, and writes them in the buckets' order.
@@ -955,7 +958,8 @@ spgemm_smem_kernel(const int* __restrict__ rows, CsrIn in, int n, const unsigned
   double scale = 1.0;
   if constexpr (NUMERIC && kIsFloat<T>) {
     double s = 0.0;
-    for (unsigned p = (unsigned)ab + tid; p < (unsigned)ae; p += NT) s += fabs((double)static_cast<const T*>(in.Aval)[p]);
+    const T* Aval = static_cast<const T*>(in.Aval);
+    for (unsigned p = (unsigned)ab + tid; p < (unsigned)ae; p += NT) s += fabs((double)Aval[p]);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(FULL, s, o);
     if (lane == 0) s_abs[warp] = s;
@@ -1056,8 +1060,10 @@ spgemm_smem_kernel(const int* __restrict__ rows, CsrIn in, int n, const unsigned
       }
       out.crd[at] = col;
       T value;
-      if constexpr (kIsFloat<T>) value = fixed ? (T)((double)(long long)v * inv) : (T)__longlong_as_double((long long)v);
-      else value = (T)v;
+      if constexpr (kIsFloat<T>)
+        value = fixed ? (T)((double)(long long)v * inv) : (T)__longlong_as_double((long long)v);
+      else
+        value = (T)v;
       static_cast<T*>(out.val)[at] = value;
     }
   }
@@ -1070,7 +1076,8 @@ spgemm_smem_kernel(const int* __restrict__ rows, CsrIn in, int n, const unsigned
 // left the hub rows to a warp each: 4.7 ms for 272 M entries); a thread finds the row of its entry
 // among the tile's row pointers in shared memory.  Tiles of kMoveTile entries, smaller where that leaves SMs idle
 // (1.1 M entries: 15.3 us in 136 tiles of 8192, 9.4 in 542 of 2048).
-// The places of kMoveAhead entries are found before the first is loaded: 284 M entries 1.06 ms one by one, 0.76 so = 6.0 TB/s.
+// The places of kMoveAhead entries are found before the first is loaded: 284 M entries 1.06 ms one by one, 0.76 so =
+// 6.0 TB/s.
 constexpr int kMoveTile = 8192, kMoveRows = 1024, kMoveAhead = 4;
 template <typename T>
 __global__ void __launch_bounds__(256)
@@ -1304,8 +1311,8 @@ static int big_rows(const WsLayout& w, const std::vector<int4>& info, int64_t n,
   for (const int4& x : info) total += x.y > w.products ? 0 : x.y;
   const int64_t target = total / std::max<int64_t>(1, ceil_div(total, w.products));
   // products per task: small enough to give every SM a few tasks
-  const int64_t task_products =
-      std::min<int64_t>(kTurnProducts, std::max<int64_t>(kScatterCta, total / (4 * sm_count()) / kScatterCta * kScatterCta));
+  const int64_t share = total / (4 * sm_count()) / kScatterCta * kScatterCta;
+  const int64_t task_products = std::min<int64_t>(kTurnProducts, std::max<int64_t>(kScatterCta, share));
   auto flush = [&]() -> int {
     if (row.empty()) return SB_OK;
     const int rc = big_batch<T, NUMERIC>(w, row, p0, shift, tasks, n, in, out, st);
@@ -1399,7 +1406,9 @@ static int launch_bins(const WsLayout& w, const long long* counts, int64_t m, in
     if (counts[4] > 0) rc = max_abs<T>(w, in, kb, st);
     if (rc != SB_OK) return rc;
   }
-  // (the long rows' list is read back ahead of the other bins, which run while the host plans the long rows' tasks)
+  // (the long rows' list is read back ahead of the other bins, which run while the host plans the long rows' tasks.
+  // A plan of more than 64 KB, which comes from pageable memory, is copied once the stream has come to it: from there
+  // on the host waits for the bins, once per batch.)
   std::vector<int4> info;
   if (counts[4] > 0 && !in_smem) rc = big_list(w, counts[4], m, in, info, st);
   if (rc != SB_OK) return rc;
@@ -1631,11 +1640,12 @@ int sb_spgemm_finish(int dtype, int64_t m, int64_t nnz, const int32_t* off, cons
   if (m == 0 || nnz == 0) return SB_OK;
   SB_CHECK_ARG(off && tcrd && tval && Cpos && Ccrd && Cval, "spgemm_finish: null pointer");
   cudaStream_t st = (cudaStream_t)stream;
-  const int tile = (int)std::min<int64_t>(kMoveTile, std::max<int64_t>(256 * kMoveAhead, ceil_div(ceil_div(nnz, 4 * sm_count()), 256) * 256));
+  const int64_t share = ceil_div(ceil_div(nnz, 4 * sm_count()), 256) * 256;
+  const int tile = (int)std::min<int64_t>(kMoveTile, std::max<int64_t>(256 * kMoveAhead, share));
   const unsigned grid = (unsigned)ceil_div(nnz, tile);
   if (dtype == SB_F32 || dtype == SB_I32)
-    spgemm_move_kernel<unsigned><<<grid, 256, 0, st>>>((int)m, (int)nnz, tile, off, Cpos, tcrd, (const unsigned*)tval, Ccrd,
-                                                       (unsigned*)Cval);
+    spgemm_move_kernel<unsigned><<<grid, 256, 0, st>>>((int)m, (int)nnz, tile, off, Cpos, tcrd, (const unsigned*)tval,
+                                                       Ccrd, (unsigned*)Cval);
   else
     spgemm_move_kernel<unsigned long long><<<grid, 256, 0, st>>>(
         (int)m, (int)nnz, tile, off, Cpos, tcrd, (const unsigned long long*)tval, Ccrd, (unsigned long long*)Cval);

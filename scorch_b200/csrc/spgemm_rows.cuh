@@ -276,7 +276,8 @@ struct ExpandSmem {
 // `turn(first, total, find)` is called per NT entries, with the number of the first product and of products; find(q)
 // = entry of the turn's product q.
 template <typename T, bool NUMERIC, int NT, typename F>
-__device__ __forceinline__ void expand_turns(const CsrIn& in, int ab, int ae, ExpandSmem<T, NT>& sm, int tid, F&& turn) {
+__device__ __forceinline__ void expand_turns(const CsrIn& in, int ab, int ae, ExpandSmem<T, NT>& sm, int tid,
+                                             F&& turn) {
   const int warp = tid >> 5, lane = tid & 31;
   // (unsigned: what is looked at ahead of A's last entries, up to 2^31 - 1 of them, lies beyond an int)
   const unsigned a0 = ab, a1 = ae;

@@ -32,13 +32,13 @@ constexpr int kUnit = 512;             // a window's last row or unit reaches up
 // ones gain by having their start-up spread over twice as many (0.8 M entries in rows of 8, 64 columns: 27.0 us, 22.9
 // with 3072).
 // 8-byte types, whose entries take 16 bytes: as much as lets three CTAs stay within 196 KB of shared memory.
-// Beyond that 23 KB are left to L1 in place of 55 and the gathers wait for it (120,000 rows of 27 entries, 16
-// float64 columns: 47.9 us with 3072, 43.2 with this).
+// Beyond that 23 KB are left to L1 in place of 55 and the gathers wait for it (120,000 rows of 27 entries, the same
+// operands over and over: 16 float64 columns 47.0 us with 3072, 42.7 with this, 3 columns 41.5, 34.5).
 constexpr int tile_window(int L, int size = 4) { return L == 32 ? 1536 : size == 8 ? 2560 : 3072; }
 // Rows of up to this length go to a lane group.  32 lets the warp's other groups help with a row of
 // a power-law graph (2 M rows, 64 columns: 6.10 ms with 64, 5.66 with 32); the 8 groups of four
-// lanes have too little of a 33-entry row each (27 entries per row, 16 float64 columns: 51.4 us
-// with 32, 47.9 with 40 and with 64; power law of mean 20, 8 columns: 29.0, 29.6, 31.7).
+// lanes have too little of a 33-entry row each (the same 16 float64 columns: 46.6 us with 32, 42.7 with 40, 43.1
+// with 64; power law of mean 20, 8 columns: 27.6, 28.0, 30.0).
 template <int L>
 constexpr int kGroupRow = L == 4 ? 40 : 32;
 constexpr int kWarpRow = 192;
@@ -51,8 +51,9 @@ constexpr int kUnitList = tile_window(L, SIZE) / kWarpRow + tile_window(L, SIZE)
 // Classes of similar length among the rows that a lane group takes.  A warp's groups take rows of one class,
 // the longest first: in the order of the matrix they waited for the longest of their 2 to 8 rows.  (GCN
 // layer of 2 M rows, 202 M entries, 64-column panels: 20.4 ms in the matrix's order, 19.1 by class; power law
-// of mean 12, 32 columns: 46.8 us, 39.8; 60,000 rows of 16, 7 columns: 15.0, 13.1.  Taken as one stream of entries per group across the rows' ends,
-// an operand row fetched for every one added, the same rows took 1.7 to 2 times as long.)
+// of mean 12, 32 columns: 46.8 us, 39.8; 60,000 rows of 16, 7 columns: 15.0, 13.1.  Taken as one stream of entries
+// per group across the rows' ends, an operand row fetched for every one added, the same rows took 1.7 to 2 times as
+// long.)
 constexpr int kShortClasses = 4;
 
 // Resident CTAs per SM the kernels are compiled for (64 / 80 registers; measured per lane count).
