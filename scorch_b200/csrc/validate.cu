@@ -26,11 +26,12 @@ __global__ void validate_crd_kernel(int m, int n, const int* __restrict__ pos, c
                                     int sorted_unique, unsigned long long* key) {
   const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (row >= m) return;
-  const int b = pos[row], e = pos[row + 1];
-  for (int p = b + lane; p < e; p += 32) {
+  // (unsigned: entries may end at 2^31 - 1, and the step behind the last one wraps an int)
+  const unsigned b = pos[row], e = pos[row + 1];
+  for (unsigned p = b + lane; p < e; p += 32) {
     const int c = crd[p];
     if (c < 0 || c >= n || (sorted_unique && p > b && crd[p - 1] >= c))
-      atomicMin(key, ((unsigned long long)(unsigned)row << 32) | (unsigned)p);
+      atomicMin(key, ((unsigned long long)(unsigned)row << 32) | p);
   }
 }
 

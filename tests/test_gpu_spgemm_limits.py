@@ -99,3 +99,18 @@ def test_last_rows_of_the_largest_matrix(largest, kind):
         got = K.spgemm_csr(pos, largest["crd"], largest["val"], *B, n, timings=timings)
         assert torch.equal(got[0][4096:], want[0]) and not got[0][:4096].any()
         assert torch.equal(got[1], want[1]) and torch.equal(got[2], want[2])     # the same bits
+
+
+def test_check_of_the_largest_matrix(largest):
+    # what SCORCH_B200_VALIDATE=1 runs on the operands: the last row ends at entry 2^31 - 2
+    from scorch_b200 import kernels as K
+    pos = torch.linspace(0, MOST, 8193, dtype=torch.float64, device="cuda").long()
+    pos[-1] = MOST
+    largest["crd"][-16384:] = 0
+    assert K.csr_validate(pos.int(), largest["crd"], 6001, sorted_unique=False) is None
+    largest["crd"][-1] = 6001
+    try:
+        assert K.csr_validate(pos.int(), largest["crd"], 6001, sorted_unique=False) == (
+            "column index out of range", 8191, MOST - 1, 6001)
+    finally:
+        largest["crd"][-1] = 0
