@@ -727,7 +727,7 @@ class GcnSharded(Workload):
             cut = [b.columns[1] if b.columns else None for b in split.blocks]
             products = sum(len(c.counts) * -(-k // K.SPLIT_PANEL) if c is not None else 1 for c in cut)
             ends = [min(o, self.shard.rows) for o in split.offsets]
-            transforms = sum(b - a >= K.DENSE_MATMUL_MIN_ROWS for a, b in zip(ends, ends[1:]))
+            transforms = sum(K.dense_on_tensor_cores(b - a, self.K1, k) for a, b in zip(ends, ends[1:]))
             return 2 * products + 2 * transforms
         return launches(self.shard.splits[0], self.K1) + launches(self.shard.splits[-1], self.K2)
 

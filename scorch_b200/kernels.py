@@ -478,18 +478,20 @@ DENSE_MATMUL_WORK_COLUMNS, DENSE_MATMUL_WORK_K = 65, 28
 DENSE_MATMUL_MAX_K = 256
 
 
+def dense_on_tensor_cores(m: int, k: int, n: int) -> bool:
+    """Whether ``dense_matmul`` computes an (m x k) by (k x n) product on the tensor cores, by its sizes."""
+    return (0 < k <= DENSE_MATMUL_MAX_K and k % 4 == 0 and n > 0 and n % 8 == 0
+            and (m >= DENSE_MATMUL_MIN_ROWS
+                 or (m >= 4096 and m * k * n >= DENSE_MATMUL_MIN_WORK
+                     and n >= DENSE_MATMUL_WORK_COLUMNS and k >= DENSE_MATMUL_WORK_K)))
+
+
 def dense_matmul(X: torch.Tensor, W: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """X @ W in fp32 for a tall X: on the tensor cores in fp32 accuracy (``sb_dense_matmul_f32``) where
-    the operands have the layout it takes, else ``torch.matmul``."""
-    if (X.dim() != 2 or W.dim() != 2
-            or (X.shape[0] < DENSE_MATMUL_MIN_ROWS
-                and (X.shape[0] < 4096 or X.numel() * W.shape[1] < DENSE_MATMUL_MIN_WORK
-                     or W.shape[1] < DENSE_MATMUL_WORK_COLUMNS or X.shape[1] < DENSE_MATMUL_WORK_K))
-            or X.dtype != torch.float32
-            or W.dtype != torch.float32 or not X.is_cuda or W.device != X.device or X.shape[1] != W.shape[0]
-            or not X.is_contiguous() or not W.is_contiguous() or not 0 < X.shape[1] <= DENSE_MATMUL_MAX_K
-            or X.shape[1] % 4
-            or W.shape[1] == 0 or W.shape[1] % 8 or X.data_ptr() % 16
+    the operands have the sizes and the layout it takes, else ``torch.matmul``."""
+    if (X.dim() != 2 or W.dim() != 2 or X.shape[1] != W.shape[0] or not dense_on_tensor_cores(*X.shape, W.shape[1])
+            or X.dtype != torch.float32 or W.dtype != torch.float32 or not X.is_cuda or W.device != X.device
+            or not X.is_contiguous() or not W.is_contiguous() or X.data_ptr() % 16
             or (out is not None and (out.shape != (X.shape[0], W.shape[1]) or out.dtype != torch.float32
                                      or out.device != X.device or not out.is_contiguous() or out.data_ptr() % 32))):
         return torch.matmul(X, W, out=out)
