@@ -523,6 +523,13 @@ SPLIT_CHUNK_ENTRIES = 17.5
 # 2 M 4: 15.1 | 15.4 and as whole forwards alike; 3 M 5: 26.4 | 23.8; d = 101, 4 M 8: 62.5 | 64.3. By the rule above
 # it says as well that a chunk fits L2: 17.5 / 13 * 86 MB = 116 MB.
 SPLIT_MIN_ENTRIES = 13
+# Chunks' worth of operand from which a product is cut at all: what L2 nearly holds is multiplied in one pass.
+SPLIT_MIN_OPERAND = 1.3
+
+
+def split_pays(n: int, k: int) -> bool:
+    """Whether a product with an (n x k) operand uses a column split of its matrix, if there is one."""
+    return 4 * n * k > SPLIT_MIN_OPERAND * SPLIT_CHUNK_BYTES
 
 
 def split_chunks(m: int, n: int, nnz: int, k: int) -> int:
@@ -530,7 +537,7 @@ def split_chunks(m: int, n: int, nnz: int, k: int) -> int:
     least, for operands larger than L2 holds.  2 M rows, 100 entries each, 256 columns: 25.0 ms in one pass,
     20.0 in six."""
     row = 4 * min(k, SPLIT_PANEL)
-    if m <= 0 or n * row <= SPLIT_CHUNK_BYTES or 4 * n * k <= 1.3 * SPLIT_CHUNK_BYTES:
+    if m <= 0 or n * row <= SPLIT_CHUNK_BYTES or not split_pays(n, k):
         return 0
     chunks = round(math.sqrt(n * row / SPLIT_CHUNK_BYTES * nnz / m / SPLIT_CHUNK_ENTRIES))
     return chunks if 1 < chunks <= 64 and nnz >= SPLIT_MIN_ENTRIES * chunks * m and m * chunks < 2 ** 31 - 4096 else 0

@@ -81,8 +81,7 @@ def gcn_forward(pos, crd, val, X, W1, W2, plan: Optional[K.CsrPlan] = None) -> t
     matrix run over equal tiles of its entries."""
     n, hidden, width = X.shape[0], W1.shape[1], W2.shape[1]
     split = K.ColumnSplit.of(pos, crd, val, n, max(hidden, width)) if W1.is_cuda and X.dtype == torch.float32 else None
-    # (an operand that L2 nearly holds whole is multiplied in one pass)
-    product = lambda B, relu: (split.matmul(B, relu) if split is not None and 4 * n * B.shape[1] > 1.3 * K.SPLIT_CHUNK_BYTES
+    product = lambda B, relu: (split.matmul(B, relu) if split is not None and K.split_pays(n, B.shape[1])
                                else K.spmm_csr(pos, crd, val, B, relu=relu))
     return product(K.dense_matmul(product(K.dense_matmul(X, W1), True), W2), False)
 

@@ -273,8 +273,7 @@ def _split_by_chunk(local: CsrBlock, bounds: List[int], offsets: List[int]) -> L
 def _default_spmm(block: CsrBlock, B: torch.Tensor, out: torch.Tensor, relu: bool,
                   accumulate: bool = False) -> None:
     from . import kernels as K
-    # (an operand that L2 nearly holds whole is multiplied in one pass)
-    if B.is_contiguous() and out.is_contiguous() and 4 * B.numel() > 1.3 * K.SPLIT_CHUNK_BYTES:
+    if B.is_contiguous() and out.is_contiguous() and K.split_pays(*B.shape):
         split = block.columns_for(B.shape[0], B.shape[1])
         if split is not None:
             split.matmul(B, relu, out=out, accumulate=accumulate)

@@ -35,7 +35,8 @@ def test_neighbouring_sizes_differ_by_one_chunk(d, k):
     assert all(a <= b <= a + 1 for a, b in zip(split, split[1:]))
 
 
-@pytest.mark.parametrize("n,k", [(0, 64), (1000, 256), (300_000, 64), (600_000, 40), (1_700_000, 16)])
+@pytest.mark.parametrize("n,k", [(0, 64), (1000, 256), (300_000, 64), (600_000, 40), (1_700_000, 16),
+                                 (400_000, 64), (430_000, 64), (690_000, 40)])
 def test_operands_that_l2_holds_are_not_split(n, k):
     assert K.split_chunks(n, n, n * 400, k) == 0
 
