@@ -267,12 +267,12 @@ __device__ __noinline__ void topk_row_radix(int n, int k, const unsigned* __rest
 
 // One CTA per row.  The k-th largest of the threads' own maxima is a lower bound of the k-th largest
 // element, and for values in no particular order a close one (32 of 32768: some 33 elements reach
-// it).  So the row is read twice - a maximum per thread, then the few elements that reach the bound
-// - and the exact selection is a ranking of those few by counting.  Rows where more than kTopkCands
-// elements reach the bound (many equal values, values sorted against the threads) and k beyond
-// kTopkFastK take the radix passes.
-// Bound: DRAM on one read of the matrix; the second read mostly hits L2.  Four CTAs of 512 threads
-// per SM, four loads in flight per thread: the phases of one row (two reads, 16 barriers of the
+// it).  So the row is read once for a maximum per thread; then the threads whose part has elements that
+// reach the bound (some 33 of the 512) read that part again and collect them, and the exact selection is
+// a ranking of those few by counting.  Rows where more than kTopkCands elements reach the bound (many
+// equal values, values sorted against the threads) and k beyond kTopkFastK take the radix passes.
+// Bound: DRAM on one read of the matrix; the parts that are read again come from L2.  Four CTAs of 512
+// threads per SM, four loads in flight per thread: the phases of one row (the reads, 16 barriers of the
 // bound, the ranking) overlap with the reads of others.  8192 x 32768, k = 32: 210 us = 5.1 TB/s
 // (292 us with two CTAs per SM, 1.86 ms with five reads, histogram atomics and a block scan per 256
 // elements).

@@ -1391,11 +1391,14 @@ static int launch_split_bin(const int* rows, int64_t count, const WsLayout& w, c
                              : launch_split_rows<T, NUMERIC, 512>(rows, count, w, in, n, out, st);
 }
 
-// All rows; the longest first, so that the short ones fill in behind them: a bin's kernel lets the
-// next one start as soon as its own CTAs have (they do not depend on one another) and ends after the
-// one before it.  The first of them is an ordinary launch: it begins behind the completed work of the
-// stream (max |b|, the operands), and so do all that begin after it, which read these without a wait
-// of their own.  A key holds the column above the product's ordinal: 32 bits where both fit.
+// All rows.  Bins 3 to 0 in this order, so that the short rows fill in behind the longer ones: a bin's
+// kernel lets the next one start as soon as its own CTAs have (they do not depend on one another) and ends
+// after the one before it.  The first of them is an ordinary launch: it begins behind the completed work of
+// the stream (max |b|, the operands), and so do all that begin after it, which read these without a wait
+// of their own.  The long rows of bin 4 come last.  In shared memory, theirs is one more such kernel.  By
+// buckets, they are a chain of ordinary launches, which the stream holds until all the bins are done: their
+// tasks are planned by the host, and planned behind the bins' launches that work keeps no GPU waiting.
+// A key holds the column above the product's ordinal: 32 bits where both fit.
 template <typename T, bool NUMERIC>
 static int launch_bins(const WsLayout& w, const long long* counts, int64_t m, int64_t kb, int64_t n,
                        const CsrIn& in, const RowsOut& out, cudaStream_t st) {
@@ -1406,9 +1409,9 @@ static int launch_bins(const WsLayout& w, const long long* counts, int64_t m, in
     if (counts[4] > 0) rc = max_abs<T>(w, in, kb, st);
     if (rc != SB_OK) return rc;
   }
-  // (the long rows' list is read back ahead of the other bins, which run while the host plans the long rows' tasks.
+  // (The long rows' list is read back ahead of the other bins, which run while the host plans the long rows' tasks.
   // A plan of more than 64 KB, which comes from pageable memory, is copied once the stream has come to it: from there
-  // on the host waits for the bins, once per batch.)
+  // on the host waits for the bins, and for the batch before with every further one.)
   std::vector<int4> info;
   if (counts[4] > 0 && !in_smem) rc = big_list(w, counts[4], m, in, info, st);
   if (rc != SB_OK) return rc;

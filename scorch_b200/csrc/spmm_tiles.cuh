@@ -8,8 +8,9 @@
 //                              length side by side in a warp
 //   up to kWarpRow             the lane groups of a warp, a slice each
 //   longer                     all lane groups of the CTA, in units of kUnit entries; the unit sums
-//                              of a row of several units are added in order by a second launch
-//                              (which also writes the rows without entries)
+//                              of a row of several units are added by a second launch, every eighth
+//                              one in order, then these eight sums (it also writes the rows without
+//                              entries)
 // Nothing is built beforehand and no host decision depends on the matrix.  Which sums are formed in
 // which order depends on a row's own length only, not on where the row lies: the same bits on every
 // run, and for a block of rows the same as for the whole matrix.
@@ -251,7 +252,8 @@ spmm_tile_kernel(SpmmArgs<T> a, TileArgs<T> t) {
         // entry was dealt with by the turn before)
         int u = b >= next ? 0 : (next == e0 ? (e0 - b + kUnit - 1) / kUnit : INT32_MAX / kUnit);
         for (; u < (len + kUnit - 1) / kUnit && b + u * kUnit < e1; u++)
-          sm.by_cta[atomicAdd(&sm.n_cta, 1)] = TileUnit{r0 + i, b + u * kUnit, min(kUnit, len - u * kUnit), len <= kUnit};
+          sm.by_cta[atomicAdd(&sm.n_cta, 1)] =
+              TileUnit{r0 + i, b + u * kUnit, min(kUnit, len - u * kUnit), len <= kUnit};
       }
     }
     int n_short[kShortClasses];          // (rows up to the class's end)
@@ -395,7 +397,9 @@ spmm_tile_rows_kernel(SpmmArgs<T> a, TileArgs<T> t) {
   }
   if (by_cta) s_rows[atomicAdd(&s_n, 1)] = (int)(r0 + lane);
   asm volatile("griddepcontrol.wait;" ::: "memory");   // the tile kernel's results
-  auto unit_sum = [&](int rb, int u, int col) { return (u ? t.rest : t.first)[((long long)(rb / kUnit) + u) * a.k + col]; };
+  auto unit_sum = [&](int rb, int u, int col) {
+    return (u ? t.rest : t.first)[((long long)(rb / kUnit) + u) * a.k + col];
+  };
   auto store = [&](T* c, int col, T s) {
     Pack<T, 1> x;
     x.v[0] = s + (a.accumulate ? *c : T(0));
@@ -488,8 +492,8 @@ static int launch_tiles(const SpmmArgs<T>& a, int64_t nnz, void* ws, cudaStream_
   // that, which is sound behind the tile kernel, whose CTAs have waited for whatever made them; a
   // matrix without entries has no tile kernel, and an ordinary launch)
   const dim3 grid((unsigned)ceil_div(a.m, kTileThreadsMm), (unsigned)std::min<int64_t>(ceil_div(a.k, 32), 64));
-  SB_CUDA(launch_kernel(t.tiles > 0, nnz >= kSharedSums ? spmm_tile_rows_kernel<T, true> : spmm_tile_rows_kernel<T, false>,
-                        grid, kTileThreadsMm, 0, st, a, t));
+  auto rows_kernel = nnz >= kSharedSums ? spmm_tile_rows_kernel<T, true> : spmm_tile_rows_kernel<T, false>;
+  SB_CUDA(launch_kernel(t.tiles > 0, rows_kernel, grid, kTileThreadsMm, 0, st, a, t));
   return SB_OK;
 }
 
