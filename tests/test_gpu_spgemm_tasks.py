@@ -4,6 +4,7 @@ from __future__ import annotations
 
 import numpy as np
 import pytest
+import torch
 
 from test_gpu_spgemm_bins import _check, _csr
 
@@ -35,10 +36,12 @@ def test_row_of_more_buckets_than_are_counted_together(dtype):
     _check(_csr([100, 3], 100, rng, dtype), B, n, dtype)
 
 
-@pytest.mark.parametrize("rows", [148, 149])
+@pytest.mark.parametrize("beyond", [0, 1])
 @pytest.mark.parametrize("n", [64, 65, 3000, 1 << 21])
-def test_cta_rows_of_both_sizes(rows, n):
-    # 2049 to 8192 products; 64 and 65 columns: segments of one and two columns
+def test_cta_rows_of_both_sizes(beyond, n):
+    # 2049 to 8192 products; as many rows as SMs, which a CTA of 1024 threads takes each, and one more, where CTAs have
+    # 512.  64 and 65 columns: segments of one and two columns
+    rows = torch.cuda.get_device_properties(0).multi_processor_count + beyond
     rng = np.random.default_rng(rows)
     B = _csr([min(n, 50)] * 150, n, rng, np.float32)
     _check(_csr([int(x) for x in rng.integers(45, 140, rows)], 150, rng, np.float32), B, n, np.float32)
