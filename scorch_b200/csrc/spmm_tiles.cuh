@@ -368,17 +368,19 @@ spmm_tile_kernel(SpmmArgs<T> a, TileArgs<T> t) {
 
 // Rows without entries (zeros, or act(bias)), and rows of several units: their unit sums, every eighth one added in
 // order, then these eight sums.  A warp looks at 32 rows and takes those that need something, a lane per column.
-// SHARED: rows of more than eight units are taken by the CTA, a warp per eighth: by one warp the rows of 90,000
-// entries of a power-law matrix kept the product waiting (150,000 rows, 128 columns: 186 us, 172 so).  Products of
-// fewer than kSharedSums entries have few units and go without the barriers (layer of 2,500 rows: 8.2 us with, 7.9).
-constexpr int kWarpUnits = 8;
+// Rows of more than kCtaUnits units are taken by the CTA, a warp per eighth: by one warp the rows of 90,000
+// entries of a power-law matrix kept the product waiting (150,000 rows, 128 columns: 186 us, 172 so; one row of
+// 130,000, 8 columns: 50.9 us, 10.6).  Shorter ones stay with the warps, which take eight rows at a time (200 rows
+// of 5,000 entries, 8 columns, us: 170.9 with 8 units as the limit, 38.5 with 16; 30 of 4,200: 30.1, 26.6; 30 of
+// 9,000: 38.4 both).  Small products take this form too: one without the CTA's part, whose row pointers were
+// waited for behind the tile kernel, took longer (2,500 rows of 5 entries, 8 columns: 5.0 us, 4.5 this way).
+constexpr int kWarpUnits = 8, kCtaUnits = 16;
 static_assert(kWarpUnits == kTileWarps, "a warp per part");
-constexpr int64_t kSharedSums = 1 << 17;
-template <typename T, bool SHARED>
+template <typename T>
 __global__ void __launch_bounds__(kTileThreadsMm)
 spmm_tile_rows_kernel(SpmmArgs<T> a, TileArgs<T> t) {
-  __shared__ int s_rows[SHARED ? kTileThreadsMm : 1], s_n;
-  __shared__ T s_part[SHARED ? kTileWarps : 1][32];
+  __shared__ int s_rows[kTileThreadsMm], s_n;
+  __shared__ T s_part[kTileWarps][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // (what follows waits for this kernel's end)
   const long long r0 = ((long long)blockIdx.x * kTileWarps + warp) * 32;
@@ -388,13 +390,10 @@ spmm_tile_rows_kernel(SpmmArgs<T> a, TileArgs<T> t) {
     len = __ldg(a.pos + r0 + lane + 1) - b;
   }
   // (an empty row of an accumulating product without bias or ReLU stays what it is)
-  const bool keep_empty = a.accumulate && !a.bias && !a.relu, by_cta = SHARED && len > kWarpUnits * kUnit;
+  const bool keep_empty = a.accumulate && !a.bias && !a.relu, by_cta = len > kCtaUnits * kUnit;
   unsigned todo = __ballot_sync(FULL, (len == 0 && !keep_empty) || (len > kUnit && !by_cta));
-  bool some = false;
-  if constexpr (SHARED) {
-    if (threadIdx.x == 0) s_n = 0;
-    some = __syncthreads_or(by_cta);
-  }
+  if (threadIdx.x == 0) s_n = 0;
+  const bool some = __syncthreads_or(by_cta);
   if (by_cta) s_rows[atomicAdd(&s_n, 1)] = (int)(r0 + lane);
   asm volatile("griddepcontrol.wait;" ::: "memory");   // the tile kernel's results
   auto unit_sum = [&](int rb, int u, int col) {
@@ -426,7 +425,7 @@ spmm_tile_rows_kernel(SpmmArgs<T> a, TileArgs<T> t) {
       store(crow + col, col, sum);
     }
   }
-  if (!SHARED || !some) return;
+  if (!some) return;
   __syncthreads();
   for (int i = 0; i < s_n; i++) {
     const int r = s_rows[i], rb = __ldg(a.pos + r), units = (__ldg(a.pos + r + 1) - rb + kUnit - 1) / kUnit;
@@ -436,13 +435,13 @@ spmm_tile_rows_kernel(SpmmArgs<T> a, TileArgs<T> t) {
         T s = unit_sum(rb, warp, col);
 #pragma unroll 8
         for (int u = warp + kWarpUnits; u < units; u += kWarpUnits) s += unit_sum(rb, u, col);
-        s_part[SHARED ? warp : 0][lane] = s;
+        s_part[warp][lane] = s;
       }
       __syncthreads();
       if (warp == 0 && col < a.k) {
         T s = s_part[0][lane];
 #pragma unroll
-        for (int w = 1; w < (SHARED ? kTileWarps : 1); w++) s += s_part[w][lane];
+        for (int w = 1; w < kTileWarps; w++) s += s_part[w][lane];
         store(a.C + (long long)r * a.ldc + col, col, s);
       }
       __syncthreads();
@@ -492,8 +491,7 @@ static int launch_tiles(const SpmmArgs<T>& a, int64_t nnz, void* ws, cudaStream_
   // that, which is sound behind the tile kernel, whose CTAs have waited for whatever made them; a
   // matrix without entries has no tile kernel, and an ordinary launch)
   const dim3 grid((unsigned)ceil_div(a.m, kTileThreadsMm), (unsigned)std::min<int64_t>(ceil_div(a.k, 32), 64));
-  auto rows_kernel = nnz >= kSharedSums ? spmm_tile_rows_kernel<T, true> : spmm_tile_rows_kernel<T, false>;
-  SB_CUDA(launch_kernel(t.tiles > 0, rows_kernel, grid, kTileThreadsMm, 0, st, a, t));
+  SB_CUDA(launch_kernel(t.tiles > 0, spmm_tile_rows_kernel<T>, grid, kTileThreadsMm, 0, st, a, t));
   return SB_OK;
 }
 
