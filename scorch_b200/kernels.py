@@ -523,8 +523,18 @@ SPLIT_CHUNK_ENTRIES = 17.5
 # 2 M 4: 15.1 | 15.4 and as whole forwards alike; 3 M 5: 26.4 | 23.8; d = 101, 4 M 8: 62.5 | 64.3. By the rule above
 # it says as well that a chunk fits L2: 17.5 / 13 * 86 MB = 116 MB.
 SPLIT_MIN_ENTRIES = 13
-# Chunks' worth of operand from which a product is cut at all: what L2 nearly holds is multiplied in one pass.
+# Chunks' worth of operand from which a product is cut at all: what L2 nearly holds is multiplied in one pass.  (One
+# pass | two chunks and the cut | two chunks, ms, 64 columns, d = 50: 0.34 M rows, 86 MB 0.37 | 0.57 | 0.39; 0.44 M,
+# 112 MB 0.53 | 0.72 | 0.51; 0.49 M, 125 MB 0.61 | 0.78 | 0.57.)
 SPLIT_MIN_OPERAND = 1.3
+# A cut costs 0.1 ms and 4.3 ns per 1000 entries, which the panels multiplied with it have to earn: one, two and three
+# of them from so many chunks on, counted by the rule above and not rounded, more of them always.  (A cut that is kept
+# counts as three panels more.)  The lines lie between graphs whose columns are uniform and such with hubs among their
+# columns too, which L2 serves better in one pass.  Whole forwards about there, one pass | chunks with the cut, ms,
+# uniform; with hubs: one panel, 0.8 to 1 M rows, d = 100 4.72 | 4.37; 3.17 | 3.27; two, 0.52 to 0.6 M, d = 71 to 88
+# 3.95 | 3.73; 2.24 | 2.26; three, 0.8 to 1 M, d = 50 5.37 | 4.89; 3.48 | 3.55; four, 0.4 M, d = 31 2.23 | 1.99; 1.87 |
+# 1.95; five, 0.48 M, d = 31 2.77 | 2.43; 2.30 | 2.35.
+SPLIT_LEAST, SPLIT_KEPT_PANELS = (3.6, 2.6, 2.5), 3
 
 
 def split_pays(n: int, k: int) -> bool:
@@ -532,15 +542,20 @@ def split_pays(n: int, k: int) -> bool:
     return 4 * n * k > SPLIT_MIN_OPERAND * SPLIT_CHUNK_BYTES
 
 
-def split_chunks(m: int, n: int, nnz: int, k: int) -> int:
+def split_chunks(m: int, n: int, nnz: int, k: int, panels: Optional[int] = None) -> int:
     """Column chunks for the product of an (m x n) matrix with an (n x k) operand, 0 for none: as many as cost
-    least, for operands larger than L2 holds.  2 M rows, 100 entries each, 256 columns: 25.0 ms in one pass,
+    least, for operands larger than L2 holds.  ``panels``: panels of up to 64 columns that are multiplied before the
+    matrix is cut anew; None where the cut is kept.  2 M rows, 100 entries each, 256 columns: 25.0 ms in one pass,
     20.0 in six."""
     row = 4 * min(k, SPLIT_PANEL)
     if m <= 0 or n * row <= SPLIT_CHUNK_BYTES or not split_pays(n, k):
         return 0
-    chunks = round(math.sqrt(n * row / SPLIT_CHUNK_BYTES * nnz / m / SPLIT_CHUNK_ENTRIES))
-    return chunks if 1 < chunks <= 64 and nnz >= SPLIT_MIN_ENTRIES * chunks * m and m * chunks < 2 ** 31 - 4096 else 0
+    best = math.sqrt(n * row / SPLIT_CHUNK_BYTES * nnz / m / SPLIT_CHUNK_ENTRIES)
+    panels = -(-k // SPLIT_PANEL) + SPLIT_KEPT_PANELS if panels is None else panels
+    if panels == 0 or (panels <= len(SPLIT_LEAST) and best < SPLIT_LEAST[panels - 1]):
+        return 0
+    chunks = max(2, round(best))
+    return chunks if chunks <= 64 and nnz >= SPLIT_MIN_ENTRIES * chunks * m and m * chunks < 2 ** 31 - 4096 else 0
 
 
 class ColumnSplit:
@@ -564,15 +579,15 @@ class ColumnSplit:
         self.stream = torch.cuda.current_stream(dev)
 
     @staticmethod
-    def of(pos, crd, val, n: int, k: int) -> Optional["ColumnSplit"]:
-        """The split for products with operands of up to ``k`` columns, or None where it does not pay, or
-        the columns do not ascend, or memory for the copy is not there.  None too while the stream is
-        captured into a graph: the split waits for the device, and a graph would go on reading a copy of the
-        matrix as it was."""
+    def of(pos, crd, val, n: int, k: int, panels: Optional[int] = None) -> Optional["ColumnSplit"]:
+        """The split for products with operands of up to ``k`` columns (``panels``: how many panels, of a split
+        that is not kept, see ``split_chunks``), or None where it does not pay, or the columns do not ascend, or
+        memory for the copy is not there.  None too while the stream is captured into a graph: the split waits
+        for the device, and a graph would go on reading a copy of the matrix as it was."""
         if not (val.dtype == torch.float32 and pos.dtype == crd.dtype == torch.int32 and val.numel() == crd.numel()
                 and all(t.is_cuda and t.is_contiguous() for t in (pos, crd, val))):
             return None
-        chunks = split_chunks(pos.numel() - 1, n, crd.numel(), k)
+        chunks = split_chunks(pos.numel() - 1, n, crd.numel(), k, panels)
         if not chunks or torch.cuda.is_current_stream_capturing():
             return None
         _validated(pos, crd, n, "ColumnSplit")

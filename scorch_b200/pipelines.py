@@ -80,7 +80,9 @@ def gcn_forward(pos, crd, val, X, W1, W2, plan: Optional[K.CsrPlan] = None) -> t
     with the operand in L2 (``kernels.split_chunks``).  ``plan`` is accepted and not needed: products of one
     matrix run over equal tiles of its entries."""
     n, hidden, width = X.shape[0], W1.shape[1], W2.shape[1]
-    split = K.ColumnSplit.of(pos, crd, val, n, max(hidden, width)) if W1.is_cuda and X.dtype == torch.float32 else None
+    panels = sum(-(-k // K.SPLIT_PANEL) for k in (hidden, width) if K.split_pays(n, k))
+    split = (K.ColumnSplit.of(pos, crd, val, n, max(hidden, width), panels)
+             if W1.is_cuda and X.dtype == torch.float32 else None)
     product = lambda B, relu: (split.matmul(B, relu) if split is not None and K.split_pays(n, B.shape[1])
                                else K.spmm_csr(pos, crd, val, B, relu=relu))
     return product(K.dense_matmul(product(K.dense_matmul(X, W1), True), W2), False)

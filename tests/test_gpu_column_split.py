@@ -238,3 +238,27 @@ def test_split_dropped_while_another_stream_multiplies_it():
     torch.cuda.synchronize()
     assert all((t == 0).all() for t in fresh)
     assert torch.allclose(out, want, rtol=1e-4, atol=1e-4)
+
+
+@pytest.mark.parametrize("hidden,width", [(64, 40), (64, 64), (256, 64)])
+def test_forward_that_cuts_on_every_call(monkeypatch, hidden, width):
+    from scorch_b200 import kernels as K, pipelines as P
+    monkeypatch.setattr(K, "SPLIT_CHUNK_BYTES", 1e5)
+    products, matmul = [], K.ColumnSplit.matmul
+    monkeypatch.setattr(K.ColumnSplit, "matmul",
+                        lambda self, B, *a, **kw: products.append(B.shape[1]) or matmul(self, B, *a, **kw))
+    pos, crd, val = _csr([100] * 2000, 2000, seed=10)
+    g = torch.Generator().manual_seed(6)
+    X, W1, W2 = (torch.randn(s, generator=g).cuda() for s in ((2000, 32), (32, hidden), (hidden, width)))
+    d = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    A = torch.sparse_csr_tensor(d(pos), d(crd), d(val), size=(2000, 2000)).to_dense().double()
+    want = A @ (torch.relu(A @ (X.double() @ W1.double())) @ W2.double())
+    got = P.gcn_forward(d(pos), d(crd), d(val), X, W1, W2)
+    assert products == [hidden, width] and ((got.double() - want).norm() / want.norm()).item() < 1e-6
+    flip = lambda a: a.reshape(2000, 100)[:, ::-1].reshape(-1)           # columns that do not ascend: one pass
+    got = P.gcn_forward(d(pos), d(flip(crd)), d(flip(val)), X, W1, W2)
+    assert len(products) == 2 and ((got.double() - want).norm() / want.norm()).item() < 1e-6
+    crd[-1] = 2000
+    monkeypatch.setenv("SCORCH_B200_VALIDATE", "1")
+    with pytest.raises(ValueError, match="column index out of range"):
+        P.gcn_forward(d(pos), d(crd), d(val), X, W1, W2)
